@@ -601,11 +601,13 @@ static int run_prefill(fa::PrefillParams& p, int D, cudaStream_t stream) {
     return fail(FA_ERR_UNSUPPORTED, "the tcgen05 prefill kernel supports D = 64 and 128 only");
   if (p.in_bf16 && !tc5_ok)
     return fail(FA_ERR_UNSUPPORTED, "bfloat16 prefill is served by the tcgen05 kernel: head dimension up to 128");
-  if (tc5_ok && (g_prefill_impl != 1 || p.in_bf16)) {
+  const bool wide_ok = fa::prefill_wide_supported(p);
+  if ((tc5_ok || wide_ok) && (g_prefill_impl != 1 || p.in_bf16)) {
     EncodeTiledFn enc;
     rc = get_encode(&enc);
     if (rc != FA_OK) return rc;
-    e = fa::launch_prefill_tc5(p, D, reinterpret_cast<void*>(enc), stream);
+    e = tc5_ok ? fa::launch_prefill_tc5(p, D, reinterpret_cast<void*>(enc), stream)
+               : fa::launch_prefill_wide(p, di.sm_count, reinterpret_cast<void*>(enc), stream);
   } else {
     e = fa::launch_prefill_mma(p, D, stream);
   }

@@ -34,6 +34,9 @@ cudaError_t launch_prefill_mma(const PrefillParams& p, int D, cudaStream_t strea
 bool prefill_tc5_supported(const PrefillParams& p, int D);
 cudaError_t launch_prefill_tc5(const PrefillParams& p, int D, void* encode_fn, cudaStream_t stream);
 void prefill_tc5_set_poly(bool on);
+// tcgen05 kernel of wide heads: 128 < D_real <= 256, fp16.
+bool prefill_wide_supported(const PrefillParams& p);
+cudaError_t launch_prefill_wide(const PrefillParams& p, int sm_count, void* encode_fn, cudaStream_t stream);
 cudaError_t prefill_status(int* host_out, cudaStream_t stream);
 cudaError_t prefill_status_ptr(int** out);  // device address of the status word (current device)
 cudaError_t prefill_status_clear(cudaStream_t stream);

@@ -1,9 +1,9 @@
 // Tiled GQA prefill on mma.sync tensor cores (dense [B,H,N,D] and packed varlen).
 //
 // Replaces the reference's one-thread-per-query-row prefill kernels
-// (flash_attn_kernel.cu:1138-1299, 2471-2605, 3005-3148).  This is the general
-// path (any supported D, any length); the tcgen05 kernel in prefill_tc5.cu takes
-// the D = 128 / D = 64 cases when it is enabled.
+// (flash_attn_kernel.cu:1138-1299, 2471-2605, 3005-3148).  The tcgen05
+// kernels (prefill_tc5.cu up to D = 128, prefill_wide.cu above) take over unless this
+// one is asked for (fa_prefill_set_impl(1)): it is what they are checked against.
 //
 // One CTA = BM query rows of one (sequence, query head); each warp owns 16 rows.
 // K/V tiles of 64 keys are double-buffered in shared memory with cp.async and an
