@@ -13,7 +13,6 @@ bf16; the attention operators run in fp16 (q, k, v are cast by the fused QK-norm
 """
 from __future__ import annotations
 
-import ctypes
 from typing import Optional
 
 import torch
@@ -24,7 +23,7 @@ from .config import ModelConfig
 
 
 def _p(t):
-    return ctypes.c_void_p(t.data_ptr())
+    return t.data_ptr()
 
 
 class GreedyHead:
@@ -104,7 +103,7 @@ class TPDecoder(GreedyHead):
 
     # ---- small wrappers over the C ABI -------------------------------------------------
     def _stream(self):
-        return ctypes.c_void_p(torch.cuda.current_stream(self.device).cuda_stream)
+        return torch.cuda.current_stream(self.device).cuda_stream
 
     def _add_rmsnorm(self, x, delta, w):
         out = torch.empty_like(x)

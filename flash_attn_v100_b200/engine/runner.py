@@ -11,6 +11,19 @@ import torch
 from .model import Segments, TPDecoder
 
 
+def _upload(parts: Sequence[torch.Tensor], device) -> List[torch.Tensor]:
+    """Host vectors on `device`, each at a multiple of 64 bytes of one buffer that is copied on the current stream."""
+    at = [0]
+    for t in parts:
+        at.append(at[-1] + (t.numel() * t.element_size() + 63) // 64 * 64)
+    host = torch.empty(at[-1], dtype=torch.uint8, pin_memory=device.type == "cuda")
+    places = [slice(a, a + t.numel() * t.element_size()) for a, t in zip(at, parts)]
+    for place, t in zip(places, parts):
+        host[place].view(t.dtype).copy_(t)
+    there = host.to(device, non_blocking=True)
+    return [there[place].view(t.dtype) for place, t in zip(places, parts)]
+
+
 class GenerationRunner:
     def __init__(self, model, max_batch: int, max_seq_len: int, use_cuda_graph: bool = True,
                  peer_collectives: bool = False, num_blocks: int = 0):
@@ -57,22 +70,30 @@ class GenerationRunner:
 
     def _pass_args(self, request_ids: Sequence[str], tokens: Sequence[Sequence[int]], want: Optional[List[int]]):
         """forward() arguments for the requests' next tokens, from where their caches end."""
-        m, kv, dev = self.model, self.kv, self.model.device
+        # One copy from pinned memory on the current stream takes everything over: a copy from pageable memory waits for the
+        # pass before, and the launches of this one would start only then.
+        kv, dev = self.kv, self.model.device
         past = [kv.get_cache_len(r) for r in request_ids]
         lens = [len(t) for t in tokens]
-        table, slots = kv.batch_view(request_ids)
-        flat = torch.tensor([t for ts in tokens for t in ts], dtype=torch.int64).to(dev)
-        rows = torch.tensor([kv.row_of(r) for r in request_ids], dtype=torch.int32).to(dev)
-        args = dict(token_ids=flat, kv=kv, block_table=table, slots=slots, max_blocks=self.max_blocks, state_rows=rows,
-                    want=None if want is None else torch.tensor(want, dtype=torch.int64).to(dev))
-        if all(n == 1 for n in lens) and all(past):
-            return dict(args, positions=slots)               # decode step
-        cu = [0]
-        for n in lens:
-            cu.append(cu[-1] + n)
-        pos = torch.cat([torch.arange(p, p + n, dtype=torch.int32) for p, n in zip(past, lens)]).to(dev)
-        return dict(args, positions=pos, cu_seqlens=torch.tensor(cu, dtype=torch.int32).to(dev), max_seqlen=max(lens), lens=lens,
-                    past=past)
+        order = [kv.row_of(r) for r in request_ids]
+        decode = all(n == 1 for n in lens) and all(past)
+        parts = [torch.tensor([t for ts in tokens for t in ts], dtype=torch.int64)]
+        if want is not None:
+            parts.append(torch.tensor(want, dtype=torch.int64))
+        parts += [torch.tensor(past, dtype=torch.int32), torch.tensor(order, dtype=torch.int32)]
+        if not decode:
+            cu = [0]
+            for n in lens:
+                cu.append(cu[-1] + n)
+            parts += [torch.cat([torch.arange(p, p + n, dtype=torch.int32) for p, n in zip(past, lens)]), torch.tensor(cu, dtype=torch.int32)]
+        on_device = iter(_upload(parts, dev))
+        args = dict(token_ids=next(on_device), kv=kv, max_blocks=self.max_blocks, want=None if want is None else next(on_device),
+                    slots=next(on_device), state_rows=next(on_device))
+        B = len(order)
+        args["block_table"] = kv.block_table[:B] if order == list(range(B)) else kv.block_table.index_select(0, args["state_rows"])
+        if decode:
+            return dict(args, positions=args["slots"])
+        return dict(args, positions=next(on_device), cu_seqlens=next(on_device), max_seqlen=max(lens), lens=lens, past=past)
 
     @torch.no_grad()
     def step(self, entries: Sequence[Tuple[str, Sequence[int], Sequence[int]]]) -> List[torch.Tensor]:
@@ -93,7 +114,7 @@ class GenerationRunner:
             past = kv.get_cache_len(r)
             if past + len(toks) > self.max_seq_len:
                 raise ValueError(f"request {r!r} would hold {past + len(toks)} tokens, more than max_seq_len={self.max_seq_len}")
-            kv.reserve(r, past + len(toks))
+            kv.reserve(r, past + len(toks), wait=False)     # the pass reads the table on this stream
         out: List[Optional[torch.Tensor]] = [None] * len(entries)
         single = [i for i, (r, toks, _) in enumerate(entries) if len(toks) == 1 and kv.get_cache_len(r) > 0]
         other = [i for i in range(len(entries)) if i not in single]

@@ -111,8 +111,9 @@ class BlockManager:
             raise
         return self._row[request_id]
 
-    def reserve(self, request_id: str, new_total_tokens: int) -> None:
-        """Grow the request's block table so that `new_total_tokens` tokens fit (manager.py:336-344)."""
+    def reserve(self, request_id: str, new_total_tokens: int, wait: bool = True) -> None:
+        """Grow the request's block table so that `new_total_tokens` tokens fit (manager.py:336-344).  With `wait` the
+        device's table holds the new entries when the call returns; without, once the current stream gets there."""
         table = self._tables[request_id]
         need = (new_total_tokens + BLOCK_SIZE - 1) // BLOCK_SIZE
         if need > self.max_blocks_per_seq:
@@ -122,7 +123,9 @@ class BlockManager:
             extra = self._take_blocks(need - len(table))
             table.extend(extra)
             row = self._row[request_id]
-            self.block_table[row, first_new:need] = torch.tensor(extra, dtype=torch.int32)  # only the new entries
+            async_copy = not wait and self.device.type == "cuda"
+            new = torch.tensor(extra, dtype=torch.int32, pin_memory=async_copy)  # only the new entries
+            self.block_table[row, first_new:need].copy_(new, non_blocking=async_copy)
 
     def commit(self, request_id: str, num_new_tokens: int) -> None:
         """Advance the token count after the step's tokens were written into every layer; with a sliding

@@ -15,6 +15,7 @@ from __future__ import annotations
 
 import contextlib
 import ctypes
+import functools
 import threading
 from typing import Dict, Tuple
 
@@ -44,14 +45,23 @@ def _entry(lib, f16_name):
     return getattr(lib, f16_name[:-3] + "bf16") if _elem() == torch.bfloat16 else getattr(lib, f16_name)
 
 
-@contextlib.contextmanager
+class _Bf16Elements:
+    """Within it, the wrappers of this thread take bfloat16 (reentrant; one shared instance)."""
+
+    def __enter__(self):
+        stack = _elem_state.__dict__.setdefault("stack", [])
+        stack.append(_elem())
+        _elem_state.dtype = torch.bfloat16
+
+    def __exit__(self, *exc):
+        _elem_state.dtype = _elem_state.stack.pop()
+
+
+_BF16 = _Bf16Elements()
+
+
 def _bf16_elements():
-    prev = _elem()
-    _elem_state.dtype = torch.bfloat16
-    try:
-        yield
-    finally:
-        _elem_state.dtype = prev
+    return _BF16
 
 
 _workspaces: Dict[Tuple[int, int], torch.Tensor] = {}
@@ -118,13 +128,39 @@ def _check_gqa_heads(H_Q, H_KV):
 
 
 def _ptr(t):
-    return ctypes.c_void_p(t.data_ptr())
+    return t.data_ptr()      # the entry points' argument types turn it into a pointer
+
+
+# The host side of a call is what bounds small batches (a decode of four short sequences runs about 8 us on the GPU), so
+# the wrappers look at each tensor once: `_plain` and a comparison of shapes accept what the detailed checks accept, and
+# only a call that fails them goes through those, for the message.  Measured per call, before and after: paged decode
+# of four sequences 31.0 and 17.7 us, packed prefill of three short prompts 32.9 and 22.5 us.
+def _plain(t, dtype, dims, dev):
+    """Whether `t` is a contiguous tensor of that type and number of dimensions on CUDA device `dev`."""
+    return isinstance(t, torch.Tensor) and t.is_cuda and t.get_device() == dev and t.dtype is dtype and t.dim() == dims and t.is_contiguous()
+
+
+def _cuda_index(t):
+    return t.get_device() if isinstance(t, torch.Tensor) and t.is_cuda else -1
+
+
+_HERE = contextlib.nullcontext()
+
+
+def _on(device):
+    """Context with `device` current; nothing to do where it is already."""
+    return _HERE if torch.cuda.current_device() == device.index else torch.cuda.device(device)
 
 
 def _stream_ptr(device, stream_int=None):
     if stream_int is None:
-        stream_int = torch.cuda.current_stream(device).cuda_stream
+        stream_int = torch._C._cuda_getCurrentRawStream(device.index)
     return int(stream_int)
+
+
+@functools.lru_cache(maxsize=1024)
+def _decode_workspace_bytes(B, H_Q, H_KV, D):
+    return int(_lib.load().fa_decode_workspace_bytes(B, H_Q, H_KV, D))
 
 
 def _workspace(device, stream_int, B, H_Q, H_KV, D):
@@ -142,7 +178,7 @@ def _workspace(device, stream_int, B, H_Q, H_KV, D):
     lib = _lib.load()
     _chk(8 <= D <= 256 and D % 8 == 0,
          f"head dimension {D} is not built (decode serves multiples of 8 up to 256)")
-    need = int(lib.fa_decode_workspace_bytes(B, H_Q, H_KV, D))
+    need = _decode_workspace_bytes(B, H_Q, H_KV, D)
     _chk(need > 0, f"unsupported decode configuration B={B} H_Q={H_Q} H_KV={H_KV} D={D}")
     dev_index = device.index if device.index is not None else torch.cuda.current_device()
     key = (dev_index, stream_int)
@@ -158,7 +194,7 @@ def _workspace(device, stream_int, B, H_Q, H_KV, D):
             ev = torch.cuda.Event()
             ev.record(current)
             torch.cuda.ExternalStream(stream_int, device=device).wait_event(ev)
-        _lib.check(lib.fa_decode_workspace_init(_ptr(ws), ws.numel(), ctypes.c_void_p(stream_int)))
+        _lib.check(lib.fa_decode_workspace_init(_ptr(ws), ws.numel(), stream_int))
         _workspaces[key] = ws
     return ws
 
@@ -172,7 +208,7 @@ def check_async_errors(device=None) -> None:
             continue
         with torch.cuda.device(dev):
             st = ctypes.c_int(0)
-            _lib.check(lib.fa_decode_status(_ptr(ws), ctypes.c_void_p(stream_int), ctypes.byref(st)))
+            _lib.check(lib.fa_decode_status(_ptr(ws), stream_int, ctypes.byref(st)))
 
 
 def set_prefill_impl(impl: int = 0) -> None:
@@ -187,7 +223,7 @@ def check_prefill_errors(device=None, clear: bool = True) -> None:
     with torch.cuda.device(dev):
         st = ctypes.c_int(0)
         s = torch.cuda.current_stream(dev).cuda_stream
-        _lib.check(lib.fa_prefill_status(ctypes.c_void_p(s), ctypes.byref(st), 1 if clear else 0))
+        _lib.check(lib.fa_prefill_status(s, ctypes.byref(st), 1 if clear else 0))
 
 
 def set_decode_tuning(warps: int = 0, stages: int = 0, ctas_per_sm: int = 0) -> None:
@@ -197,21 +233,31 @@ def set_decode_tuning(warps: int = 0, stages: int = 0, ctas_per_sm: int = 0) -> 
 # --------------------------------------------------------------------------
 # decode
 # --------------------------------------------------------------------------
+def _decode_inputs(q, k, v, dtype):
+    """q [B, H_Q, 1, D] and k, v [B, H_KV, N, D] of that type, contiguous, on one CUDA device."""
+    dev = _cuda_index(q)
+    if not (dev >= 0 and _plain(q, dtype, 4, dev) and _plain(k, dtype, 4, dev) and _plain(v, dtype, 4, dev)):
+        return False
+    qs, ks = q.shape, k.shape
+    return qs[2] == 1 and ks == v.shape and qs[0] == ks[0] and qs[3] == ks[3]
+
+
 def _decode_gqa(out, q, k, v, causal, cache_len, stream_int=None):
-    for t, n in ((q, "q"), (k, "k"), (v, "v")):
-        _check_input(t, n)
-    _check_decode_gqa_shapes(q, k, v)
-    if out is not None:
-        # check_decode_gqa_output_tensor (flash_attn_kernel.cu:226-239)
-        _check_input(out, "out")
-        _check_dim(out, 4, "out")
-        _same_device(out, q, "out", "q"); _same_dtype(out, q, "out", "q")
-        _chk(out.size(0) == q.size(0), "out batch size must match q")
-        _chk(out.size(1) == q.size(1), "out head count must match q")
-        _chk(out.size(2) == 1, "out sequence length must be 1 for decode mode")
-        _chk(out.size(3) == q.size(3), "out head dimension must match q")
-    _chk(q.dtype == _elem(), f"q, k, v must be {_elem_name()}")
-    _chk(q.size(2) == 1, "q sequence length must be 1 for decode mode")
+    if not (_decode_inputs(q, k, v, _elem()) and (out is None or (_plain(out, _elem(), 4, q.get_device()) and out.shape == q.shape))):
+        for t, n in ((q, "q"), (k, "k"), (v, "v")):
+            _check_input(t, n)
+        _check_decode_gqa_shapes(q, k, v)
+        if out is not None:
+            # check_decode_gqa_output_tensor (flash_attn_kernel.cu:226-239)
+            _check_input(out, "out")
+            _check_dim(out, 4, "out")
+            _same_device(out, q, "out", "q"); _same_dtype(out, q, "out", "q")
+            _chk(out.size(0) == q.size(0), "out batch size must match q")
+            _chk(out.size(1) == q.size(1), "out head count must match q")
+            _chk(out.size(2) == 1, "out sequence length must be 1 for decode mode")
+            _chk(out.size(3) == q.size(3), "out head dimension must match q")
+        _chk(q.dtype == _elem(), f"q, k, v must be {_elem_name()}")
+        _chk(q.size(2) == 1, "q sequence length must be 1 for decode mode")
     B, H_Q, _, D = q.shape
     H_KV, N = k.size(1), k.size(2)
     _check_gqa_heads(H_Q, H_KV)
@@ -219,13 +265,13 @@ def _decode_gqa(out, q, k, v, causal, cache_len, stream_int=None):
     cache_len = int(cache_len)
     _check_cache_len(cache_len, N)
     lib = _lib.load()
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         if out is None:
             out = torch.empty((B, H_Q, 1, D), dtype=q.dtype, device=q.device)
         s = _stream_ptr(q.device, stream_int)
         ws = _workspace(q.device, s, B, H_Q, H_KV, D)
         _lib.check(_entry(lib, "fa_decode_gqa_f16")(_ptr(q), _ptr(k), _ptr(v), _ptr(out), B, H_Q, H_KV, N, D,
-                                         1 if causal else 0, cache_len, _ptr(ws), ws.numel(), ctypes.c_void_p(s)))
+                                         1 if causal else 0, cache_len, _ptr(ws), ws.numel(), s))
     return out
 
 
@@ -263,35 +309,32 @@ def forward_decode_sliding_window_gqa(q, k, v, causal, cache_len, window_size, s
     j < sink_size or window_start <= j <= cache_len, window_start = max(0, min(cache_len+1, N) - window_size)
     (:4386-4387, :4410-4412).  `causal` has no effect, as in the reference; like the reference, no
     bound is checked on cache_len, window_size or sink_size."""
-    for t, n in ((q, "q"), (k, "k"), (v, "v")):
-        _check_input(t, n)
-    _chk(q.dtype == torch.float16, "q must be float16")
-    _chk(k.dtype == torch.float16 and v.dtype == torch.float16, "k and v must be float16")
-    _chk(q.dim() == 4 and k.dim() == 4 and v.dim() == 4, "q, k, v must be 4D tensors")
-    _chk(q.size(2) == 1, "q sequence length must be 1 for decode mode")
-    _same_device(q, k, "q", "k"); _same_device(q, v, "q", "v")
-    _chk(k.shape == v.shape, "k and v must have the same shape")
-    _chk(k.size(0) == q.size(0) and k.size(3) == q.size(3), "k must match q in batch size and head dimension")
+    if not _decode_inputs(q, k, v, torch.float16):
+        for t, n in ((q, "q"), (k, "k"), (v, "v")):
+            _check_input(t, n)
+        _chk(q.dtype == torch.float16, "q must be float16")
+        _chk(k.dtype == torch.float16 and v.dtype == torch.float16, "k and v must be float16")
+        _chk(q.dim() == 4 and k.dim() == 4 and v.dim() == 4, "q, k, v must be 4D tensors")
+        _chk(q.size(2) == 1, "q sequence length must be 1 for decode mode")
+        _same_device(q, k, "q", "k"); _same_device(q, v, "q", "v")
+        _chk(k.shape == v.shape, "k and v must have the same shape")
+        _chk(k.size(0) == q.size(0) and k.size(3) == q.size(3), "k must match q in batch size and head dimension")
     B, H_Q, _, D = q.shape
     H_KV, N = k.size(1), k.size(2)
     _check_gqa_heads(H_Q, H_KV)
     _chk(D <= MAX_D_LARGE, "D must be <= MAX_D_LARGE(256)")
     lib = _lib.load()
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         out = torch.empty((B, H_Q, 1, D), dtype=q.dtype, device=q.device)
         s = _stream_ptr(q.device)
         ws = _workspace(q.device, s, B, H_Q, H_KV, D)
         _lib.check(lib.fa_decode_sliding_window_gqa_f16(
             _ptr(q), _ptr(k), _ptr(v), _ptr(out), B, H_Q, H_KV, N, D, int(cache_len), int(window_size),
-            int(sink_size), _ptr(ws), ws.numel(), ctypes.c_void_p(s)))
+            int(sink_size), _ptr(ws), ws.numel(), s))
     return out
 
 
-def forward_decode_int8_kv_cache_gqa(q, k_int8, v_int8, k_scale, v_scale, cache_len):
-    """flash_attn_forward_decode_int8_kv_cache_gqa (flash_attn_kernel.cu:4164-4221).
-    q [B,H_Q,1,D] fp16; k_int8/v_int8 [B,H_KV,N,D] int8; k_scale/v_scale [B,H_KV,N] fp16 (one scale per
-    cached token) -> new [B,H_Q,1,D] fp16.  Elements are dequantised as fp16(float(int8) * float(scale))
-    (:4083-4086) and keys j <= cache_len are attended (:4094-4098)."""
+def _check_int8_kv(q, k_int8, v_int8, k_scale, v_scale):
     for t, n in ((q, "q"), (k_int8, "k_int8"), (v_int8, "v_int8"), (k_scale, "k_scale"), (v_scale, "v_scale")):
         _check_input(t, n)
     _chk(q.dtype == torch.float16, "q must be float16")
@@ -315,14 +358,31 @@ def forward_decode_int8_kv_cache_gqa(q, k_int8, v_int8, k_scale, v_scale, cache_
     _chk(v_scale.size(2) == N, "v_scale size mismatch")
     _chk(tuple(k_scale.shape) == (B, H_KV, N) and tuple(v_scale.shape) == (B, H_KV, N),
          "k_scale and v_scale must be [B, H_KV, N]")
+
+
+def forward_decode_int8_kv_cache_gqa(q, k_int8, v_int8, k_scale, v_scale, cache_len):
+    """flash_attn_forward_decode_int8_kv_cache_gqa (flash_attn_kernel.cu:4164-4221).
+    q [B,H_Q,1,D] fp16; k_int8/v_int8 [B,H_KV,N,D] int8; k_scale/v_scale [B,H_KV,N] fp16 (one scale per
+    cached token) -> new [B,H_Q,1,D] fp16.  Elements are dequantised as fp16(float(int8) * float(scale))
+    (:4083-4086) and keys j <= cache_len are attended (:4094-4098)."""
+    dev = _cuda_index(q)
+    if not (dev >= 0 and _plain(q, torch.float16, 4, dev) and _plain(k_int8, torch.int8, 4, dev) and _plain(v_int8, torch.int8, 4, dev)
+            and _plain(k_scale, torch.float16, 3, dev) and _plain(v_scale, torch.float16, 3, dev) and q.size(2) == 1
+            and k_int8.shape == v_int8.shape and q.size(0) == k_int8.size(0) and q.size(3) == k_int8.size(3)
+            and k_scale.shape == k_int8.shape[:3] and v_scale.shape == k_int8.shape[:3]):
+        _check_int8_kv(q, k_int8, v_int8, k_scale, v_scale)
+    B, H_Q, _, D = q.shape
+    H_KV, N = k_int8.size(1), k_int8.size(2)
+    _check_gqa_heads(H_Q, H_KV)
+    _chk(D <= MAX_D_LARGE, "D must be <= MAX_D_LARGE(256)")
     lib = _lib.load()
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         out = torch.empty((B, H_Q, 1, D), dtype=q.dtype, device=q.device)
         s = _stream_ptr(q.device)
         ws = _workspace(q.device, s, B, H_Q, H_KV, D)
         _lib.check(lib.fa_decode_int8_kv_cache_gqa(
             _ptr(q), _ptr(k_int8), _ptr(v_int8), _ptr(k_scale), _ptr(v_scale), _ptr(out), B, H_Q, H_KV, N, D,
-            int(cache_len), _ptr(ws), ws.numel(), ctypes.c_void_p(s)))
+            int(cache_len), _ptr(ws), ws.numel(), s))
     return out
 
 
@@ -330,40 +390,41 @@ def forward_continuous_batching_fp16(q, k, v, cache_lens, causal):
     """flash_attn_forward_continuous_batching_fp16 (continuous_batching_kernel.cu:338-406).
     q [B,H_Q,1,D], k/v [B,H_KV,max_N,D] fp16, cache_lens [B] int32; sequence b attends
     keys [0, min(cache_lens[b]+1, max_N)).  `causal` has no effect (as in the reference)."""
-    for t, n in ((q, "q"), (k, "k"), (v, "v"), (cache_lens, "cache_lens")):
-        _check_input(t, n)
-    _chk(q.dtype == torch.float16, "q must be float16")
-    _chk(k.dtype == torch.float16 and v.dtype == torch.float16, "k and v must be float16")
-    _chk(q.dim() == 4 and k.dim() == 4 and v.dim() == 4, "q, k, v must be 4D tensors")
-    _chk(q.size(2) == 1, "q sequence length must be 1 for decode mode")
-    _chk(cache_lens.dim() == 1, "cache_lens must be 1D tensor")
-    _chk(cache_lens.size(0) == q.size(0), "cache_lens size must match batch size")
-    # the reference reads cache_lens through data_ptr<int>() (:394); other dtypes would be misread
-    _chk(cache_lens.dtype == torch.int32, "cache_lens must be int32")
-    _same_device(q, k, "q", "k"); _same_device(q, v, "q", "v"); _same_device(q, cache_lens, "q", "cache_lens")
-    _chk(k.shape == v.shape, "k and v must have the same shape")
-    _chk(k.size(0) == q.size(0) and k.size(3) == q.size(3), "k must match q in batch size and head dimension")
+    if not (_decode_inputs(q, k, v, torch.float16) and _plain(cache_lens, torch.int32, 1, q.get_device())
+            and cache_lens.size(0) == q.size(0)):
+        for t, n in ((q, "q"), (k, "k"), (v, "v"), (cache_lens, "cache_lens")):
+            _check_input(t, n)
+        _chk(q.dtype == torch.float16, "q must be float16")
+        _chk(k.dtype == torch.float16 and v.dtype == torch.float16, "k and v must be float16")
+        _chk(q.dim() == 4 and k.dim() == 4 and v.dim() == 4, "q, k, v must be 4D tensors")
+        _chk(q.size(2) == 1, "q sequence length must be 1 for decode mode")
+        _chk(cache_lens.dim() == 1, "cache_lens must be 1D tensor")
+        _chk(cache_lens.size(0) == q.size(0), "cache_lens size must match batch size")
+        # the reference reads cache_lens through data_ptr<int>() (:394); other dtypes would be misread
+        _chk(cache_lens.dtype == torch.int32, "cache_lens must be int32")
+        _same_device(q, k, "q", "k"); _same_device(q, v, "q", "v"); _same_device(q, cache_lens, "q", "cache_lens")
+        _chk(k.shape == v.shape, "k and v must have the same shape")
+        _chk(k.size(0) == q.size(0) and k.size(3) == q.size(3), "k must match q in batch size and head dimension")
     B, H_Q, _, D = q.shape
     H_KV, max_N = k.size(1), k.size(2)
     _check_gqa_heads(H_Q, H_KV)
     _chk(D <= MAX_D_LARGE, "D must be <= MAX_D_CB_LARGE(256)")
     lib = _lib.load()
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         out = torch.empty((B, H_Q, 1, D), dtype=q.dtype, device=q.device)
         s = _stream_ptr(q.device)
         ws = _workspace(q.device, s, B, H_Q, H_KV, D)
         _lib.check(lib.fa_decode_varlen_f16(_ptr(q), _ptr(k), _ptr(v), _ptr(out), _ptr(cache_lens), B, H_Q, H_KV,
-                                            max_N, D, 1 if causal else 0, _ptr(ws), ws.numel(), ctypes.c_void_p(s)))
+                                            max_N, D, 1 if causal else 0, _ptr(ws), ws.numel(), s))
     return out
 
 
-def forward_paged_decode_gqa_fp16(q, k_cache, v_cache, block_table, seq_lens, max_num_blocks, out_dtype=None):
-    """flash_attn_forward_paged_decode_gqa_fp16 (flash_attn_kernel.cu:3516-3584).
-    q [B,H_Q,1,D]; k_cache/v_cache [pages,H_KV,16,D] fp16; block_table [B,*] int32 with
-    row stride `max_num_blocks` (:3438); seq_lens [B] int32.  seq_len 0 gives zeros.
-    `out_dtype=torch.bfloat16` (an addition) returns the result rounded to bfloat16 instead of fp16."""
-    _chk(out_dtype in (None, torch.float16, torch.bfloat16), "out_dtype must be float16 or bfloat16")
-    bf16_out = out_dtype == torch.bfloat16 and _elem() == torch.float16
+def _paged_shapes_fit(qs, ks, vs, tables, lens):
+    return (qs[2] == 1 and ks == vs and ks[2] == PAGE_BLOCK_SIZE and qs[3] == ks[3] <= MAX_D_LARGE and qs[0] == tables == lens
+            and qs[1] >= ks[1] > 0 and qs[1] % ks[1] == 0)
+
+
+def _check_paged(q, k_cache, v_cache, block_table, seq_lens):
     for t, n in ((q, "q"), (k_cache, "k_cache"), (v_cache, "v_cache"), (block_table, "block_table"),
                  (seq_lens, "seq_lens")):
         _check_input(t, n)
@@ -387,12 +448,28 @@ def forward_paged_decode_gqa_fp16(q, k_cache, v_cache, block_table, seq_lens, ma
     _chk(seq_lens.size(0) == B, "seq_lens batch size must match q")
     _chk(k_cache.shape == v_cache.shape, "k_cache and v_cache must have the same shape")
     _chk(k_cache.size(3) == D, "k_cache head dimension must match q")
+
+
+def forward_paged_decode_gqa_fp16(q, k_cache, v_cache, block_table, seq_lens, max_num_blocks, out_dtype=None):
+    """flash_attn_forward_paged_decode_gqa_fp16 (flash_attn_kernel.cu:3516-3584).
+    q [B,H_Q,1,D]; k_cache/v_cache [pages,H_KV,16,D] fp16; block_table [B,*] int32 with
+    row stride `max_num_blocks` (:3438); seq_lens [B] int32.  seq_len 0 gives zeros.
+    `out_dtype=torch.bfloat16` (an addition) returns the result rounded to bfloat16 instead of fp16."""
+    _chk(out_dtype in (None, torch.float16, torch.bfloat16), "out_dtype must be float16 or bfloat16")
+    bf16_out = out_dtype == torch.bfloat16 and _elem() == torch.float16
+    elem, dev = _elem(), _cuda_index(q)
+    if not (dev >= 0 and _plain(q, elem, 4, dev) and _plain(k_cache, elem, 4, dev) and _plain(v_cache, elem, 4, dev)
+            and _plain(block_table, torch.int32, 2, dev) and _plain(seq_lens, torch.int32, 1, dev)
+            and _paged_shapes_fit(q.shape, k_cache.shape, v_cache.shape, block_table.size(0), seq_lens.size(0))):
+        _check_paged(q, k_cache, v_cache, block_table, seq_lens)
+    B, H_Q, _, D = q.shape
+    H_KV = k_cache.size(1)
     max_num_blocks = int(max_num_blocks)
     _chk(max_num_blocks > 0, "max_num_blocks must be positive")
     _chk((B - 1) * max_num_blocks + min(max_num_blocks, block_table.size(1)) <= block_table.numel(),
          "max_num_blocks (row stride) is larger than block_table allows")
     lib = _lib.load()
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         out = torch.empty((B, H_Q, 1, D), dtype=torch.bfloat16 if bf16_out else q.dtype, device=q.device)
         s = _stream_ptr(q.device)
         ws = _workspace(q.device, s, B, H_Q, H_KV, D)
@@ -400,15 +477,11 @@ def forward_paged_decode_gqa_fp16(q, k_cache, v_cache, block_table, seq_lens, ma
         entry = lib.fa_paged_decode_gqa_f16_out_bf16 if bf16_out else _entry(lib, "fa_paged_decode_gqa_f16")
         _lib.check(entry(_ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(out), _ptr(block_table),
                                                _ptr(seq_lens), B, H_Q, H_KV, D, k_cache.size(0), max_num_blocks,
-                                               max_len, _ptr(ws), ws.numel(), ctypes.c_void_p(s)))
+                                               max_len, _ptr(ws), ws.numel(), s))
     return out
 
 
-def forward_decode_int8_gqa(q, k, v, q_scale, k_scale, cache_len, return_scores=False):
-    """flash_attn_forward_decode_int8_gqa (flash_attn_kernel.cu:2941-3003).
-    q [B,H_Q,1,D], k/v [B,H_KV,N,D] fp16, q_scale [B,H_Q] fp32, k_scale [B,H_KV,N] fp32
-    (per cached token).  With `return_scores=True` (an addition) also returns the raw
-    int32 QK^T accumulators [B,H_Q,N] (entries past cache_len are zero)."""
+def _check_int8_qk(q, k, v, q_scale, k_scale):
     for t, n in ((q, "q"), (k, "k"), (v, "v"), (q_scale, "q_scale"), (k_scale, "k_scale")):
         _check_input(t, n)
     _check_decode_gqa_shapes(q, k, v)
@@ -424,10 +497,24 @@ def forward_decode_int8_gqa(q, k, v, q_scale, k_scale, cache_len, return_scores=
     _chk(k_scale.dim() == 3 and k_scale.size(0) == B and k_scale.size(1) == H_KV and k_scale.size(2) == N,
          "k_scale must be [B, H_KV, N]")
     _same_device(q, q_scale, "q", "q_scale"); _same_device(q, k_scale, "q", "k_scale")
+
+
+def forward_decode_int8_gqa(q, k, v, q_scale, k_scale, cache_len, return_scores=False):
+    """flash_attn_forward_decode_int8_gqa (flash_attn_kernel.cu:2941-3003).
+    q [B,H_Q,1,D], k/v [B,H_KV,N,D] fp16, q_scale [B,H_Q] fp32, k_scale [B,H_KV,N] fp32
+    (per cached token).  With `return_scores=True` (an addition) also returns the raw
+    int32 QK^T accumulators [B,H_Q,N] (entries past cache_len are zero)."""
+    if not (_decode_inputs(q, k, v, torch.float16) and _plain(q_scale, torch.float32, 2, q.get_device())
+            and _plain(k_scale, torch.float32, 3, q.get_device()) and q_scale.shape == q.shape[:2] and k_scale.shape == k.shape[:3]):
+        _check_int8_qk(q, k, v, q_scale, k_scale)
+    B, H_Q, _, D = q.shape
+    H_KV, N = k.size(1), k.size(2)
+    _check_gqa_heads(H_Q, H_KV)
+    _chk(D <= MAX_D_LARGE, "D must be <= MAX_D_LARGE(256)")
     cache_len = int(cache_len)
     _check_cache_len(cache_len, N)
     lib = _lib.load()
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         out = torch.empty((B, H_Q, 1, D), dtype=q.dtype, device=q.device)
         scores = torch.zeros((B, H_Q, N), dtype=torch.int32, device=q.device) if return_scores else None
         s = _stream_ptr(q.device)
@@ -435,7 +522,7 @@ def forward_decode_int8_gqa(q, k, v, q_scale, k_scale, cache_len, return_scores=
         _lib.check(lib.fa_decode_int8_gqa(_ptr(q), _ptr(k), _ptr(v), _ptr(out), _ptr(q_scale), _ptr(k_scale),
                                           B, H_Q, H_KV, N, D, cache_len,
                                           _ptr(scores) if scores is not None else None,
-                                          _ptr(ws), ws.numel(), ctypes.c_void_p(s)))
+                                          _ptr(ws), ws.numel(), s))
     return (out, scores) if return_scores else out
 
 
@@ -446,12 +533,12 @@ def _prefill_dense(out, q, k, v, causal):
     B, H_Q, N, D = q.shape
     H_KV = k.size(1)
     lib = _lib.load()
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         if out is None:
             out = torch.empty((B, H_Q, N, D), dtype=q.dtype, device=q.device)
         s = _stream_ptr(q.device)
         _lib.check(_entry(lib, "fa_prefill_dense_f16")(_ptr(q), _ptr(k), _ptr(v), _ptr(out), B, H_Q, H_KV, N, D,
-                                            1 if causal else 0, ctypes.c_void_p(s)))
+                                            1 if causal else 0, s))
     return out
 
 
@@ -472,16 +559,19 @@ def forward_fp16(q, k, v, causal):
 
 
 def _prefill_gqa(out, q, k, v, causal):
-    for t, n in ((q, "q"), (k, "k"), (v, "v")):
-        _check_input(t, n)
-    _check_prefill_gqa_shapes(q, k, v)
-    if out is not None:
-        # check_prefill_gqa_output_tensor (flash_attn_kernel.cu:241-250)
-        _check_input(out, "out")
-        _check_dim(out, 4, "out")
-        _same_device(out, q, "out", "q"); _same_dtype(out, q, "out", "q")
-        _chk(out.shape == q.shape, "out shape must match q shape for prefill mode")
-    _chk(q.dtype == _elem(), f"q, k, v must be {_elem_name()}")
+    elem, dev = _elem(), _cuda_index(q)
+    if not (dev >= 0 and _plain(q, elem, 4, dev) and _plain(k, elem, 4, dev) and _plain(v, elem, 4, dev) and k.shape == v.shape
+            and q.size(0) == k.size(0) and q.shape[2:] == k.shape[2:] and (out is None or (_plain(out, elem, 4, dev) and out.shape == q.shape))):
+        for t, n in ((q, "q"), (k, "k"), (v, "v")):
+            _check_input(t, n)
+        _check_prefill_gqa_shapes(q, k, v)
+        if out is not None:
+            # check_prefill_gqa_output_tensor (flash_attn_kernel.cu:241-250)
+            _check_input(out, "out")
+            _check_dim(out, 4, "out")
+            _same_device(out, q, "out", "q"); _same_dtype(out, q, "out", "q")
+            _chk(out.shape == q.shape, "out shape must match q shape for prefill mode")
+        _chk(q.dtype == _elem(), f"q, k, v must be {_elem_name()}")
     _check_gqa_heads(q.size(1), k.size(1))
     _chk(q.size(3) <= MAX_D_LARGE, "D must be <= MAX_D_LARGE(256)")
     return _prefill_dense(out, q, k, v, causal)
@@ -498,18 +588,21 @@ def forward_prefill_gqa_fp16_out(out, q, k, v, causal):
 
 
 def _varlen(q, k, v, cu_seqlens, max_seqlen, causal, stream_int=None, bf16_out=False):
-    for t, n in ((q, "q"), (k, "k"), (v, "v"), (cu_seqlens, "cu_seqlens")):
-        _check_input(t, n)
-    # check_varlen_prefill_input_shapes (flash_attn_kernel.cu:195-219); the head-count
-    # equality of the reference (:217) is relaxed to GQA: H_Q % H_KV == 0.
-    _check_dim(q, 3, "q"); _check_dim(k, 3, "k"); _check_dim(v, 3, "v"); _check_dim(cu_seqlens, 1, "cu_seqlens")
-    _same_device(q, k, "q", "k"); _same_device(q, v, "q", "v"); _same_device(q, cu_seqlens, "q", "cu_seqlens")
-    _same_dtype(q, k, "q", "k"); _same_dtype(q, v, "q", "v")
-    _chk(k.size(0) == q.size(0) and v.size(0) == q.size(0), "k and v total length must match q")
-    _chk(k.size(1) == v.size(1), "k and v must have the same number of heads")
-    _chk(k.size(2) == q.size(2) and v.size(2) == q.size(2), "k and v head dimension must match q")
-    _chk(q.dtype == _elem(), f"q, k, v must be {_elem_name()}")
-    _chk(cu_seqlens.dtype == torch.int32, "cu_seqlens must be int32")
+    elem, dev = _elem(), _cuda_index(q)
+    if not (dev >= 0 and _plain(q, elem, 3, dev) and _plain(k, elem, 3, dev) and _plain(v, elem, 3, dev) and _plain(cu_seqlens, torch.int32, 1, dev)
+            and k.shape == v.shape and q.size(0) == k.size(0) and q.size(2) == k.size(2)):
+        for t, n in ((q, "q"), (k, "k"), (v, "v"), (cu_seqlens, "cu_seqlens")):
+            _check_input(t, n)
+        # check_varlen_prefill_input_shapes (flash_attn_kernel.cu:195-219); the head-count
+        # equality of the reference (:217) is relaxed to GQA: H_Q % H_KV == 0.
+        _check_dim(q, 3, "q"); _check_dim(k, 3, "k"); _check_dim(v, 3, "v"); _check_dim(cu_seqlens, 1, "cu_seqlens")
+        _same_device(q, k, "q", "k"); _same_device(q, v, "q", "v"); _same_device(q, cu_seqlens, "q", "cu_seqlens")
+        _same_dtype(q, k, "q", "k"); _same_dtype(q, v, "q", "v")
+        _chk(k.size(0) == q.size(0) and v.size(0) == q.size(0), "k and v total length must match q")
+        _chk(k.size(1) == v.size(1), "k and v must have the same number of heads")
+        _chk(k.size(2) == q.size(2) and v.size(2) == q.size(2), "k and v head dimension must match q")
+        _chk(q.dtype == _elem(), f"q, k, v must be {_elem_name()}")
+        _chk(cu_seqlens.dtype == torch.int32, "cu_seqlens must be int32")
     bf16_out = bf16_out and _elem() == torch.float16
     total, H_Q, D = q.shape
     H_KV = k.size(1)
@@ -520,7 +613,7 @@ def _varlen(q, k, v, cu_seqlens, max_seqlen, causal, stream_int=None, bf16_out=F
     _chk(max_seqlen > 0, "max_seqlen must be positive")
     _chk(batch > 0, "cu_seqlens must contain at least one sequence")
     lib = _lib.load()
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         # rows outside every sequence stay zero, as in the reference (:3373)
         out = torch.zeros(q.shape, dtype=torch.bfloat16 if bf16_out else q.dtype, device=q.device)
         s = _stream_ptr(q.device, stream_int)
@@ -531,7 +624,7 @@ def _varlen(q, k, v, cu_seqlens, max_seqlen, causal, stream_int=None, bf16_out=F
             torch.cuda.ExternalStream(stream_int, device=q.device).wait_event(ev)
         entry = lib.fa_prefill_varlen_f16_out_bf16 if bf16_out else _entry(lib, "fa_prefill_varlen_f16")
         _lib.check(entry(_ptr(q), _ptr(k), _ptr(v), _ptr(out), _ptr(cu_seqlens), batch, total,
-                         H_Q, H_KV, D, max_seqlen, 1 if causal else 0, ctypes.c_void_p(s)))
+                         H_Q, H_KV, D, max_seqlen, 1 if causal else 0, s))
     return out
 
 
@@ -614,7 +707,7 @@ def rope_append_paged_fp16(q, k, v, cos, sin, k_cache, v_cache, block_table, pos
         _check_input(positions, "positions")
         _chk(positions.dtype == torch.int32 and positions.numel() == batch, "positions must be int32 [batch]")
     lib = _lib.load()
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         q_out = torch.empty_like(q)
         k_out = torch.empty_like(k) if return_k else None
         s = _stream_ptr(q.device)
@@ -623,7 +716,7 @@ def rope_append_paged_fp16(q, k, v, cos, sin, k_cache, v_cache, block_table, pos
             _ptr(k_cache) if has_cache else None, _ptr(v_cache) if has_cache else None,
             _ptr(block_table) if has_cache else None, _ptr(positions) if positions is not None else None,
             _ptr(cu_seqlens) if packed else None, T, batch, H_Q, H_KV, D, R,
-            k_cache.size(0) if has_cache else 0, int(max_num_blocks) if has_cache else 0, ctypes.c_void_p(s)))
+            k_cache.size(0) if has_cache else 0, int(max_num_blocks) if has_cache else 0, s))
     return (q_out, k_out) if return_k else q_out
 
 

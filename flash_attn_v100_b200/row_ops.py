@@ -12,11 +12,11 @@ _DTYPE = {torch.float32: 0, torch.bfloat16: 1}
 
 
 def _p(t):
-    return None if t is None else ctypes.c_void_p(t.data_ptr())
+    return None if t is None else t.data_ptr()      # the entry points' argument types turn it into a pointer
 
 
 def _stream(t):
-    return ctypes.c_void_p(torch.cuda.current_stream(t.device).cuda_stream)
+    return torch._C._cuda_getCurrentRawStream(t.get_device())
 
 
 def _check(t, name, dtype, contiguous=True):
