@@ -667,6 +667,15 @@ static int prefill_varlen_impl(const void* q, const void* k, const void* v, void
   return run_prefill(p, D, static_cast<cudaStream_t>(stream));
 }
 
+int fa_prefill_varlen_clear(void* out, const int32_t* cu_seqlens, int batch, int64_t total, int max_seqlen,
+                            int64_t row_bytes, void* stream) {
+  FA_REQUIRE(out != nullptr && cu_seqlens != nullptr, "null pointer");
+  FA_REQUIRE(batch > 0 && total > 0 && max_seqlen > 0 && row_bytes > 0, "batch, total, max_seqlen and row_bytes must be positive");
+  FA_REQUIRE(row_bytes % 16 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0, "out and its rows must be 16-byte aligned");
+  FA_CUDA(fa::launch_varlen_clear(out, cu_seqlens, batch, total, max_seqlen, row_bytes, static_cast<cudaStream_t>(stream)));
+  return FA_OK;
+}
+
 int fa_prefill_varlen_bf16(const void* q, const void* k, const void* v, void* out, const int32_t* cu_seqlens,
                            int batch, int64_t total, int H_Q, int H_KV, int D, int max_seqlen, int causal,
                            void* stream) {

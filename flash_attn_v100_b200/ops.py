@@ -614,14 +614,16 @@ def _varlen(q, k, v, cu_seqlens, max_seqlen, causal, stream_int=None, bf16_out=F
     _chk(batch > 0, "cu_seqlens must contain at least one sequence")
     lib = _lib.load()
     with _on(q.device):
-        # rows outside every sequence stay zero, as in the reference (:3373)
-        out = torch.zeros(q.shape, dtype=torch.bfloat16 if bf16_out else q.dtype, device=q.device)
+        out = torch.empty(q.shape, dtype=torch.bfloat16 if bf16_out else q.dtype, device=q.device)
         s = _stream_ptr(q.device, stream_int)
         if stream_int is not None and stream_int != torch.cuda.current_stream(q.device).cuda_stream:
-            # zeros_like ran on the current stream; order the foreign stream after it
+            # the block may have been released by work still queued on the current stream: order the foreign stream after it
             ev = torch.cuda.Event()
             ev.record()
             torch.cuda.ExternalStream(stream_int, device=q.device).wait_event(ev)
+        if total > 0 and D % 8 == 0:      # (the attention refuses the rest)
+            # rows outside every sequence are zero, as in the reference (:3373)
+            _lib.check(lib.fa_prefill_varlen_clear(_ptr(out), _ptr(cu_seqlens), batch, total, max_seqlen, H_Q * D * 2, s))
         entry = lib.fa_prefill_varlen_f16_out_bf16 if bf16_out else _entry(lib, "fa_prefill_varlen_f16")
         _lib.check(entry(_ptr(q), _ptr(k), _ptr(v), _ptr(out), _ptr(cu_seqlens), batch, total,
                          H_Q, H_KV, D, max_seqlen, 1 if causal else 0, s))

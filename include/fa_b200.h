@@ -266,6 +266,13 @@ int fa_prefill_dense_f16(const void* q, const void* k, const void* v, void* out,
 int fa_prefill_varlen_f16(const void* q, const void* k, const void* v, void* out,
                           const int32_t* cu_seqlens, int batch, int64_t total,
                           int H_Q, int H_KV, int D, int max_seqlen, int causal, void* stream);
+/*
+ * Zeros in the rows of a packed output [total, row_bytes] that no sequence covers: before cu_seqlens[0],
+ * behind the first max_seqlen rows of a longer sequence, from cu_seqlens[batch] on.  Launched on the stream
+ * before the attention it makes the whole output defined.
+ */
+int fa_prefill_varlen_clear(void* out, const int32_t* cu_seqlens, int batch, int64_t total,
+                            int max_seqlen, int64_t row_bytes, void* stream);
 /* fa_prefill_varlen_f16 with the output stored as bfloat16 (see fa_paged_decode_gqa_f16_out_bf16). */
 int fa_prefill_varlen_f16_out_bf16(const void* q, const void* k, const void* v, void* out,
                           const int32_t* cu_seqlens, int batch, int64_t total,
