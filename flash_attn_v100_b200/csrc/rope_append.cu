@@ -159,124 +159,194 @@ __global__ void __launch_bounds__(256) rope_append_kernel(const RopeAppendParams
   }
 }
 
-// qkv projection output -> attention inputs.  One warp per (token, head); lane L holds D/32 consecutive
+// PER 16-bit elements as one access.
+template <int PER> struct Packed;
+template <> struct Packed<2> { using V = uint32_t; };
+template <> struct Packed<4> { using V = uint2; };
+template <> struct Packed<8> { using V = uint4; };
+
+// Pairs of elements.  A product or sum of two 16-bit numbers, rounded once, is what the fp32 operation and a rounding to 16 bits give
+// (fp32 has at least 2 * 11 + 2 bits), so the packed instructions leave every bit as it was.
+template <typename T> struct Two;
+template <> struct Two<__half> {
+  using V = __half2;
+  static __device__ __forceinline__ V from(float a, float b) { return __floats2half2_rn(a, b); }
+};
+template <> struct Two<__nv_bfloat16> {
+  using V = __nv_bfloat162;
+  static __device__ __forceinline__ V from(float a, float b) { return __floats2bfloat162_rn(a, b); }
+};
+template <typename V> __device__ __forceinline__ uint32_t bits(V v) { return *reinterpret_cast<const uint32_t*>(&v); }
+template <typename V> __device__ __forceinline__ V of_bits(uint32_t b) { return *reinterpret_cast<const V*>(&b); }
+
+// qkv projection output -> attention inputs.  A warp takes HPW consecutive heads of a token; lane L holds D/32 consecutive
 // elements, its rotary partner (the element half a head away) lives in lane L ^ 16.  The arithmetic is that
 // of the per-head norm kernel followed by the rotary kernel above, value for value, so the fused launch is
 // bit-identical to the two it replaces.
-template <int PER, typename T>
+//
+// Bound by memory and, with 16-bit elements, by the instructions per element.  What a token's heads share (its place in the cache, cosines and
+// sines) is fetched once per HPW heads, every access is PER elements wide (VEC false: element by element, for bases that are not aligned to
+// that) and the rotation works on pairs.  3307 tokens of 32 query heads on 8 of 128: 72 us with one head per warp and 2-byte accesses, 56 us with
+// four and whole accesses, 37 us with pairs as well.
+template <int PER, typename T, int HPW, bool VEC>
 __global__ void __launch_bounds__(256) qkv_rope_append_kernel(const QkvRopeAppendParams p) {
+  using V = typename Packed<PER>::V;
+  using V2 = typename Two<T>::V;
+  constexpr int NP = PER / 2;
+  union Row {
+    V v;
+    __nv_bfloat16 b[PER];
+    __nv_bfloat162 b2[NP];
+    T t[PER];
+    V2 t2[NP];
+    __device__ Row() {}
+  };
   const RopeAppendParams& r = p.r;
   const int D = r.D, heads = r.H_Q + 2 * r.H_KV;
+  const int groups = (heads + HPW - 1) / HPW;
   const long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
-  if (wid >= (long long)r.T * heads) return;
-  const int tok = (int)(wid / heads);
-  const int hh = (int)(wid - (long long)tok * heads);
-  int kind, h;   // 0 = q, 1 = k, 2 = v
-  if (hh < r.H_Q) { kind = 0; h = hh; }
-  else if (hh < r.H_Q + r.H_KV) { kind = 1; h = hh - r.H_Q; }
-  else { kind = 2; h = hh - r.H_Q - r.H_KV; }
-  const __nv_bfloat16* src = static_cast<const __nv_bfloat16*>(p.qkv) + ((long long)tok * heads + hh) * D + lane * PER;
-  float f[PER];
-  float ss = 0.f;
+  if (wid >= (long long)r.T * groups) return;
+  const int tok = (int)(wid / groups);
+  const int hh0 = (int)(wid - (long long)tok * groups) * HPW;
+  auto load = [&](const __nv_bfloat16* src, Row& to) {
+    if constexpr (VEC) {
+      to.v = *reinterpret_cast<const V*>(src);
+    } else {
 #pragma unroll
-  for (int i = 0; i < PER; ++i) {
-    f[i] = __bfloat162float(src[i]);
-    ss += f[i] * f[i];
-  }
-  const __nv_bfloat16* w = kind == 0 ? static_cast<const __nv_bfloat16*>(p.q_weight)
-                         : kind == 1 ? static_cast<const __nv_bfloat16*>(p.k_weight) : nullptr;
-  if (w != nullptr) {
+      for (int i = 0; i < PER; ++i) to.b[i] = src[i];
+    }
+  };
+  auto store = [&](T* dst, const Row& from) {
+    if constexpr (VEC) {
+      *reinterpret_cast<V*>(dst) = from.v;
+    } else {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    const float inv = rsqrtf(ss / (float)D + p.eps);
+      for (int i = 0; i < PER; ++i) dst[i] = from.t[i];
+    }
+  };
+  Row in[HPW];
 #pragma unroll
-    for (int i = 0; i < PER; ++i) {
-      const __nv_bfloat16 nb = __float2bfloat16(f[i] * inv);
-      f[i] = __bfloat162float(__float2bfloat16(__bfloat162float(w[lane * PER + i]) * __bfloat162float(nb)));
+  for (int u = 0; u < HPW; ++u)
+    if (hh0 + u < heads) load(static_cast<const __nv_bfloat16*>(p.qkv) + ((long long)tok * heads + hh0 + u) * D + lane * PER, in[u]);
+  V2 cs[NP], sn[NP];
+  if (hh0 < r.H_Q + r.H_KV) {
+    // cos / sin at the element's own index (the tables hold cat(freqs, freqs))
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+      const float *c = r.cos + (long long)tok * D + lane * PER + 2 * i, *s = r.sin + (long long)tok * D + lane * PER + 2 * i;
+      cs[i] = Two<T>::from(__ldg(c), __ldg(c + 1));
+      sn[i] = Two<T>::from(__ldg(s), __ldg(s + 1));
     }
   }
-  T x[PER];
-#pragma unroll
-  for (int i = 0; i < PER; ++i) x[i] = el_from<T>(f[i]);
-
-  // sequence and cache slot of this token
-  int seq, pos;
-  if (r.cu_seqlens != nullptr) {
-    int lo = 0, hi = r.batch;
-    while (hi - lo > 1) {
-      const int mid = (lo + hi) >> 1;
-      if (__ldg(r.cu_seqlens + mid) <= tok) lo = mid; else hi = mid;
+  // sequence and cache slot of this token (query heads go to neither)
+  long long slot = -1;      // page * 16 + row
+  if (hh0 + HPW > r.H_Q && r.k_cache != nullptr) {
+    int seq, pos;
+    if (r.cu_seqlens != nullptr) {
+      int lo = 0, hi = r.batch;
+      while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (__ldg(r.cu_seqlens + mid) <= tok) lo = mid; else hi = mid;
+      }
+      seq = lo;
+      pos = tok - __ldg(r.cu_seqlens + seq) + (r.positions ? __ldg(r.positions + seq) : 0);
+    } else {
+      seq = tok;
+      pos = __ldg(r.positions + seq);
     }
-    seq = lo;
-    pos = tok - __ldg(r.cu_seqlens + seq) + (r.positions ? __ldg(r.positions + seq) : 0);
-  } else {
-    seq = tok;
-    pos = __ldg(r.positions + seq);
-  }
-  T* dst_page = nullptr;
-  if (kind != 0 && r.k_cache != nullptr) {
     const int blk = pos >> 4;
     int page = -1;
     if (pos >= 0 && blk < r.bt_stride) page = __ldg(r.block_table + (long long)seq * r.bt_stride + blk);
-    if (page >= 0 && (long long)page < r.num_pages) {
+    if (page >= 0 && (long long)page < r.num_pages) slot = (long long)page * 16 + (pos & 15);
+    else if (lane == 0) atomicOr(r.status, kStatusBadPageId);   // no slot for this token: reported, nothing written
+  }
+#pragma unroll
+  for (int u = 0; u < HPW; ++u) {
+    const int hh = hh0 + u;
+    if (hh >= heads) break;
+    int kind, h;   // 0 = q, 1 = k, 2 = v
+    if (hh < r.H_Q) { kind = 0; h = hh; }
+    else if (hh < r.H_Q + r.H_KV) { kind = 1; h = hh - r.H_Q; }
+    else { kind = 2; h = hh - r.H_Q - r.H_KV; }
+    float2 f[NP];
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+      f[i] = __bfloat1622float2(in[u].b2[i]);
+      ss += f[i].x * f[i].x;
+      ss += f[i].y * f[i].y;
+    }
+    const __nv_bfloat16* w = kind == 0 ? static_cast<const __nv_bfloat16*>(p.q_weight)
+                           : kind == 1 ? static_cast<const __nv_bfloat16*>(p.k_weight) : nullptr;
+    if (w != nullptr) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      const float inv = rsqrtf(ss / (float)D + p.eps);
+      Row wr;
+      load(w + lane * PER, wr);
+#pragma unroll
+      for (int i = 0; i < NP; ++i) f[i] = __bfloat1622float2(__hmul2_rn(wr.b2[i], __floats2bfloat162_rn(f[i].x * inv, f[i].y * inv)));
+    }
+    Row o;
+#pragma unroll
+    for (int i = 0; i < NP; ++i) o.t2[i] = Two<T>::from(f[i].x, f[i].y);
+    if (kind != 2) {
+      // rotary: first half (lanes 0-15) x1 * cos + (-x2) * sin, second half x2 * cos + x1 * sin, with the partner
+      // element from lane ^ 16
+#pragma unroll
+      for (int i = 0; i < NP; ++i) {
+        const uint32_t other = __shfl_xor_sync(0xffffffffu, bits(o.t2[i]), 16) ^ (lane < 16 ? 0x80008000u : 0u);
+        o.t2[i] = __hadd2_rn(__hmul2_rn(o.t2[i], cs[i]), __hmul2_rn(of_bits<V2>(other), sn[i]));
+      }
+    }
+    T* dst_lin = nullptr;
+    if (kind == 0) dst_lin = reinterpret_cast<T*>(r.q_out) + ((long long)tok * r.H_Q + h) * D + lane * PER;
+    else if (kind == 1 && r.k_out != nullptr) dst_lin = reinterpret_cast<T*>(r.k_out) + ((long long)tok * r.H_KV + h) * D + lane * PER;
+    else if (kind == 2 && p.v_out != nullptr) dst_lin = reinterpret_cast<T*>(p.v_out) + ((long long)tok * r.H_KV + h) * D + lane * PER;
+    if (dst_lin) store(dst_lin, o);
+    if (kind != 0 && slot >= 0) {
       T* base = reinterpret_cast<T*>((kind == 1) ? r.k_cache : r.v_cache);
-      dst_page = base + (((long long)page * r.H_KV + h) * 16 + (pos & 15)) * D + lane * PER;
-    } else if (lane == 0) {
-      atomicOr(r.status, kStatusBadPageId);   // no slot for this token: reported, nothing written
+      store(base + (((slot >> 4) * r.H_KV + h) * 16 + (slot & 15)) * D + lane * PER, o);
     }
   }
-  T o[PER];
-  if (kind == 2) {
-#pragma unroll
-    for (int i = 0; i < PER; ++i) o[i] = x[i];
+}
+
+bool aligned_to(const void* p, size_t bytes) { return (reinterpret_cast<uintptr_t>(p) & (bytes - 1)) == 0; }
+
+template <int PER, typename T>
+cudaError_t launch_qkv_t(const QkvRopeAppendParams& p, cudaStream_t stream) {
+  const int heads = p.r.H_Q + 2 * p.r.H_KV;
+  bool vec = true;
+  for (const void* q : {p.qkv, p.q_weight, p.k_weight, (const void*)p.r.q_out, (const void*)p.r.k_out, (const void*)p.v_out,
+                        (const void*)p.r.k_cache, (const void*)p.r.v_cache})
+    vec = vec && aligned_to(q, PER * 2);
+  // A few tokens (a decode step) take one head per warp: more warps, each with one chain of loads; from about four warps per scheduler
+  // on (148 SMs x 4 x 4), sharing a token's tables and place among four heads is worth more.
+  const bool many = (long long)p.r.T * heads > 4 * 2368;
+  const int hpw = many ? 4 : 1;
+  const long long warps = (long long)p.r.T * ((heads + hpw - 1) / hpw);
+  const unsigned blocks = (unsigned)((warps * 32 + 255) / 256);
+  if (!vec) {
+    if (many) qkv_rope_append_kernel<PER, T, 4, false><<<blocks, 256, 0, stream>>>(p);
+    else qkv_rope_append_kernel<PER, T, 1, false><<<blocks, 256, 0, stream>>>(p);
   } else {
-    // rotary: first half (lanes 0-15) x1 * cos - x2 * sin, second half x2 * cos + x1 * sin, with the partner
-    // element from lane ^ 16 and cos / sin at the element's own index (the tables hold cat(freqs, freqs))
-    const float* cs = r.cos + (long long)tok * D + lane * PER;
-    const float* sn = r.sin + (long long)tok * D + lane * PER;
-#pragma unroll
-    for (int i = 0; i < PER; ++i) {
-      const unsigned short mine = *reinterpret_cast<const unsigned short*>(&x[i]);
-      const unsigned short got = (unsigned short)__shfl_xor_sync(0xffffffffu, (unsigned int)mine, 16);
-      const T other = *reinterpret_cast<const T*>(&got);
-      const T c = el_from<T>(__ldg(cs + i)), s = el_from<T>(__ldg(sn + i));
-      o[i] = lane < 16 ? rope_lo(x[i], other, c, s) : rope_hi(other, x[i], c, s);
-    }
+    if (many) qkv_rope_append_kernel<PER, T, 4, true><<<blocks, 256, 0, stream>>>(p);
+    else qkv_rope_append_kernel<PER, T, 1, true><<<blocks, 256, 0, stream>>>(p);
   }
-  T* dst_lin = nullptr;
-  if (kind == 0) dst_lin = reinterpret_cast<T*>(r.q_out) + ((long long)tok * r.H_Q + h) * D + lane * PER;
-  else if (kind == 1 && r.k_out != nullptr) dst_lin = reinterpret_cast<T*>(r.k_out) + ((long long)tok * r.H_KV + h) * D + lane * PER;
-  else if (kind == 2 && p.v_out != nullptr) dst_lin = reinterpret_cast<T*>(p.v_out) + ((long long)tok * r.H_KV + h) * D + lane * PER;
-#pragma unroll
-  for (int i = 0; i < PER; ++i) {
-    if (dst_lin) dst_lin[i] = o[i];
-    if (dst_page) dst_page[i] = o[i];
-  }
+  return cudaGetLastError();
 }
 
 }  // namespace
 
 cudaError_t launch_qkv_rope_append(const QkvRopeAppendParams& p, cudaStream_t stream) {
-  const long long warps = (long long)p.r.T * (p.r.H_Q + 2 * p.r.H_KV);
-  if (warps == 0) return cudaSuccess;
-  const unsigned blocks = (unsigned)((warps * 32 + 255) / 256);
-  if (p.r.bf16) {
-    switch (p.r.D) {
-      case 64: qkv_rope_append_kernel<2, __nv_bfloat16><<<blocks, 256, 0, stream>>>(p); break;
-      case 128: qkv_rope_append_kernel<4, __nv_bfloat16><<<blocks, 256, 0, stream>>>(p); break;
-      case 256: qkv_rope_append_kernel<8, __nv_bfloat16><<<blocks, 256, 0, stream>>>(p); break;
-      default: return cudaErrorInvalidValue;
-    }
-    return cudaGetLastError();
-  }
+  if (p.r.T == 0) return cudaSuccess;
   switch (p.r.D) {
-    case 64: qkv_rope_append_kernel<2, __half><<<blocks, 256, 0, stream>>>(p); break;
-    case 128: qkv_rope_append_kernel<4, __half><<<blocks, 256, 0, stream>>>(p); break;
-    case 256: qkv_rope_append_kernel<8, __half><<<blocks, 256, 0, stream>>>(p); break;
+    case 64: return p.r.bf16 ? launch_qkv_t<2, __nv_bfloat16>(p, stream) : launch_qkv_t<2, __half>(p, stream);
+    case 128: return p.r.bf16 ? launch_qkv_t<4, __nv_bfloat16>(p, stream) : launch_qkv_t<4, __half>(p, stream);
+    case 256: return p.r.bf16 ? launch_qkv_t<8, __nv_bfloat16>(p, stream) : launch_qkv_t<8, __half>(p, stream);
     default: return cudaErrorInvalidValue;
   }
-  return cudaGetLastError();
 }
 
 cudaError_t launch_rope_append(const RopeAppendParams& p, int sm_count, cudaStream_t stream) {
