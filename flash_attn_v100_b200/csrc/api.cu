@@ -240,7 +240,9 @@ int run_decode(const DecodeCall& c) {
   p.scale_log2 = p.scale * 1.4426950408889634f;
   long long n_cta = (long long)di.sm_count * cfg.ctas_per_sm;
   if (n_cta > kMaxDecodeCtas) n_cta = kMaxDecodeCtas;
-  if (c.max_units > 0 && c.max_units < n_cta) n_cta = c.max_units;
+  p.parts = fa::decode_parts(c.B, p.HV, (int)n_cta, c.max_units / ((long long)c.B * p.HV), c.mode == fa::kModeContigFixed, cfg.warps * cfg.stages);
+  if (p.parts > 0) n_cta = (long long)c.B * p.HV * p.parts;
+  else if (c.max_units > 0 && c.max_units < n_cta) n_cta = c.max_units;
   if (n_cta < 1) n_cta = 1;
   p.n_cta = (int)n_cta;
 

@@ -28,6 +28,7 @@
 // ldmatrix from the swizzled tiles; softmax is fp32, base-2, online.
 #include "common.cuh"
 #include "decode_splitkv.cuh"
+#include "smem_limit.cuh"
 
 #include <math.h>
 
@@ -363,7 +364,20 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap,
   long long per = (T + p.n_cta - 1) / p.n_cta;
   if (per < 1) per = 1;
   long long u = (long long)blockIdx.x * per;
-  const long long u1 = (u + per < T) ? (u + per) : T;
+  long long u1 = (u + per < T) ? (u + per) : T;
+  int part_pages = 0;
+  if (p.parts > 0) {
+    // a segment is cut into parts of equal length (at least what the rings hold), one per CTA: see decode_parts
+    const int seg = (int)blockIdx.x / p.parts;
+    if (seg >= p.B * p.HV) return;
+    const int bb = seg / p.HV, np = pre[bb + 1] - pre[bb];
+    part_pages = (np + p.parts - 1) / p.parts;
+    if (part_pages < W * S) part_pages = W * S;
+    const int lo = ((int)blockIdx.x - seg * p.parts) * part_pages;
+    if (lo >= np) return;
+    u = (long long)p.HV * pre[bb] + (long long)(seg - bb * p.HV) * np + lo;
+    u1 = u + (part_pages < np - lo ? part_pages : np - lo);
+  }
   if (u >= u1) return;
 
   const uint64_t policy = l2_policy_evict_first();
@@ -996,7 +1010,8 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap,
       // The segment is shared with neighbouring CTAs.  Publish the partial, count the arrival;
       // whoever arrives last merges all partials of the segment.
       const long long seg_start = (long long)p.HV * pre[b] + (long long)hv * np;
-      const int first = (int)(seg_start / per), last = (int)((seg_start + np - 1) / per);
+      const int first = p.parts > 0 ? (b * p.HV + hv) * p.parts : (int)(seg_start / per);
+      const int last = p.parts > 0 ? first + (np - 1) / part_pages : (int)((seg_start + np - 1) / per);
       const unsigned int n_parts = (unsigned int)(last - first + 1);
       __threadfence();
       __syncthreads();
@@ -1026,7 +1041,7 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap,
           // merge the longest part of such launches.)
           constexpr int MB = 8;
           auto part_row = [&](int c) -> const float* {
-            const int slot = ((long long)c * per >= seg_start) ? 0 : 1;
+            const int slot = (p.parts > 0 || (long long)c * per >= seg_start) ? 0 : 1;
             return p.partials + ((size_t)c * 2 + slot) * p.slot_rows * ROWLEN + row * ROWLEN;
           };
           float M = -INFINITY;
@@ -1071,7 +1086,8 @@ cudaError_t launch_t(const CUtensorMap& kmap, const CUtensorMap& vmap, const Dec
                      int warps, size_t smem_bytes, cudaStream_t stream) {
   auto kern = decode_splitkv_kernel<D, KIND, HM>;
   if (warps * 32 > DecodeOccupancy<D, KIND, HM>::kThreads) return cudaErrorInvalidConfiguration;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
+  static SharedMemoryLimit limit;
+  cudaError_t e = limit.raise(reinterpret_cast<const void*>(kern), (int)smem_bytes);
   if (e != cudaSuccess) return e;
   if (p.B + 1 > kMaxSmemPrefix) decode_plan_kernel<<<1, 1024, 0, stream>>>(p);  // else scanned in-kernel
   kern<<<p.n_cta, warps * 32, smem_bytes, stream>>>(kmap, vmap, p);
@@ -1098,6 +1114,22 @@ size_t decode_workspace_bytes(int B, int H_Q, int H_KV, int D, int max_ctas) {
   bytes += ((size_t)(B + 1) * 4 + 255) & ~(size_t)255;
   bytes += (size_t)max_ctas * 2 * slot_rows * (D + 2) * 4;
   return (bytes + 255) & ~(size_t)255;
+}
+
+// CTAs per segment where every segment is cut into equal parts, one per CTA; 0: the even cut of all pages.
+//
+// Few pages: with the even cut a CTA works on the ends of two segments, one after the other, and nearly every segment is merged through
+// global memory, two round trips that take as long as the pages themselves.  With parts a CTA has one piece, and a segment whose pages the
+// rings of one CTA hold all at once is not cut.  The line: the longest part is no longer than the rings, so that all its copies are in
+// flight together (beyond that the parts of unequal sequences would keep CTAs waiting for the longest); where every sequence has the same
+// length, no longer than an even share.  Decode of 4 sequences of up to 101 tokens, 8 KV heads of 128: 10.7 us with the even cut, 6.3 with parts.
+int decode_parts(int B, int HV, int n_cta, long long longest_pages, bool equal_lengths, int ring_pages) {
+  const long long segs = (long long)B * HV;
+  if (segs <= 0 || segs > n_cta || longest_pages <= 0 || B + 1 > kMaxSmemPrefix) return 0;
+  const long long k = n_cta / segs, most = (longest_pages + k - 1) / k;
+  const long long share = (segs * longest_pages + n_cta - 1) / n_cta;
+  if (most <= ring_pages) return (int)((longest_pages + ring_pages - 1) / ring_pages);     // (more CTAs would have nothing to do)
+  return equal_lengths && most <= share ? (int)k : 0;
 }
 
 cudaError_t launch_decode(const CUtensorMap& kmap, const CUtensorMap& vmap, const DecodeParams& p,

@@ -49,6 +49,7 @@ struct DecodeParams {
   int bt_stride;
   long long num_pages;
   int n_cta, stages, slot_rows;
+  int parts;                   // CTAs per segment where segments are cut into equal parts (decode_parts), 0: the even cut
   float scale;                 // 1 / sqrt(D)
   float scale_log2;            // scale * log2(e)
 };
@@ -77,6 +78,8 @@ constexpr size_t kWsInitBytes = kWsPrefixOffset;   // what fa_decode_workspace_i
 // cache, [rows, D] bytes with a min(D, 128)-column x 16-row box (128-byte swizzle, none for D = 64).
 cudaError_t launch_decode(const CUtensorMap& kmap, const CUtensorMap& vmap, const DecodeParams& p,
                           int D, int kind, int warps, size_t smem_bytes, cudaStream_t stream);
+
+int decode_parts(int B, int HV, int n_cta, long long longest_pages, bool equal_lengths, int ring_pages);
 
 size_t decode_smem_bytes(int D, int warps, int stages, int slot_rows, int B, int kv_elem_bytes);
 

@@ -1,6 +1,7 @@
 // Launcher of the tcgen05 prefill kernel (prefill_tc5_kernel.cuh) for the dense and packed attention operators.
 #include "prefill.cuh"
 #include "prefill_tc5_kernel.cuh"
+#include "smem_limit.cuh"
 
 namespace fa {
 
@@ -51,7 +52,8 @@ cudaError_t launch_tc5_t(const PrefillParams& pp, void* encode_fn, cudaStream_t 
   p.scale_log2 = pp.scale_log2;
   const size_t smem = Tc5Layout<D / 64, 0, D>::BYTES;
   Tc5Kernel kern = pp.in_bf16 ? pick_kernel_bf16<D>() : pick_kernel<D>();
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  static SharedMemoryLimit limits[4];
+  cudaError_t e = limits[(pp.in_bf16 ? 2 : 0) + (g_tc5_poly ? 1 : 0)].raise(reinterpret_cast<const void*>(kern), (int)smem);
   if (e != cudaSuccess) return e;
   const int max_len = dense ? pp.N : pp.max_seqlen;
   dim3 grid;
@@ -62,8 +64,10 @@ cudaError_t launch_tc5_t(const PrefillParams& pp, void* encode_fn, cudaStream_t 
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   grid = dim3((unsigned)(n_items < sms ? n_items : sms));
-  e = next_item_counter(&p.item_counter, stream);
-  if (e != cudaSuccess) return e;
+  if (n_items > sms) {           // (else CTA i has item i, and the launch that zeroes the counter is not needed: three short prompts 16.2 -> 12.4 us)
+    e = next_item_counter(&p.item_counter, stream);
+    if (e != cudaSuccess) return e;
+  }
   kern<<<grid, 640, smem, stream>>>(qmap, kmap, vmap, qmap, kmap, p);
   return cudaGetLastError();
 }

@@ -86,7 +86,7 @@ struct Tc5Params {
   int dense;
   int out_bf16;    // store O as bfloat16 instead of fp16
   int n_hg, n_rb;  // head groups and row blocks of the item grid (items = n_rb * batch * n_hg)
-  unsigned long long* item_counter;  // next unclaimed item of this launch (zeroed in-stream before it)
+  unsigned long long* item_counter;  // next unclaimed item of this launch (zeroed in-stream before it); null: CTA i has item i
   float scale_log2;
 };
 // Builds with a shared key part (a type of its own: the wider parameter block costs the plain builds registers).
@@ -595,13 +595,16 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_consta
     // sequence) and publishes the others through the item queue, up to kItemQ items ahead of the slowest
     // role: the latency of the global atomic stays off every other role's path.
     if (lane == 0) {
+      bool first = true;
       for (uint32_t ic = 0;; ++ic) {
         if (*abort_flag) break;
         Tc5Item it;
         long long item;
         bool have = false;
         while (true) {
-          item = (long long)atomicAdd(p.item_counter, 1ULL);
+          if (p.item_counter != nullptr) item = (long long)atomicAdd(p.item_counter, 1ULL);
+          else item = first ? (long long)blockIdx.x : n_items;
+          first = false;
           if (item >= n_items) break;
           if (tc5_decode_item<EXT>(p, item, it)) { have = true; break; }
         }

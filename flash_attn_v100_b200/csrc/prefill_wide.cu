@@ -21,6 +21,7 @@
 // the MMA batch that read it (a tcgen05.commit costs the tensor pipe about as much as an MMA).
 #include "prefill.cuh"
 #include "prefill_tc5_kernel.cuh"
+#include "smem_limit.cuh"
 
 namespace fa {
 
@@ -511,7 +512,8 @@ cudaError_t launch_prefill_wide(const PrefillParams& pp, int sm_count, void* enc
   p.n_rb = ((dense ? pp.N : pp.max_seqlen) + 127) / 128;
   cudaError_t e = prefill_status_ptr(&p.status);
   if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(prefill_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kWideSmem);
+  static SharedMemoryLimit limit;
+  e = limit.raise(reinterpret_cast<const void*>(prefill_wide_kernel), kWideSmem);
   if (e != cudaSuccess) return e;
   const long long n_items = (long long)p.n_rb * pp.batch * pp.H_Q;
   if (n_items > sm_count) {
