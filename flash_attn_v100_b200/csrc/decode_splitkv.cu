@@ -114,42 +114,21 @@ __device__ __forceinline__ int seq_len_of(const DecodeParams& p, int b) {
   return n < 0 ? 0 : (int)n;
 }
 
-// MMA on the query-head block.  HM ("half M"): the block has at most 8 heads, so fragment rows 8-15 are
-// all-zero padding: their A registers are passed as zero and their accumulators are not kept.
-template <bool HM, bool BF = false>
-__device__ __forceinline__ void mma_rows(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  if constexpr (HM && BF) {
-    float d2, d3;
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%5}, {%7,%8}, "
-        "{%0,%1,%9,%9};"
-        : "+f"(c[0]), "+f"(c[1]), "=f"(d2), "=f"(d3)
-        : "r"(a[0]), "r"(0u), "r"(a[2]), "r"(b0), "r"(b1), "f"(0.f));
-  } else if constexpr (HM) {
-    float d2, d3;
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%5}, {%7,%8}, "
-        "{%0,%1,%9,%9};"
-        : "+f"(c[0]), "+f"(c[1]), "=f"(d2), "=f"(d3)
-        : "r"(a[0]), "r"(0u), "r"(a[2]), "r"(b0), "r"(b1), "f"(0.f));
-  } else if constexpr (BF) {
-    mma_bf16_16816(c, a, b0, b1);
-  } else {
-    mma_f16_16816(c, a, b0, b1);
-  }
+// MMAs.  Builds for at most 8 query heads per KV head (HM) have the tokens (scores) and the head dimensions (output) in the 16 rows of the MMA
+// and the heads in its 8 columns: S^T = K Q^T, O^T = V^T P^T.  The others have the heads in the rows.
+// (With the heads in the rows half of every MMA worked on rows of zeros, and the accumulators' empty halves had to be cleared before each
+// one.  32 sequences, 32 heads on 8 of 128: int8 cache of 8192 tokens 138.6 us so, 120.7 turned; scores in whole numbers over 4096 124.5 and 121.9.)
+template <bool BF>
+__device__ __forceinline__ void mma_f(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  const uint32_t a[4] = {a0, a1, a2, a3};
+  if constexpr (BF) mma_bf16_16816(c, a, b0, b1);
+  else mma_f16_16816(c, a, b0, b1);
 }
-template <bool HM>
-__device__ __forceinline__ void mma_s8_rows(int (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  if constexpr (HM) {
-    int d2, d3;
-    asm volatile(
-        "mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%5}, {%7,%8}, "
-        "{%0,%1,%5,%5};"
-        : "+r"(c[0]), "+r"(c[1]), "=r"(d2), "=r"(d3)
-        : "r"(a[0]), "r"(0u), "r"(a[2]), "r"(b0), "r"(b1));
-  } else {
-    mma_s8_16832(c, a, b0, b1);
-  }
+// 8 x 8 tile of 16-bit elements, transposed across the warp (two elements of a row per lane).
+__device__ __forceinline__ uint32_t transpose_8x8(uint32_t x) {
+  uint32_t y;
+  asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y) : "r"(x));
+  return y;
 }
 
 // ---- int8 KV cache helpers ---------------------------------------------------
@@ -199,17 +178,18 @@ __device__ __forceinline__ void load_v_row(const uint8_t* vptr, int tok, int g, 
   }
 }
 
-// Byte J of the words of four token rows (2c, 2c+1 | 2c+8, 2c+9) -> the B fragment of one output
-// tile, dequantised as in dequant_k4, then acc += P * V.
-template <int J, bool HM>
-__device__ __forceinline__ void dequant_v_pair(uint32_t wa, uint32_t wb, uint32_t wc, uint32_t wd, uint32_t sc_lo,
-                                               uint32_t sc_hi, const uint32_t (&pa)[4], float (&acc)[4]) {
+// Byte J of the words of four token rows (2c, 2c+1 | 2c+8, 2c+9), dequantised as in hsub_hmul: one output column's pairs of tokens.
+template <int J>
+__device__ __forceinline__ void dequant_v_pair(uint32_t wa, uint32_t wb, uint32_t wc, uint32_t wd, uint32_t sc_lo, uint32_t sc_hi, uint32_t& lo,
+                                               uint32_t& hi) {
   constexpr uint32_t sel = ((4u + J) << 12) | ((4u + J) << 8) | (J << 4) | J;  // [a.bJ, a.bJ, b.bJ, b.bJ]
-  uint32_t lo = __byte_perm(wa, wb, sel), hi = __byte_perm(wc, wd, sel);
+  lo = __byte_perm(wa, wb, sel);
+  hi = __byte_perm(wc, wd, sel);
   // low byte of each half: x ^ 0x80; high byte: 0x64   (f = a ? (t ^ b) : b, lut 0x6a)
   asm("lop3.b32 %0, %0, 0x00ff00ff, 0x64806480, 0x6a;" : "+r"(lo));
   asm("lop3.b32 %0, %0, 0x00ff00ff, 0x64806480, 0x6a;" : "+r"(hi));
-  mma_rows<HM>(acc, pa, hsub_hmul(lo, 0x64806480u, sc_lo), hsub_hmul(hi, 0x64806480u, sc_hi));
+  lo = hsub_hmul(lo, 0x64806480u, sc_lo);
+  hi = hsub_hmul(hi, 0x64806480u, sc_hi);
 }
 
 __device__ __forceinline__ int pages_of(const DecodeParams& p, int b) {
@@ -289,7 +269,7 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap,
   constexpr bool INT8 = KIND == kKindInt8QK;   // fp16 cache, K and Q quantised on the fly for the scores
   constexpr bool KV8 = KIND == kKindInt8KV;    // int8 cache with per-token fp16 scales
   constexpr bool BF = KIND == kKindBF16;       // bfloat16 q / cache: the fp16 path with bfloat16 MMAs and P
-  constexpr int NR = HM ? 2 : 4;               // live accumulator registers per fragment (rows g | g, g + 8)
+  constexpr int NACC = HM ? D / 16 : D / 8;    // output fragments: 16 dimensions x 8 heads, or 16 heads x 8 dimensions
   constexpr int PAGE_BYTES = 16 * D * (KV8 ? 1 : 2);
   // One TMA box: 16 rows x 128 bytes (64 fp16 or 128 int8 columns), 128-byte swizzle;
   // D = 64 int8 rows are 64 bytes wide and are copied unswizzled.
@@ -467,7 +447,7 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap,
     // a lane then reads 16 consecutive int8 of a token row for four k-steps.  Q uses the same map.
     constexpr int KPS = (D >= 128) ? 8 : 4;
     uint32_t qa[QREGS][4];
-    float q_s0 = 1.f, q_s1 = 1.f;
+    float q_s0 = 1.f, q_s1 = 1.f, qc_s0 = 1.f, qc_s1 = 1.f;
     float kbias0 = 0.f, kbias1 = 0.f;  // KV8 only
     {
       // D is the padded head dimension the kernel is built for, Dr the real one: columns [Dr, D) of K and V
@@ -498,6 +478,10 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap,
         kbias1 += __shfl_xor_sync(0xffffffffu, kbias1, 2);
         kbias0 *= 1152.f;
         kbias1 *= 1152.f;
+        if constexpr (HM) {       // ... of heads cq and cq + 1
+          kbias1 = __shfl_sync(0xffffffffu, kbias0, (cq + 1) * 4);
+          kbias0 = __shfl_sync(0xffffffffu, kbias0, cq * 4);
+        }
       } else if constexpr (!INT8) {
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk) {
@@ -509,6 +493,10 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap,
         }
       } else {
         if (v0) q_s0 = __ldg(p.q_scale + (size_t)b * p.H_Q + head0 + g);
+        if constexpr (HM) {       // the scores' columns are heads cq and cq + 1
+          if (cq < Gb) qc_s0 = __ldg(p.q_scale + (size_t)b * p.H_Q + head0 + cq);
+          if (cq + 1 < Gb) qc_s1 = __ldg(p.q_scale + (size_t)b * p.H_Q + head0 + cq + 1);
+        }
         if (v1) q_s1 = __ldg(p.q_scale + (size_t)b * p.H_Q + head0 + g + 8);
         // Slot 4c+i of k-step kk of the int8 MMA stands for head dimension
         // 32*kk + {2c, 2c+1, 8+2c, 9+2c}[i], slot 16+4c+i for the same plus 16: these are the values a
@@ -535,9 +523,9 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap,
       }
     }
 
-    float acc[NT][4];
+    float acc[NACC][4];
 #pragma unroll
-    for (int i = 0; i < NT; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+    for (int i = 0; i < NACC; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
     float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
 
     // Block-table entries of this warp's pages, 32 at a time, one batch ahead.
@@ -661,7 +649,7 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap,
       // ---- S = Q K^T : [16 heads x 16 tokens] ------------------------------------
       if constexpr (KV8) {
 #pragma unroll
-        for (int j = 0; j < 2; ++j) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
+        for (int j = 0; j < (HM ? 1 : 2); ++j) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
         const uint8_t* kptr = my_stages + (size_t)st * (2 * PAGE_BYTES);
 #pragma unroll
         for (int q4 = 0; q4 < D / 64; ++q4) {  // 16 bytes = four k-steps per load; token g and token g + 8
@@ -672,32 +660,46 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap,
           const uint32_t w1[4] = {wb.x, wb.y, wb.z, wb.w};
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            uint32_t b0, b1;
+            const uint32_t (&q)[4] = qa[q4 * 4 + i];
+            uint32_t b0, b1, c0, c1;
             dequant_k4_biased(w0[i], b0, b1);
-            mma_rows<HM>(s[0], qa[q4 * 4 + i], b0, b1);
-            dequant_k4_biased(w1[i], b0, b1);
-            mma_rows<HM>(s[1], qa[q4 * 4 + i], b0, b1);
+            dequant_k4_biased(w1[i], c0, c1);
+            if constexpr (HM) {
+              mma_f<false>(s[0], b0, c0, b1, c1, q[0], q[2]);
+            } else {
+              mma_f16_16816(s[0], q, b0, b1);
+              mma_f16_16816(s[1], q, c0, c1);
+            }
           }
         }
         // score = (raw - 1152 * sum q) * k_scale[token] / sqrt(D), in fp32, to base 2.  The per-element
         // product k * k_scale is not rounded to fp16 first: the score is the exact-dequantisation score
         // up to fp32 rounding.
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          const uint32_t ka = __shfl_sync(0xffffffffu, sc_cur, 8 * j + cq);
-          const uint32_t kb = __shfl_sync(0xffffffffu, sc_cur, 8 * j + cq + 1);
+        if constexpr (HM) {
+          const uint32_t ka = __shfl_sync(0xffffffffu, sc_cur, g);
+          const uint32_t kb = __shfl_sync(0xffffffffu, sc_cur, g + 8);
           const float ta = __half2float(__ushort_as_half((unsigned short)ka)) * p.scale_log2;
           const float tb = __half2float(__ushort_as_half((unsigned short)kb)) * p.scale_log2;
-          s[j][0] = (s[j][0] - kbias0) * ta;
-          s[j][1] = (s[j][1] - kbias0) * tb;
-          if constexpr (!HM) {
+          s[0][0] = (s[0][0] - kbias0) * ta;
+          s[0][1] = (s[0][1] - kbias1) * ta;
+          s[0][2] = (s[0][2] - kbias0) * tb;
+          s[0][3] = (s[0][3] - kbias1) * tb;
+        } else {
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            const uint32_t ka = __shfl_sync(0xffffffffu, sc_cur, 8 * j + cq);
+            const uint32_t kb = __shfl_sync(0xffffffffu, sc_cur, 8 * j + cq + 1);
+            const float ta = __half2float(__ushort_as_half((unsigned short)ka)) * p.scale_log2;
+            const float tb = __half2float(__ushort_as_half((unsigned short)kb)) * p.scale_log2;
+            s[j][0] = (s[j][0] - kbias0) * ta;
+            s[j][1] = (s[j][1] - kbias0) * tb;
             s[j][2] = (s[j][2] - kbias1) * ta;
             s[j][3] = (s[j][3] - kbias1) * tb;
           }
         }
       } else if constexpr (!INT8) {
 #pragma unroll
-        for (int j = 0; j < 2; ++j) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
+        for (int j = 0; j < (HM ? 1 : 2); ++j) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
         const int mi = lane >> 3;
         const int r = (lane & 7) + (mi >> 1) * 8;
 #pragma unroll
@@ -706,13 +708,17 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap,
           const uint32_t addr = kbase + (chunk >> 3) * SLAB_BYTES + r * 128 + (((chunk & 7) ^ (r & 7)) << 4);
           uint32_t kb[4];
           ldmatrix_x4(kb, addr);
-          mma_rows<HM, BF>(s[0], qa[kk], kb[0], kb[1]);
-          mma_rows<HM, BF>(s[1], qa[kk], kb[2], kb[3]);
+          if constexpr (HM) {
+            mma_f<BF>(s[0], kb[0], kb[2], kb[1], kb[3], qa[kk][0], qa[kk][2]);
+          } else {
+            mma_f<BF>(s[0], qa[kk][0], qa[kk][1], qa[kk][2], qa[kk][3], kb[0], kb[1]);
+            mma_f<BF>(s[1], qa[kk][0], qa[kk][1], qa[kk][2], qa[kk][3], kb[2], kb[3]);
+          }
         }
 #pragma unroll
-        for (int j = 0; j < 2; ++j)
+        for (int j = 0; j < (HM ? 1 : 2); ++j)
 #pragma unroll
-          for (int e = 0; e < NR; ++e) s[j][e] *= p.scale_log2;
+          for (int e = 0; e < 4; ++e) s[j][e] *= p.scale_log2;
       } else {
         int si[2][4];
 #pragma unroll
@@ -777,29 +783,41 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap,
         }
 #pragma unroll
         for (int kk = 0; kk < D / 32; ++kk) {
-          mma_s8_rows<HM>(si[0], qa[kk], bq[0][kk][0], bq[0][kk][1]);
-          mma_s8_rows<HM>(si[1], qa[kk], bq[1][kk][0], bq[1][kk][1]);
+          if constexpr (HM) {
+            const uint32_t ka[4] = {bq[0][kk][0], bq[1][kk][0], bq[0][kk][1], bq[1][kk][1]};
+            mma_s8_16832(si[0], ka, qa[kk][0], qa[kk][2]);
+          } else {
+            mma_s8_16832(si[0], qa[kk], bq[0][kk][0], bq[0][kk][1]);
+            mma_s8_16832(si[1], qa[kk], bq[1][kk][0], bq[1][kk][1]);
+          }
         }
+        // score = float(dot) * q_s * k_s * scale, then to base 2
+        if constexpr (HM) {
+          s[0][0] = ((static_cast<float>(si[0][0]) * qc_s0) * ksr0) * p.scale * 1.4426950408889634f;
+          s[0][1] = ((static_cast<float>(si[0][1]) * qc_s1) * ksr0) * p.scale * 1.4426950408889634f;
+          s[0][2] = ((static_cast<float>(si[0][2]) * qc_s0) * ksr1) * p.scale * 1.4426950408889634f;
+          s[0][3] = ((static_cast<float>(si[0][3]) * qc_s1) * ksr1) * p.scale * 1.4426950408889634f;
+        } else {
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          const float ks_a = __shfl_sync(0xffffffffu, ks_cur, 8 * j + cq);
-          const float ks_b = __shfl_sync(0xffffffffu, ks_cur, 8 * j + cq + 1);
-          // score = float(dot) * q_s * k_s * scale, then to base 2
-          s[j][0] = ((static_cast<float>(si[j][0]) * q_s0) * ks_a) * p.scale * 1.4426950408889634f;
-          s[j][1] = ((static_cast<float>(si[j][1]) * q_s0) * ks_b) * p.scale * 1.4426950408889634f;
-          if constexpr (!HM) {
+          for (int j = 0; j < 2; ++j) {
+            const float ks_a = __shfl_sync(0xffffffffu, ks_cur, 8 * j + cq);
+            const float ks_b = __shfl_sync(0xffffffffu, ks_cur, 8 * j + cq + 1);
+            s[j][0] = ((static_cast<float>(si[j][0]) * q_s0) * ks_a) * p.scale * 1.4426950408889634f;
+            s[j][1] = ((static_cast<float>(si[j][1]) * q_s0) * ks_b) * p.scale * 1.4426950408889634f;
             s[j][2] = ((static_cast<float>(si[j][2]) * q_s1) * ks_a) * p.scale * 1.4426950408889634f;
             s[j][3] = ((static_cast<float>(si[j][3]) * q_s1) * ks_b) * p.scale * 1.4426950408889634f;
           }
-          if (p.scores_out != nullptr) {
+        }
+        if (p.scores_out != nullptr) {
 #pragma unroll
-            for (int e = 0; e < NR; ++e) {
-              const int row = g + (e >> 1) * 8;
-              const int tin = 8 * j + cq + (e & 1);
+          for (int j = 0; j < (HM ? 1 : 2); ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const int row = HM ? cq + (e & 1) : g + (e >> 1) * 8;
+              const int tin = HM ? g + (e >> 1) * 8 : 8 * j + cq + (e & 1);
               if (row < Gb && ((vmask >> tin) & 1u))
                 p.scores_out[((size_t)b * p.H_Q + head0 + row) * p.N + page * 16 + tin] = si[j][e];
             }
-          }
         }
       }
 
@@ -818,56 +836,69 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap,
 
       if (vmask != 0xffffu) {
 #pragma unroll
-        for (int j = 0; j < 2; ++j)
+        for (int j = 0; j < (HM ? 1 : 2); ++j)
 #pragma unroll
-          for (int e = 0; e < NR; ++e)
-            if (!((vmask >> (8 * j + cq + (e & 1))) & 1u)) s[j][e] = -INFINITY;
+          for (int e = 0; e < 4; ++e)
+            if (!((vmask >> (HM ? g + (e >> 1) * 8 : 8 * j + cq + (e & 1))) & 1u)) s[j][e] = -INFINITY;
       }
 
-      // ---- online softmax (base 2) ----------------------------------------------
-      float mx0 = fmaxf(fmaxf(s[0][0], s[0][1]), fmaxf(s[1][0], s[1][1]));
-      mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1));
-      mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
-      const float mn0 = fmaxf(m0, mx0);
-      const float a0 = fast_exp2(m0 - mn0);
-      m0 = mn0;
-      float pr[2][4];
+      // ---- online softmax (base 2): of heads cq and cq + 1 (HM), or g and g + 8 ----------
+      float mx0, mx1;
+      if constexpr (HM) {
+        mx0 = fmaxf(s[0][0], s[0][2]);
+        mx1 = fmaxf(s[0][1], s[0][3]);
 #pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        pr[j][0] = fast_exp2(s[j][0] - mn0);
-        pr[j][1] = fast_exp2(s[j][1] - mn0);
-      }
-      l0 = l0 * a0 + (pr[0][0] + pr[0][1] + pr[1][0] + pr[1][1]);
-      float a1 = 1.f;
-      uint32_t pa[4];
-      pa[0] = BF ? pack_bf162(pr[0][0], pr[0][1]) : pack_half2(pr[0][0], pr[0][1]);
-      pa[2] = BF ? pack_bf162(pr[1][0], pr[1][1]) : pack_half2(pr[1][0], pr[1][1]);
-      pa[1] = pa[3] = 0u;
-      if constexpr (!HM) {
-        float mx1 = fmaxf(fmaxf(s[0][2], s[0][3]), fmaxf(s[1][2], s[1][3]));
+        for (int o = 4; o < 32; o <<= 1) {
+          mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, o));
+          mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, o));
+        }
+      } else {
+        mx0 = fmaxf(fmaxf(s[0][0], s[0][1]), fmaxf(s[1][0], s[1][1]));
+        mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1));
+        mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
+        mx1 = fmaxf(fmaxf(s[0][2], s[0][3]), fmaxf(s[1][2], s[1][3]));
         mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
         mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
-        const float mn1 = fmaxf(m1, mx1);
-        a1 = fast_exp2(m1 - mn1);
-        m1 = mn1;
+      }
+      const float mn0 = fmaxf(m0, mx0), mn1 = fmaxf(m1, mx1);
+      const float a0 = fast_exp2(m0 - mn0), a1 = fast_exp2(m1 - mn1);
+      m0 = mn0;
+      m1 = mn1;
+      float pr[2][4];
+      uint32_t pa[4];
+      auto pack2 = [](float x, float y) { return BF ? pack_bf162(x, y) : pack_half2(x, y); };
+      if constexpr (HM) {
+        pr[0][0] = fast_exp2(s[0][0] - mn0);
+        pr[0][1] = fast_exp2(s[0][1] - mn1);
+        pr[0][2] = fast_exp2(s[0][2] - mn0);
+        pr[0][3] = fast_exp2(s[0][3] - mn1);
+        l0 = l0 * a0 + (pr[0][0] + pr[0][2]);
+        l1 = l1 * a1 + (pr[0][1] + pr[0][3]);
+        pa[0] = transpose_8x8(pack2(pr[0][0], pr[0][1]));     // P^T as the MMA's second operand: head g, tokens cq, cq + 1
+        pa[2] = transpose_8x8(pack2(pr[0][2], pr[0][3]));     // ... and eight tokens on
+        pa[1] = pa[3] = 0u;
+      } else {
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
+          pr[j][0] = fast_exp2(s[j][0] - mn0);
+          pr[j][1] = fast_exp2(s[j][1] - mn0);
           pr[j][2] = fast_exp2(s[j][2] - mn1);
           pr[j][3] = fast_exp2(s[j][3] - mn1);
         }
+        l0 = l0 * a0 + (pr[0][0] + pr[0][1] + pr[1][0] + pr[1][1]);
         l1 = l1 * a1 + (pr[0][2] + pr[0][3] + pr[1][2] + pr[1][3]);
-        pa[1] = BF ? pack_bf162(pr[0][2], pr[0][3]) : pack_half2(pr[0][2], pr[0][3]);
-        pa[3] = BF ? pack_bf162(pr[1][2], pr[1][3]) : pack_half2(pr[1][2], pr[1][3]);
+        pa[0] = pack2(pr[0][0], pr[0][1]);
+        pa[1] = pack2(pr[0][2], pr[0][3]);
+        pa[2] = pack2(pr[1][0], pr[1][1]);
+        pa[3] = pack2(pr[1][2], pr[1][3]);
       }
       if (__any_sync(0xffffffffu, (a0 != 1.f) || (a1 != 1.f))) {
 #pragma unroll
-        for (int i = 0; i < NT; ++i) {
+        for (int i = 0; i < NACC; ++i) {
           acc[i][0] *= a0;
-          acc[i][1] *= a0;
-          if constexpr (!HM) {
-            acc[i][2] *= a1;
-            acc[i][3] *= a1;
-          }
+          acc[i][1] *= HM ? a1 : a0;
+          acc[i][2] *= HM ? a0 : a1;
+          acc[i][3] *= a1;
         }
       }
 
@@ -901,10 +932,18 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap,
         load_v_row<D>(vptr, c2 + 9, g, vd);
 #pragma unroll
         for (int wd = 0; wd < NW; ++wd) {
-          dequant_v_pair<0, HM>(va[wd], vb[wd], vc[wd], vd[wd], sc_lo, sc_hi, pa, acc[wd * 4 + 0]);
-          dequant_v_pair<1, HM>(va[wd], vb[wd], vc[wd], vd[wd], sc_lo, sc_hi, pa, acc[wd * 4 + 1]);
-          dequant_v_pair<2, HM>(va[wd], vb[wd], vc[wd], vd[wd], sc_lo, sc_hi, pa, acc[wd * 4 + 2]);
-          dequant_v_pair<3, HM>(va[wd], vb[wd], vc[wd], vd[wd], sc_lo, sc_hi, pa, acc[wd * 4 + 3]);
+          uint32_t lo[4], hi[4];
+          dequant_v_pair<0>(va[wd], vb[wd], vc[wd], vd[wd], sc_lo, sc_hi, lo[0], hi[0]);
+          dequant_v_pair<1>(va[wd], vb[wd], vc[wd], vd[wd], sc_lo, sc_hi, lo[1], hi[1]);
+          dequant_v_pair<2>(va[wd], vb[wd], vc[wd], vd[wd], sc_lo, sc_hi, lo[2], hi[2]);
+          dequant_v_pair<3>(va[wd], vb[wd], vc[wd], vd[wd], sc_lo, sc_hi, lo[3], hi[3]);
+          if constexpr (HM) {
+            mma_f<false>(acc[wd * 2], lo[0], lo[1], hi[0], hi[1], pa[0], pa[2]);
+            mma_f<false>(acc[wd * 2 + 1], lo[2], lo[3], hi[2], hi[3], pa[0], pa[2]);
+          } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) mma_f16_16816(acc[wd * 4 + i], pa, lo[i], hi[i]);
+          }
         }
       } else {
         const int mi = lane >> 3;
@@ -915,8 +954,12 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap,
           const uint32_t addr = vbase + (chunk >> 3) * SLAB_BYTES + r * 128 + (((chunk & 7) ^ (r & 7)) << 4);
           uint32_t vb[4];
           ldmatrix_x4_trans(vb, addr);
-          mma_rows<HM, BF>(acc[2 * c2], pa, vb[0], vb[1]);
-          mma_rows<HM, BF>(acc[2 * c2 + 1], pa, vb[2], vb[3]);
+          if constexpr (HM) {
+            mma_f<BF>(acc[c2], vb[0], vb[2], vb[1], vb[3], pa[0], pa[2]);
+          } else {
+            mma_f<BF>(acc[2 * c2], pa[0], pa[1], pa[2], pa[3], vb[0], vb[1]);
+            mma_f<BF>(acc[2 * c2 + 1], pa[0], pa[1], pa[2], pa[3], vb[2], vb[3]);
+          }
         }
       }
 
@@ -938,44 +981,47 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap,
     }
 
     // ---- merge the warps of this CTA ---------------------------------------------
-    l0 += __shfl_xor_sync(0xffffffffu, l0, 1);
-    l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
-    if constexpr (!HM) {
-      l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
-      l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
+#pragma unroll
+    for (int o = (HM ? 4 : 1); o < (HM ? 32 : 4); o <<= 1) {
+      l0 += __shfl_xor_sync(0xffffffffu, l0, o);
+      l1 += __shfl_xor_sync(0xffffffffu, l1, o);
     }
     {
       float* mb = mbuf + (size_t)warp * p.slot_rows * ROWLEN;
-      if (g < Gb) {
-        float* rowp = mb + g * ROWLEN;
+      if constexpr (HM) {
+        // fragment i: dimensions 16i + g and 16i + 8 + g (KV8: NT*g + 2i and one on) of heads cq and cq + 1
 #pragma unroll
-        for (int i = 0; i < NT; ++i) {
-          if constexpr (KV8) {
-            rowp[NT * cq + i] = acc[i][0];
-            rowp[NT * (cq + 1) + i] = acc[i][1];
-          } else {
-            *reinterpret_cast<float2*>(rowp + i * 8 + cq) = make_float2(acc[i][0], acc[i][1]);
+        for (int e = 0; e < 2; ++e) {
+          if (cq + e >= Gb) continue;
+          float* rowp = mb + (cq + e) * ROWLEN;
+#pragma unroll
+          for (int i = 0; i < NACC; ++i) {
+            rowp[KV8 ? NT * g + 2 * i : 16 * i + g] = acc[i][e];
+            rowp[KV8 ? NT * g + 2 * i + 1 : 16 * i + 8 + g] = acc[i][2 + e];
+          }
+          if (g == 0) {
+            rowp[D] = e ? m1 : m0;
+            rowp[D + 1] = e ? l1 : l0;
           }
         }
-        if ((lane & 3) == 0) {
-          rowp[D] = m0;
-          rowp[D + 1] = l0;
-        }
-      }
-      if (!HM && g + 8 < Gb) {
-        float* rowp = mb + (g + 8) * ROWLEN;
+      } else {
 #pragma unroll
-        for (int i = 0; i < NT; ++i) {
-          if constexpr (KV8) {
-            rowp[NT * cq + i] = acc[i][2];
-            rowp[NT * (cq + 1) + i] = acc[i][3];
-          } else {
-            *reinterpret_cast<float2*>(rowp + i * 8 + cq) = make_float2(acc[i][2], acc[i][3]);
+        for (int e = 0; e < 2; ++e) {
+          if (g + 8 * e >= Gb) continue;
+          float* rowp = mb + (g + 8 * e) * ROWLEN;
+#pragma unroll
+          for (int i = 0; i < NACC; ++i) {
+            if constexpr (KV8) {
+              rowp[NT * cq + i] = acc[i][2 * e];
+              rowp[NT * (cq + 1) + i] = acc[i][2 * e + 1];
+            } else {
+              *reinterpret_cast<float2*>(rowp + i * 8 + cq) = make_float2(acc[i][2 * e], acc[i][2 * e + 1]);
+            }
           }
-        }
-        if ((lane & 3) == 0) {
-          rowp[D] = m1;
-          rowp[D + 1] = l1;
+          if ((lane & 3) == 0) {
+            rowp[D] = e ? m1 : m0;
+            rowp[D + 1] = e ? l1 : l0;
+          }
         }
       }
     }
