@@ -22,8 +22,8 @@
 // goes to warp i mod W) through a private ring of shared-memory stages filled
 // by TMA (cp.async.bulk.tensor, 128-byte swizzle, completion on an mbarrier).
 // K and V of a page for one KV head are 16 x D fp16 = one contiguous 4 KB block
-// at D = 128.  All query heads of the group are processed together (they are
-// the M rows of the MMA) so each K/V byte is read from HBM exactly once.
+// at D = 128.  All query heads of the group are processed together (they share
+// every MMA) so each K/V byte is read from HBM exactly once.
 // S = Q K^T and O += P V run on mma.sync m16n8k16 (fp32 accumulate) with
 // ldmatrix from the swizzled tiles; softmax is fp32, base-2, online.
 #include "common.cuh"
@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(1024) decode_plan_kernel(const DecodeParams p)
 #define FA_F16_MINB 2
 #endif
 #ifndef FA_KV8_MINB
-#define FA_KV8_MINB 3
+#define FA_KV8_MINB 4
 #endif
 #ifndef FA_I8QK_MINB
 #define FA_I8QK_MINB 3
@@ -345,14 +345,17 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap,
   if (per < 1) per = 1;
   long long u = (long long)blockIdx.x * per;
   long long u1 = (u + per < T) ? (u + per) : T;
-  int part_pages = 0;
+  // pages per part of a sequence of np pages (computed where it is used: nothing of it stays in registers through the loop)
+  auto part_pages_of = [&](int np) {
+    const int n = (np + p.parts - 1) / p.parts;
+    return n < W * S ? W * S : n;
+  };
   if (p.parts > 0) {
     // a segment is cut into parts of equal length (at least what the rings hold), one per CTA: see decode_parts
     const int seg = (int)blockIdx.x / p.parts;
     if (seg >= p.B * p.HV) return;
     const int bb = seg / p.HV, np = pre[bb + 1] - pre[bb];
-    part_pages = (np + p.parts - 1) / p.parts;
-    if (part_pages < W * S) part_pages = W * S;
+    const int part_pages = part_pages_of(np);
     const int lo = ((int)blockIdx.x - seg * p.parts) * part_pages;
     if (lo >= np) return;
     u = (long long)p.HV * pre[bb] + (long long)(seg - bb * p.HV) * np + lo;
@@ -1057,7 +1060,7 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap,
       // whoever arrives last merges all partials of the segment.
       const long long seg_start = (long long)p.HV * pre[b] + (long long)hv * np;
       const int first = p.parts > 0 ? (b * p.HV + hv) * p.parts : (int)(seg_start / per);
-      const int last = p.parts > 0 ? first + (np - 1) / part_pages : (int)((seg_start + np - 1) / per);
+      const int last = p.parts > 0 ? first + (np - 1) / part_pages_of(np) : (int)((seg_start + np - 1) / per);
       const unsigned int n_parts = (unsigned int)(last - first + 1);
       __threadfence();
       __syncthreads();
