@@ -295,6 +295,16 @@ recurrence_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
       }
     };
     const uint64_t khd = smem_desc(sK, SLAB, 1024), shd = smem_desc(sSh, SLAB, 1024), sld = smem_desc(sSl, SLAB, 1024);
+    auto issue_old = [&]() {                                  // Q S
+      const uint64_t qd = smem_desc(sQ, 16, 1024);
+#pragma unroll
+      for (int ks = 0; ks < 8; ++ks) {
+        const uint32_t off = (uint32_t)(ks >> 2) * (SLAB >> 4) + (uint32_t)(ks & 3) * 2u;
+        tc_mma_ss(tmem + 128u, qd + off, shd + (uint64_t)(ks * 128), IDESC_B, ks > 0 ? 1u : 0u);
+        tc_mma_ss(tmem + 128u, qd + off, sld + (uint64_t)(ks * 128), IDESC_B, 1u);
+      }
+      tc_commit(bar_1);
+    };
     auto issue_state = [&]() {
 #pragma unroll
       for (int ks = 0; ks < 8; ++ks) {
@@ -341,13 +351,7 @@ recurrence_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
           tc_mma_ss(tmem, qd + off, kd + off, IDESC_QK, ks > 0 ? 1u : 0u);
         }
         tc_commit(bar_a);
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {
-          const uint32_t off = (uint32_t)(ks >> 2) * (SLAB >> 4) + (uint32_t)(ks & 3) * 2u;
-          tc_mma_ss(tmem + 128u, qd + off, shd + (uint64_t)(ks * 128), IDESC_B, ks > 0 ? 1u : 0u);
-          tc_mma_ss(tmem + 128u, qd + off, sld + (uint64_t)(ks * 128), IDESC_B, 1u);
-        }
-        tc_commit(bar_1);
+        if constexpr (!NORM) issue_old();
       }
     }
     if (copier) {
@@ -390,7 +394,15 @@ recurrence_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
       tc_fence_before();
       __syncthreads();                                        // P is written over other warps' part of A; n has been read
       tc_fence_after();
-      if constexpr (NORM) advance_norm();
+      if constexpr (NORM) {
+        // Q S only now: its operands would take shared-memory cycles from the sums for the normaliser (16 x 1024 tokens, 32 heads of 128: 245.6 us
+        // with Q S right behind Q K^T, 242.7 so; the sums on mma.sync, which waits for the same tensor cores, 268)
+        if (warp == 0) {
+          __syncwarp();
+          issue_old();
+        }
+        advance_norm();
+      }
       const int over = row - cg * 32;                         // my columns up to this one are at or before my row
       const bool below = __any_sync(0xffffffffu, over >= 0);
 #pragma unroll
