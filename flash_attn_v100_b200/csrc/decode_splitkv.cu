@@ -118,6 +118,8 @@ __device__ __forceinline__ int seq_len_of(const DecodeParams& p, int b) {
 // and the heads in its 8 columns: S^T = K Q^T, O^T = V^T P^T.  The others have the heads in the rows.
 // (With the heads in the rows half of every MMA worked on rows of zeros, and the accumulators' empty halves had to be cleared before each
 // one.  32 sequences, 32 heads on 8 of 128: int8 cache of 8192 tokens 138.6 us so, 120.7 turned; scores in whole numbers over 4096 124.5 and 121.9.)
+// The scores' products are two chains of half the length: with one, 21 sequences of up to 559 tokens, 8 heads on 2 of 256, took 36.9 us against
+// 34.8 with the heads in the rows (which had two); with two, 35.0 against 37.4 on another day's clock.
 template <bool BF>
 __device__ __forceinline__ void mma_f(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   const uint32_t a[4] = {a0, a1, a2, a3};
@@ -262,7 +264,8 @@ struct DecodeOccupancy {
       !HM ? 1 : (D == 64 ? 4 : (D == 256 ? 2 : ((KIND == kKindF16 || KIND == kKindBF16) ? FA_F16_MINB : (KIND == kKindInt8KV ? FA_KV8_MINB : FA_I8QK_MINB))));
 };
 
-template <int D, int KIND, bool HM>
+// PARTS: segments are cut into equal parts (a build of its own: the branches cost the large batches 0.6 %).
+template <int D, int KIND, bool HM, bool PARTS>
 __global__ void __launch_bounds__(DecodeOccupancy<D, KIND, HM>::kThreads, DecodeOccupancy<D, KIND, HM>::kMinBlocks)
 decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap,
                       const __grid_constant__ CUtensorMap vmap, const DecodeParams p) {
@@ -345,12 +348,11 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap,
   if (per < 1) per = 1;
   long long u = (long long)blockIdx.x * per;
   long long u1 = (u + per < T) ? (u + per) : T;
-  // pages per part of a sequence of np pages (computed where it is used: nothing of it stays in registers through the loop)
-  auto part_pages_of = [&](int np) {
+  auto part_pages_of = [&](int np) {       // pages per part of a sequence of np pages
     const int n = (np + p.parts - 1) / p.parts;
     return n < W * S ? W * S : n;
   };
-  if (p.parts > 0) {
+  if constexpr (PARTS) {
     // a segment is cut into parts of equal length (at least what the rings hold), one per CTA: see decode_parts
     const int seg = (int)blockIdx.x / p.parts;
     if (seg >= p.B * p.HV) return;
@@ -652,7 +654,7 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap,
       // ---- S = Q K^T : [16 heads x 16 tokens] ------------------------------------
       if constexpr (KV8) {
 #pragma unroll
-        for (int j = 0; j < (HM ? 1 : 2); ++j) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
+        for (int j = 0; j < 2; ++j) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
         const uint8_t* kptr = my_stages + (size_t)st * (2 * PAGE_BYTES);
 #pragma unroll
         for (int q4 = 0; q4 < D / 64; ++q4) {  // 16 bytes = four k-steps per load; token g and token g + 8
@@ -668,7 +670,7 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap,
             dequant_k4_biased(w0[i], b0, b1);
             dequant_k4_biased(w1[i], c0, c1);
             if constexpr (HM) {
-              mma_f<false>(s[0], b0, c0, b1, c1, q[0], q[2]);
+              mma_f<false>(s[i & 1], b0, c0, b1, c1, q[0], q[2]);       // (two chains of half the length)
             } else {
               mma_f16_16816(s[0], q, b0, b1);
               mma_f16_16816(s[1], q, c0, c1);
@@ -683,10 +685,10 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap,
           const uint32_t kb = __shfl_sync(0xffffffffu, sc_cur, g + 8);
           const float ta = __half2float(__ushort_as_half((unsigned short)ka)) * p.scale_log2;
           const float tb = __half2float(__ushort_as_half((unsigned short)kb)) * p.scale_log2;
-          s[0][0] = (s[0][0] - kbias0) * ta;
-          s[0][1] = (s[0][1] - kbias1) * ta;
-          s[0][2] = (s[0][2] - kbias0) * tb;
-          s[0][3] = (s[0][3] - kbias1) * tb;
+          s[0][0] = (s[0][0] + s[1][0] - kbias0) * ta;
+          s[0][1] = (s[0][1] + s[1][1] - kbias1) * ta;
+          s[0][2] = (s[0][2] + s[1][2] - kbias0) * tb;
+          s[0][3] = (s[0][3] + s[1][3] - kbias1) * tb;
         } else {
 #pragma unroll
           for (int j = 0; j < 2; ++j) {
@@ -702,7 +704,7 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap,
         }
       } else if constexpr (!INT8) {
 #pragma unroll
-        for (int j = 0; j < (HM ? 1 : 2); ++j) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
+        for (int j = 0; j < 2; ++j) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
         const int mi = lane >> 3;
         const int r = (lane & 7) + (mi >> 1) * 8;
 #pragma unroll
@@ -712,16 +714,21 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap,
           uint32_t kb[4];
           ldmatrix_x4(kb, addr);
           if constexpr (HM) {
-            mma_f<BF>(s[0], kb[0], kb[2], kb[1], kb[3], qa[kk][0], qa[kk][2]);
+            mma_f<BF>(s[kk & 1], kb[0], kb[2], kb[1], kb[3], qa[kk][0], qa[kk][2]);       // (two chains of half the length)
           } else {
             mma_f<BF>(s[0], qa[kk][0], qa[kk][1], qa[kk][2], qa[kk][3], kb[0], kb[1]);
             mma_f<BF>(s[1], qa[kk][0], qa[kk][1], qa[kk][2], qa[kk][3], kb[2], kb[3]);
           }
         }
+        if constexpr (HM) {
 #pragma unroll
-        for (int j = 0; j < (HM ? 1 : 2); ++j)
+          for (int e = 0; e < 4; ++e) s[0][e] = (s[0][e] + s[1][e]) * p.scale_log2;
+        } else {
 #pragma unroll
-          for (int e = 0; e < 4; ++e) s[j][e] *= p.scale_log2;
+          for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) s[j][e] *= p.scale_log2;
+        }
       } else {
         int si[2][4];
 #pragma unroll
@@ -788,11 +795,15 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap,
         for (int kk = 0; kk < D / 32; ++kk) {
           if constexpr (HM) {
             const uint32_t ka[4] = {bq[0][kk][0], bq[1][kk][0], bq[0][kk][1], bq[1][kk][1]};
-            mma_s8_16832(si[0], ka, qa[kk][0], qa[kk][2]);
+            mma_s8_16832(si[kk & 1], ka, qa[kk][0], qa[kk][2]);
           } else {
             mma_s8_16832(si[0], qa[kk], bq[0][kk][0], bq[0][kk][1]);
             mma_s8_16832(si[1], qa[kk], bq[1][kk][0], bq[1][kk][1]);
           }
+        }
+        if constexpr (HM) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) si[0][e] += si[1][e];
         }
         // score = float(dot) * q_s * k_s * scale, then to base 2
         if constexpr (HM) {
@@ -1059,8 +1070,8 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap,
       // The segment is shared with neighbouring CTAs.  Publish the partial, count the arrival;
       // whoever arrives last merges all partials of the segment.
       const long long seg_start = (long long)p.HV * pre[b] + (long long)hv * np;
-      const int first = p.parts > 0 ? (b * p.HV + hv) * p.parts : (int)(seg_start / per);
-      const int last = p.parts > 0 ? first + (np - 1) / part_pages_of(np) : (int)((seg_start + np - 1) / per);
+      const int first = PARTS ? (b * p.HV + hv) * p.parts : (int)(seg_start / per);
+      const int last = PARTS ? first + (np - 1) / part_pages_of(np) : (int)((seg_start + np - 1) / per);
       const unsigned int n_parts = (unsigned int)(last - first + 1);
       __threadfence();
       __syncthreads();
@@ -1090,7 +1101,7 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap,
           // merge the longest part of such launches.)
           constexpr int MB = 8;
           auto part_row = [&](int c) -> const float* {
-            const int slot = (p.parts > 0 || (long long)c * per >= seg_start) ? 0 : 1;
+            const int slot = (PARTS || (long long)c * per >= seg_start) ? 0 : 1;
             return p.partials + ((size_t)c * 2 + slot) * p.slot_rows * ROWLEN + row * ROWLEN;
           };
           float M = -INFINITY;
@@ -1133,10 +1144,10 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap,
 template <int D, int KIND, bool HM>
 cudaError_t launch_t(const CUtensorMap& kmap, const CUtensorMap& vmap, const DecodeParams& p,
                      int warps, size_t smem_bytes, cudaStream_t stream) {
-  auto kern = decode_splitkv_kernel<D, KIND, HM>;
+  auto kern = p.parts > 0 ? decode_splitkv_kernel<D, KIND, HM, true> : decode_splitkv_kernel<D, KIND, HM, false>;
   if (warps * 32 > DecodeOccupancy<D, KIND, HM>::kThreads) return cudaErrorInvalidConfiguration;
-  static SharedMemoryLimit limit;
-  cudaError_t e = limit.raise(reinterpret_cast<const void*>(kern), (int)smem_bytes);
+  static SharedMemoryLimit limits[2];
+  cudaError_t e = limits[p.parts > 0].raise(reinterpret_cast<const void*>(kern), (int)smem_bytes);
   if (e != cudaSuccess) return e;
   if (p.B + 1 > kMaxSmemPrefix) decode_plan_kernel<<<1, 1024, 0, stream>>>(p);  // else scanned in-kernel
   kern<<<p.n_cta, warps * 32, smem_bytes, stream>>>(kmap, vmap, p);
