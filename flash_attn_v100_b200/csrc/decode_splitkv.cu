@@ -118,8 +118,8 @@ __device__ __forceinline__ int seq_len_of(const DecodeParams& p, int b) {
 // and the heads in its 8 columns: S^T = K Q^T, O^T = V^T P^T.  The others have the heads in the rows.
 // (With the heads in the rows half of every MMA worked on rows of zeros, and the accumulators' empty halves had to be cleared before each
 // one.  32 sequences, 32 heads on 8 of 128: int8 cache of 8192 tokens 138.6 us so, 120.7 turned; scores in whole numbers over 4096 124.5 and 121.9.)
-// The scores' products are two chains of half the length: with one, 21 sequences of up to 559 tokens, 8 heads on 2 of 256, took 36.9 us against
-// 34.8 with the heads in the rows (which had two); with two, 35.0 against 37.4 on another day's clock.
+// The scores' products are two chains of half the length.  21 sequences of up to 559 tokens, 8 heads on 2 of 256: with the heads in the rows, which
+// has two chains by itself, 34.8 us against 36.9 turned with one chain; 37.4 against 35.0 (measured together) turned with two.
 template <bool BF>
 __device__ __forceinline__ void mma_f(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   const uint32_t a[4] = {a0, a1, a2, a3};
