@@ -138,8 +138,14 @@ fa::DecodeLaunchConfig pick_decode_config(int D, int G, int slot_rows, int B, in
                                           const DeviceInfo& di) {
   fa::DecodeLaunchConfig c;
   const bool half_m = G <= 8;  // kernels for at most 8 query heads per KV head: 128 threads, more CTAs per SM
-  if (kv_elem_bytes == 1) c = {4, 2, (half_m && D <= 128) ? 4 : (D == 256 ? 1 : 2)};  // dequantisation-bound: a fourth CTA hides its latency (120.7 -> 119.3 us)
-  else if (int8_qk && half_m && D == 128) c = {4, 2, 3};   // quantisation-bound: a third CTA hides its latency
+  // The int8 kinds are bound by instructions, so as many CTAs per SM as registers and shared memory allow, up to where the rings of more CTAs only
+  // cut the work finer.  20 sequences of 3000 tokens, 16 heads on 4 (one CTA per SM fewer, or the former choice, in brackets): int8 cache 64
+  // columns 23.6 us (four CTAs: 25.2), 256 columns 49.9 (56.1); scores in whole numbers, 64 columns 35.2 (40.0), 256 columns, where three warps of up to
+  // five heads leave shared memory for a second CTA, 112.5 (126.2).  At 128 columns, 32 x 8192 tokens: 119.3 (120.7).
+  if (kv_elem_bytes == 1 && half_m) c = {4, 2, D == 64 ? 3 : (D == 128 ? 4 : 2)};
+  else if (kv_elem_bytes == 1) c = {4, 2, D == 256 ? 1 : 2};
+  else if (int8_qk && half_m && D < 256) c = {4, 2, D == 64 ? 4 : 3};
+  else if (int8_qk && half_m && (fa::decode_smem_bytes(D, 3, 2, slot_rows, B, 2) + 1024) * 2 <= (size_t)di.max_smem_optin + 1024) c = {3, 2, 2};
   else if (D == 256) c = {4, 2, 1};
   else if (D == 128) c = {4, 2, 2};
   else c = {4, 4, 2};
