@@ -73,6 +73,11 @@ __device__ unsigned long long g_tc5_prof[5 * 16];
 #endif
 
 constexpr uint32_t kTc5MaxPolls = 1u << 21;
+// Batch barriers per query tile, used in turn.  A wait by parity tells a phase from its neighbours only, so a barrier must not complete two phases
+// before everyone who waits for the first has seen it.  Behind an item's last batch it could, were there one barrier: the next item's first QK needs nothing from
+// the softmax of its tile, so it may be complete before a softmax warp looks for the last batch (a cold instruction cache in the epilogue is enough), and
+// that warp would wait for a third phase, which needs its own P.  With two barriers the next phase of the same one needs P from every warp of the tile.
+constexpr int kBatchBars = 2;
 
 struct Tc5Params {
   __half* out;
@@ -323,9 +328,10 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_consta
   // barrier indices
   constexpr int B_QFULL = 0, B_QEMPTY = 2, B_KFULL = B_QEMPTY + 2, B_KEMPTY = B_KFULL + K_STAGES,
                 B_VFULL = B_KEMPTY + K_STAGES, B_VEMPTY = B_VFULL + V_STAGES, B_SFULL = B_VEMPTY + V_STAGES,
-                B_PFULL = B_SFULL + 2, B_TOKEN = B_PFULL + 2,
+                B_PFULL = B_SFULL + 2 * kBatchBars, B_TOKEN = B_PFULL + 2,
                 B_IFULL = B_TOKEN + 2, B_IEMPTY = B_IFULL + kItemQ, B_PAIR = B_IEMPTY + kItemQ,
                 B_DRAIN = B_PAIR + 8, B_TURN = B_DRAIN + 2, B_COUNT = B_TURN + 2;
+  static_assert(B_COUNT + kItemQ + 1 <= 64, "barriers, item slots and the tensor-memory slot share 64 words");
   volatile long long* item_slot = reinterpret_cast<volatile long long*>(bars + B_COUNT);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + B_COUNT + kItemQ);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -356,7 +362,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_consta
     for (int t = 0; t < 2; ++t) {
       mbar_init(bar(B_QFULL + t), 1);
       mbar_init(bar(B_QEMPTY + t), 1);
-      mbar_init(bar(B_SFULL + t), 1);
+      for (int i = 0; i < kBatchBars; ++i) mbar_init(bar(B_SFULL + t * kBatchBars + i), 1);
       mbar_init(bar(B_PFULL + t), 8);     // one arrival per softmax warp of the tile
       mbar_init(bar(B_TOKEN + t), 1);
       mbar_init(bar(B_DRAIN + t), 1);
@@ -497,6 +503,8 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_consta
         }
       };
       uint32_t kv_it = 0, q_cnt = 0, blk = 0, tok_waits = 0;
+      uint32_t batches = 0;                      // committed so far
+      auto commit_batch = [&]() { tc_commit(bar(B_SFULL + t * kBatchBars + (int)(batches++ % kBatchBars))); };
       for (uint32_t ic = 0;; ++ic) {
         if (*abort_flag) break;
         const int slot = ic % kItemQ;
@@ -528,7 +536,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_consta
             if (t == 1) take_token();
             issue_qk(st);
             pass_token();
-            tc_commit(bar(B_SFULL + t));
+            commit_batch();
           }
           for (int j = 0; j < n_mine; ++j, ++blk) {
             const uint32_t g = kv_it + (uint32_t)j;
@@ -553,7 +561,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_consta
             // ONE commit per batch (a tcgen05.commit costs the tensor pipe about as much as an MMA): the
             // batch barrier tells the softmax group that S(j+1) is complete and O holds PV(j); that group
             // passes the news on to the copy lane (K / V stages and the Q buffer that have become free)
-            tc_commit(bar(B_SFULL + t));
+            commit_batch();
             PROF_STAMP(t);
             PROF_MARK(prof_t_c);
             PROF_SPAN(1 + t, 11, prof_t_i, prof_t_c);   // issue of PV_hi + QK + commit
@@ -577,9 +585,12 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_consta
         for (int j = n_mine; j < it.n_max; ++j) {
           const uint32_t g = kv_it + (uint32_t)j;
           const int st = g % K_STAGES, sv = g % V_STAGES;
+          // (every lane has seen it: a lane left behind could miss two phases and wait for good)
           PROF_WAIT(1 + t, 8, wait_or_abort(bar(B_KFULL + st), (g / K_STAGES) & 1u, abort_flag));
+          __syncwarp();
           if (lane == 0) mbar_arrive(bar(B_KEMPTY + st));
           PROF_WAIT(1 + t, 8, wait_or_abort(bar(B_VFULL + sv), (g / V_STAGES) & 1u, abort_flag));
+          __syncwarp();
           if (lane == 0) mbar_arrive(bar(B_VEMPTY + sv));
         }
         kv_it += (uint32_t)it.n_max;
@@ -683,7 +694,11 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_consta
       if (lane == 0) mbar_arrive(bar(B_TURN + (t ^ 1)));
     };
     const float2 sc2 = make_float2(p.scale_log2, p.scale_log2);
-    uint32_t sph = 0;        // completed phases of B_SFULL[t] that this thread has consumed
+    uint32_t sph = 0;        // batches of this tile that this thread has seen complete
+    auto wait_batch = [&]() {
+      wait_or_abort(bar(B_SFULL + t * kBatchBars + (int)(sph % kBatchBars)), (sph / kBatchBars) & 1u, abort_flag);
+      ++sph;
+    };
     uint32_t pph = 0;        // KV steps of this tile so far: tags of the redo vote, slots of the exchange
     uint32_t kv_it = 0;      // KV tiles of all items so far: ring stage of K / V
     // What a completed MMA batch implies is passed on to the copy lane by this role, as soon as the batch
@@ -732,8 +747,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_consta
       };
       for (int j = 0; j < n_mine; ++j, ++pph) {
         PROF_COUNT(3 + t, 14);
-        PROF_WAIT(3 + t, 1, wait_or_abort(bar(B_SFULL + t), sph & 1u, abort_flag));
-        ++sph;
+        PROF_WAIT(3 + t, 1, wait_batch());
         if (j > 0) PROF_SINCE(3 + t, 8, t);   // commit issued by the MMA lane -> batch seen complete here
         PROF_MARK(prof_t_s);
         tc_fence_after();
@@ -888,8 +902,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_consta
       // ---- epilogue: O / l -> fp16 -> global, my half of the columns.  The batch barrier of the last step
       // covers PV(n-1).  The next item's first PV of this tile cannot be issued before these threads have
       // produced its P, i.e. after these loads have completed.
-      PROF_WAIT(3 + t, 3, wait_or_abort(bar(B_SFULL + t), sph & 1u, abort_flag));
-      ++sph;
+      PROF_WAIT(3 + t, 3, wait_batch());
       PROF_MARK(prof_t_o);
       tc_fence_after();
       if (fwd == 1) mbar_arrive(bar(B_VEMPTY + (int)((kv0 + (uint32_t)n_mine - 1u) % V_STAGES)));
