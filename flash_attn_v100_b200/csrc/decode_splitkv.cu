@@ -343,6 +343,12 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap,
       for (int e = threadIdx.x; e < p.H_Q * p.D_real; e += blockDim.x) o[e] = __float2half_rn(0.f);
     }
   }
+  // A piece: the pages [p0, p0 + cnt) of one (sequence, KV-head block) unit, the part of this CTA's range
+  // [u, u1) that lies in that unit.
+  struct Piece {
+    int b, np, hv, p0, cnt;
+  };
+  Piece only;                              // PARTS: the one piece of this CTA
   const long long T = (long long)p.HV * pre[p.B];
   long long per = (T + p.n_cta - 1) / p.n_cta;
   if (per < 1) per = 1;
@@ -354,14 +360,15 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap,
   };
   if constexpr (PARTS) {
     // a segment is cut into parts of equal length (at least what the rings hold), one per CTA: see decode_parts
-    const int seg = (int)blockIdx.x / p.parts;
+    const int seg = p.parts == 1 ? (int)blockIdx.x : (int)blockIdx.x / p.parts;
     if (seg >= p.B * p.HV) return;
     const int bb = seg / p.HV, np = pre[bb + 1] - pre[bb];
-    const int part_pages = part_pages_of(np);
+    const int part_pages = p.parts == 1 ? np : part_pages_of(np);
     const int lo = ((int)blockIdx.x - seg * p.parts) * part_pages;
     if (lo >= np) return;
-    u = (long long)p.HV * pre[bb] + (long long)(seg - bb * p.HV) * np + lo;
-    u1 = u + (part_pages < np - lo ? part_pages : np - lo);
+    only = {bb, np, seg - bb * p.HV, lo, part_pages < np - lo ? part_pages : np - lo};
+    u = 0;
+    u1 = only.cnt;
   }
   if (u >= u1) return;
 
@@ -372,8 +379,8 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap,
   uint32_t st_issue = 0, st_cons = 0, par_cons = 0;
 
   // locate the sequence that holds unit u: largest b with HV * pre[b] <= u
-  int b;
-  {
+  int b = 0;
+  if constexpr (!PARTS) {
     int lo = 0, hi = p.B;  // invariant: HV*pre[lo] <= u < HV*pre[hi]
     while (hi - lo > 1) {
       int mid = (lo + hi) >> 1;
@@ -382,11 +389,6 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap,
     b = lo;
   }
 
-  // A piece: the pages [p0, p0 + cnt) of one (sequence, KV-head block) unit, the part of this CTA's range
-  // [u, u1) that lies in that unit.
-  struct Piece {
-    int b, np, hv, p0, cnt;
-  };
   auto locate = [&](long long uu, int bb) -> Piece {
     Piece q;
     while ((long long)p.HV * pre[bb + 1] <= uu) ++bb;  // also skips empty sequences
@@ -432,7 +434,7 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap,
 
   int piece = 0;
   while (u < u1) {
-    const Piece pc = locate(u, b);
+    const Piece pc = PARTS ? only : locate(u, b);
     b = pc.b;
     const int np = pc.np, hv = pc.hv, p0 = pc.p0, cnt = pc.cnt;
     const bool complete = (p0 == 0) && (cnt == np);
@@ -554,7 +556,7 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap,
 
     // The piece after this one (if this CTA has one): where it lies, this warp's share of it and the
     // block-table entries of its first pages, fetched now so that they are at hand when the ring has room.
-    const bool has_next = u + cnt < u1;
+    const bool has_next = !PARTS && u + cnt < u1;
     Piece nx = pc;
     int nx_n_my = 0, nx_tbl = 0, nx_h_kv = 0;
     long long nx_row0 = 0;
@@ -1092,45 +1094,66 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap,
       if (s_last_flag) {
         __threadfence();
         __half* outp = p.out + ((size_t)b * p.H_Q + head0) * p.D_real;
-        for (int e = threadIdx.x; e < Gb * D; e += blockDim.x) {
-          const int row = e / D, d = e - row * D;
-          if (d >= p.D_real) continue;
-          // The partials sit in L2 (other CTAs wrote them): every read costs an L2 round trip, so the reads
-          // of eight partials are issued together before any of them is used.  (A segment is split over
-          // up to hundreds of CTAs when few sequences fill the grid; one dependent read per partial made the
-          // merge the longest part of such launches.)
-          constexpr int MB = 8;
+        // The partials sit in L2 (other CTAs wrote them), and every read that waits for another one costs a round trip there: a segment is split
+        // over up to hundreds of CTAs when few sequences fill the grid.  A warp takes a row (or 128 of its columns); its lanes fetch the maxima and
+        // sums of 32 parts at a time and hand the weights round, and the values of eight parts are under way together.  (With a
+        // thread per element, which walks through all parts once per row: 8 sequences of up to 8000 tokens, 16 heads on 2 of 128, 76 us against 26 so; one
+        // of 8000, 5 heads on 1, 46 and 20; int8 cache of 256 columns, 2 of 8000, 16 heads on 2, 130 and 38.)  The sums run over the parts in
+        // order, so the split of the work does not show in the bits.
+        constexpr int MB = 8, COLS = D < 128 ? 64 : 128, NV = COLS / 64;
+        const int first_slot = (PARTS || (long long)first * per >= seg_start) ? 0 : 1;
+        for (int unit = warp; unit < Gb * (D / COLS); unit += W) {
+          const int row = unit / (D / COLS), col = (unit - row * (D / COLS)) * COLS + lane * 2;
           auto part_row = [&](int c) -> const float* {
-            const int slot = (PARTS || (long long)c * per >= seg_start) ? 0 : 1;
-            return p.partials + ((size_t)c * 2 + slot) * p.slot_rows * ROWLEN + row * ROWLEN;
+            const int slot = c == first ? first_slot : 0;
+            return p.partials + (((size_t)c * 2 + slot) * p.slot_rows + row) * ROWLEN;
           };
-          float M = -INFINITY;
-          for (int c0 = first; c0 <= last; c0 += MB) {
-            float mv[MB];
+          // maximum and sum of part c + lane; values of the parts c to c + MB - 1
+          auto stats = [&](int c) -> float2 {
+            return c + lane <= last ? __ldcg(reinterpret_cast<const float2*>(part_row(c + lane) + D)) : make_float2(-INFINITY, 0.f);
+          };
+          float2 v[MB][NV];
+          auto fetch = [&](int c) {
 #pragma unroll
-            for (int k = 0; k < MB; ++k) mv[k] = (c0 + k <= last) ? __ldcg(part_row(c0 + k) + D) : -INFINITY;
+            for (int k = 0; k < MB; ++k)
 #pragma unroll
-            for (int k = 0; k < MB; ++k) M = fmaxf(M, mv[k]);
-          }
-          float L = 0.f, O = 0.f;
-          for (int c0 = first; c0 <= last; c0 += MB) {
-            float mv[MB], lv[MB], ov[MB];
+              for (int i = 0; i < NV; ++i)
+                v[k][i] = (c + k <= last && col + i * 64 < p.D_real) ? __ldcg(reinterpret_cast<const float2*>(part_row(c + k) + col + i * 64))
+                                                                     : make_float2(0.f, 0.f);
+          };
+          float2 ml = stats(first);
+          fetch(first);
+          float M = ml.x;
+          for (int c = first + 32; c <= last; c += 32) M = fmaxf(M, stats(c).x);
 #pragma unroll
-            for (int k = 0; k < MB; ++k) {
-              const bool in = c0 + k <= last;
-              const float* pr = part_row(in ? c0 + k : last);
-              mv[k] = in ? __ldcg(pr + D) : -INFINITY;
-              lv[k] = in ? __ldcg(pr + D + 1) : 0.f;
-              ov[k] = in ? __ldcg(pr + d) : 0.f;
+          for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+          float f = 0.f, L = 0.f;
+          float2 O[NV];
+#pragma unroll
+          for (int i = 0; i < NV; ++i) O[i] = make_float2(0.f, 0.f);
+          for (int c = first; c <= last; c += MB) {
+            const int at = (c - first) & 31;
+            if (at == 0) {
+              if (c > first) ml = stats(c);
+              f = ml.x == -INFINITY ? 0.f : fast_exp2(ml.x - M);
             }
 #pragma unroll
             for (int k = 0; k < MB; ++k) {
-              const float f = (mv[k] == -INFINITY) ? 0.f : fast_exp2(mv[k] - M);
-              L += lv[k] * f;
-              O += ov[k] * f;
+              const float fk = __shfl_sync(0xffffffffu, f, at + k);
+              L += __shfl_sync(0xffffffffu, ml.y, at + k) * fk;
+#pragma unroll
+              for (int i = 0; i < NV; ++i) {
+                O[i].x += v[k][i].x * fk;
+                O[i].y += v[k][i].y * fk;
+              }
             }
+            if (c + MB <= last) fetch(c + MB);
           }
-          outp[(size_t)row * p.D_real + d] = to_out16(O / L, p.out_bf16 != 0);
+#pragma unroll
+          for (int i = 0; i < NV; ++i)
+            if (col + i * 64 < p.D_real)
+              *reinterpret_cast<__half2*>(outp + (size_t)row * p.D_real + col + i * 64) =
+                  __halves2half2(to_out16(O[i].x / L, p.out_bf16 != 0), to_out16(O[i].y / L, p.out_bf16 != 0));
         }
       }
     }
