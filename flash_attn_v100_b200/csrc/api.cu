@@ -680,7 +680,10 @@ int fa_prefill_varlen_clear(void* out, const int32_t* cu_seqlens, int batch, int
   FA_REQUIRE(out != nullptr && cu_seqlens != nullptr, "null pointer");
   FA_REQUIRE(batch > 0 && total > 0 && max_seqlen > 0 && row_bytes > 0, "batch, total, max_seqlen and row_bytes must be positive");
   FA_REQUIRE(row_bytes % 16 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0, "out and its rows must be 16-byte aligned");
-  FA_CUDA(fa::launch_varlen_clear(out, cu_seqlens, batch, total, max_seqlen, row_bytes, static_cast<cudaStream_t>(stream)));
+  DeviceInfo di;
+  int rc = device_info(&di);
+  if (rc != FA_OK) return rc;
+  FA_CUDA(fa::launch_varlen_clear(out, cu_seqlens, batch, total, max_seqlen, row_bytes, di.sm_count, static_cast<cudaStream_t>(stream)));
   return FA_OK;
 }
 

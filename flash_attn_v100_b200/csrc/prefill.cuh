@@ -39,7 +39,7 @@ bool prefill_wide_supported(const PrefillParams& p);
 cudaError_t launch_prefill_wide(const PrefillParams& p, int sm_count, void* encode_fn, cudaStream_t stream);
 // Zeros in the rows of a packed [total, row_bytes] output that no sequence covers.
 cudaError_t launch_varlen_clear(void* out, const int32_t* cu_seqlens, int batch, long long total, int max_seqlen, long long row_bytes,
-                                cudaStream_t stream);
+                                int sm_count, cudaStream_t stream);
 cudaError_t prefill_status(int* host_out, cudaStream_t stream);
 cudaError_t prefill_status_ptr(int** out);  // device address of the status word (current device)
 cudaError_t prefill_status_clear(cudaStream_t stream);

@@ -25,16 +25,52 @@ def test_uncovered_rows_are_zero(D, dtype, cu, behind, longest):
         del got
 
 
-@pytest.mark.parametrize("rows,row_bytes", [(1, 16), (1000, 8192), (40000, 8192)])
-def test_clear_touches_nothing_else(rows, row_bytes):
+def _clear(out, cu, longest):
     from flash_attn_v100_b200 import _lib
     lib = _lib.load()
-    out = torch.ones(rows, row_bytes, dtype=torch.uint8, device="cuda")
+    _lib.check(lib.fa_prefill_varlen_clear(out.data_ptr(), cu.data_ptr(), cu.numel() - 1, out.size(0), longest, out.size(1), torch.cuda.current_stream().cuda_stream))
+
+
+# (2000003 rows of 16 bytes: a block's share is more than it marks at a time)
+@pytest.mark.parametrize("rows,row_bytes", [(1, 16), (1000, 8192), (40000, 8192), (2000003, 16), (33, 512), (5000, 528)])
+@pytest.mark.parametrize("offsets", ["few", "many", "out of order"])
+def test_clear_touches_nothing_else(rows, row_bytes, offsets):
     cu = [rows // 10, rows // 3, rows // 3, rows // 2]
-    longest = max(1, rows // 8)
-    _lib.check(lib.fa_prefill_varlen_clear(out.data_ptr(), torch.tensor(cu, dtype=torch.int32, device="cuda").data_ptr(), 3, rows, longest, row_bytes,
-                                           torch.cuda.current_stream().cuda_stream))
-    want = torch.zeros(rows, dtype=torch.uint8)
+    if offsets == "many":
+        cu = sorted((torch.rand(700, generator=torch.Generator().manual_seed(rows)) * rows).int().tolist())
+    elif offsets == "out of order":
+        cu = [rows // 3, rows // 10, rows // 2, rows // 4]
+    longest = max(1, rows // 8 if offsets != "many" else rows // 700)
+    memory = torch.ones(rows + 2, row_bytes, dtype=torch.uint8, device="cuda")       # a row on either side that must stay
+    out = memory[1:-1]
+    _clear(out, torch.tensor(cu, dtype=torch.int32, device="cuda"), longest)
+    gap, covered = torch.zeros(rows, dtype=torch.bool), torch.zeros(rows, dtype=torch.bool)
+    gap[:cu[0]] = gap[cu[-1]:] = True
     for a, e in zip(cu, cu[1:]):
-        want[a:min(e, a + longest)] = 1
-    assert torch.equal(out.cpu(), want[:, None].expand(rows, row_bytes))
+        covered[a:min(e, a + longest)] = True
+        gap[a + longest:e] = True
+    assert bool((gap | covered).all())                       # what no sequence covers lies in a gap
+    rows_of = memory.cpu().view(rows + 2, row_bytes)
+    assert bool(rows_of[0].all()) and bool(rows_of[-1].all())
+    assert torch.equal(rows_of[1:-1], (~gap).to(torch.uint8)[:, None].expand(rows, row_bytes))
+
+
+@pytest.mark.parametrize("batch", [1, 64, 300, 2000])
+def test_long_gap_at_the_rate_of_a_fill(batch):
+    """A buffer padded to a fixed size: the gap behind the sequences is nearly all of it.  A fill is the time it took before there was
+    a clear; the line is four of them, and the clear by few blocks took up to 60."""
+    rows, row_bytes = 65536, 8192
+    out = torch.ones(rows, row_bytes, dtype=torch.uint8, device="cuda")
+    cu = torch.arange(batch + 1, dtype=torch.int32, device="cuda")
+
+    def fastest(fn):
+        times = []
+        for _ in range(8):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            fn()
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b))
+        return min(times)
+    assert fastest(lambda: _clear(out, cu, 1)) < 4 * fastest(out.zero_)
