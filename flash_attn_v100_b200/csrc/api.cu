@@ -135,17 +135,20 @@ int make_rows_map_u8(CUtensorMap* map, const void* base, long long rows, int D) 
 fa::DecodeLaunchConfig g_cfg_override = {0, 0, 0};
 
 fa::DecodeLaunchConfig pick_decode_config(int D, int G, int slot_rows, int B, int kv_elem_bytes, bool int8_qk,
-                                          const DeviceInfo& di) {
+                                          long long segments, long long units, const DeviceInfo& di) {
   fa::DecodeLaunchConfig c;
   const bool half_m = G <= 8;  // kernels for at most 8 query heads per KV head: 128 threads, more CTAs per SM
   // The int8 kinds are bound by instructions, so as many CTAs per SM as registers and shared memory allow, up to where the rings of more CTAs only
-  // cut the work finer.  20 sequences of 3000 tokens, 16 heads on 4 (one CTA per SM fewer, or the former choice, in brackets): int8 cache 64
-  // columns 23.6 us (four CTAs: 25.2), 256 columns 49.9 (56.1); scores in whole numbers, 64 columns 35.2 (40.0), 256 columns, where three warps of up to
-  // five heads leave shared memory for a second CTA, 112.5 (126.2).  At 128 columns, 32 x 8192 tokens: 119.3 (120.7).
+  // cut the work finer.  Over 235 shapes each (1 to 32 sequences of 16 to 8000 tokens; 32 heads on 8, 4 on 4, 16 on 4, 16 on 2, 5 on 1), times of the choice
+  // against one CTA per SM fewer: int8 cache 128 columns 0.98 (0.90 to 1.03 by length), 256 columns 0.94 (0.84 to 1.01); scores in whole
+  // numbers, 64 columns 0.97 (0.89 to 1.03).  At 256 columns, scores in whole numbers, two CTAs fit only with three warps each (and up to five or six heads), whose
+  // longer chain per warp pays from about 20 pages per SM on, or where there are more segments than SMs: 0.44 to 0.98 times, but for 8 segments of 500
+  // pages (1.0 to 1.1); below that 1.0 to 1.3 times (16 heads on 4, 16 sequences of 3000 tokens: 91.3 us, and 103.6 with four warps; 4 of 100: 27.2, and 22.6).
   if (kv_elem_bytes == 1 && half_m) c = {4, 2, D == 64 ? 3 : (D == 128 ? 4 : 2)};
   else if (kv_elem_bytes == 1) c = {4, 2, D == 256 ? 1 : 2};
   else if (int8_qk && half_m && D < 256) c = {4, 2, D == 64 ? 4 : 3};
-  else if (int8_qk && half_m && (fa::decode_smem_bytes(D, 3, 2, slot_rows, B, 2) + 1024) * 2 <= (size_t)di.max_smem_optin + 1024) c = {3, 2, 2};
+  else if (int8_qk && half_m && (segments > di.sm_count || units >= 20ll * di.sm_count) &&
+           (fa::decode_smem_bytes(D, 3, 2, slot_rows, B, 2) + 1024) * 2 <= (size_t)di.max_smem_optin + 1024) c = {3, 2, 2};
   else if (D == 256) c = {4, 2, 1};
   else if (D == 128) c = {4, 2, 2};
   else c = {4, 4, 2};
@@ -209,7 +212,7 @@ int run_decode(const DecodeCall& c) {
   if (c.rows_total >= (1ll << 31)) return fail(FA_ERR_UNSUPPORTED, "KV cache has too many rows for one tensor map");
 
   const int kv_elem_bytes = c.kv8 ? 1 : 2;
-  fa::DecodeLaunchConfig cfg = pick_decode_config(Dp, G, slot_rows, c.B, kv_elem_bytes, c.int8, di);
+  fa::DecodeLaunchConfig cfg = pick_decode_config(Dp, G, slot_rows, c.B, kv_elem_bytes, c.int8, (long long)c.B * c.H_KV * ((G + 15) / 16), c.max_units, di);
   fa::DecodeParams p;
   memset(&p, 0, sizeof(p));
   p.q = static_cast<const __half*>(c.q);

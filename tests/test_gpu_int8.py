@@ -17,6 +17,10 @@ def _scales(q, k):
 @pytest.mark.parametrize("B,H_Q,H_KV,N,D,cache_len", [
     (2, 8, 2, 70, 64, 69), (1, 32, 8, 257, 128, 256), (2, 16, 16, 33, 128, 20), (1, 8, 1, 129, 256, 128),
     (3, 32, 8, 1000, 128, 999), (1, 40, 2, 50, 64, 49),
+    # 256 columns, where the warps and CTAs per SM depend on the heads of a group, and the column counts padded to them; lengths at the edge of what
+    # the rings hold (six and eight pages), cut into parts, and cut evenly
+    (2, 2, 2, 95, 256, 94), (2, 4, 1, 96, 256, 95), (1, 5, 1, 97, 256, 96), (2, 6, 1, 97, 256, 96), (3, 10, 2, 130, 192, 127), (2, 5, 1, 700, 256, 699),
+    (2, 12, 2, 700, 192, 650), (1, 4, 1, 9000, 256, 8999), (40, 20, 4, 300, 256, 299), (40, 6, 1, 129, 136, 128),
 ])
 def test_int8_scores_bit_exact_and_output_close(B, H_Q, H_KV, N, D, cache_len):
     import flash_attn_v100 as fa
