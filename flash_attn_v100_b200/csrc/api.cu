@@ -789,7 +789,10 @@ static int qkv_rope_append_impl(const void* qkv, const void* q_weight, const voi
   p.r.bt_stride = block_table_stride; p.r.num_pages = num_pages;
   p.r.bf16 = bf16 ? 1 : 0;
   FA_CUDA(fa::prefill_status_ptr(&p.r.status));
-  cudaError_t e = fa::launch_qkv_rope_append(p, static_cast<cudaStream_t>(stream));
+  DeviceInfo di;
+  int rc = device_info(&di);
+  if (rc != FA_OK) return rc;
+  cudaError_t e = fa::launch_qkv_rope_append(p, di.sm_count, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return fail(FA_ERR_CUDA, "qkv norm/rope/append launch failed: %s", cudaGetErrorString(e));
   return FA_OK;
 }

@@ -315,15 +315,15 @@ __global__ void __launch_bounds__(256) qkv_rope_append_kernel(const QkvRopeAppen
 bool aligned_to(const void* p, size_t bytes) { return (reinterpret_cast<uintptr_t>(p) & (bytes - 1)) == 0; }
 
 template <int PER, typename T>
-cudaError_t launch_qkv_t(const QkvRopeAppendParams& p, cudaStream_t stream) {
+cudaError_t launch_qkv_t(const QkvRopeAppendParams& p, int sm_count, cudaStream_t stream) {
   const int heads = p.r.H_Q + 2 * p.r.H_KV;
   bool vec = true;
   for (const void* q : {p.qkv, p.q_weight, p.k_weight, (const void*)p.r.q_out, (const void*)p.r.k_out, (const void*)p.v_out,
                         (const void*)p.r.k_cache, (const void*)p.r.v_cache})
     vec = vec && aligned_to(q, PER * 2);
-  // A few tokens (a decode step) take one head per warp: more warps, each with one chain of loads; from about four warps per scheduler
-  // on (148 SMs x 4 x 4), sharing a token's tables and place among four heads is worth more.
-  const bool many = (long long)p.r.T * heads > 4 * 2368;
+  // A few tokens (a decode step) take one head per warp: more warps, each with one chain of loads; from four warps per scheduler on
+  // with four heads each (16 warps per SM), sharing a token's tables and place among them is worth more.
+  const bool many = (long long)p.r.T * heads > 4 * 16ll * sm_count;
   const int hpw = many ? 4 : 1;
   const long long warps = (long long)p.r.T * ((heads + hpw - 1) / hpw);
   const unsigned blocks = (unsigned)((warps * 32 + 255) / 256);
@@ -339,12 +339,12 @@ cudaError_t launch_qkv_t(const QkvRopeAppendParams& p, cudaStream_t stream) {
 
 }  // namespace
 
-cudaError_t launch_qkv_rope_append(const QkvRopeAppendParams& p, cudaStream_t stream) {
+cudaError_t launch_qkv_rope_append(const QkvRopeAppendParams& p, int sm_count, cudaStream_t stream) {
   if (p.r.T == 0) return cudaSuccess;
   switch (p.r.D) {
-    case 64: return p.r.bf16 ? launch_qkv_t<2, __nv_bfloat16>(p, stream) : launch_qkv_t<2, __half>(p, stream);
-    case 128: return p.r.bf16 ? launch_qkv_t<4, __nv_bfloat16>(p, stream) : launch_qkv_t<4, __half>(p, stream);
-    case 256: return p.r.bf16 ? launch_qkv_t<8, __nv_bfloat16>(p, stream) : launch_qkv_t<8, __half>(p, stream);
+    case 64: return p.r.bf16 ? launch_qkv_t<2, __nv_bfloat16>(p, sm_count, stream) : launch_qkv_t<2, __half>(p, sm_count, stream);
+    case 128: return p.r.bf16 ? launch_qkv_t<4, __nv_bfloat16>(p, sm_count, stream) : launch_qkv_t<4, __half>(p, sm_count, stream);
+    case 256: return p.r.bf16 ? launch_qkv_t<8, __nv_bfloat16>(p, sm_count, stream) : launch_qkv_t<8, __half>(p, sm_count, stream);
     default: return cudaErrorInvalidValue;
   }
 }

@@ -37,6 +37,6 @@ struct QkvRopeAppendParams {
   __half* v_out;              // optional [T, H_KV, D] fp16 copy of v (prefill attention reads it)
   RopeAppendParams r;         // cos, sin, q_out, k_out, caches, tables, sizes (q / k / v unused; rot_dim == D)
 };
-cudaError_t launch_qkv_rope_append(const QkvRopeAppendParams& p, cudaStream_t stream);
+cudaError_t launch_qkv_rope_append(const QkvRopeAppendParams& p, int sm_count, cudaStream_t stream);
 
 }  // namespace fa
