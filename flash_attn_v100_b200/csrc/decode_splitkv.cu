@@ -254,8 +254,8 @@ __global__ void __launch_bounds__(1024) decode_plan_kernel(const DecodeParams p)
 #ifndef FA_I8QK_MINB
 #define FA_I8QK_MINB 3
 #endif
-// Threads per CTA and CTAs per SM the kernel is compiled for.  The half-M variants keep half the
-// accumulators, which leaves room for more resident CTAs (more pages in flight, more warps to hide
+// Threads per CTA and CTAs per SM the kernel is compiled for.  The turned variants (HM) hold
+// 8 heads, half the accumulators of 16, which leaves room for more resident CTAs (more pages in flight, more warps to hide
 // the dequantisation latency); they run with at most 4 warps.
 template <int D, int KIND, bool HM>
 struct DecodeOccupancy {
@@ -447,7 +447,7 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap,
     // ---- this warp's share of the piece: pages p0 + warp + n*W -------------------
     const int n_my = cnt > warp ? (cnt - warp + W - 1) / W : 0;
 
-    // Q fragments (A operand).  Rows >= Gb are zero.
+    // Q fragments: the A operand, 16 heads in its rows, or (HM, registers 0 and 2) the B operand, 8 heads in its columns.  Heads >= Gb are zero.
     constexpr int QREGS = INT8 ? (D / 32) : (D / 16);
     // KV8: the contraction index of k-step t, fragment slot pair (2c,2c+1 | 2c+8,2c+9) of lane c = lane & 3
     // stands for head dimensions d0 .. d0+3 with d0 = 128 * (t / KPS) + 4 * KPS * c + 4 * (t % KPS):
@@ -653,7 +653,7 @@ decode_splitkv_kernel(const __grid_constant__ CUtensorMap kmap,
       const uint32_t sc_cur = ps.sc;
       const uint32_t kbase = stage0 + st * (2 * PAGE_BYTES);
       (void)vmask; (void)page; (void)ks_cur; (void)sc_cur; (void)kbase;
-      // ---- S = Q K^T : [16 heads x 16 tokens] ------------------------------------
+      // ---- S = Q K^T : [16 heads x 16 tokens], or (HM) S^T = K Q^T : [16 tokens x 8 heads], all of it in s[0] ------------------
       if constexpr (KV8) {
 #pragma unroll
         for (int j = 0; j < 2; ++j) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
