@@ -3,15 +3,20 @@
 // Replaces the reference's prefill kernels (flash_attn_kernel.cu:1138-1299, 2471-2605, 3005-3148) for those head dimensions, dense
 // [B,H,N,D] and packed varlen [total,H,D], fp16 operands.
 //
-// What bounds it: the tensor cores.  A step of 128 rows x 128 keys is 1024 cycles of QK and 1024 of PV at D = 256 against 1024
-// cycles of exponentials, so one 128-row query tile per CTA keeps the tensor pipe busy if the softmax of one step runs under the MMAs of
-// its neighbours; and one tile is what tensor memory holds (an output of 256 columns and two score buffers of 128 fill its 512).
-// The issue order is QK(j+1), PV(j), QK(j+2), ...: from the end of QK(j) to the start of PV(j) the softmax has the length of PV(j-1) and
-// QK(j+1), 2048 cycles.  P is handed over in two halves of 64 keys, so that PV(j) starts while the second half is exponentiated.
+// What bounds it: the softmax of a step, then the tensor cores.  A step of 128 rows x 128 keys is 1024 cycles of QK and 2048 of PV at D = 256 (the
+// weights and their rests, below) against 1024 cycles of exponentials, so one 128-row query tile per CTA keeps the tensor pipe busy if the softmax
+// of one step runs under the MMAs of its neighbours; and one tile is what tensor memory holds (an output of 256 columns and two score buffers of 128 fill
+// its 512).  The issue order is QK(j+1), PV(j), QK(j+2), ...: from the end of QK(j) to the start of PV(j) the softmax has the length of PV(j-1) and
+// QK(j+1).  P is handed over in two halves of 64 keys, so that PV(j) starts while the second half is exponentiated.
 //
-// Measured: 2 x 2048 tokens, 16 heads on 8 of 256, causal: 105 us (654 TFLOP/s) against 403 us (171) of the mma.sync kernel
-// (prefill_mma.cu); 8192 tokens, not causal: 1180 TFLOP/s, 0.87 of the sustained cuBLAS rate.  The smallest launch takes 12 us.  Releasing
-// every unit with a commit of its own, 512 cycles earlier, changed nothing.
+// Weights in two fp16 terms.  A row's reference exponent lags behind its maximum (see the softmax), so the largest weight is not exactly 1, as it is
+// under an exact running maximum, and rounding the weights to fp16 alone costs 2 to 4 % of the error against 64 bits, 20 % with peaked scores, above the mma.sync
+// kernel's.  What the rounding leaves is a second operand beside the first: 0.73 to 0.94 of the mma.sync kernel's error, for 128 to 8192 tokens,
+// 136 to 256 columns, flat and peaked scores.  The other way, an exact maximum with O scaled in tensor memory before every PV, is as slow: PV, scale, PV is a
+// serial chain (1 x 4096 tokens, 16 heads on 8, not causal: 375 us; two terms 374; one term 252).
+//
+// Measured: 16 x 2048 tokens, 2 heads of 256, causal: 134 us against 401 of the mma.sync kernel (prefill_mma.cu); 1 x 2048, 16 heads on 8: 79 and 229; 4
+// x 1024, 8 on 1: 51 and 127.  The smallest launch takes 12 us.  Releasing every unit with a commit of its own, earlier, changed nothing.
 //
 // Warps: 0 copies (TMA), 1 issues the MMAs, 2 owns tensor memory and claims work, 4-7 and 8-11 softmax of the even and of the odd steps (a
 // thread per row, its 128 scores in registers), 12-15 write the output of a finished tile while the softmax is on the next one.  (With one
@@ -91,6 +96,23 @@ __device__ __forceinline__ bool wide_item(const WideParams& p, long long item, W
   return true;
 }
 
+// One 32-column chunk of a score row: P = exp2(s * scale - m) in two fp16 terms, the weight and what its rounding left, written to tensor memory
+// at `taddr` and 32 columns on (16 columns each); the fp32 sum of the chunk is added to `rs`.
+__device__ __forceinline__ void exp_chunk_two(const float (&s)[32], float2 sc2, float2 nm2, float2& rs, uint32_t taddr) {
+  uint32_t hi[16], lo[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const float2 x = ffma2(make_float2(s[2 * i], s[2 * i + 1]), sc2, nm2);
+    const float2 e = make_float2(fast_exp2(x.x), fast_exp2(x.y));
+    rs = fadd2(rs, e);
+    hi[i] = pack_half2(e.x, e.y);
+    const float2 h = __half22float2(*reinterpret_cast<const __half2*>(&hi[i]));
+    lo[i] = pack_half2(e.x - h.x, e.y - h.y);
+  }
+  tc_st16(taddr, hi);
+  tc_st16(taddr + 32, lo);
+}
+
 __global__ void __launch_bounds__(kWideThreads, 1)
 prefill_wide_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap kmap,
                     const __grid_constant__ CUtensorMap vmap, const WideParams p) {
@@ -142,7 +164,7 @@ prefill_wide_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;                // S_0 [0,128) S_1 [128,256) O [256,512); P (64 columns) over the start of its S
+  const uint32_t tmem = *tmem_slot;                // S_0 [0,128) S_1 [128,256) O [256,512); P over its S: per 64 keys 32 columns and 32 of their rests
   auto next_item = [&](uint32_t ic) -> long long {
     const int slot = ic % kWideItemQ;
     wait_or_abort(bar(kIFull + slot), (ic / kWideItemQ) & 1u, abort_flag);
@@ -266,10 +288,10 @@ prefill_wide_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
           wait_or_abort(bar((half ? kPHi : kPLo) + (int)(cnt & 1u)), (cnt >> 1) & 1u, abort_flag);
           tc_fence_after();
           __syncwarp();
-          const uint32_t a = tmem + (cnt & 1u) * 128u + (uint32_t)half * 32u;
+          const uint32_t a = tmem + (cnt & 1u) * 128u + (uint32_t)half * 64u;
 #pragma unroll
-          for (int ks = 0; ks < 4; ++ks)
-            tc_mma_ts(tmem + 256u, a + (uint32_t)ks * 8u, vd + (uint64_t)(u * (kUnitBytes >> 4) + (uint32_t)ks * 128u), idesc_pv,
+          for (int ks = 0; ks < 8; ++ks)             // the weights, and their rests, by the same rows of V
+            tc_mma_ts(tmem + 256u, a + (uint32_t)ks * 8u, vd + (uint64_t)(u * (kUnitBytes >> 4) + (uint32_t)(ks & 3) * 128u), idesc_pv,
                       (j | half | ks) ? 1u : 0u);
         }
         tc_commit(bar(kODone + (int)(cnt & 1u)));
@@ -304,7 +326,7 @@ prefill_wide_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
   } else if (warp < 12) {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 176;");
     // ---- softmax: thread = row.  m is the reference exponent of the row (raised, with O rescaled, when the maximum grows by more than
-    // 2^8: P stays within fp16 and a stale reference cancels in O / l); l is this group's part of the row sum, relative to its last m.  The
+    // 2^8: P stays within fp16, and a stale reference cancels in O / l up to the rounding of P, which the second term takes in); l is this group's part of the row sum, relative to its last m.  The
     // groups take turns: a step's reference comes from the step before through shared memory, as soon as that step has its maximum.
     const int grp = (warp - 4) >> 2, wq = warp & 3;
     const int row = wq * 32 + lane;
@@ -385,7 +407,7 @@ prefill_wide_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
         const float2 nm2 = make_float2(neg_m, neg_m);
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-          exp_chunk_store<0, false>(s[c], sc2, nm2, l2, tS + c * 16);
+          exp_chunk_two(s[c], sc2, nm2, l2, tS + (c >> 1) * 64 + (c & 1) * 16);
           if (c & 1) {
             tc_wait_st();                              // O's rescale as well
             tc_fence_before();
