@@ -607,13 +607,16 @@ static int run_prefill(fa::PrefillParams& p, int D, cudaStream_t stream) {
   p.scale_log2 = 1.4426950408889634f / sqrtf((float)D);
   D = Dp;
   cudaError_t e;
-  const bool tc5_ok = fa::prefill_tc5_supported(p, D);
-  if (g_prefill_impl == 2 && !tc5_ok)
-    return fail(FA_ERR_UNSUPPORTED, "the tcgen05 prefill kernel supports D = 64 and 128 only");
+  const bool tc5_ok = fa::prefill_tc5_supported(p, D), wide_ok = fa::prefill_wide_supported(p);
+  if (g_prefill_impl == 2 && !tc5_ok && !wide_ok)
+    return fail(FA_ERR_UNSUPPORTED, "no tcgen05 prefill kernel supports this call");
   if (p.in_bf16 && !tc5_ok)
     return fail(FA_ERR_UNSUPPORTED, "bfloat16 prefill is served by the tcgen05 kernel: head dimension up to 128");
-  const bool wide_ok = fa::prefill_wide_supported(p);
-  if ((tc5_ok || wide_ok) && (g_prefill_impl != 1 || p.in_bf16)) {
+  // Wide heads: the mma.sync kernel keeps the short prompts.  Its blocks of 64 rows and 64 keys are done sooner than one step of 128 x 128 and the
+  // hand-overs of the tcgen05 kernel: up to 64 tokens 0.58 to 0.80 times its time, whatever the batch; of 72 to 128 tokens 0.9 to 1.2 times with few
+  // heads in all, 1.4 to 2 times where they fill half the SMs; from 144 on more than its time.
+  const bool wide = wide_ok && (g_prefill_impl == 2 || p.max_seqlen > ((long long)p.batch * p.H_Q * 2 > di.sm_count ? 64 : 128));
+  if ((tc5_ok || wide) && (g_prefill_impl != 1 || p.in_bf16)) {
     EncodeTiledFn enc;
     rc = get_encode(&enc);
     if (rc != FA_OK) return rc;

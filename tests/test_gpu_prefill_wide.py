@@ -1,5 +1,6 @@
 """Prefill of wide heads (128 < D <= 256, `csrc/prefill_wide.cu`): edges of its 128-row and 128-key tiles, of the 64-key halves and of
-the 64-column slabs, one item per CTA and many, against the fp32 oracle and the mma.sync kernel."""
+the 64-column slabs, one item per CTA and many, against the fp32 oracle and the mma.sync kernel; its error against 64 bits; and which lengths
+go to which kernel."""
 import pytest
 import torch
 
@@ -12,10 +13,12 @@ pytestmark = pytest.mark.gpu
 TOL = 2e-3
 
 
-@pytest.fixture(scope="module")
+@pytest.fixture
 def fa():
+    """The module with the tcgen05 kernels required, so that nothing here can pass on the other kernel."""
     import flash_attn_v100
     from flash_attn_v100_b200 import ops
+    ops.set_prefill_impl(2)
     yield flash_attn_v100
     ops.set_prefill_impl(0)
 
@@ -26,7 +29,7 @@ def _by(impl, fn):
     try:
         return fn()
     finally:
-        ops.set_prefill_impl(0)
+        ops.set_prefill_impl(2)
 
 
 def _dense(B, HQ, HKV, N, D, seed):
@@ -59,9 +62,7 @@ def test_packed_against_oracle_and_other_kernel(fa, causal, D):
     args = (q.cuda(), k.cuda(), v.cuda(), cu.cuda(), max(lens), causal)
     got = fa.forward_varlen_prefill_fp16(*args)
     bf = fa.forward_varlen_prefill_fp16(*args, out_dtype=torch.bfloat16)
-    ops.set_prefill_impl(1)
-    other = fa.forward_varlen_prefill_fp16(*args)
-    ops.set_prefill_impl(0)
+    other = _by(1, lambda: fa.forward_varlen_prefill_fp16(*args))
     a, e = int(cu[0]), int(cu[-1])
     assert not got[:a].any() and not got[e:].any()
     ref = orc.varlen_prefill(q[a:e], k[a:e], v[a:e], cu - a, causal, final_cast=False)
@@ -114,3 +115,13 @@ def test_error_no_larger_than_the_other_kernels(fa, N, D, spread, causal):
     q = (q.float() * spread).half()
     run = lambda: fa.forward_prefill_gqa_fp16(q, k, v, causal)
     assert _error(run(), q, k, v, causal) <= _error(_by(1, run), q, k, v, causal)
+
+
+@pytest.mark.parametrize("B,HQ,N,wide", [(1, 2, 64, False), (1, 2, 128, False), (1, 2, 129, True), (2, 64, 64, False), (2, 64, 65, True), (3, 100, 16, False)])
+def test_short_prompts_stay_with_the_other_kernel(fa, B, HQ, N, wide):
+    """Which kernel a length goes to shows in the bits: the rounding of the two differs in some element of every such output."""
+    q, k, v = (t.cuda() for t in _dense(B, HQ, HQ // 2, N, 256, N + HQ))
+    run = lambda: fa.forward_prefill_gqa_fp16(q, k, v, True)
+    mma, tc = _by(1, run), run()
+    assert not torch.equal(mma, tc)
+    assert torch.equal(_by(0, run), tc if wide else mma)
