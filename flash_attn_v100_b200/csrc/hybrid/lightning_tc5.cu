@@ -233,24 +233,13 @@ __global__ void __launch_bounds__(kThreads, 1) lightning_tc5_kernel(const Lightn
       const uint64_t vd = smem_desc(sV, SLAB, 1024), khd = smem_desc(sKh, SLAB, 1024), kld = smem_desc(sKl, SLAB, 1024);
       const uint64_t shd = smem_desc(sSh, SLAB, 1024), sld = smem_desc(sSl, SLAB, 1024);
       if (!STATE_ONLY) {
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {
-          const uint32_t off = (uint32_t)(ks >> 2) * (SLAB >> 4) + (uint32_t)(ks & 3) * 2u;
-          tc_mma_ss(tmem, qd + off, kd + off, IDESC_QK, ks > 0 ? 1u : 0u);
-        }
+        tc_mma_ss8<StepsAlongK<SLAB, SLAB>>(tmem, qd, kd, IDESC_QK, 0u);
         tc_commit(bar_a);
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {
-          const uint32_t off = (uint32_t)(ks >> 2) * (SLAB >> 4) + (uint32_t)(ks & 3) * 2u;
-          tc_mma_ss(tmem + 128u, qd + off, shd + (uint64_t)(ks * 128), IDESC_B, ks > 0 ? 1u : 0u);
-          tc_mma_ss(tmem + 128u, qd + off, sld + (uint64_t)(ks * 128), IDESC_B, 1u);
-        }
+        tc_mma_ss8<StepsByRowsB<SLAB>>(tmem + 128u, qd, shd, IDESC_B, 0u);
+        tc_mma_ss8<StepsByRowsB<SLAB>>(tmem + 128u, qd, sld, IDESC_B, 1u);
       }
-#pragma unroll
-      for (int ks = 0; ks < 8; ++ks) {
-        tc_mma_ss(tmem + 384u, khd + (uint64_t)(ks * 128), vd + (uint64_t)(ks * 128), IDESC_AB, ks > 0 ? 1u : 0u);
-        tc_mma_ss(tmem + 384u, kld + (uint64_t)(ks * 128), vd + (uint64_t)(ks * 128), IDESC_AB, 1u);
-      }
+      tc_mma_ss8<StepsByRows>(tmem + 384u, khd, vd, IDESC_AB, 0u);
+      tc_mma_ss8<StepsByRows>(tmem + 384u, kld, vd, IDESC_AB, 1u);
       tc_commit(bar_s);
     }
     if (!STATE_ONLY) {
@@ -283,11 +272,8 @@ __global__ void __launch_bounds__(kThreads, 1) lightning_tc5_kernel(const Lightn
         tc_fence_after();
         __syncwarp();
         const uint64_t vd = smem_desc(sV, SLAB, 1024);
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {
-          tc_mma_ts(tmem + 256u, tmem + (uint32_t)ks * 8u, vd + (uint64_t)(ks * 128), IDESC_B, ks > 0 ? 1u : 0u);
-          tc_mma_ts(tmem + 256u, tmem + 64u + (uint32_t)ks * 8u, vd + (uint64_t)(ks * 128), IDESC_B, 1u);
-        }
+        tc_mma_ts8<StepsTmemA<>>(tmem + 256u, tmem, vd, IDESC_B, 0u);
+        tc_mma_ts8<StepsTmemA<>>(tmem + 256u, tmem + 64u, vd, IDESC_B, 1u);
         tc_commit(bar_o);
       }
     }

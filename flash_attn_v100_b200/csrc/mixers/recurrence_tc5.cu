@@ -297,20 +297,13 @@ recurrence_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
     const uint64_t khd = smem_desc(sK, SLAB, 1024), shd = smem_desc(sSh, SLAB, 1024), sld = smem_desc(sSl, SLAB, 1024);
     auto issue_old = [&]() {                                  // Q S
       const uint64_t qd = smem_desc(sQ, 16, 1024);
-#pragma unroll
-      for (int ks = 0; ks < 8; ++ks) {
-        const uint32_t off = (uint32_t)(ks >> 2) * (SLAB >> 4) + (uint32_t)(ks & 3) * 2u;
-        tc_mma_ss(tmem + 128u, qd + off, shd + (uint64_t)(ks * 128), IDESC_B, ks > 0 ? 1u : 0u);
-        tc_mma_ss(tmem + 128u, qd + off, sld + (uint64_t)(ks * 128), IDESC_B, 1u);
-      }
+      tc_mma_ss8<StepsByRowsB<SLAB>>(tmem + 128u, qd, shd, IDESC_B, 0u);
+      tc_mma_ss8<StepsByRowsB<SLAB>>(tmem + 128u, qd, sld, IDESC_B, 1u);
       tc_commit(bar_1);
     };
     auto issue_state = [&]() {
-#pragma unroll
-      for (int ks = 0; ks < 8; ++ks) {
-        tc_mma_ss(tmem + 384u, khd + (uint64_t)(ks * 128), shd + (uint64_t)(ks * 128), IDESC_AB, ks > 0 ? 1u : 0u);
-        tc_mma_ss(tmem + 384u, khd + (uint64_t)(ks * 128), sld + (uint64_t)(ks * 128), IDESC_AB, 1u);
-      }
+      tc_mma_ss8<StepsByRows>(tmem + 384u, khd, shd, IDESC_AB, 0u);
+      tc_mma_ss8<StepsByRows>(tmem + 384u, khd, sld, IDESC_AB, 1u);
       tc_commit(bar_s);
     };
 
@@ -345,11 +338,7 @@ recurrence_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
         issue_state();
       } else {
         const uint64_t qd = smem_desc(sQ, 16, 1024), kd = smem_desc(sK, 16, 1024);
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {
-          const uint32_t off = (uint32_t)(ks >> 2) * (SLAB >> 4) + (uint32_t)(ks & 3) * 2u;
-          tc_mma_ss(tmem, qd + off, kd + off, IDESC_QK, ks > 0 ? 1u : 0u);
-        }
+        tc_mma_ss8<StepsAlongK<SLAB, SLAB>>(tmem, qd, kd, IDESC_QK, 0u);
         tc_commit(bar_a);
         if constexpr (!NORM) issue_old();
       }
@@ -445,11 +434,8 @@ recurrence_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
         for (int hh = 0; hh < NH; ++hh) {
           const uint64_t vh = vd + (uint64_t)(hh * (SLAB >> 4));
           const uint32_t d = tmem + 256u + (uint32_t)hh * 64u, p = tmem + (uint32_t)hh * 384u;
-#pragma unroll
-          for (int ks = 0; ks < 8; ++ks) {
-            tc_mma_ts(d, p + (uint32_t)ks * 8u, vh + (uint64_t)(ks * 128), IDESC_PV, ks > 0 ? 1u : 0u);
-            tc_mma_ts(d, p + 64u + (uint32_t)ks * 8u, vh + (uint64_t)(ks * 128), IDESC_PV, 1u);
-          }
+          tc_mma_ts8<StepsTmemA<>>(d, p, vh, IDESC_PV, 0u);
+          tc_mma_ts8<StepsTmemA<>>(d, p + 64u, vh, IDESC_PV, 1u);
         }
         tc_commit(bar_o);
       }

@@ -130,6 +130,12 @@ __device__ __forceinline__ void drain_wait(uint32_t bar, uint32_t parity, volati
   atomicOr(&g_prefill_status, kStatusWaitTimeout);
 }
 
+// P quarter i / 2 holds the keys of score chunk {0, 1, 3, 2}[i / 2]: the matching rows of V.
+struct PvSteps {
+  static constexpr uint32_t a(int i) { return (uint32_t)i * 8u; }
+  static constexpr uint32_t b(int i) { return (uint32_t)(i < 4 ? i : (i ^ 2)) * 128u; }
+};
+
 __device__ __forceinline__ float fmax3(float a, float b, float c) {
   float d;
   asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
@@ -486,21 +492,15 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_consta
         __syncwarp();   // the lanes leave their barrier waits one by one; elect.sync needs them together
         const uint64_t b0 = kd0 + (uint64_t)((uint32_t)st * (QK_BYTES >> 4));
 #pragma unroll
-        for (int ks = 0; ks < NQK * 4; ++ks) {
-          constexpr uint32_t kSlab16 = SLAB >> 4;
-          const uint32_t off = (uint32_t)(ks >> 2) * kSlab16 + (uint32_t)(ks & 3) * 2u;
-          tc_mma_ss(dS, qd + off, b0 + off, IDESC_QK, ks > 0 ? 1u : 0u);
-        }
+        for (int sl = 0; sl + 1 < NQK; sl += 2)
+          tc_mma_ss8<StepsAlongK<SLAB, SLAB>>(dS, qd + (uint64_t)(sl * (SLAB >> 4)), b0 + (uint64_t)(sl * (SLAB >> 4)), IDESC_QK, sl > 0 ? 1u : 0u);
+        if constexpr (NQK % 2 == 1)
+          tc_mma_ss4<StepsAlongK<SLAB, SLAB>>(dS, qd + (uint64_t)((NQK - 1) * (SLAB >> 4)), b0 + (uint64_t)((NQK - 1) * (SLAB >> 4)), IDESC_QK, NQK > 1 ? 1u : 0u);
       };
       auto issue_pv = [&](int st, uint32_t acc) {
         __syncwarp();
         const uint64_t b0 = vd0 + (uint64_t)((uint32_t)st * (V_BYTES >> 4));
-#pragma unroll
-        for (int ks = 0; ks < BN / 16; ++ks) {
-          // P quarter ks / 2 holds the keys of score chunk {0, 1, 3, 2}[ks / 2]: pick the matching rows of V
-          const int kv = ks < 4 ? ks : (ks ^ 2);
-          tc_mma_ts(dO, dS + P_COL + (uint32_t)ks * 8u, b0 + (uint32_t)kv * 128u, IDESC_PV, (acc | (ks > 0 ? 1u : 0u)));
-        }
+        tc_mma_ts8<PvSteps>(dO, dS + P_COL, b0, IDESC_PV, acc);
       };
       uint32_t kv_it = 0, q_cnt = 0, blk = 0, tok_waits = 0;
       uint32_t batches = 0;                      // committed so far

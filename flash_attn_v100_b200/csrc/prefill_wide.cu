@@ -261,12 +261,9 @@ prefill_wide_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
           const uint32_t u = take_unit();
           tc_fence_after();
           __syncwarp();
-          const int ks1 = (half == 0 ? 2 : n_slab - 2) * 4;
-          for (int ks = 0; ks < ks1; ++ks) {
-            const uint32_t off = (uint32_t)(ks >> 2) * (kSlabK >> 4) + (uint32_t)(ks & 3) * 2u;
-            tc_mma_ss(d, qd + (uint64_t)((uint32_t)half * 2u * (kSlabK >> 4) + off), kd + (uint64_t)(u * (kUnitBytes >> 4) + off), IDESC_QK,
-                      (half | ks) ? 1u : 0u);
-          }
+          const uint64_t a = qd + (uint64_t)((uint32_t)half * 2u * (kSlabK >> 4)), b = kd + (uint64_t)(u * (kUnitBytes >> 4));
+          if (half == 0 || n_slab == 4) tc_mma_ss8<StepsAlongK<kSlabK, kSlabK>>(d, a, b, IDESC_QK, (uint32_t)half);
+          else tc_mma_ss4<StepsAlongK<kSlabK, kSlabK>>(d, a, b, IDESC_QK, 1u);
         }
         tc_commit(bar(kSFull + (c & 1u)));
       };
@@ -289,10 +286,8 @@ prefill_wide_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
           tc_fence_after();
           __syncwarp();
           const uint32_t a = tmem + (cnt & 1u) * 128u + (uint32_t)half * 64u;
-#pragma unroll
-          for (int ks = 0; ks < 8; ++ks)             // the weights, and their rests, by the same rows of V
-            tc_mma_ts(tmem + 256u, a + (uint32_t)ks * 8u, vd + (uint64_t)(u * (kUnitBytes >> 4) + (uint32_t)(ks & 3) * 128u), idesc_pv,
-                      (j | half | ks) ? 1u : 0u);
+          // the weights, and their rests, by the same rows of V
+          tc_mma_ts8<StepsTmemA<4>>(tmem + 256u, a, vd + (uint64_t)(u * (kUnitBytes >> 4)), idesc_pv, (j | half) ? 1u : 0u);
         }
         tc_commit(bar(kODone + (int)(cnt & 1u)));
       }
