@@ -165,3 +165,20 @@ def last_error(name: str = "attention") -> str:
 def check(rc: int, name: str = "attention") -> None:
     if rc != 0:
         raise RuntimeError(last_error(name) or f"a call of the {name} library failed with status {rc}")
+
+
+def call_module(workspaces):
+    """The native host side of the calls (`_call`), bound to the library's entry points and to the scratch buffers by (device, stream); None if it has
+    not been built, or for another torch."""
+    try:
+        import torch
+
+        from . import _call
+        if _call.torch_version != torch.__version__.split("+")[0]:
+            return None
+        lib = load()
+        entries = [n for n in SIGNATURES if n.startswith(("fa_last", "fa_decode", "fa_paged", "fa_prefill"))]
+        _call.bind({n: _c.cast(getattr(lib, n), _vp).value for n in entries}, workspaces)
+        return _call
+    except ImportError:
+        return None

@@ -10,6 +10,8 @@ model needs.
     python -m flash_attn_v100_b200.build --force
     python -m flash_attn_v100_b200.build -v         # also print ptxas resource usage
 
+`_call` (csrc/host/call.cpp) is the host side of the attention operators' calls, a CPython extension built against the installed torch.
+
 Every `.cu` file is compiled to an object of its own (in parallel, cached under
 `_build/` by source time stamps and flags) and the objects of a library are linked
 together.  nvcc cross-compiles without a GPU.  The libraries link only the CUDA
@@ -83,7 +85,7 @@ def find_nvcc() -> str:
 def _run(cmd):
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
-        raise RuntimeError("nvcc failed:\n" + " ".join(cmd) + "\n" + res.stdout + res.stderr)
+        raise RuntimeError("compiler failed:\n" + " ".join(cmd) + "\n" + res.stdout + res.stderr)
     return res.stderr
 
 
@@ -122,6 +124,31 @@ def build(force: bool = False, verbose: bool = False, extra_flags=None, lib_path
     return lib_path
 
 
+CALL_SOURCE = os.path.join(CSRC, "host", "call.cpp")
+CALL_PATH = os.path.join(PKG_DIR, "_call.so")
+
+
+def build_call(force: bool = False) -> str:
+    """Compile the host side of the calls.  The operators work without it, through ctypes, at a higher cost per call."""
+    deps = (CALL_SOURCE, os.path.join(INCLUDE, "fa_b200.h"))
+    if not force and os.path.exists(CALL_PATH) and os.path.getmtime(CALL_PATH) >= max(os.path.getmtime(d) for d in deps):
+        return CALL_PATH
+    import sysconfig
+
+    import torch
+    root = os.path.join(os.path.dirname(torch.__file__), "")
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(find_nvcc())))
+    include = [root + "include", root + "include/torch/csrc/api/include", sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
+    with _build_lock():
+        part = f"{CALL_PATH}.{os.getpid()}.tmp"
+        abi = f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}"
+        _run([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", abi, *[f"-I{d}" for d in include], CALL_SOURCE, "-o", part, f"-L{root}lib",
+              "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"])
+        os.replace(part, CALL_PATH)
+    return CALL_PATH
+
+
 if __name__ == "__main__":
     for name in LIBRARIES:
         print(build(force="--force" in sys.argv, verbose="-v" in sys.argv, library=name))
+    print(build_call(force="--force" in sys.argv))

@@ -68,6 +68,18 @@ _workspaces: Dict[Tuple[int, int], torch.Tensor] = {}
 _retired_workspaces: list = []
 
 
+_UNSET = object()
+_call_mod = _UNSET
+
+
+def _native(name, *args):
+    """The call `name` of the native host side with these arguments; None if it is not for it (or not there)."""
+    global _call_mod
+    if _call_mod is _UNSET:
+        _call_mod = _lib.call_module(_workspaces)
+    return None if _call_mod is None else getattr(_call_mod, name)(*args)
+
+
 def _chk(cond: bool, msg: str) -> None:
     if not cond:
         raise RuntimeError(msg)
@@ -131,8 +143,8 @@ def _ptr(t):
     return t.data_ptr()      # the entry points' argument types turn it into a pointer
 
 
-# The host side of a call is what bounds small batches (a decode of four short sequences runs 6 us on the GPU), so
-# the wrappers look at each tensor once: `_plain` and a comparison of shapes accept what the detailed checks accept, and
+# The host side of a call is what bounds small batches (a decode of four short sequences runs 6 us on the GPU).  Plain calls go through the native
+# host side (csrc/host/call.cpp); for the rest, and without it, the wrappers look at each tensor once: `_plain` and a comparison of shapes accept what the detailed checks accept, and
 # only a call that fails them goes through those, for the message.  Measured per call, before and after: paged decode
 # of four sequences 31.0 and 17.7 us, packed prefill of three short prompts 32.9 and 22.5 us.
 def _plain(t, dtype, dims, dev):
@@ -243,6 +255,10 @@ def _decode_inputs(q, k, v, dtype):
 
 
 def _decode_gqa(out, q, k, v, causal, cache_len, stream_int=None):
+    if out is None and stream_int is None:
+        done = _native("decode", q, k, v, causal, cache_len, _elem() is torch.bfloat16)
+        if done is not None:
+            return done
     if not (_decode_inputs(q, k, v, _elem()) and (out is None or (_plain(out, _elem(), 4, q.get_device()) and out.shape == q.shape))):
         for t, n in ((q, "q"), (k, "k"), (v, "v")):
             _check_input(t, n)
@@ -309,6 +325,9 @@ def forward_decode_sliding_window_gqa(q, k, v, causal, cache_len, window_size, s
     j < sink_size or window_start <= j <= cache_len, window_start = max(0, min(cache_len+1, N) - window_size)
     (:4386-4387, :4410-4412).  `causal` has no effect, as in the reference; like the reference, no
     bound is checked on cache_len, window_size or sink_size."""
+    done = _native("window", q, k, v, cache_len, window_size, sink_size)
+    if done is not None:
+        return done
     if not _decode_inputs(q, k, v, torch.float16):
         for t, n in ((q, "q"), (k, "k"), (v, "v")):
             _check_input(t, n)
@@ -365,6 +384,9 @@ def forward_decode_int8_kv_cache_gqa(q, k_int8, v_int8, k_scale, v_scale, cache_
     q [B,H_Q,1,D] fp16; k_int8/v_int8 [B,H_KV,N,D] int8; k_scale/v_scale [B,H_KV,N] fp16 (one scale per
     cached token) -> new [B,H_Q,1,D] fp16.  Elements are dequantised as fp16(float(int8) * float(scale))
     (:4083-4086) and keys j <= cache_len are attended (:4094-4098)."""
+    done = _native("int8_kv", q, k_int8, v_int8, k_scale, v_scale, cache_len)
+    if done is not None:
+        return done
     dev = _cuda_index(q)
     if not (dev >= 0 and _plain(q, torch.float16, 4, dev) and _plain(k_int8, torch.int8, 4, dev) and _plain(v_int8, torch.int8, 4, dev)
             and _plain(k_scale, torch.float16, 3, dev) and _plain(v_scale, torch.float16, 3, dev) and q.size(2) == 1
@@ -390,6 +412,9 @@ def forward_continuous_batching_fp16(q, k, v, cache_lens, causal):
     """flash_attn_forward_continuous_batching_fp16 (continuous_batching_kernel.cu:338-406).
     q [B,H_Q,1,D], k/v [B,H_KV,max_N,D] fp16, cache_lens [B] int32; sequence b attends
     keys [0, min(cache_lens[b]+1, max_N)).  `causal` has no effect (as in the reference)."""
+    done = _native("contig", q, k, v, cache_lens, causal)
+    if done is not None:
+        return done
     if not (_decode_inputs(q, k, v, torch.float16) and _plain(cache_lens, torch.int32, 1, q.get_device())
             and cache_lens.size(0) == q.size(0)):
         for t, n in ((q, "q"), (k, "k"), (v, "v"), (cache_lens, "cache_lens")):
@@ -458,6 +483,9 @@ def forward_paged_decode_gqa_fp16(q, k_cache, v_cache, block_table, seq_lens, ma
     _chk(out_dtype in (None, torch.float16, torch.bfloat16), "out_dtype must be float16 or bfloat16")
     bf16_out = out_dtype == torch.bfloat16 and _elem() == torch.float16
     elem, dev = _elem(), _cuda_index(q)
+    done = _native("paged", q, k_cache, v_cache, block_table, seq_lens, max_num_blocks, elem is torch.bfloat16, bf16_out)
+    if done is not None:
+        return done
     if not (dev >= 0 and _plain(q, elem, 4, dev) and _plain(k_cache, elem, 4, dev) and _plain(v_cache, elem, 4, dev)
             and _plain(block_table, torch.int32, 2, dev) and _plain(seq_lens, torch.int32, 1, dev)
             and _paged_shapes_fit(q.shape, k_cache.shape, v_cache.shape, block_table.size(0), seq_lens.size(0))):
@@ -504,6 +532,10 @@ def forward_decode_int8_gqa(q, k, v, q_scale, k_scale, cache_len, return_scores=
     q [B,H_Q,1,D], k/v [B,H_KV,N,D] fp16, q_scale [B,H_Q] fp32, k_scale [B,H_KV,N] fp32
     (per cached token).  With `return_scores=True` (an addition) also returns the raw
     int32 QK^T accumulators [B,H_Q,N] (entries past cache_len are zero)."""
+    if not return_scores:
+        done = _native("int8_qk", q, k, v, q_scale, k_scale, cache_len)
+        if done is not None:
+            return done
     if not (_decode_inputs(q, k, v, torch.float16) and _plain(q_scale, torch.float32, 2, q.get_device())
             and _plain(k_scale, torch.float32, 3, q.get_device()) and q_scale.shape == q.shape[:2] and k_scale.shape == k.shape[:3]):
         _check_int8_qk(q, k, v, q_scale, k_scale)
@@ -560,6 +592,10 @@ def forward_fp16(q, k, v, causal):
 
 def _prefill_gqa(out, q, k, v, causal):
     elem, dev = _elem(), _cuda_index(q)
+    if out is None:
+        done = _native("dense", q, k, v, causal, elem is torch.bfloat16)
+        if done is not None:
+            return done
     if not (dev >= 0 and _plain(q, elem, 4, dev) and _plain(k, elem, 4, dev) and _plain(v, elem, 4, dev) and k.shape == v.shape
             and q.size(0) == k.size(0) and q.shape[2:] == k.shape[2:] and (out is None or (_plain(out, elem, 4, dev) and out.shape == q.shape))):
         for t, n in ((q, "q"), (k, "k"), (v, "v")):
@@ -589,6 +625,10 @@ def forward_prefill_gqa_fp16_out(out, q, k, v, causal):
 
 def _varlen(q, k, v, cu_seqlens, max_seqlen, causal, stream_int=None, bf16_out=False):
     elem, dev = _elem(), _cuda_index(q)
+    if stream_int is None:
+        done = _native("varlen", q, k, v, cu_seqlens, max_seqlen, causal, elem is torch.bfloat16, bf16_out and elem is torch.float16)
+        if done is not None:
+            return done
     if not (dev >= 0 and _plain(q, elem, 3, dev) and _plain(k, elem, 3, dev) and _plain(v, elem, 3, dev) and _plain(cu_seqlens, torch.int32, 1, dev)
             and k.shape == v.shape and q.size(0) == k.size(0) and q.size(2) == k.size(2)):
         for t, n in ((q, "q"), (k, "k"), (v, "v"), (cu_seqlens, "cu_seqlens")):
@@ -727,21 +767,33 @@ def rope_append_paged_fp16(q, k, v, cos, sin, k_cache, v_cache, block_table, pos
 # are bfloat16; everything else — shapes, checks, errors — is that of the fp16 function named in the body.
 # --------------------------------------------------------------------------
 def forward_decode_gqa_bf16(q, k, v, causal, cache_len):
+    done = _native("decode", q, k, v, causal, cache_len, True)
+    if done is not None:
+        return done
     with _bf16_elements():
         return forward_decode_gqa_fp16(q, k, v, causal, cache_len)
 
 
 def forward_paged_decode_gqa_bf16(q, k_cache, v_cache, block_table, seq_lens, max_num_blocks):
+    done = _native("paged", q, k_cache, v_cache, block_table, seq_lens, max_num_blocks, True, False)
+    if done is not None:
+        return done
     with _bf16_elements():
         return forward_paged_decode_gqa_fp16(q, k_cache, v_cache, block_table, seq_lens, max_num_blocks)
 
 
 def forward_prefill_gqa_bf16(q, k, v, causal):
+    done = _native("dense", q, k, v, causal, True)
+    if done is not None:
+        return done
     with _bf16_elements():
         return forward_prefill_gqa_fp16(q, k, v, causal)
 
 
 def forward_varlen_prefill_bf16(q, k, v, cu_seqlens, max_seqlen, causal):
+    done = _native("varlen", q, k, v, cu_seqlens, max_seqlen, causal, True, False)
+    if done is not None:
+        return done
     with _bf16_elements():
         return forward_varlen_prefill_fp16(q, k, v, cu_seqlens, max_seqlen, causal)
 
