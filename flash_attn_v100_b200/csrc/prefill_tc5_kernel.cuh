@@ -335,7 +335,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_consta
   constexpr int B_QFULL = 0, B_QEMPTY = 2, B_KFULL = B_QEMPTY + 2, B_KEMPTY = B_KFULL + K_STAGES,
                 B_VFULL = B_KEMPTY + K_STAGES, B_VEMPTY = B_VFULL + V_STAGES, B_SFULL = B_VEMPTY + V_STAGES,
                 B_PFULL = B_SFULL + 2 * kBatchBars, B_TOKEN = B_PFULL + 2,
-                B_IFULL = B_TOKEN + 2, B_IEMPTY = B_IFULL + kItemQ, B_PAIR = B_IEMPTY + kItemQ,
+                B_IFULL = B_TOKEN + 2, B_IEMPTY = B_IFULL + kItemQ, B_CLAIM = B_IEMPTY + kItemQ, B_PAIR = B_CLAIM + 1,
                 B_DRAIN = B_PAIR + 8, B_TURN = B_DRAIN + 2, B_COUNT = B_TURN + 2;
   static_assert(B_COUNT + kItemQ + 1 <= 64, "barriers, item slots and the tensor-memory slot share 64 words");
   volatile long long* item_slot = reinterpret_cast<volatile long long*>(bars + B_COUNT);
@@ -379,6 +379,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_consta
       mbar_init(bar(B_IFULL + i), 1);
       mbar_init(bar(B_IEMPTY + i), kItemConsumers);
     }
+    mbar_init(bar(B_CLAIM), 1);
     *abort_flag = 0;
     for (int i = 0; i < 8; ++i) redo_tag[i] = 0u;
     mbar_fence_init();
@@ -437,6 +438,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_consta
           ++q_used[t];
         }
         for (int j = 0; j < it.n_max; ++j, ++kv_it) {
+          if (j == (it.n_max > 2 ? it.n_max - 3 : 0)) mbar_arrive(bar(B_CLAIM));
           const int st = kv_it % K_STAGES, sv = kv_it % V_STAGES;
           const uint32_t ph = (kv_it / K_STAGES) & 1u, phv = (kv_it / V_STAGES) & 1u;
           if (kv_it >= K_STAGES) PROF_WAIT(0, 3, wait_or_abort(bar(B_KEMPTY + st), ph ^ 1u, abort_flag));
@@ -603,8 +605,9 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_consta
     asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
     // ============================ item claimer ======================================
     // Claims work items from the global counter, skips the empty ones (row blocks past the end of a
-    // sequence) and publishes the others through the item queue, up to kItemQ items ahead of the slowest
-    // role: the latency of the global atomic stays off every other role's path.
+    // sequence) and publishes the others through the item queue: an item is claimed while the copies of the last three
+    // KV tiles of the one before are issued, which keeps the latency of the global atomic off every other role's path.
+    // Claims of up to kItemQ items ahead dealt the items out in turn, whatever they cost, where a CTA has few of them.
     if (lane == 0) {
       bool first = true;
       for (uint32_t ic = 0;; ++ic) {
@@ -612,6 +615,8 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_consta
         Tc5Item it;
         long long item;
         bool have = false;
+        // not before the copies of the last steps of the item before begin: earlier claims would deal the items out in turn, whatever they cost
+        if (ic > 0) wait_or_abort(bar(B_CLAIM), (ic - 1) & 1u, abort_flag);
         while (true) {
           if (p.item_counter != nullptr) item = (long long)atomicAdd(p.item_counter, 1ULL);
           else item = first ? (long long)blockIdx.x : n_items;
