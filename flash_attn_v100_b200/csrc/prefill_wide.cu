@@ -40,7 +40,7 @@ constexpr int kQBytes = 64 * 1024;
 constexpr int kWideItemQ = 4;
 constexpr int kWideConsumers = 1 + 1 + 8 + 4;             // copy lane, MMA warp, softmax and output warps
 enum WideBar { kQFull = 0, kUFull = 1, kSFull = kUFull + kUnits, kPLo = kSFull + 2, kPHi = kPLo + 2, kODone = kPHi + 2, kOEmpty = kODone + 2, kLFull, kMReady,
-               kIFull = kMReady + 2, kIEmpty = kIFull + kWideItemQ, kWideBars = kIEmpty + kWideItemQ };
+               kIFull = kMReady + 2, kIEmpty = kIFull + kWideItemQ, kClaim = kIEmpty + kWideItemQ, kWideBars };
 constexpr int kWideSmem = kQBytes + kUnits * kUnitBytes + kWideBars * 8 + kWideItemQ * 8 + 4 * 128 * 4 + 16;
 static_assert(kWideSmem <= 227 * 1024, "shared memory plan exceeds the SM");
 
@@ -145,6 +145,7 @@ prefill_wide_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
       mbar_init(bar(kODone + b), 1);
     }
     mbar_init(bar(kOEmpty), 4);
+    mbar_init(bar(kClaim), 1);
     mbar_init(bar(kLFull), 8);
     for (int i = 0; i < kWideItemQ; ++i) {
       mbar_init(bar(kIFull + i), 1);
@@ -224,6 +225,7 @@ prefill_wide_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
         };
         load_k(0);
         for (int j = 0; j < it.n_kv; ++j) {
+          if (j == (it.n_kv > 2 ? it.n_kv - 3 : 0)) mbar_arrive(bar(kClaim));
           if (j + 1 < it.n_kv) load_k(j + 1);
           load_v(j);
         }
@@ -302,6 +304,8 @@ prefill_wide_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
         if (*abort_flag) break;
         WideItem it;
         long long item = -1;
+        // an item is claimed when the copies of the last steps of the one before begin: earlier claims would deal the items out in turn, whatever they cost
+        if (ic > 0) wait_or_abort(bar(kClaim), (ic - 1) & 1u, abort_flag);
         while (true) {
           if (p.item_counter != nullptr) item = (long long)atomicAdd(p.item_counter, 1ULL);
           else item = first ? (long long)blockIdx.x : n_items;
