@@ -130,6 +130,14 @@ __device__ __forceinline__ void drain_wait(uint32_t bar, uint32_t parity, volati
   atomicOr(&g_prefill_status, kStatusWaitTimeout);
 }
 
+// The next item of a launch; `n_items` or more: there is none.  Every CTA gets exactly one such answer, so the one that is given out last is known, and whoever
+// gets it puts the counter back to zero for the next launch.
+__device__ __forceinline__ long long claim_item(unsigned long long* counter, long long n_items) {
+  const long long item = (long long)atomicAdd(counter, 1ULL);
+  if (item == n_items + gridDim.x - 1) atomicExch(counter, 0ULL);
+  return item;
+}
+
 // P quarter i / 2 holds the keys of score chunk {0, 1, 3, 2}[i / 2]: the matching rows of V.
 struct PvSteps {
   static constexpr uint32_t a(int i) { return (uint32_t)i * 8u; }
@@ -609,7 +617,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_consta
     // KV tiles of the one before are issued, which keeps the latency of the global atomic off every other role's path.
     // Claims of up to kItemQ items ahead dealt the items out in turn, whatever they cost, where a CTA has few of them.
     if (lane == 0) {
-      bool first = true;
+      bool first = true, ended = p.item_counter == nullptr;
       for (uint32_t ic = 0;; ++ic) {
         if (*abort_flag) break;
         Tc5Item it;
@@ -618,10 +626,10 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_consta
         // not before the copies of the last steps of the item before begin: earlier claims would deal the items out in turn, whatever they cost
         if (ic > 0) wait_or_abort(bar(B_CLAIM), (ic - 1) & 1u, abort_flag);
         while (true) {
-          if (p.item_counter != nullptr) item = (long long)atomicAdd(p.item_counter, 1ULL);
+          if (p.item_counter != nullptr) item = claim_item(p.item_counter, n_items);
           else item = first ? (long long)blockIdx.x : n_items;
           first = false;
-          if (item >= n_items) break;
+          if (item >= n_items) { ended = true; break; }
           if (tc5_decode_item<EXT>(p, item, it)) { have = true; break; }
         }
         const int slot = ic % kItemQ;
@@ -630,6 +638,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_consta
         mbar_arrive(bar(B_IFULL + slot));
         if (!have) break;
       }
+      while (!ended) ended = claim_item(p.item_counter, n_items) >= n_items;      // (left early: the counter is put back all the same)
     }
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
@@ -1016,16 +1025,16 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_consta
   }
 }
 
-// Item counters of in-flight launches (one per launch, used round-robin, zeroed in-stream before
-// the kernel).  More than kCounterPool prefill launches in flight at once on one device would share
-// a counter; launches ordered on one stream never do.
+// Item counters of in-flight launches (one per launch, used round-robin).  A launch finds its counter at zero and leaves it so (claim_item), so none of
+// them has to be cleared by a launch of its own (2 to 3 us of a prefill of 40).  More than kCounterPool prefill launches in flight at once on
+// one device would share a counter; launches ordered on one stream never do.
 constexpr int kCounterPool = 64;
 __device__ unsigned long long g_tc5_item_counters[kCounterPool];
 unsigned long long* g_counter_base[64] = {nullptr};
 std::atomic<unsigned int> g_counter_next{0};
 std::mutex g_counter_mu;
 
-cudaError_t next_item_counter(unsigned long long** out, cudaStream_t stream) {
+cudaError_t next_item_counter(unsigned long long** out) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
@@ -1039,10 +1048,8 @@ cudaError_t next_item_counter(unsigned long long** out, cudaStream_t stream) {
       g_counter_base[dev] = static_cast<unsigned long long*>(ptr);
     }
   }
-  unsigned long long* c = g_counter_base[dev] + (g_counter_next.fetch_add(1) % kCounterPool);
-  e = cudaMemsetAsync(c, 0, sizeof(unsigned long long), stream);
-  *out = c;
-  return e;
+  *out = g_counter_base[dev] + (g_counter_next.fetch_add(1) % kCounterPool);
+  return cudaSuccess;
 }
 
 }  // namespace

@@ -299,7 +299,7 @@ prefill_wide_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
   } else if (warp == 2) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
     if (lane == 0) {
-      bool first = true;
+      bool first = true, ended = p.item_counter == nullptr;
       for (uint32_t ic = 0;; ++ic) {
         if (*abort_flag) break;
         WideItem it;
@@ -307,10 +307,10 @@ prefill_wide_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
         // an item is claimed when the copies of the last steps of the one before begin: earlier claims would deal the items out in turn, whatever they cost
         if (ic > 0) wait_or_abort(bar(kClaim), (ic - 1) & 1u, abort_flag);
         while (true) {
-          if (p.item_counter != nullptr) item = (long long)atomicAdd(p.item_counter, 1ULL);
+          if (p.item_counter != nullptr) item = claim_item(p.item_counter, n_items);
           else item = first ? (long long)blockIdx.x : n_items;
           first = false;
-          if (item >= n_items) { item = -1; break; }
+          if (item >= n_items) { item = -1; ended = true; break; }
           if (wide_item(p, item, it)) break;
         }
         const int slot = ic % kWideItemQ;
@@ -319,6 +319,7 @@ prefill_wide_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
         mbar_arrive(bar(kIFull + slot));
         if (item < 0) break;
       }
+      while (!ended) ended = claim_item(p.item_counter, n_items) >= n_items;      // (left early: the counter is put back all the same)
     }
   } else if (warp == 3) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
@@ -538,7 +539,7 @@ cudaError_t launch_prefill_wide(const PrefillParams& pp, int sm_count, void* enc
   if (e != cudaSuccess) return e;
   const long long n_items = (long long)p.n_rb * pp.batch * pp.H_Q;
   if (n_items > sm_count) {
-    e = next_item_counter(&p.item_counter, stream);
+    e = next_item_counter(&p.item_counter);
     if (e != cudaSuccess) return e;
   }
   prefill_wide_kernel<<<(unsigned)(n_items < sm_count ? n_items : sm_count), kWideThreads, kWideSmem, stream>>>(qmap, kmap, vmap, p);
