@@ -196,6 +196,9 @@ class TPDecoder(GreedyHead):
         st["peer"] = peer
         fused = peer is not None and len(peer) == 4    # peer[2]: residual stream x, peer[3]: normed activations h
         n_layers = len(self.w["layers"])
+        # Prefill: behind the last layer's attention only the rows that are returned go on (its keys and values are in the cache by then).  Where none are
+        # wanted, all rows do, as operators do not take empty tensors.
+        narrow = prefill and (want is None or want.numel() > 0)
 
         def first():
             if fused:
@@ -244,6 +247,9 @@ class TPDecoder(GreedyHead):
                     attn = ops.forward_paged_decode_gqa_fp16(q_rot, kv.k_pools[l], kv.v_pools[l], block_table,
                                                              st["lens"], max_blocks, out_dtype=torch.bfloat16)
                 a = attn.reshape(x.size(0), self.ql * cfg.head_dim)   # bf16 straight from the attention epilogue
+                if narrow and l + 1 == n_layers:
+                    rows = want if want is not None else (cu_seqlens[1:] - 1).long()
+                    a, st["x"] = a[rows], x[rows]
                 if peer is None:
                     st["o"] = a @ lw["wo"].t()
                 elif fused:                # GEMM into the peer buffer; sum over the ranks, x += sum, h = ln2(x)
@@ -271,11 +277,9 @@ class TPDecoder(GreedyHead):
             if fused:                      # the last all-reduce has applied the final norm
                 st["hidden"] = st["h"] if want is None else st["h"][want]
                 return
-            if prefill or want is not None:
-                idx = want if want is not None else (cu_seqlens[1:] - 1).long()
-                x_last, d_last = st["x"][idx].contiguous(), st["delta"][idx].contiguous()
-            else:
-                x_last, d_last = st["x"], st["delta"]
+            x_last, d_last = st["x"], st["delta"]
+            if want is not None and not narrow:
+                x_last, d_last = x_last[want].contiguous(), d_last[want].contiguous()
             st["hidden"] = self._add_rmsnorm(x_last, d_last, self.w["final_ln"])   # final norm of (x + last MLP)
 
         return st, first, layers, last
