@@ -660,7 +660,7 @@ int fa_prefill_dense_bf16(const void* q, const void* k, const void* v, void* out
 
 static int prefill_varlen_impl(const void* q, const void* k, const void* v, void* out, const int32_t* cu_seqlens,
                                int batch, int64_t total, int H_Q, int H_KV, int D, int max_seqlen, int causal,
-                               void* stream, bool out_bf16, bool in_bf16 = false) {
+                               void* stream, bool out_bf16, bool in_bf16 = false, bool clear = false) {
   int rc = check_decode_common(q, k, v, out, batch, H_Q, H_KV, D);
   if (rc != FA_OK) return rc;
   FA_REQUIRE(cu_seqlens != nullptr, "null cu_seqlens");
@@ -678,7 +678,19 @@ static int prefill_varlen_impl(const void* q, const void* k, const void* v, void
   p.causal = causal ? 1 : 0;
   p.out_bf16 = out_bf16 ? 1 : 0;
   p.in_bf16 = in_bf16 ? 1 : 0;
+  if (clear) {
+    rc = fa_prefill_varlen_clear(out, cu_seqlens, batch, total, max_seqlen, (int64_t)H_Q * D * 2, stream);
+    if (rc != FA_OK) return rc;
+    p.after_clear = 1;
+  }
   return run_prefill(p, D, static_cast<cudaStream_t>(stream));
+}
+
+int fa_prefill_varlen_zeroed(const void* q, const void* k, const void* v, void* out, const int32_t* cu_seqlens,
+                             int batch, int64_t total, int H_Q, int H_KV, int D, int max_seqlen, int causal,
+                             int in_bf16, int out_bf16, void* stream) {
+  return prefill_varlen_impl(q, k, v, out, cu_seqlens, batch, total, H_Q, H_KV, D, max_seqlen, causal, stream, in_bf16 != 0 || out_bf16 != 0,
+                             in_bf16 != 0, true);
 }
 
 int fa_prefill_varlen_clear(void* out, const int32_t* cu_seqlens, int batch, int64_t total, int max_seqlen,

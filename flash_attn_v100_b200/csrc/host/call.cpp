@@ -33,8 +33,7 @@ struct Entries {
   decltype(&fa_decode_int8_kv_cache_gqa) int8_kv;
   decltype(&fa_decode_int8_gqa) int8_qk;
   decltype(&fa_prefill_dense_f16) dense, dense_bf16;
-  decltype(&fa_prefill_varlen_clear) clear;
-  decltype(&fa_prefill_varlen_f16) varlen, varlen_bf16, varlen_out_bf16;
+  decltype(&fa_prefill_varlen_zeroed) varlen;
 };
 Entries g;
 PyObject* g_workspaces = nullptr;      // ops._workspaces: (device, stream) -> uint8 tensor
@@ -304,12 +303,8 @@ PyObject* varlen(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const cudaStream_t s = stream_of(c.dev);
   const int batch = (int)cu->size(0) - 1, HQ = (int)q->size(1), D = (int)q->size(2);
   int rc;
-  Py_BEGIN_ALLOW_THREADS
-  rc = g.clear(out.data_ptr(), cu->data_ptr<int32_t>(), batch, q->size(0), longest, (int64_t)HQ * D * 2, s);   // rows outside every sequence are zero
-  if (rc == 0)
-    rc = (bf ? g.varlen_bf16 : (out_bf ? g.varlen_out_bf16 : g.varlen))(q->data_ptr(), k->data_ptr(), v->data_ptr(), out.data_ptr(), cu->data_ptr<int32_t>(),
-                                                                        batch, q->size(0), HQ, (int)k->size(1), D, longest, causal, s);
-  Py_END_ALLOW_THREADS
+  FA_LAUNCH(g.varlen(q->data_ptr(), k->data_ptr(), v->data_ptr(), out.data_ptr(), cu->data_ptr<int32_t>(), batch, q->size(0), HQ, (int)k->size(1), D, longest,
+                     causal, bf, out_bf, s));
   return result(rc, out);
   END_HANDLE_TH_ERRORS
 }
@@ -340,10 +335,7 @@ PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
   get("fa_decode_int8_gqa", g.int8_qk);
   get("fa_prefill_dense_f16", g.dense);
   get("fa_prefill_dense_bf16", g.dense_bf16);
-  get("fa_prefill_varlen_clear", g.clear);
-  get("fa_prefill_varlen_f16", g.varlen);
-  get("fa_prefill_varlen_bf16", g.varlen_bf16);
-  get("fa_prefill_varlen_f16_out_bf16", g.varlen_out_bf16);
+  get("fa_prefill_varlen_zeroed", g.varlen);
   if (!ok) {
     if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, "an entry point is missing");
     return nullptr;

@@ -26,7 +26,26 @@ struct PrefillParams {
   int D_real;                 // head dimension of the tensors; the kernels are built for 64 / 128 / 256 columns
                               // and take the columns [D_real, D) as zeros
   float scale_log2;           // log2(e) / sqrt(D_real)
+  int after_clear;            // launched directly behind launch_varlen_clear on the same stream
 };
+
+// Launch of an attention kernel; `overlap`: beside the end of the clear in front of it, which lets its successor start as soon as its own blocks have.  That clear
+// started behind everything before it, so the attention may read its inputs at once; before its first store it waits for the clear (wait_for_clear), whose rows it
+// may share where offsets overlap.
+template <class Kernel, class... Args>
+cudaError_t launch_attention(bool overlap, Kernel kern, unsigned grid, unsigned threads, size_t smem, cudaStream_t stream, const Args&... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = overlap ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, args...);
+}
 
 cudaError_t launch_prefill_mma(const PrefillParams& p, int D, cudaStream_t stream);
 

@@ -68,8 +68,7 @@ cudaError_t launch_tc5_t(const PrefillParams& pp, void* encode_fn, cudaStream_t 
     e = next_item_counter(&p.item_counter);
     if (e != cudaSuccess) return e;
   }
-  kern<<<grid, 640, smem, stream>>>(qmap, kmap, vmap, qmap, kmap, p);
-  return cudaGetLastError();
+  return launch_attention(pp.after_clear != 0, kern, grid.x, 640, smem, stream, qmap, kmap, vmap, qmap, kmap, p);
 }
 
 }  // namespace

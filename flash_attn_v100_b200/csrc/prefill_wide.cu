@@ -434,6 +434,7 @@ prefill_wide_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
     const int wq = warp & 3, row = wq * 32 + lane;
     const uint32_t tO = tmem + 256u + ((uint32_t)(wq * 32) << 16);
     uint32_t cnt = 0;
+    wait_for_clear();
     for (uint32_t ic = 0;; ++ic) {
       if (*abort_flag) break;
       const long long item = next_item(ic);
@@ -542,8 +543,8 @@ cudaError_t launch_prefill_wide(const PrefillParams& pp, int sm_count, void* enc
     e = next_item_counter(&p.item_counter);
     if (e != cudaSuccess) return e;
   }
-  prefill_wide_kernel<<<(unsigned)(n_items < sm_count ? n_items : sm_count), kWideThreads, kWideSmem, stream>>>(qmap, kmap, vmap, p);
-  return cudaGetLastError();
+  return launch_attention(pp.after_clear != 0, prefill_wide_kernel, (unsigned)(n_items < sm_count ? n_items : sm_count), kWideThreads, kWideSmem, stream, qmap, kmap,
+                          vmap, p);
 }
 
 }  // namespace fa

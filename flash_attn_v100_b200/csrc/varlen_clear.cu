@@ -10,13 +10,14 @@ constexpr int kThreads = 256, kRows = 1024, kAhead = 4;      // kRows: rows that
 // sequence.  A block has an equal share of the rows, marks which of them lie in a gap and clears those, a warp per row: one gap that is most
 // of the output, as a buffer padded to a fixed size has it, then keeps every SM writing.  (65536 rows of 32 heads of 128, 300 sequences of 4
 // tokens at their start: the packed prefill takes 290 us so, 340 over a fill of the whole output, and took 4400 with the blocks dealt out to the gaps, two
-// for each.)  Every gap is looked at, not searched for, so offsets in any order are served as they were by a fill; the attention is launched behind
-// this one, so where offsets overlap its rows win.  Usually all gaps are empty: 16 prompts of up to 4096 tokens, 32 heads of 128, took 1046 us with the
+// for each.)  Every gap is looked at, not searched for, so offsets in any order are served as they were by a fill; the attention waits for
+// this one before it stores, so where offsets overlap its rows win.  Usually all gaps are empty: 16 prompts of up to 4096 tokens, 32 heads of 128, took 1046 us with the
 // fill, 67 of them the fill, and the clear takes 3.
 __global__ void __launch_bounds__(kThreads)
 varlen_clear_kernel(uint4* out, const int32_t* cu, int batch, long long total, int max_seqlen, long long units, long long share) {
   __shared__ uint32_t in_gap[kRows / 32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the attention may be launched (see launch_attention)
   const long long first = (long long)blockIdx.x * share, end = first + share < total ? first + share : total;
   for (long long r0 = first; r0 < end; r0 += kRows) {
     const int n = (int)(end - r0 < kRows ? end - r0 : kRows);

@@ -661,12 +661,9 @@ def _varlen(q, k, v, cu_seqlens, max_seqlen, causal, stream_int=None, bf16_out=F
             ev = torch.cuda.Event()
             ev.record()
             torch.cuda.ExternalStream(stream_int, device=q.device).wait_event(ev)
-        if total > 0 and D % 8 == 0:      # (the attention refuses the rest)
-            # rows outside every sequence are zero, as in the reference (:3373)
-            _lib.check(lib.fa_prefill_varlen_clear(_ptr(out), _ptr(cu_seqlens), batch, total, max_seqlen, H_Q * D * 2, s))
-        entry = lib.fa_prefill_varlen_f16_out_bf16 if bf16_out else _entry(lib, "fa_prefill_varlen_f16")
-        _lib.check(entry(_ptr(q), _ptr(k), _ptr(v), _ptr(out), _ptr(cu_seqlens), batch, total,
-                         H_Q, H_KV, D, max_seqlen, 1 if causal else 0, s))
+        # rows outside every sequence are zero, as in the reference (:3373)
+        _lib.check(lib.fa_prefill_varlen_zeroed(_ptr(q), _ptr(k), _ptr(v), _ptr(out), _ptr(cu_seqlens), batch, total, H_Q, H_KV, D, max_seqlen,
+                                                1 if causal else 0, 1 if elem == torch.bfloat16 else 0, 1 if bf16_out else 0, s))
     return out
 
 

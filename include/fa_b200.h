@@ -273,6 +273,13 @@ int fa_prefill_varlen_f16(const void* q, const void* k, const void* v, void* out
  */
 int fa_prefill_varlen_clear(void* out, const int32_t* cu_seqlens, int batch, int64_t total,
                             int max_seqlen, int64_t row_bytes, void* stream);
+/*
+ * fa_prefill_varlen_clear and the attention in one call, the attention's launch beside the clear: every row of
+ * `out` is defined afterwards.  q, k, v fp16, or bfloat16 with in_bf16; out in their type, or bfloat16 with out_bf16.
+ */
+int fa_prefill_varlen_zeroed(const void* q, const void* k, const void* v, void* out,
+                             const int32_t* cu_seqlens, int batch, int64_t total, int H_Q, int H_KV, int D,
+                             int max_seqlen, int causal, int in_bf16, int out_bf16, void* stream);
 /* fa_prefill_varlen_f16 with the output stored as bfloat16 (see fa_paged_decode_gqa_f16_out_bf16). */
 int fa_prefill_varlen_f16_out_bf16(const void* q, const void* k, const void* v, void* out,
                           const int32_t* cu_seqlens, int batch, int64_t total,
