@@ -1,5 +1,6 @@
 // Attention over the cached latent rows (see latent_attention.cu, latent_decode.cu).
 #pragma once
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -37,8 +38,13 @@ template <typename T> cudaError_t launch_latent_attention(const LatentAttentionA
 
 // Tensor cores (bfloat16; kv_rank + rot_dim <= 576, both multiples of 8).
 bool latent_decode_supported(const LatentAttentionArgs& a);
-int latent_decode_ctas(int heads, int sm_count);   // per head block
+int latent_decode_ctas(int heads, int kv_rank, int rot_dim, int sm_count);   // per head block
 cudaError_t launch_latent_decode(const LatentAttentionArgs& a, void* encode_fn, cudaStream_t s);   // cuTensorMapEncodeTiled
+
+// The kernel of latents of 128 to 512 columns in blocks of 128, with rotated parts of 16 to 64 columns (latent_decode_tc5.cu).
+bool latent_decode_tc5_supported(int kv_rank, int rot_dim);
+int latent_decode_tc5_ctas(int heads, int kv_rank, int sm_count);
+cudaError_t launch_latent_decode_tc5(const LatentAttentionArgs& a, const CUtensorMap& pool_map, cudaStream_t s);
 
 }  // namespace hybrid
 }  // namespace fa

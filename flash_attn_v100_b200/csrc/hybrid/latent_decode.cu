@@ -1,5 +1,5 @@
 // Attention in the latent space on the tensor cores (mma.sync, bfloat16 operands, fp32 scores, weights' sums and
-// accumulators), sm_100a: decode steps and short portions of prompts.
+// accumulators), sm_100a: decode steps and short portions of prompts, of the sizes that latent_decode_tc5.cu does not serve.
 //
 // All heads read the same cached rows, so a key tile (64 tokens) is fetched once and serves every head of the block (16 or
 // 32, the M rows of the MMAs) as key and as value.  The (row, key tile) units of the batch are numbered row by row and cut
@@ -16,6 +16,7 @@
 #include "../smem_limit.cuh"
 #include "hybrid_common.cuh"
 #include "latent_attention.cuh"
+#include "latent_run.cuh"
 
 namespace fa {
 namespace hybrid {
@@ -25,7 +26,6 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
                                   CUtensorMapFloatOOBfill);
 
-constexpr int KT = 64;         // keys per tile
 constexpr int kCompute = 512;  // threads that compute
 constexpr int kThreads = kCompute + 32;
 constexpr int kWarps = kThreads / 32;
@@ -40,27 +40,6 @@ __device__ __forceinline__ uint32_t key_off(int key, int u) {
 template <int UNITS>
 __device__ __forceinline__ uint32_t q_off(int row, int u) {
   return (uint32_t)((row * UNITS + ((u & ~7) | ((u ^ row) & 7))) * 16);
-}
-
-__device__ __forceinline__ int row_tiles_of(const LatentAttentionArgs& a, long long row) {
-  const int n = a.positions[row] + 1;
-  return n > 0 ? (n + KT - 1) / KT : 1;
-}
-
-// Inclusive scan over the block of one int per thread; `buf` holds one int per warp.
-__device__ __forceinline__ int block_scan(int v, int* buf) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int t = __shfl_up_sync(0xffffffffu, v, o);
-    if (lane >= o) v += t;
-  }
-  if (lane == 31) buf[warp] = v;
-  __syncthreads();
-  int add = 0;
-  for (int i = 0; i < warp; ++i) add += buf[i];
-  __syncthreads();
-  return v + add;
 }
 
 // KS: slabs of 64 columns = 16-column steps per warp quarter (4 * 16 * KS >= kv_rank + rot_dim); MB: 16-head blocks.
@@ -90,36 +69,8 @@ __global__ void __launch_bounds__(kThreads, 1) latent_decode_kernel(const __grid
   const int R = a.kv_rank, D = R + a.rot_dim;
 
   // ---- my run of units --------------------------------------------------------------------------
-  int total = 0, mine = 0, upto = 0;               // of my row in the last block of rows: its tiles, tiles up to and with it
-  for (long long r0 = 0; r0 < a.rows; r0 += kThreads) {
-    mine = r0 + tid < a.rows ? row_tiles_of(a, r0 + tid) : 0;
-    upto = total + block_scan(mine, scan_buf);
-    if (cta == 0 && blockIdx.y == 0 && r0 + tid < a.rows) a.row_tiles[r0 + tid + 1] = upto;
-    if (tid == kThreads - 1) found[0] = upto;
-    __syncthreads();
-    total = found[0];
-    __syncthreads();
-  }
-  if (cta == 0 && blockIdx.y == 0 && tid == 0) a.row_tiles[0] = 0;
-  const int per = (total + a.n_cta - 1) / a.n_cta;
-  const int u0 = cta * per, u1 = min(u0 + per, total);
-  if (u0 >= u1) return;
-  if (a.rows <= kThreads) {
-    if (mine > 0 && upto - mine <= u0 && u0 < upto) { found[0] = tid; found[1] = upto - mine; }
-    __syncthreads();
-  } else {
-    int base = 0;
-    for (long long r0 = 0; r0 < a.rows; r0 += kThreads) {
-      const int v = r0 + tid < a.rows ? row_tiles_of(a, r0 + tid) : 0;
-      const int inc = base + block_scan(v, scan_buf);
-      if (v > 0 && inc - v <= u0 && u0 < inc) { found[0] = (int)(r0 + tid); found[1] = inc - v; }
-      if (tid == kThreads - 1) scan_buf[0] = inc;
-      __syncthreads();
-      base = scan_buf[0];
-      __syncthreads();
-      if (base > u0) break;
-    }
-  }
+  int u0, u1;
+  if (!find_run<kThreads>(a, scan_buf, found, u0, u1)) return;
   const int first_row = found[0];
   if (tid == 0) {
     mbar_init(bars, 4 * KS);                        // one arrival per box
@@ -131,12 +82,6 @@ __global__ void __launch_bounds__(kThreads, 1) latent_decode_kernel(const __grid
     tma_prefetch_desc(&pool_map);
   }
   __syncthreads();
-  struct Cursor { int row, tile, tiles, n; };
-  auto start_row = [&](Cursor& c, int row) { c.row = row; c.tile = 0; c.n = a.positions[row] + 1; c.tiles = c.n > 0 ? (c.n + KT - 1) / KT : 1; };
-  auto advance = [&](Cursor& c) {
-    if (++c.tile == c.tiles && c.row + 1 < a.rows) start_row(c, c.row + 1);
-  };
-
   bool late = false;
   auto wait = [&](uint32_t bar, uint32_t parity) {
     if (!late) late = !mbar_wait(bar, parity);
@@ -146,16 +91,9 @@ __global__ void __launch_bounds__(kThreads, 1) latent_decode_kernel(const __grid
     // ---- copies: lane l fetches boxes l and l + 32 of every tile ------------------------------------
     constexpr int NB = (4 * KS + 31) / 32;
     bool bad = false;
-    // page of the cursor's tile that a box comes from, checked when it is used; keys past the end: the tile's first page (any
-    // finite rows will do, their weights are zero)
-    auto box_page = [&](const Cursor& c, int box) {
-      const int seq = a.tok_seq[c.row];
-      int blk = c.tile * (KT / 16) + box / KS;
-      if (blk * 16 >= c.n) blk = c.tile * (KT / 16);
-      return seq >= 0 && seq < a.n_seq && c.n > 0 && blk < a.max_blocks ? a.block_table[(long long)seq * a.max_blocks + blk] : -1;
-    };
+    auto box_page = [&](const Cursor& c, int box) { return page_of(a, c, box / KS); };   // (checked when it is used)
     Cursor nxt;
-    start_row(nxt, first_row);
+    start_row(a, nxt, first_row);
     nxt.tile = u0 - found[1];
     int page[NB];
 #pragma unroll
@@ -175,7 +113,7 @@ __global__ void __launch_bounds__(kThreads, 1) latent_decode_kernel(const __grid
         }
       }
       if (u + 1 < u1) {
-        advance(nxt);
+        advance(a, nxt);
 #pragma unroll
         for (int i = 0; i < NB; ++i)
           if (lane + 32 * i < 4 * KS) page[i] = box_page(nxt, lane + 32 * i);
@@ -232,7 +170,7 @@ __global__ void __launch_bounds__(kThreads, 1) latent_decode_kernel(const __grid
   const float sc = a.scale * 1.4426950408889634f;
 
   Cursor cur;
-  start_row(cur, first_row);
+  start_row(a, cur, first_row);
   cur.tile = u0 - found[1];
   int piece_tile0 = cur.tile;
   load_q(cur.row);
@@ -383,7 +321,7 @@ __global__ void __launch_bounds__(kThreads, 1) latent_decode_kernel(const __grid
         piece_tile0 = 0;
       }
     }
-    if (u + 1 < u1) advance(cur);
+    if (u + 1 < u1) advance(a, cur);
   }
   if (late && lane == 0) atomicOr(a.status, kStatusWaitTimeout);
 }
@@ -442,13 +380,15 @@ cudaError_t launch_t(const LatentAttentionArgs& a, const CUtensorMap& map, cudaS
   cudaError_t e = limit.raise(reinterpret_cast<const void*>(latent_decode_kernel<KS, MB>), smem);
   if (e != cudaSuccess) return e;
   latent_decode_kernel<KS, MB><<<dim3((unsigned)a.n_cta, (unsigned)((a.heads + M - 1) / M)), kThreads, smem, s>>>(map, a);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  // Launched while the decode still runs (its blocks take the places that finished ones leave) and held at its first instruction until
-  // all of the decode's writes are there: 0.5 to 1 us of launch latency less.  Not beside the decode of the widest rows, whose shared memory leaves little of the SM's
-  // memory as L1, where few rows are cut into many pieces, so that the merge is long: it then reads the pieces more slowly than one that
-  // starts on free SMs.  32 heads of 512 + 64, early (behind the decode): 1 row of 8192 cached tokens 32.1 us (27.0), 2 of 4096 1.15 times, 8 of
-  // 4096 1.02, 12 of 1000 1.04 times; from 16 rows on 0.96 to 1.00 times.  256 + 32, any rows: 0.85 to 1.05 times, 0.96 on average.
+  return cudaGetLastError();
+}
+
+// Launched while the decode still runs (its blocks take the places that finished ones leave) and held at its first instruction until
+// all of the decode's writes are there: 0.5 to 1 us of launch latency less.  Not beside the decode of the widest rows, whose shared memory leaves little of the SM's
+// memory as L1, where few rows are cut into many pieces, so that the merge is long: it then reads the pieces more slowly than one that
+// starts on free SMs.  32 heads of 512 + 64, early (behind the decode): 1 row of 8192 cached tokens 32.1 us (27.0), 2 of 4096 1.15 times, 8 of
+// 4096 1.02, 12 of 1000 1.04 times; from 16 rows on 0.96 to 1.00 times.  256 + 32, any rows: 0.85 to 1.05 times, 0.96 on average.
+cudaError_t launch_merge(const LatentAttentionArgs& a, cudaStream_t s) {
   cudaLaunchAttribute early;
   early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   early.val.programmaticStreamSerializationAllowed = 1;
@@ -458,7 +398,7 @@ cudaError_t launch_t(const LatentAttentionArgs& a, const CUtensorMap& map, cudaS
   cfg.dynamicSmemBytes = a.n_cta * sizeof(float);
   cfg.stream = s;
   cfg.attrs = &early;
-  cfg.numAttrs = KS < 9 || a.rows >= 16 ? 1 : 0;
+  cfg.numAttrs = a.kv_rank + a.rot_dim <= 320 || a.rows >= 16 ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, latent_decode_merge_kernel, a);
 }
 
@@ -472,7 +412,8 @@ bool latent_decode_supported(const LatentAttentionArgs& a) {
          (reinterpret_cast<uintptr_t>(a.out) & 15) == 0;
 }
 
-int latent_decode_ctas(int heads, int sm_count) {
+int latent_decode_ctas(int heads, int kv_rank, int rot_dim, int sm_count) {
+  if (latent_decode_tc5_supported(kv_rank, rot_dim)) return latent_decode_tc5_ctas(heads, kv_rank, sm_count);
   const int blocks = heads <= 16 ? 1 : (heads + 31) / 32;
   const int n = sm_count / blocks;
   return n > 0 ? n : 1;
@@ -488,17 +429,12 @@ cudaError_t launch_latent_decode(const LatentAttentionArgs& a, void* encode_fn, 
                                                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                                                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return cudaErrorInvalidValue;
+  cudaError_t e;
   const int ks = ks_of(a.kv_rank + a.rot_dim);
-  if (a.heads <= 16) {
-    if (ks == 2) return launch_t<2, 1>(a, map, s);
-    if (ks == 3) return launch_t<3, 1>(a, map, s);
-    if (ks == 5) return launch_t<5, 1>(a, map, s);
-    return launch_t<9, 1>(a, map, s);
-  }
-  if (ks == 2) return launch_t<2, 2>(a, map, s);
-  if (ks == 3) return launch_t<3, 2>(a, map, s);
-  if (ks == 5) return launch_t<5, 2>(a, map, s);
-  return launch_t<9, 2>(a, map, s);
+  if (latent_decode_tc5_supported(a.kv_rank, a.rot_dim)) e = launch_latent_decode_tc5(a, map, s);
+  else if (a.heads <= 16) e = ks == 2 ? launch_t<2, 1>(a, map, s) : (ks == 3 ? launch_t<3, 1>(a, map, s) : (ks == 5 ? launch_t<5, 1>(a, map, s) : launch_t<9, 1>(a, map, s)));
+  else e = ks == 2 ? launch_t<2, 2>(a, map, s) : (ks == 3 ? launch_t<3, 2>(a, map, s) : (ks == 5 ? launch_t<5, 2>(a, map, s) : launch_t<9, 2>(a, map, s)));
+  return e == cudaSuccess ? launch_merge(a, s) : e;
 }
 
 }  // namespace hybrid
