@@ -114,7 +114,7 @@ int fah_latent_attention(const void* q_abs, const void* q, int q_stride, int q_o
     a.row_tiles = reinterpret_cast<int32_t*>(a.part_ml + (int64_t)a.n_cta * 2 * heads * 2);
     void* enc = tensor_map_encode();
     if (enc == nullptr) return fail(FAH_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
-    return done(fa::hybrid::launch_latent_decode(a, enc, st(stream)), "latent_decode");
+    return done(fa::hybrid::launch_latent_decode(a, sm_count(), enc, st(stream)), "latent_decode");
   }
   return done(FAH_DISPATCH(dtype, fa::hybrid::launch_latent_attention, a, st(stream)), "latent_attention");
 }

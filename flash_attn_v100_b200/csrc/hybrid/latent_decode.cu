@@ -326,11 +326,14 @@ __global__ void __launch_bounds__(kThreads, 1) latent_decode_kernel(const __grid
   if (late && lane == 0) atomicOr(a.status, kStatusWaitTimeout);
 }
 
-// Rows that several CTAs worked on: log-sum-exp merge of their partial sums.  One CTA per (row, head).
+// Rows that several CTAs worked on: log-sum-exp merge of their partial sums.  One CTA per (row, head), or (SPLIT) per (row, head, 128 columns) with
+// a quarter of the pieces per warp: few rows are cut into many pieces, whose sums one after the other were most of the time.
 constexpr int kMergeThreads = 128;
+template <bool SPLIT>
 __global__ void __launch_bounds__(kMergeThreads) latent_decode_merge_kernel(const LatentAttentionArgs a) {
   extern __shared__ float weight[];                 // [pieces of the row] (n_cta at most)
   __shared__ float red[2 * kMergeThreads / 32];
+  __shared__ float4 parts[SPLIT ? kMergeThreads : 1];
   const long long row = blockIdx.x;
   const int head = blockIdx.y, tid = threadIdx.x;
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -356,6 +359,32 @@ __global__ void __launch_bounds__(kMergeThreads) latent_decode_merge_kernel(cons
   float f = l > 0.f ? 1.f / l : 0.f;
   if (a.gate != nullptr) f *= sigmoid_f(to_f(static_cast<const bf16*>(a.gate)[row * a.gate_stride + head]));
   bf16* out = static_cast<bf16*>(a.out) + (row * a.heads + head) * a.kv_rank;
+  if constexpr (SPLIT) {
+    const int warp = tid >> 5, i = blockIdx.z * 128 + (tid & 31) * 4;
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    if (i < a.kv_rank) {
+#pragma unroll 8
+      for (int c = warp; c < n; c += kMergeThreads / 32) {
+        float v[4];
+        load_n<4>(a.part_o + piece(c) * a.kv_rank + i, v);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[j] += weight[c] * v[j];
+      }
+    }
+    parts[tid] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    __syncthreads();
+    if (warp == 0 && i < a.kv_rank) {
+#pragma unroll
+      for (int w = 1; w < kMergeThreads / 32; ++w) {
+        const float4 v = parts[w * 32 + tid];
+        acc[0] += v.x; acc[1] += v.y; acc[2] += v.z; acc[3] += v.w;
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[j] *= f;
+      store_n<4>(out + i, acc);
+    }
+    return;
+  }
   for (int i = tid * 4; i < a.kv_rank; i += kMergeThreads * 4) {
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 8
@@ -388,18 +417,21 @@ cudaError_t launch_t(const LatentAttentionArgs& a, const CUtensorMap& map, cudaS
 // memory as L1, where few rows are cut into many pieces, so that the merge is long: it then reads the pieces more slowly than one that
 // starts on free SMs.  32 heads of 512 + 64, early (behind the decode): 1 row of 8192 cached tokens 32.1 us (27.0), 2 of 4096 1.15 times, 8 of
 // 4096 1.02, 12 of 1000 1.04 times; from 16 rows on 0.96 to 1.00 times.  256 + 32, any rows: 0.85 to 1.05 times, 0.96 on average.
-cudaError_t launch_merge(const LatentAttentionArgs& a, cudaStream_t s) {
+cudaError_t launch_merge(const LatentAttentionArgs& a, int sm_count, cudaStream_t s) {
   cudaLaunchAttribute early;
   early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   early.val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)a.rows, (unsigned)a.heads);
+  // From three blocks of a whole row and head per SM on these are enough.  32 heads of 512 + 64, split (whole): 1 row of up to 8192 cached tokens 26.5 us
+  // (35.8), 8 of 4096 28.6 (30.7), 12 of 1000 24.5 (24.5); 9 rows of 1000, 130 heads 36.8 (32.7).
+  const bool split = a.rows * a.heads < 3ll * sm_count;
+  cfg.gridDim = dim3((unsigned)a.rows, (unsigned)a.heads, split ? (unsigned)((a.kv_rank + 127) / 128) : 1u);
   cfg.blockDim = dim3(kMergeThreads);
   cfg.dynamicSmemBytes = a.n_cta * sizeof(float);
   cfg.stream = s;
   cfg.attrs = &early;
   cfg.numAttrs = a.kv_rank + a.rot_dim <= 320 || a.rows >= 16 ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, latent_decode_merge_kernel, a);
+  return split ? cudaLaunchKernelEx(&cfg, latent_decode_merge_kernel<true>, a) : cudaLaunchKernelEx(&cfg, latent_decode_merge_kernel<false>, a);
 }
 
 int ks_of(int D) { return D <= 128 ? 2 : (D <= 192 ? 3 : (D <= 320 ? 5 : 9)); }
@@ -419,7 +451,7 @@ int latent_decode_ctas(int heads, int kv_rank, int rot_dim, int sm_count) {
   return n > 0 ? n : 1;
 }
 
-cudaError_t launch_latent_decode(const LatentAttentionArgs& a, void* encode_fn, cudaStream_t s) {
+cudaError_t launch_latent_decode(const LatentAttentionArgs& a, int sm_count, void* encode_fn, cudaStream_t s) {
   if (a.rows == 0) return cudaSuccess;
   CUtensorMap map;
   const cuuint64_t dims[2] = {(cuuint64_t)a.pool_stride, (cuuint64_t)a.n_blocks * 16};
@@ -434,7 +466,7 @@ cudaError_t launch_latent_decode(const LatentAttentionArgs& a, void* encode_fn, 
   if (latent_decode_tc5_supported(a.kv_rank, a.rot_dim)) e = launch_latent_decode_tc5(a, map, s);
   else if (a.heads <= 16) e = ks == 2 ? launch_t<2, 1>(a, map, s) : (ks == 3 ? launch_t<3, 1>(a, map, s) : (ks == 5 ? launch_t<5, 1>(a, map, s) : launch_t<9, 1>(a, map, s)));
   else e = ks == 2 ? launch_t<2, 2>(a, map, s) : (ks == 3 ? launch_t<3, 2>(a, map, s) : (ks == 5 ? launch_t<5, 2>(a, map, s) : launch_t<9, 2>(a, map, s)));
-  return e == cudaSuccess ? launch_merge(a, s) : e;
+  return e == cudaSuccess ? launch_merge(a, sm_count, s) : e;
 }
 
 }  // namespace hybrid
