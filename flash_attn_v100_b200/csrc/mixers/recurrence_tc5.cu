@@ -8,18 +8,27 @@
 //     S  <- e^(L_C) S + dS                 S stays in the threads' registers, fp32
 // Decays and weights act on rows of V' and P and on columns of S only, never on Q and K: the 128 value columns of a CTA can
 // belong to two heads with the same queries and keys (NH = 2, heads of up to 64 value columns), which share A.
-// The normaliser (NORM): n stays in shared memory, fp32; n_i . q_i = e^(L_i) (n . q_i) + sum_j P_ij from the P in registers.
+// The normaliser (NORM), n <- e^(L_C) n + sum_j w_j k_j with the weights w of V', is a column beside the state's: n_i . q_i = e^(L_i) (n . q_i) +
+// sum_j P_ij, the second sum from the P in registers. n and w enter their products as three bfloat16 parts each, which hold all 24 bits, in columns 0-2
+// and 16-18 of a tile of their own (two products of N = 32); n stays in registers, fp32.  (As sums in the threads, which read Q and K from shared
+// memory once more, they took 2950 cycles of a chunk.)
 //
-// CTA = (segment of a sequence, head or pair of heads, 128 value columns), sixteen warps, all of them with the same role: a warp
-// owns 32 lanes (rows) x 32 columns of whatever is in tensor memory; warp 0 issues the MMAs.  Segments let few long sequences
-// fill the GPU: a first launch computes what every segment adds to the state, a scan over the segments turns that into the state
-// at the start of each, and the main launch then runs all segments side by side.
+// CTA = (segment of a sequence, head or pair of heads, 128 value columns), eighteen warps.  Sixteen compute: a warp owns 32 lanes (rows) x 32 columns of
+// whatever is in tensor memory.  One issues the MMAs and one the copies, and works out the gates of the next chunk.  They meet at mbarriers, the four warps
+// that share rows at named ones: with the MMAs issued by one of the computing warps and all of them at block barriers, everybody waited for that warp at
+// every hand-over, since an issue blocks while the tensor queue is full.  16 x 1024 tokens, 32 heads of 128, with the normaliser's sums moved to the MMAs
+// and Q K^T of the next chunk issued behind the state's product: 235 -> 209 us for gates and recurrence; 8700 cycles per chunk where it took 11 700. What
+// bounds it now: the chain S -> tiles -> V' -> state of a chunk, its shared-memory traffic (a third of the cycles), and 6 of the 43 us of a CTA
+// before its first and behind its last chunk.
+// Segments let few long sequences fill the GPU: a first launch computes what every segment adds to the state, a scan over the segments turns that into
+// the state at the start of each, and the main launch then runs all segments side by side.
 //
-// Tensor memory, 512 columns: A / P of the first head [0, 128)  O1 [128, 256)  O2 [256, 384)  P of the second head / dS [384, 512).
+// Tensor memory, 512 columns: A / P of the first head [0, 128)  O1 [128, 256)  O2 [256, 384), before P V the normaliser's products  P of the second head / dS
+// [384, 512).
 // Shared memory: six tiles of 128 x 128 bfloat16, each two 128-byte-swizzled slabs of 64 columns: Q, K twice, V, and S high and low,
 // whose place V' takes once O1 is done.  Q, K and V come by TMA (the next K while this chunk is computed, the next Q once O1 is done,
 // the next V once the output, which takes V's place, has been stored, also by TMA).  Rows past a sequence's end have the weight 0.
-// Waits are bounded: one that runs out sets the status word and the CTA leaves after another bounded wait for its MMAs and copies.
+// Waits are bounded: one that runs out sets the status word, and every role runs on to its end without waiting.
 #include "../hybrid/hybrid_common.cuh"
 #include "../tc5.cuh"
 #include "../tma3.cuh"
@@ -34,7 +43,8 @@ namespace {
 
 constexpr int C = 128;         // tokens per chunk
 constexpr int N = 128;         // key and value columns per CTA (padded with zeros)
-constexpr int kThreads = 512;
+constexpr int kCompute = 512;  // threads that compute
+constexpr int kThreads = kCompute + 64;
 constexpr int SLAB = 128 * 128;
 constexpr int TILE = 2 * SLAB;
 constexpr float kLog2e = 1.4426950408889634f;
@@ -43,15 +53,17 @@ struct Small {                 // behind the tiles
   float2 lb[2][2][C];          // [buffer][head]: running log2 decay and weight of every token
   float wk[2][2][C];           // weight of every token in the state after the chunk
   float dec[2][2];             // log2 decay over the chunk
-  float n[N];                  // normaliser
-  float n_add[kThreads / 32][N];
   float den[4][C];             // partial n . q of every row, by column group
-  uint64_t bars[8];
+  uint64_t bars[16];
   uint32_t tmem_slot;
+  volatile int gave_up;
 };
+// Barriers: a copy has landed; MMAs are done; the computing warps have written (or, the last, may be read) what the name says; gates are there.
+enum Bar { kFullQ, kFullV, kFullK, kScores = kFullK + 2, kOld, kNew, kState, kStateIn, kWeights, kValues, kOut, kGates, kDrain = kGates + 2, kBars };
+static_assert(kBars <= 16, "barriers");
 constexpr int kTiles = 6;
-constexpr int kSmem = 1024 + kTiles * TILE + (int)sizeof(Small);
-static_assert(kSmem <= 227 * 1024, "shared memory plan exceeds the SM");
+constexpr int smem_bytes(bool norm) { return 1024 + kTiles * TILE + (norm ? SLAB : 0) + (int)sizeof(Small); }
+static_assert(smem_bytes(true) <= 227 * 1024, "shared memory plan exceeds the SM");
 
 // Byte offset of 16-byte unit `u` (0..15) of row `row` in a tile.
 __device__ __forceinline__ uint32_t tile_off(int row, int u) {
@@ -74,6 +86,11 @@ __device__ __forceinline__ void split2(float2 v, uint32_t& hi, uint32_t& lo) {
   const float2 r = ffma2(unpack2(hi), make_float2(-1.f, -1.f), v);
   lo = pack_bf162(r.x, r.y);
 }
+// One fp32 number as the sum of three bfloat16 numbers, the first three of a unit.
+__device__ __forceinline__ uint4 split3(float v) {
+  const float hi = __bfloat162float(__float2bfloat16_rn(v)), mid = __bfloat162float(__float2bfloat16_rn(v - hi));
+  return make_uint4(pack_bf162(hi, mid), pack_bf162((v - hi) - mid, 0.f), 0u, 0u);
+}
 
 template <bool STATE_ONLY, int NH, bool NORM>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -85,13 +102,13 @@ recurrence_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
   constexpr uint32_t N128 = (uint32_t)(N >> 3) << 17, NPV = (uint32_t)((N / NH) >> 3) << 17;
   constexpr uint32_t IDESC_QK = IDESC | N128, IDESC_B = IDESC | N128 | (1u << 16), IDESC_PV = IDESC | NPV | (1u << 16),
                      IDESC_AB = IDESC | N128 | (1u << 15) | (1u << 16);
+  constexpr uint32_t N32 = (uint32_t)(32 >> 3) << 17, IDESC_B32 = IDESC | N32 | (1u << 16), IDESC_AB32 = IDESC | N32 | (1u << 15) | (1u << 16);
   extern __shared__ uint8_t smem_dyn[];
   const uint32_t raw_base = smem_u32(smem_dyn);
   uint8_t* smem = smem_dyn + ((1024u - (raw_base & 1023u)) & 1023u);
-  const uint32_t sQ = smem_u32(smem), sK0 = sQ + TILE, sV = sK0 + 2 * TILE, sSh = sV + TILE, sSl = sSh + TILE;
-  Small& sm = *reinterpret_cast<Small*>(smem + kTiles * TILE);
+  const uint32_t sQ = smem_u32(smem), sK0 = sQ + TILE, sV = sK0 + 2 * TILE, sSh = sV + TILE, sSl = sSh + TILE, sE = sSl + TILE;
+  Small& sm = *reinterpret_cast<Small*>(smem + kTiles * TILE + (NORM ? SLAB : 0));
   auto bar = [&](int i) { return smem_u32(&sm.bars[i]); };
-  const uint32_t bar_a = bar(0), bar_1 = bar(1), bar_o = bar(2), bar_s = bar(3), full_q = bar(4), full_v = bar(5), full_k = bar(6);   // full_k: two
 
   const int seq = blockIdx.x / a.max_segs, seg = blockIdx.x - seq * a.max_segs;
   const int head0 = blockIdx.y * NH, c0 = blockIdx.z * N, grp = head0 / a.kv_rep;
@@ -115,85 +132,91 @@ recurrence_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
   const bool segmented = a.max_segs > 1;
   const long long seg_at = ((long long)seq * a.max_segs + seg) * a.heads;      // + head
 
-  // ---- copies: one thread issues them all ------------------------------------------------------------
-  const bool copier = tid == kThreads - 32;
+  // ---- roles: the first sixteen warps compute, then one issues the MMAs and one the copies (and works out the gates) ----------
   const bool wide_k = a.dk > 64, wide_v = NH == 2 || a.dv - c0 > 64;           // the tile's second slab has columns
+  const bool mma_warp = warp == kCompute / 32, copy_warp = warp == kCompute / 32 + 1;
   auto load_tile = [&](const CUtensorMap* map, uint32_t dst, uint32_t full, bool wide, int col, int head, int col2, int head2, long long t) {
     mbar_expect_tx(full, wide ? TILE : SLAB);
     tma_load_3d(dst, map, col, head, (int)t, full);
     if (wide) tma_load_3d(dst + SLAB, map, col2, head2, (int)t, full);
   };
-  auto load_q = [&](int chunk) { load_tile(&qmap, sQ, full_q, wide_k, 0, grp, 64, grp, t0 + (long long)chunk * C); };
+  auto load_q = [&](int chunk) { load_tile(&qmap, sQ, bar(kFullQ), wide_k, 0, grp, 64, grp, t0 + (long long)chunk * C); };
   auto load_k = [&](int chunk) {
-    load_tile(&kmap, sK0 + (chunk & 1) * TILE, full_k + (chunk & 1) * 8, wide_k, 0, grp, 64, grp, t0 + (long long)chunk * C);
+    load_tile(&kmap, sK0 + (chunk & 1) * TILE, bar(kFullK + (chunk & 1)), wide_k, 0, grp, 64, grp, t0 + (long long)chunk * C);
   };
   auto load_v = [&](int chunk) {
-    if (NH == 2) load_tile(&vmap, sV, full_v, true, 0, head0, 0, head0 + 1, t0 + (long long)chunk * C);
-    else load_tile(&vmap, sV, full_v, wide_v, c0, head0, c0 + 64, head0, t0 + (long long)chunk * C);
+    if (NH == 2) load_tile(&vmap, sV, bar(kFullV), true, 0, head0, 0, head0 + 1, t0 + (long long)chunk * C);
+    else load_tile(&vmap, sV, bar(kFullV), wide_v, c0, head0, c0 + 64, head0, t0 + (long long)chunk * C);
   };
-  int n_q = 0, n_k = 0, n_v = 0;                   // (copier) loads issued
-  if (copier) {
-    for (int i = 0; i < 8; ++i) mbar_init(bar(i), 1);
+  if (copy_warp && lane == 0) {
+    for (int i = 0; i < kBars; ++i) mbar_init(bar(i), i >= kStateIn && i < kStateIn + 4 ? kCompute / 32 : 1);
+    sm.gave_up = 0;
     mbar_fence_init();
     fence_proxy_async();
-    if (!STATE_ONLY) { load_q(0); ++n_q; }
-    load_k(0); ++n_k;
-    load_v(0); ++n_v;
+    if (!STATE_ONLY) load_q(0);
+    load_k(0);
+    load_v(0);
   }
-  if (warp == 0) {
+  if (mma_warp) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sm.tmem_slot)), "r"(512u) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
 
-  // ---- decays: warp h < NH turns the chunk's la and b of head h into sums, four tokens per lane -----
-  float gl[4], gb[4];
+  // ---- decays: la and b of a chunk turned into sums, four tokens per lane -----
+  float gl[NH][4], gb[NH][4];
   auto fetch_gates = [&](int chunk) {
-    const long long tb = t0 + (long long)chunk * C + lane * 4, at = (long long)(head0 + warp) * a.total + tb;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const bool in = tb + i < t1;
-      gl[i] = in ? a.la[at + i] : 0.f;
-      gb[i] = in ? a.b[at + i] : 0.f;
+    for (int h = 0; h < NH; ++h) {
+      const long long tb = t0 + (long long)chunk * C + lane * 4, at = (long long)(head0 + h) * a.total + tb;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const bool in = tb + i < t1;
+        gl[h][i] = in ? a.la[at + i] : 0.f;
+        gb[h][i] = in ? a.b[at + i] : 0.f;
+      }
     }
   };
   auto put_gates = [&](int buf) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) gl[i] *= kLog2e;
-    float up = gl[0] + gl[1] + gl[2] + gl[3], down = up;       // sums up to my last token, and from my first token on
+    for (int h = 0; h < NH; ++h) {
+      float* g = gl[h];
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const float u = __shfl_up_sync(0xffffffffu, up, o), d = __shfl_down_sync(0xffffffffu, down, o);
-      if (lane >= o) up += u;
-      if (lane + o < 32) down += d;
-    }
-    if (lane == 31) sm.dec[buf][warp] = up;
-    float before = __shfl_up_sync(0xffffffffu, up, 1), after = __shfl_down_sync(0xffffffffu, down, 1);
-    if (lane == 0) before = 0.f;
-    if (lane == 31) after = 0.f;
+      for (int i = 0; i < 4; ++i) g[i] *= kLog2e;
+      float up = g[0] + g[1] + g[2] + g[3], down = up;         // sums up to my last token, and from my first token on
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      before += gl[i];
-      sm.lb[buf][warp][lane * 4 + i] = make_float2(before, gb[i]);
-    }
+      for (int o = 1; o < 32; o <<= 1) {
+        const float u = __shfl_up_sync(0xffffffffu, up, o), d = __shfl_down_sync(0xffffffffu, down, o);
+        if (lane >= o) up += u;
+        if (lane + o < 32) down += d;
+      }
+      if (lane == 31) sm.dec[buf][h] = up;
+      float before = __shfl_up_sync(0xffffffffu, up, 1), after = __shfl_down_sync(0xffffffffu, down, 1);
+      if (lane == 0) before = 0.f;
+      if (lane == 31) after = 0.f;
 #pragma unroll
-    for (int i = 3; i >= 0; --i) {                              // (summed from the end: the tokens that matter have small sums)
-      sm.wk[buf][warp][lane * 4 + i] = fast_exp2(after) * gb[i];
-      after += gl[i];
+      for (int i = 0; i < 4; ++i) {
+        before += g[i];
+        sm.lb[buf][h][lane * 4 + i] = make_float2(before, gb[h][i]);
+      }
+#pragma unroll
+      for (int i = 3; i >= 0; --i) {                            // (summed from the end: the tokens that matter have small sums)
+        sm.wk[buf][h][lane * 4 + i] = fast_exp2(after) * gb[h][i];
+        after += g[i];
+      }
     }
   };
-  if (warp < NH) {
+  if (copy_warp) {
     fetch_gates(0);
     put_gates(0);
+    if (n_chunk > 1) fetch_gates(1);
   }
-  if (NORM && tid < N) {
-    float v = 0.f;
-    if (!STATE_ONLY && tid < a.dk)
-      v = segmented ? a.seg_norm[(seg_at + head0) * a.dk + tid] : a.n0[((long long)seq * a.heads + head0) * a.dk + tid];
-    sm.n[tid] = v;
+  if (NORM && tid < kCompute) {                                // the columns that are never written
+    for (int i = tid; i < SLAB / 16; i += kCompute) st_shared(sE + i * 16, make_uint4(0, 0, 0, 0));
+    fence_proxy_async();
   }
-  if (!wide_k || !wide_v) {                                    // slabs that no copy fills
+  if ((!wide_k || !wide_v) && tid < kCompute) {                // slabs that no copy fills
     const uint4 z = make_uint4(0, 0, 0, 0);
-    for (int i = tid; i < SLAB / 16; i += kThreads) {
+    for (int i = tid; i < SLAB / 16; i += kCompute) {
       if (!wide_k) {
         st_shared(sQ + SLAB + i * 16, z);
         st_shared(sK0 + SLAB + i * 16, z);
@@ -208,228 +231,50 @@ recurrence_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
   tc_fence_after();
   const uint32_t tmem = sm.tmem_slot;
 
-  // my place in tensor memory: lane (row) and 32 columns
-  const int row = (warp & 3) * 32 + lane, cg = warp >> 2;
-  const uint32_t tl = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)cg * 32u;
-  const uint32_t tA = tl, tO1 = tl + 128u, tO2 = tl + 256u, tS = tl + 384u;
-  const uint32_t tP = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)cg * 16u;     // high part; low part 64 columns on
-  // ... and what the columns are: a head and its columns from mc on
-  const int mh = NH == 2 ? cg >> 1 : 0, mc = NH == 2 ? (cg & 1) * 32 : c0 + cg * 32;
-
-  // ---- state: row `row`, my columns ----------------------------------------------------------------
-  float* cache = slot_ok ? a.state + ((long long)slot * a.heads + head0 + mh) * hs + (long long)row * a.dv : nullptr;
-  float* segst = segmented ? a.seg_state + (seg_at + head0 + mh) * hs + (long long)row * a.dv : nullptr;
-  float S[32];
-  {
-    const float* init = nullptr;
-    if (!STATE_ONLY) {
-      if (segmented) init = segst;
-      else if (a.starts[seq] != 0) init = cache;
-    }
-#pragma unroll
-    for (int i = 0; i < 32; i += 4) {
-      const float4 v = init != nullptr && row < a.dk && mc + i < a.dv ? *reinterpret_cast<const float4*>(init + mc + i)
-                                                                     : make_float4(0.f, 0.f, 0.f, 0.f);
-      S[i] = v.x; S[i + 1] = v.y; S[i + 2] = v.z; S[i + 3] = v.w;
-    }
-  }
-
-  // 16-byte unit n of mine where tiles are worked on row by row: row urow + 32 n, unit tid & 15
-  const int cu8 = (tid & 15) * 8, urow = tid >> 4;
-  const int uh = NH == 2 ? cu8 >> 6 : 0, uc = NH == 2 ? cu8 & 63 : c0 + cu8;     // as value columns: a head and its columns
-
-  const float skip = a.skip != nullptr ? a.skip[head0 + mh] : 0.f;
-  float log_sum = 0.f;                                        // (STATE_ONLY) log2 decay over the segment
+  // A wait that runs out, here or elsewhere in the CTA, turns `ok` false; the role goes on without waiting (the computing warps meet at barriers),
+  // arriving or copying.
   bool ok = true;
-  uint32_t phase = 0;
-  int chunk = 0;
-  for (; chunk < n_chunk; ++chunk, phase ^= 1u) {
-    const int buf = chunk & 1;
-    const bool more = chunk + 1 < n_chunk;
-    const uint32_t sK = sK0 + (uint32_t)buf * TILE;
-    const uint32_t kphase = (uint32_t)(chunk >> 1) & 1u;
-    auto k_full = [&] { return mbar_wait(full_k + (uint32_t)buf * 8u, kphase); };
-
-    // v' = weight * v of the units of mine, high and low part, to the state's tiles
-    auto put_weighted = [&]() {
-#pragma unroll
-      for (int n = 0; n < 4; ++n) {
-        const uint32_t off = tile_off(urow + 32 * n, tid & 15);
-        const float w1 = sm.wk[buf][uh][urow + 32 * n];
-        const float2 w = make_float2(w1, w1);
-        const uint4 v = ld_shared(sV + off);
-        uint4 h, l;
-        split2(fmul2(unpack2(v.x), w), h.x, l.x);
-        split2(fmul2(unpack2(v.y), w), h.y, l.y);
-        split2(fmul2(unpack2(v.z), w), h.z, l.z);
-        split2(fmul2(unpack2(v.w), w), h.w, l.w);
-        st_shared(sSh + off, h);
-        st_shared(sSl + off, l);
-      }
-    };
-    auto put_norm_sums = [&]() {                              // what the chunk adds to n, by warp
-      float2 add[4] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-#pragma unroll
-      for (int n = 0; n < 4; ++n) {
-        const float w1 = sm.wk[buf][0][urow + 32 * n];
-        const float2 w = make_float2(w1, w1);
-        const uint4 k = ld_shared(sK + tile_off(urow + 32 * n, tid & 15));
-        add[0] = ffma2(unpack2(k.x), w, add[0]);
-        add[1] = ffma2(unpack2(k.y), w, add[1]);
-        add[2] = ffma2(unpack2(k.z), w, add[2]);
-        add[3] = ffma2(unpack2(k.w), w, add[3]);
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        add[i].x += __shfl_xor_sync(0xffffffffu, add[i].x, 16);
-        add[i].y += __shfl_xor_sync(0xffffffffu, add[i].y, 16);
-        if (lane < 16) *reinterpret_cast<float2*>(&sm.n_add[warp][cu8 + 2 * i]) = add[i];
-      }
-    };
-    auto advance_norm = [&]() {
-      if (tid < N) {
-        float v = sm.n[tid] * fast_exp2(sm.dec[buf][0]);
-#pragma unroll
-        for (int w = 0; w < kThreads / 32; ++w) v += sm.n_add[w][tid];
-        sm.n[tid] = v;
-      }
-    };
-    const uint64_t khd = smem_desc(sK, SLAB, 1024), shd = smem_desc(sSh, SLAB, 1024), sld = smem_desc(sSl, SLAB, 1024);
-    auto issue_old = [&]() {                                  // Q S
-      const uint64_t qd = smem_desc(sQ, 16, 1024);
-      tc_mma_ss8<StepsByRowsB<SLAB>>(tmem + 128u, qd, shd, IDESC_B, 0u);
-      tc_mma_ss8<StepsByRowsB<SLAB>>(tmem + 128u, qd, sld, IDESC_B, 1u);
-      tc_commit(bar_1);
-    };
-    auto issue_state = [&]() {
-      tc_mma_ss8<StepsByRows>(tmem + 384u, khd, shd, IDESC_AB, 0u);
-      tc_mma_ss8<StepsByRows>(tmem + 384u, khd, sld, IDESC_AB, 1u);
-      tc_commit(bar_s);
-    };
-
-    // ---- the state's tiles: S, or (STATE_ONLY) V' at once ------------------------------------------------
-    if constexpr (STATE_ONLY) {
-      ok = mbar_wait(full_v, phase) && ok;
-      ok = k_full() && ok;
-      put_weighted();
-      if constexpr (NORM) put_norm_sums();
-    } else {
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        uint4 h, l;
-        split2(make_float2(S[8 * u], S[8 * u + 1]), h.x, l.x);
-        split2(make_float2(S[8 * u + 2], S[8 * u + 3]), h.y, l.y);
-        split2(make_float2(S[8 * u + 4], S[8 * u + 5]), h.z, l.z);
-        split2(make_float2(S[8 * u + 6], S[8 * u + 7]), h.w, l.w);
-        const uint32_t off = tile_off(row, cg * 4 + u);
-        st_shared(sSh + off, h);
-        st_shared(sSl + off, l);
-      }
+  auto wait = [&](int which, uint32_t parity) {
+    if (!ok) return;
+    for (uint32_t i = 0; i < kMaxBarrierPolls; ++i) {
+      if (mbar_try_wait(bar(which), parity)) return;
+      if ((i & 255u) == 255u && sm.gave_up) break;
     }
-    fence_proxy_async();
-    tc_fence_before();                                        // the last chunk's tensor-memory reads are done
-    __syncthreads();
-    if (warp == 0) {
-      if constexpr (!STATE_ONLY) ok = mbar_wait(full_q, phase) && ok;
-      ok = k_full() && ok;
+    sm.gave_up = 1;
+    ok = false;
+  };
+  // Every barrier below completes one phase per chunk, that of chunk c with parity c & 1; the two that alternate (K, gates) one per two chunks.
+  if (mma_warp) {
+    const uint64_t qd = smem_desc(sQ, 16, 1024), qkd = smem_desc(sK0, 16, 1024), khd = smem_desc(sK0, SLAB, 1024), vd = smem_desc(sV, SLAB, 1024);
+    const uint64_t shd = smem_desc(sSh, SLAB, 1024), sld = smem_desc(sSl, SLAB, 1024), ed = smem_desc(sE, SLAB, 1024);
+    auto issue_scores = [&](int c) {
+      wait(kFullQ, (uint32_t)c & 1u);
+      wait(kFullK + (c & 1), (uint32_t)(c >> 1) & 1u);
       tc_fence_after();
       __syncwarp();
-      if constexpr (STATE_ONLY) {
-        issue_state();
-      } else {
-        const uint64_t qd = smem_desc(sQ, 16, 1024), kd = smem_desc(sK, 16, 1024);
-        tc_mma_ss8<StepsAlongK<SLAB, SLAB>>(tmem, qd, kd, IDESC_QK, 0u);
-        tc_commit(bar_a);
-        if constexpr (!NORM) issue_old();
-      }
-    }
-    if (copier) {
-      if (more) { load_k(chunk + 1); ++n_k; }                 // (its last readers were done before the last chunk's end)
-      if (!STATE_ONLY && chunk > 0) {                         // the output has left V's place
-        tma_store_wait_read();
-        load_v(chunk);
-        ++n_v;
-      }
-      if (STATE_ONLY && more) { load_v(chunk + 1); ++n_v; }   // V has become V'
-    }
-    __syncwarp();
-    if (warp < NH && more) fetch_gates(chunk + 1);
-    if constexpr (!STATE_ONLY) {
-      float floor = 0.f, den = 0.f;
-      if constexpr (NORM) {
-        const long long t = t0 + (long long)chunk * C + row;
-        if (t < t1) floor = a.floor[(long long)head0 * a.total + t];
-        ok = mbar_wait(full_q, phase) && ok;
-        ok = k_full() && ok;
-        put_norm_sums();
-        float2 d2 = make_float2(0.f, 0.f);
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const uint4 q = ld_shared(sQ + tile_off(row, cg * 4 + u));
-          const float4 n0 = *reinterpret_cast<const float4*>(sm.n + cg * 32 + u * 8), n1 = *reinterpret_cast<const float4*>(sm.n + cg * 32 + u * 8 + 4);
-          d2 = ffma2(unpack2(q.x), make_float2(n0.x, n0.y), d2);
-          d2 = ffma2(unpack2(q.y), make_float2(n0.z, n0.w), d2);
-          d2 = ffma2(unpack2(q.z), make_float2(n1.x, n1.y), d2);
-          d2 = ffma2(unpack2(q.w), make_float2(n1.z, n1.w), d2);
-        }
-        den = (d2.x + d2.y) * fast_exp2(sm.lb[buf][0][row].x);
-      }
-      // ---- A -> P ------------------------------------------------------------------------------------
-      ok = mbar_wait(bar_a, phase) && ok;
-      tc_fence_after();
-      float s[32];
-      tc_ld32(tA, s);
-      tc_wait_ld();
-      tc_fence_before();
-      __syncthreads();                                        // P is written over other warps' part of A; n has been read
-      tc_fence_after();
-      if constexpr (NORM) {
-        // Q S only now: its operands would take shared-memory cycles from the sums for the normaliser (16 x 1024 tokens, 32 heads of 128: 245.6 us
-        // with Q S right behind Q K^T, 242.7 so; the sums on mma.sync, which waits for the same tensor cores, 268)
-        if (warp == 0) {
-          __syncwarp();
-          issue_old();
-        }
-        advance_norm();
-      }
-      const int over = row - cg * 32;                         // my columns up to this one are at or before my row
-      const bool below = __any_sync(0xffffffffu, over >= 0);
-#pragma unroll
-      for (int hh = 0; hh < NH; ++hh) {
-        const float2* lb = sm.lb[buf][hh] + cg * 32;
-        const float li = sm.lb[buf][hh][row].x;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          uint32_t ph[8], pl[8];
-          if (below) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              const int j = h * 16 + 2 * i;
-              const float4 w = *reinterpret_cast<const float4*>(lb + j);
-              const float2 e = make_float2(fast_exp2(li - w.x), fast_exp2(li - w.z));
-              float2 p = fmul2(make_float2(s[j], s[j + 1]), fmul2(e, make_float2(w.y, w.w)));
-              p.x = j <= over ? p.x : 0.f;                    // (a selection: what is dropped may have overflowed)
-              p.y = j + 1 <= over ? p.y : 0.f;
-              if constexpr (NORM) den += p.x + p.y;
-              split2(p, ph[i], pl[i]);
-            }
-          } else {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) ph[i] = pl[i] = 0u;
-          }
-          tc_st8(tP + hh * 384u + h * 8u, ph);
-          tc_st8(tP + hh * 384u + 64u + h * 8u, pl);
-        }
-      }
-      if constexpr (NORM) sm.den[cg][row] = den;
-      tc_wait_st();
-      tc_fence_before();
-      __syncthreads();
-      if (warp == 0) {
-        ok = mbar_wait(full_v, phase) && ok;
+      tc_mma_ss8<StepsAlongK<SLAB, SLAB>>(tmem, qd, qkd + (uint64_t)((c & 1) * (TILE >> 4)), IDESC_QK, 0u);
+      tc_commit(bar(kScores));
+    };
+    if constexpr (!STATE_ONLY) issue_scores(0);
+#pragma unroll 1
+    for (int c = 0; c < n_chunk; ++c) {
+      const uint32_t ph = (uint32_t)c & 1u;
+      const uint64_t kc = khd + (uint64_t)((c & 1) * (TILE >> 4));
+      if constexpr (!STATE_ONLY) {
+        wait(kStateIn, ph);
         tc_fence_after();
         __syncwarp();
-        const uint64_t vd = smem_desc(sV, SLAB, 1024);
+        tc_mma_ss8<StepsByRowsB<SLAB>>(tmem + 128u, qd, shd, IDESC_B, 0u);
+        tc_mma_ss8<StepsByRowsB<SLAB>>(tmem + 128u, qd, sld, IDESC_B, 1u);
+        if constexpr (NORM) {
+          tc_mma_ss8<StepsByRowsB<SLAB>>(tmem + 256u, qd, ed, IDESC_B32, 0u);
+          tc_mma_ss8<StepsByRows>(tmem + 288u, kc, ed, IDESC_AB32, 0u);
+        }
+        tc_commit(bar(kOld));
+        wait(kWeights, ph);
+        wait(kFullV, ph);
+        tc_fence_after();
+        __syncwarp();
 #pragma unroll
         for (int hh = 0; hh < NH; ++hh) {
           const uint64_t vh = vd + (uint64_t)(hh * (SLAB >> 4));
@@ -437,135 +282,328 @@ recurrence_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
           tc_mma_ts8<StepsTmemA<>>(d, p, vh, IDESC_PV, 0u);
           tc_mma_ts8<StepsTmemA<>>(d, p + 64u, vh, IDESC_PV, 1u);
         }
-        tc_commit(bar_o);
+        tc_commit(bar(kNew));
       }
-      // ---- V' over the state's tiles ----------------------------------------------------------------
-      ok = mbar_wait(bar_1, phase) && ok;
-      ok = mbar_wait(full_v, phase) && ok;
-      if (copier && more) { load_q(chunk + 1); ++n_q; }
-      __syncwarp();
-      put_weighted();
-      fence_proxy_async();
-      __syncthreads();
-      if (warp == 0) {                                        // (in order behind the products that read the second head's P there)
-        tc_fence_after();
-        __syncwarp();
-        issue_state();
-      }
-      // ---- output, over V --------------------------------------------------------------------------------
-      const float e = fast_exp2(sm.lb[buf][mh][row].x) * a.q_scale;
-      float f2 = a.q_scale, f1 = e;
-      if constexpr (NORM) {
-        const float dn = a.q_scale * (sm.den[0][row] + sm.den[1][row] + sm.den[2][row] + sm.den[3][row]);
-        const float inv = 1.f / (fmaxf(fabsf(dn), floor) + a.norm_eps);
-        f1 *= inv;
-        f2 *= inv;
-      }
-      ok = mbar_wait(bar_o, phase) && ok;
+      wait(kValues, ph);
+      if constexpr (STATE_ONLY) wait(kFullK + (c & 1), (uint32_t)(c >> 1) & 1u);
       tc_fence_after();
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        float x[16], y[16];
-        tc_ld16(tO1 + h * 16u, x);
-        tc_ld16(tO2 + h * 16u, y);
-        tc_wait_ld();
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const uint32_t off = tile_off(row, cg * 4 + h * 2 + u);
-          uint32_t p[4];
-          uint4 vu = make_uint4(0, 0, 0, 0);
-          if (!NORM) vu = ld_shared(sV + off);
-          const uint32_t vv[4] = {vu.x, vu.y, vu.z, vu.w};
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int j = u * 8 + 2 * i;
-            float2 r = ffma2(make_float2(x[j], x[j + 1]), make_float2(f1, f1), fmul2(make_float2(y[j], y[j + 1]), make_float2(f2, f2)));
-            if (!NORM) r = ffma2(unpack2(vv[i]), make_float2(skip, skip), r);
-            p[i] = pack_bf162(r.x, r.y);
-          }
-          st_shared(sV + off, make_uint4(p[0], p[1], p[2], p[3]));
-        }
-      }
-      fence_proxy_async();
-    } else {
-      if constexpr (NORM) advance_norm();
+      __syncwarp();
+      tc_mma_ss8<StepsByRows>(tmem + 384u, kc, shd, IDESC_AB, 0u);       // (in order behind the products that read the second head's P there)
+      tc_mma_ss8<StepsByRows>(tmem + 384u, kc, sld, IDESC_AB, 1u);
+      if constexpr (NORM && STATE_ONLY) tc_mma_ss8<StepsByRows>(tmem + 288u, kc, ed, IDESC_AB32, 0u);
+      tc_commit(bar(kState));
+      if constexpr (!STATE_ONLY)
+        if (c + 1 < n_chunk) issue_scores(c + 1);               // over P, in order behind P V
     }
-    // ---- state ---------------------------------------------------------------------------------------
-    ok = mbar_wait(bar_s, phase) && ok;
-    tc_fence_after();
-    {
-      const float ld = sm.dec[buf][mh], dc = fast_exp2(ld);
-      if (STATE_ONLY) log_sum += ld;
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        float t[16];
-        tc_ld16(tS + h * 16u, t);
-        tc_wait_ld();
-#pragma unroll
-        for (int i = 0; i < 16; i += 2) {
-          const float2 r = ffma2(make_float2(S[h * 16 + i], S[h * 16 + i + 1]), make_float2(dc, dc), make_float2(t[i], t[i + 1]));
-          S[h * 16 + i] = r.x;
-          S[h * 16 + i + 1] = r.y;
-        }
-      }
-    }
-    if (warp < NH && more) put_gates(buf ^ 1);
-    if (__syncthreads_or(ok ? 0 : 1)) break;                  // a wait ran out somewhere in the CTA
-    if constexpr (!STATE_ONLY) {
-      const int rows = n_tok - chunk * C;
-      const long long tb = t0 + (long long)chunk * C;
-      if (rows >= C) {
-        if (copier) {
-          if (NH == 2) {
-            tma_store_3d(&omap, 0, head0, (int)tb, sV);
-            tma_store_3d(&omap, 0, head0 + 1, (int)tb, sV + SLAB);
-          } else {
-            tma_store_3d(&omap, c0, head0, (int)tb, sV);
-            if (wide_v) tma_store_3d(&omap, c0 + 64, head0, (int)tb, sV + SLAB);
-          }
-          tma_store_commit();
-        }
+    // every MMA is done before shared and tensor memory are given up
+    tc_commit(bar(kDrain));
+    if (!mbar_wait(bar(kDrain), 0u)) sm.gave_up = 1;
+  } else if (copy_warp) {
+    int n_q = 1, n_v = 1, n_k = 1;                              // loads issued
+#pragma unroll 1
+    for (int c = 0; c < n_chunk; ++c) {
+      const uint32_t ph = (uint32_t)c & 1u;
+      const bool more = c + 1 < n_chunk;
+      wait(STATE_ONLY ? kValues : kStateIn, ph);                // every warp has begun the chunk: what only the one before used is free
+      ok = __all_sync(0xffffffffu, ok);
+      if (more) {
+        if (lane == 0 && ok) { load_k(c + 1); ++n_k; }
         __syncwarp();
-      } else {                                                // the last chunk of a sequence: its rows only
-        bf16* p = static_cast<bf16*>(a.out) + (tb + urow) * ((long long)a.heads * a.dv) + (long long)(head0 + uh) * a.dv + uc;
+        put_gates((c + 1) & 1);
+        __syncwarp();
+        if (ok && lane == 0) mbar_arrive(bar(kGates + ((c + 1) & 1)));
+        if (c + 2 < n_chunk) fetch_gates(c + 2);
+      }
+      if constexpr (STATE_ONLY) {
+        if (more && lane == 0 && ok) { load_v(c + 1); ++n_v; }  // V has become V'
+      } else {
+        if (more) {
+          wait(kOld, ph);
+          ok = __all_sync(0xffffffffu, ok);
+          if (lane == 0 && ok) { load_q(c + 1); ++n_q; }
+        }
+        wait(kOut, ph);
+        ok = __all_sync(0xffffffffu, ok);
+        if (lane == 0 && ok) {
+          const long long tb = t0 + (long long)c * C;
+          if (n_tok - c * C >= C) {
+            if (NH == 2) {
+              tma_store_3d(&omap, 0, head0, (int)tb, sV);
+              tma_store_3d(&omap, 0, head0 + 1, (int)tb, sV + SLAB);
+            } else {
+              tma_store_3d(&omap, c0, head0, (int)tb, sV);
+              if (wide_v) tma_store_3d(&omap, c0 + 64, head0, (int)tb, sV + SLAB);
+            }
+            tma_store_commit();
+          }
+          if (more) {
+            tma_store_wait_read();
+            load_v(c + 1);
+            ++n_v;
+          }
+        }
+      }
+      __syncwarp();
+    }
+    if (lane == 0) {                                            // copies into and out of this CTA's shared memory
+      bool in = STATE_ONLY || mbar_wait(bar(kFullQ), (uint32_t)(n_q - 1) & 1u);
+      in = mbar_wait(bar(kFullK + ((n_k - 1) & 1)), (uint32_t)((n_k - 1) >> 1) & 1u) && in;
+      in = mbar_wait(bar(kFullV), (uint32_t)(n_v - 1) & 1u) && in;
+      if (!in) sm.gave_up = 1;
+      tma_store_wait_read();
+    }
+  } else {
+    // my place in tensor memory: lane (row) and 32 columns
+    const int row = (warp & 3) * 32 + lane, cg = warp >> 2;
+    const uint32_t tl = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)cg * 32u;
+    const uint32_t tA = tl, tO1 = tl + 128u, tO2 = tl + 256u, tS = tl + 384u;
+    const uint32_t tP = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)cg * 16u;     // high part; low part 64 columns on
+    // ... and what the columns are: a head and its columns from mc on
+    const int mh = NH == 2 ? cg >> 1 : 0, mc = NH == 2 ? (cg & 1) * 32 : c0 + cg * 32;
+    auto row_sync = [&]() {                                     // the four warps that share my rows
+      tc_fence_before();
+      asm volatile("bar.sync %0, 128;" ::"r"(1 + (warp & 3)) : "memory");
+      tc_fence_after();
+    };
+    auto done = [&](int which) {                                // one arrival per warp, behind its writes of shared and tensor memory
+      tc_fence_before();
+      __syncwarp();
+      if (ok && lane == 0) mbar_arrive(bar(which));
+    };
+
+    // ---- state: row `row`, my columns ----------------------------------------------------------------
+    float* cache = slot_ok ? a.state + ((long long)slot * a.heads + head0 + mh) * hs + (long long)row * a.dv : nullptr;
+    float* segst = segmented ? a.seg_state + (seg_at + head0 + mh) * hs + (long long)row * a.dv : nullptr;
+    float S[32];
+    {
+      const float* init = nullptr;
+      if (!STATE_ONLY) {
+        if (segmented) init = segst;
+        else if (a.starts[seq] != 0) init = cache;
+      }
 #pragma unroll
-        for (int n = 0; n < 4; ++n)
-          if (uc < a.dv && urow + 32 * n < rows)
-            *reinterpret_cast<uint4*>(p + (long long)(32 * n) * a.heads * a.dv) = ld_shared(sV + tile_off(urow + 32 * n, tid & 15));
+      for (int i = 0; i < 32; i += 4) {
+        const float4 v = init != nullptr && row < a.dk && mc + i < a.dv ? *reinterpret_cast<const float4*>(init + mc + i)
+                                                                       : make_float4(0.f, 0.f, 0.f, 0.f);
+        S[i] = v.x; S[i + 1] = v.y; S[i + 2] = v.z; S[i + 3] = v.w;
       }
     }
-  }
-  if (chunk < n_chunk) {                                      // left early: wait (bounded) for what is still in flight
-    if (tid == 0) atomicOr(a.status, kStatusWaitTimeout);
-    if (!STATE_ONLY) {
-      mbar_wait(bar_a, phase);
-      mbar_wait(bar_1, phase);
-      mbar_wait(bar_o, phase);
-    }
-    mbar_wait(bar_s, phase);
-  }
-  if (copier) {                                               // copies into and out of this CTA's shared memory
-    if (n_q > 0) mbar_wait(full_q, (uint32_t)(n_q - 1) & 1u);
-    if (n_k > 0) mbar_wait(full_k + (uint32_t)((n_k - 1) & 1) * 8u, (uint32_t)((n_k - 1) >> 1) & 1u);
-    if (n_v > 0) mbar_wait(full_v, (uint32_t)(n_v - 1) & 1u);
-    tma_store_wait_read();
-  }
-  __syncwarp();
-  float* dst = STATE_ONLY ? segst : (last_seg ? cache : nullptr);
-  if (dst != nullptr && row < a.dk) {
+    // normaliser: the first 128 threads hold column `row` of it
+    float nrm = 0.f;
+    auto put_ext = [&](int unit, float v) { st_shared(sE + (uint32_t)(row * 128 + ((unit ^ row) & 7) * 16), split3(v)); };
+    if (NORM && !STATE_ONLY && cg == 0 && row < a.dk)
+      nrm = segmented ? a.seg_norm[(seg_at + head0) * a.dk + row] : a.n0[((long long)seq * a.heads + head0) * a.dk + row];
+
+    // 16-byte unit n of mine where tiles are worked on row by row: row urow + 32 n, unit tid & 15
+    const int cu8 = (tid & 15) * 8, urow = tid >> 4;
+    const int uh = NH == 2 ? cu8 >> 6 : 0, uc = NH == 2 ? cu8 & 63 : c0 + cu8;   // as value columns: a head and its columns
+    const float skip = a.skip != nullptr ? a.skip[head0 + mh] : 0.f;
+    float log_sum = 0.f;                                        // (STATE_ONLY) log2 decay over the segment
+
+#pragma unroll 1
+    for (int c = 0; c < n_chunk; ++c) {
+      const int buf = c & 1;
+      const uint32_t ph = (uint32_t)buf;
+      // v' = weight * v of the units of mine, high and low part, to the state's tiles
+      auto put_weighted = [&]() {
 #pragma unroll
-    for (int i = 0; i < 32; i += 4)
-      if (mc + i < a.dv) *reinterpret_cast<float4*>(dst + mc + i) = make_float4(S[i], S[i + 1], S[i + 2], S[i + 3]);
-  }
-  if (STATE_ONLY && blockIdx.z == 0 && row == 0 && (NH == 2 ? (cg & 1) == 0 : cg == 0)) a.seg_log[seg_at + head0 + mh] = log_sum;
-  if (NORM && blockIdx.z == 0 && tid < a.dk) {
-    if (STATE_ONLY) a.seg_norm[(seg_at + head0) * a.dk + tid] = sm.n[tid];
-    else if (last_seg && slot_ok)
-      a.norm[(((long long)slot * 2 + ((a.starts[seq] + seq_len - 1) & 1)) * a.heads + head0) * a.dk + tid] = sm.n[tid];
+        for (int n = 0; n < 4; ++n) {
+          const uint32_t off = tile_off(urow + 32 * n, tid & 15);
+          const float w1 = sm.wk[buf][uh][urow + 32 * n];
+          const float2 w = make_float2(w1, w1);
+          const uint4 v = ld_shared(sV + off);
+          uint4 h, l;
+          split2(fmul2(unpack2(v.x), w), h.x, l.x);
+          split2(fmul2(unpack2(v.y), w), h.y, l.y);
+          split2(fmul2(unpack2(v.z), w), h.z, l.z);
+          split2(fmul2(unpack2(v.w), w), h.w, l.w);
+          st_shared(sSh + off, h);
+          st_shared(sSl + off, l);
+        }
+      };
+      if (c > 0) wait(kGates + buf, (uint32_t)((c - 1) >> 1) & 1u);
+      if (NORM && cg == 0) put_ext(2, sm.wk[buf][0][row]);
+      if constexpr (!STATE_ONLY) {
+        // ---- the state's tiles ------------------------------------------------------------------------
+        if (NORM && cg == 0) put_ext(0, nrm);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          uint4 h, l;
+          split2(make_float2(S[8 * u], S[8 * u + 1]), h.x, l.x);
+          split2(make_float2(S[8 * u + 2], S[8 * u + 3]), h.y, l.y);
+          split2(make_float2(S[8 * u + 4], S[8 * u + 5]), h.z, l.z);
+          split2(make_float2(S[8 * u + 6], S[8 * u + 7]), h.w, l.w);
+          const uint32_t off = tile_off(row, cg * 4 + u);
+          st_shared(sSh + off, h);
+          st_shared(sSl + off, l);
+        }
+        fence_proxy_async();
+        done(kStateIn);
+        float floor = 0.f, den = 0.f;
+        if constexpr (NORM) {
+          const long long t = t0 + (long long)c * C + row;
+          if (t < t1) floor = a.floor[(long long)head0 * a.total + t];
+        }
+        // ---- A -> P ------------------------------------------------------------------------------------
+        wait(kScores, ph);
+        __syncwarp();
+        tc_fence_after();
+        float s[32];
+        tc_ld32(tA, s);
+        tc_wait_ld();
+        row_sync();                                             // P is written over the other warps' part of A
+        const int over = row - cg * 32;                         // my columns up to this one are at or before my row
+        const bool below = __any_sync(0xffffffffu, over >= 0);
+#pragma unroll
+        for (int hh = 0; hh < NH; ++hh) {
+          const float2* lb = sm.lb[buf][hh] + cg * 32;
+          const float li = sm.lb[buf][hh][row].x;
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            uint32_t hi[8], lo[8];
+            if (below) {
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                const int j = h * 16 + 2 * i;
+                const float4 w = *reinterpret_cast<const float4*>(lb + j);
+                const float2 e = make_float2(fast_exp2(li - w.x), fast_exp2(li - w.z));
+                float2 p = fmul2(make_float2(s[j], s[j + 1]), fmul2(e, make_float2(w.y, w.w)));
+                p.x = j <= over ? p.x : 0.f;                    // (a selection: what is dropped may have overflowed)
+                p.y = j + 1 <= over ? p.y : 0.f;
+                if constexpr (NORM) den += p.x + p.y;
+                split2(p, hi[i], lo[i]);
+              }
+            } else {
+#pragma unroll
+              for (int i = 0; i < 8; ++i) hi[i] = lo[i] = 0u;
+            }
+            tc_st8(tP + hh * 384u + h * 8u, hi);
+            tc_st8(tP + hh * 384u + 64u + h * 8u, lo);
+          }
+        }
+        wait(kOld, ph);
+        __syncwarp();
+        tc_fence_after();
+        if constexpr (NORM) {
+          if (cg == 0) {                                        // n . q and what the chunk adds to n, from where the first columns of P V will be
+            float nq[8], add[8];
+            tc_ld8(tO2, nq);
+            tc_ld8(tO2 + 48u, add);
+            tc_wait_ld();
+            den += (nq[0] + nq[1] + nq[2]) * fast_exp2(sm.lb[buf][0][row].x);
+            nrm = nrm * fast_exp2(sm.dec[buf][0]) + (add[0] + add[1] + add[2]);
+          }
+          sm.den[cg][row] = den;
+        }
+        tc_wait_st();
+        done(kWeights);
+        // ---- V' over the state's tiles ----------------------------------------------------------------
+        wait(kFullV, ph);
+        __syncwarp();
+        put_weighted();
+        fence_proxy_async();
+        done(kValues);
+        // ---- output, over V --------------------------------------------------------------------------------
+        const float e = fast_exp2(sm.lb[buf][mh][row].x) * a.q_scale;
+        float f2 = a.q_scale, f1 = e;
+        if constexpr (NORM) {
+          row_sync();
+          const float dn = a.q_scale * (sm.den[0][row] + sm.den[1][row] + sm.den[2][row] + sm.den[3][row]);
+          const float inv = 1.f / (fmaxf(fabsf(dn), floor) + a.norm_eps);
+          f1 *= inv;
+          f2 *= inv;
+        }
+        wait(kValues, ph);                                      // every warp has read V
+        wait(kNew, ph);
+        __syncwarp();
+        tc_fence_after();
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          float x[16], y[16];
+          tc_ld16(tO1 + h * 16u, x);
+          tc_ld16(tO2 + h * 16u, y);
+          tc_wait_ld();
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            const uint32_t off = tile_off(row, cg * 4 + h * 2 + u);
+            uint32_t p[4];
+            uint4 vu = make_uint4(0, 0, 0, 0);
+            if (!NORM) vu = ld_shared(sV + off);
+            const uint32_t vv[4] = {vu.x, vu.y, vu.z, vu.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const int j = u * 8 + 2 * i;
+              float2 r = ffma2(make_float2(x[j], x[j + 1]), make_float2(f1, f1), fmul2(make_float2(y[j], y[j + 1]), make_float2(f2, f2)));
+              if (!NORM) r = ffma2(unpack2(vv[i]), make_float2(skip, skip), r);
+              p[i] = pack_bf162(r.x, r.y);
+            }
+            st_shared(sV + off, make_uint4(p[0], p[1], p[2], p[3]));
+          }
+        }
+        fence_proxy_async();
+        done(kOut);
+      } else {
+        wait(kFullV, ph);
+        __syncwarp();
+        put_weighted();
+        fence_proxy_async();
+        done(kValues);
+      }
+      // ---- state ---------------------------------------------------------------------------------------
+      wait(kState, ph);
+      __syncwarp();
+      tc_fence_after();
+      {
+        const float ld = sm.dec[buf][mh], dc = fast_exp2(ld);
+        if (STATE_ONLY) log_sum += ld;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          float t[16];
+          tc_ld16(tS + h * 16u, t);
+          tc_wait_ld();
+#pragma unroll
+          for (int i = 0; i < 16; i += 2) {
+            const float2 r = ffma2(make_float2(S[h * 16 + i], S[h * 16 + i + 1]), make_float2(dc, dc), make_float2(t[i], t[i + 1]));
+            S[h * 16 + i] = r.x;
+            S[h * 16 + i + 1] = r.y;
+          }
+        }
+        if (NORM && STATE_ONLY && cg == 0) {
+          float add[8];
+          tc_ld8(tO2 + 48u, add);
+          tc_wait_ld();
+          nrm = nrm * dc + (add[0] + add[1] + add[2]);
+        }
+      }
+      if constexpr (!STATE_ONLY) {
+        const int rows = n_tok - c * C;
+        if (rows < C) {                                         // the last chunk of a sequence: its rows only
+          wait(kOut, ph);
+          bf16* p = static_cast<bf16*>(a.out) + (t0 + (long long)c * C + urow) * ((long long)a.heads * a.dv) + (long long)(head0 + uh) * a.dv + uc;
+#pragma unroll
+          for (int n = 0; n < 4; ++n)
+            if (uc < a.dv && urow + 32 * n < rows)
+              *reinterpret_cast<uint4*>(p + (long long)(32 * n) * a.heads * a.dv) = ld_shared(sV + tile_off(urow + 32 * n, tid & 15));
+        }
+      }
+    }
+    float* dst = STATE_ONLY ? segst : (last_seg ? cache : nullptr);
+    if (dst != nullptr && row < a.dk) {
+#pragma unroll
+      for (int i = 0; i < 32; i += 4)
+        if (mc + i < a.dv) *reinterpret_cast<float4*>(dst + mc + i) = make_float4(S[i], S[i + 1], S[i + 2], S[i + 3]);
+    }
+    if (STATE_ONLY && blockIdx.z == 0 && row == 0 && (NH == 2 ? (cg & 1) == 0 : cg == 0)) a.seg_log[seg_at + head0 + mh] = log_sum;
+    if (NORM && blockIdx.z == 0 && tid < a.dk) {
+      if (STATE_ONLY) a.seg_norm[(seg_at + head0) * a.dk + tid] = nrm;
+      else if (last_seg && slot_ok)
+        a.norm[(((long long)slot * 2 + ((a.starts[seq] + seq_len - 1) & 1)) * a.heads + head0) * a.dk + tid] = nrm;
+    }
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) {
+  if (tid == 0 && sm.gave_up) atomicOr(a.status, kStatusWaitTimeout);
+  if (mma_warp) {
     __syncwarp();
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
@@ -613,9 +651,9 @@ cudaError_t launch_t(const RecurrenceArgs& a, EncodeTiledFn enc, cudaStream_t st
     return cudaErrorInvalidValue;
   cudaError_t e;
   if (a.max_segs > 1) {
-    e = cudaFuncSetAttribute(recurrence_tc5_kernel<true, NH, NORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+    e = cudaFuncSetAttribute(recurrence_tc5_kernel<true, NH, NORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(NORM));
     if (e != cudaSuccess) return e;
-    recurrence_tc5_kernel<true, NH, NORM><<<grid, kThreads, kSmem, stream>>>(qmap, kmap, vmap, omap, a);
+    recurrence_tc5_kernel<true, NH, NORM><<<grid, kThreads, smem_bytes(NORM), stream>>>(qmap, kmap, vmap, omap, a);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     const long long n = (long long)a.dk * a.dv + (NORM ? a.dk : 0);
@@ -623,9 +661,9 @@ cudaError_t launch_t(const RecurrenceArgs& a, EncodeTiledFn enc, cudaStream_t st
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
-  e = cudaFuncSetAttribute(recurrence_tc5_kernel<false, NH, NORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+  e = cudaFuncSetAttribute(recurrence_tc5_kernel<false, NH, NORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(NORM));
   if (e != cudaSuccess) return e;
-  recurrence_tc5_kernel<false, NH, NORM><<<grid, kThreads, kSmem, stream>>>(qmap, kmap, vmap, omap, a);
+  recurrence_tc5_kernel<false, NH, NORM><<<grid, kThreads, smem_bytes(NORM), stream>>>(qmap, kmap, vmap, omap, a);
   return cudaGetLastError();
 }
 
