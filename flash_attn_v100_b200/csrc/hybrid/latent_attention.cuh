@@ -38,12 +38,12 @@ template <typename T> cudaError_t launch_latent_attention(const LatentAttentionA
 
 // Tensor cores (bfloat16; kv_rank + rot_dim <= 576, both multiples of 8).
 bool latent_decode_supported(const LatentAttentionArgs& a);
-int latent_decode_ctas(int heads, int kv_rank, int rot_dim, int sm_count);   // per head block
+int latent_decode_ctas(int heads, int kv_rank, int rot_dim, long long tokens, int sm_count);   // per head block
 cudaError_t launch_latent_decode(const LatentAttentionArgs& a, int sm_count, void* encode_fn, cudaStream_t s);   // cuTensorMapEncodeTiled
 
 // The kernel of latents of 128 to 512 columns in blocks of 128, with rotated parts of 16 to 64 columns (latent_decode_tc5.cu).
 bool latent_decode_tc5_supported(int kv_rank, int rot_dim);
-int latent_decode_tc5_ctas(int heads, int kv_rank, int sm_count);
+int latent_decode_tc5_ctas(int heads, int kv_rank, long long tokens, int sm_count);   // tokens: a bound on those of all rows
 cudaError_t launch_latent_decode_tc5(const LatentAttentionArgs& a, const CUtensorMap& pool_map, cudaStream_t s);
 
 }  // namespace hybrid

@@ -444,8 +444,8 @@ bool latent_decode_supported(const LatentAttentionArgs& a) {
          (reinterpret_cast<uintptr_t>(a.out) & 15) == 0;
 }
 
-int latent_decode_ctas(int heads, int kv_rank, int rot_dim, int sm_count) {
-  if (latent_decode_tc5_supported(kv_rank, rot_dim)) return latent_decode_tc5_ctas(heads, kv_rank, sm_count);
+int latent_decode_ctas(int heads, int kv_rank, int rot_dim, long long tokens, int sm_count) {
+  if (latent_decode_tc5_supported(kv_rank, rot_dim)) return latent_decode_tc5_ctas(heads, kv_rank, tokens, sm_count);
   const int blocks = heads <= 16 ? 1 : (heads + 31) / 32;
   const int n = sm_count / blocks;
   return n > 0 ? n : 1;

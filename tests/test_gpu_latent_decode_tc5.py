@@ -53,9 +53,10 @@ def test_wider_pool_rows(H, r, rot, extra):
     run(H, r, rot, LENS, AROUND, H + 1, extra=extra)
 
 
-@pytest.mark.parametrize("H,r", [(16, 256), (32, 512)])
+@pytest.mark.parametrize("H,r", [(16, 256), (32, 512), (33, 512), (64, 256), (65, 512)])
 def test_more_rows_than_threads(H, r):
-    """Every position of a sequence as a row of its own: 700 rows of 1 to 11 tiles, most of them whole within a CTA."""
+    """Every position of a sequence as a row of its own: 700 rows of 1 to 11 tiles, most of them whole within a CTA.  So many that 33 heads and more come
+    in blocks of 64; in the other tests in blocks of 32."""
     run(H, r, 64, [3, 700], [(1, p) for p in range(700)] + [(0, 2)], 5)
 
 
