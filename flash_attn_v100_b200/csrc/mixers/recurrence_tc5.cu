@@ -17,9 +17,10 @@
 // whatever is in tensor memory.  One issues the MMAs and one the copies, and works out the gates of the next chunk.  They meet at mbarriers, the four warps
 // that share rows at named ones: with the MMAs issued by one of the computing warps and all of them at block barriers, everybody waited for that warp at
 // every hand-over, since an issue blocks while the tensor queue is full.  16 x 1024 tokens, 32 heads of 128, with the normaliser's sums moved to the MMAs
-// and Q K^T of the next chunk issued behind the state's product: 235 -> 209 us for gates and recurrence; 8700 cycles per chunk where it took 11 700. What
-// bounds it now: the chain S -> tiles -> V' -> state of a chunk, its shared-memory traffic (a third of the cycles), and 6 of the 43 us of a CTA
-// before its first and behind its last chunk.
+// and Q K^T of the next chunk issued behind the state's product: 235 -> 209 us for gates and recurrence.  The least divisor of every token comes with the
+// gates, too: as a load in the computing warps, whose registers are full, it held them up for a trip to memory per chunk; 209 -> 200 us, 7900 cycles per
+// chunk where it took 8700 (11 700 at first).  What bounds it now: the chain S -> tiles -> V' -> state of a chunk, its shared-memory traffic (a third of the
+// cycles), and 6 of the 43 us of a CTA before its first and behind its last chunk.
 // Segments let few long sequences fill the GPU: a first launch computes what every segment adds to the state, a scan over the segments turns that into
 // the state at the start of each, and the main launch then runs all segments side by side.
 //
@@ -53,6 +54,7 @@ struct Small {                 // behind the tiles
   float2 lb[2][2][C];          // [buffer][head]: running log2 decay and weight of every token
   float wk[2][2][C];           // weight of every token in the state after the chunk
   float dec[2][2];             // log2 decay over the chunk
+  float floor[2][C];           // (NORM) least divisor of every token
   float den[4][C];             // partial n . q of every row, by column group
   uint64_t bars[16];
   uint32_t tmem_slot;
@@ -163,7 +165,7 @@ recurrence_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
   }
 
   // ---- decays: la and b of a chunk turned into sums, four tokens per lane -----
-  float gl[NH][4], gb[NH][4];
+  float gl[NH][4], gb[NH][4], gf[4];
   auto fetch_gates = [&](int chunk) {
 #pragma unroll
     for (int h = 0; h < NH; ++h) {
@@ -173,6 +175,7 @@ recurrence_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
         const bool in = tb + i < t1;
         gl[h][i] = in ? a.la[at + i] : 0.f;
         gb[h][i] = in ? a.b[at + i] : 0.f;
+        if (NORM && !STATE_ONLY) gf[i] = in ? a.floor[at + i] : 0.f;
       }
     }
   };
@@ -203,6 +206,7 @@ recurrence_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
         sm.wk[buf][h][lane * 4 + i] = fast_exp2(after) * gb[h][i];
         after += g[i];
       }
+      if (NORM && !STATE_ONLY) *reinterpret_cast<float4*>(&sm.floor[buf][lane * 4]) = make_float4(gf[0], gf[1], gf[2], gf[3]);
     }
   };
   if (copy_warp) {
@@ -439,11 +443,7 @@ recurrence_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
         }
         fence_proxy_async();
         done(kStateIn);
-        float floor = 0.f, den = 0.f;
-        if constexpr (NORM) {
-          const long long t = t0 + (long long)c * C + row;
-          if (t < t1) floor = a.floor[(long long)head0 * a.total + t];
-        }
+        float den = 0.f;
         // ---- A -> P ------------------------------------------------------------------------------------
         wait(kScores, ph);
         __syncwarp();
@@ -509,7 +509,7 @@ recurrence_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
         if constexpr (NORM) {
           row_sync();
           const float dn = a.q_scale * (sm.den[0][row] + sm.den[1][row] + sm.den[2][row] + sm.den[3][row]);
-          const float inv = 1.f / (fmaxf(fabsf(dn), floor) + a.norm_eps);
+          const float inv = 1.f / (fmaxf(fabsf(dn), sm.floor[buf][row]) + a.norm_eps);
           f1 *= inv;
           f2 *= inv;
         }
