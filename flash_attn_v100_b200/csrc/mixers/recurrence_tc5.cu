@@ -13,14 +13,15 @@
 // and 16-18 of a tile of their own (two products of N = 32); n stays in registers, fp32.  (As sums in the threads, which read Q and K from shared
 // memory once more, they took 2950 cycles of a chunk.)
 //
-// CTA = (segment of a sequence, head or pair of heads, 128 value columns), eighteen warps.  Sixteen compute: a warp owns 32 lanes (rows) x 32 columns of
+// CTA = (segment of a sequence, head or pair of heads, 128 value columns), eighteen warps and two idle ones.  Sixteen compute: a warp owns 32 lanes (rows) x 32 columns of
 // whatever is in tensor memory.  One issues the MMAs and one the copies, and works out the gates of the next chunk.  They meet at mbarriers, the four warps
 // that share rows at named ones: with the MMAs issued by one of the computing warps and all of them at block barriers, everybody waited for that warp at
 // every hand-over, since an issue blocks while the tensor queue is full.  16 x 1024 tokens, 32 heads of 128, with the normaliser's sums moved to the MMAs
 // and Q K^T of the next chunk issued behind the state's product: 235 -> 209 us for gates and recurrence.  The least divisor of every token comes with the
-// gates, too: as a load in the computing warps, whose registers are full, it held them up for a trip to memory per chunk; 209 -> 200 us, 7900 cycles per
-// chunk where it took 8700 (11 700 at first).  What bounds it now: the chain S -> tiles -> V' -> state of a chunk, its shared-memory traffic (a third of the
-// cycles), and 6 of the 43 us of a CTA before its first and behind its last chunk.
+// gates, too: as a load in the computing warps, whose registers are full, it held them up for a trip to memory per chunk; 209 -> 200 us.  Registers that the
+// other warps hand in (a thread may have 96 at the launch, the computing warps then have 104, with next to no spills): 200 -> 193 us; 7500 cycles per chunk
+// where it took 8700 (11 700 at first).  What bounds it now: the chain S -> tiles -> V' -> state of a chunk, its shared-memory traffic (a third of the
+// cycles), and 6 of the 40 us of a CTA before its first and behind its last chunk.
 // Segments let few long sequences fill the GPU: a first launch computes what every segment adds to the state, a scan over the segments turns that into
 // the state at the start of each, and the main launch then runs all segments side by side.
 //
@@ -45,7 +46,8 @@ namespace {
 constexpr int C = 128;         // tokens per chunk
 constexpr int N = 128;         // key and value columns per CTA (padded with zeros)
 constexpr int kCompute = 512;  // threads that compute
-constexpr int kThreads = kCompute + 64;
+constexpr int kThreads = kCompute + 128;
+static_assert(kCompute * 104 + 128 * 64 <= kThreads * 96, "registers");   // (launched with 96 a thread)
 constexpr int SLAB = 128 * 128;
 constexpr int TILE = 2 * SLAB;
 constexpr float kLog2e = 1.4426950408889634f;
@@ -249,6 +251,7 @@ recurrence_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
   };
   // Every barrier below completes one phase per chunk, that of chunk c with parity c & 1; the two that alternate (K, gates) one per two chunks.
   if (mma_warp) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
     const uint64_t qd = smem_desc(sQ, 16, 1024), qkd = smem_desc(sK0, 16, 1024), khd = smem_desc(sK0, SLAB, 1024), vd = smem_desc(sV, SLAB, 1024);
     const uint64_t shd = smem_desc(sSh, SLAB, 1024), sld = smem_desc(sSl, SLAB, 1024), ed = smem_desc(sE, SLAB, 1024);
     auto issue_scores = [&](int c) {
@@ -303,6 +306,7 @@ recurrence_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
     tc_commit(bar(kDrain));
     if (!mbar_wait(bar(kDrain), 0u)) sm.gave_up = 1;
   } else if (copy_warp) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
     int n_q = 1, n_v = 1, n_k = 1;                              // loads issued
 #pragma unroll 1
     for (int c = 0; c < n_chunk; ++c) {
@@ -356,7 +360,10 @@ recurrence_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
       if (!in) sm.gave_up = 1;
       tma_store_wait_read();
     }
+  } else if (tid >= kCompute) {                                // (two warps that only hand in their registers)
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
   } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
     // my place in tensor memory: lane (row) and 32 columns
     const int row = (warp & 3) * 32 + lane, cg = warp >> 2;
     const uint32_t tl = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)cg * 32u;
