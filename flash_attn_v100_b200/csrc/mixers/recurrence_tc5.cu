@@ -55,6 +55,7 @@ constexpr float kLog2e = 1.4426950408889634f;
 struct Small {                 // behind the tiles
   float2 lb[2][2][C];          // [buffer][head]: running log2 decay and weight of every token
   float wk[2][2][C];           // weight of every token in the state after the chunk
+  float wb[2][2][C];           // ... and in the row at the end of its block of 32 tokens, without what is decayed by then
   float dec[2][2];             // log2 decay over the chunk
   float floor[2][C];           // (NORM) least divisor of every token
   float den[4][C];             // partial n . q of every row, by column group
@@ -198,10 +199,17 @@ recurrence_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
       float before = __shfl_up_sync(0xffffffffu, up, 1), after = __shfl_down_sync(0xffffffffu, down, 1);
       if (lane == 0) before = 0.f;
       if (lane == 31) after = 0.f;
+      float own[4];                                             // running decay at my tokens
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         before += g[i];
         sm.lb[buf][h][lane * 4 + i] = make_float2(before, gb[h][i]);
+        own[i] = before;
+      }
+      if (NH == 2 && !STATE_ONLY) {
+        const float end = __shfl_sync(0xffffffffu, before, lane | 7);
+        *reinterpret_cast<float4*>(&sm.wb[buf][h][lane * 4]) = make_float4(fast_exp2(end - own[0]) * gb[h][0], fast_exp2(end - own[1]) * gb[h][1],
+                                                                           fast_exp2(end - own[2]) * gb[h][2], fast_exp2(end - own[3]) * gb[h][3]);
       }
 #pragma unroll
       for (int i = 3; i >= 0; --i) {                            // (summed from the end: the tokens that matter have small sums)
@@ -461,14 +469,32 @@ recurrence_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
         row_sync();                                             // P is written over the other warps' part of A
         const int over = row - cg * 32;                         // my columns up to this one are at or before my row
         const bool below = __any_sync(0xffffffffu, over >= 0);
+        // All of my columns' tokens are in blocks before my row's: e^(L_i - L_j) is a factor per row, from the end of the columns' block on, and one per column,
+        // which come with the gates (both at most 1), in place of an exponential per element and head.  Pairs of heads, 8 x 2048 tokens of 64 heads: 166 -> 154 us,
+        // 8 x 1024 of 32 48.4 -> 46.9; with one head per CTA the exponentials are not what a chunk waits for (157.4 and 156.3 us, long sequences 2 % slower).
+        const bool apart = NH == 2 && cg < (warp & 3);
 #pragma unroll
         for (int hh = 0; hh < NH; ++hh) {
           const float2* lb = sm.lb[buf][hh] + cg * 32;
           const float li = sm.lb[buf][hh][row].x;
+          const float *wb = sm.wb[buf][hh] + cg * 32, e1 = apart ? fast_exp2(li - lb[31].x) : 0.f;
+          const float2 e_end = make_float2(e1, e1);
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             uint32_t hi[8], lo[8];
-            if (below) {
+            if (apart) {
+#pragma unroll
+              for (int i = 0; i < 8; i += 2) {
+                const int j = h * 16 + 2 * i;
+                const float4 w = *reinterpret_cast<const float4*>(wb + j);
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                  const float2 p = fmul2(make_float2(s[j + 2 * u], s[j + 2 * u + 1]), fmul2(e_end, u == 0 ? make_float2(w.x, w.y) : make_float2(w.z, w.w)));
+                  if constexpr (NORM) den += p.x + p.y;
+                  split2(p, hi[i + u], lo[i + u]);
+                }
+              }
+            } else if (below) {
 #pragma unroll
               for (int i = 0; i < 8; ++i) {
                 const int j = h * 16 + 2 * i;
