@@ -415,7 +415,7 @@ cudaError_t launch_t(const LatentAttentionArgs& a, const CUtensorMap& map, cudaS
 // Launched while the decode still runs (its blocks take the places that finished ones leave) and held at its first instruction until
 // all of the decode's writes are there: 0.5 to 1 us of launch latency less.  Not beside the decode of the widest rows, whose shared memory leaves little of the SM's
 // memory as L1, where few rows are cut into many pieces, so that the merge is long: it then reads the pieces more slowly than one that
-// starts on free SMs.  32 heads of 512 + 64, early (behind the decode): 1 row of 8192 cached tokens 32.1 us (27.0), 2 of 4096 1.15 times, 8 of
+// starts on free SMs.  Behind the kernel above, 32 heads of 512 + 64, early (behind the decode): 1 row of 8192 cached tokens 32.1 us (27.0), 2 of 4096 1.15 times, 8 of
 // 4096 1.02, 12 of 1000 1.04 times; from 16 rows on 0.96 to 1.00 times.  256 + 32, any rows: 0.85 to 1.05 times, 0.96 on average.
 cudaError_t launch_merge(const LatentAttentionArgs& a, int sm_count, cudaStream_t s) {
   cudaLaunchAttribute early;
