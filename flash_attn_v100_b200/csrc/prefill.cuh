@@ -13,7 +13,7 @@ struct PrefillParams {
   const __half* v;
   __half* out;                // fp16, or bfloat16 bits when out_bf16 is set
   int out_bf16;
-  int in_bf16;                // q, k, v are bfloat16 (tcgen05 kernel only: bfloat16 MMAs, P rounded to bfloat16)
+  int in_bf16;                // q, k, v are bfloat16 (D <= 128: bfloat16 MMAs, P rounded to bfloat16)
   const int32_t* cu_seqlens;  // null => dense [B,H,N,D]; else packed [total,H,D]
   int batch;                  // sequences (dense: B)
   int H_Q, H_KV;
@@ -33,12 +33,12 @@ struct PrefillParams {
 // started behind everything before it, so the attention may read its inputs at once; before its first store it waits for the clear (wait_for_clear), whose rows it
 // may share where offsets overlap.
 template <class Kernel, class... Args>
-cudaError_t launch_attention(bool overlap, Kernel kern, unsigned grid, unsigned threads, size_t smem, cudaStream_t stream, const Args&... args) {
+cudaError_t launch_attention(bool overlap, Kernel kern, dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, const Args&... args) {
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
+  cfg.gridDim = grid;
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;

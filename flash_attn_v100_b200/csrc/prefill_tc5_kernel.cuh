@@ -130,9 +130,6 @@ __device__ __forceinline__ void drain_wait(uint32_t bar, uint32_t parity, volati
   atomicOr(&g_prefill_status, kStatusWaitTimeout);
 }
 
-// Until the clear that the launch overlaps is done; passes at once elsewhere.
-__device__ __forceinline__ void wait_for_clear() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 // The next item of a launch; `n_items` or more: there is none.  Every CTA gets exactly one such answer, so the one that is given out last is known, and whoever
 // gets it puts the counter back to zero for the next launch.
 __device__ __forceinline__ long long claim_item(unsigned long long* counter, long long n_items) {
