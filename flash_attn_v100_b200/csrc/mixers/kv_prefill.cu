@@ -48,9 +48,8 @@ cudaError_t launch_t(const KvPrefillArgs& a, EncodeTiledFn enc, cudaStream_t str
   constexpr int smem = Tc5Layout<NA, 0, D>::BYTES;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
-  e = next_item_counter(&p.item_counter);
-  if (e != cudaSuccess) return e;
-  kern<<<dim3((unsigned)(n_items < sms ? n_items : sms)), 640, smem, stream>>>(qmap, kmap, vmap, qmap, kmap, p);
+  p.take_over = n_items > sms ? 1 : 0;
+  kern<<<item_grid(n_items), 640, smem, stream>>>(qmap, kmap, vmap, qmap, kmap, p);
   return cudaGetLastError();
 }
 

@@ -56,19 +56,14 @@ cudaError_t launch_tc5_t(const PrefillParams& pp, void* encode_fn, cudaStream_t 
   cudaError_t e = limits[(pp.in_bf16 ? 2 : 0) + (g_tc5_poly ? 1 : 0)].raise(reinterpret_cast<const void*>(kern), (int)smem);
   if (e != cudaSuccess) return e;
   const int max_len = dense ? pp.N : pp.max_seqlen;
-  dim3 grid;
   if (p.pair_heads) { p.n_hg = pp.H_Q / 2; p.n_rb = (max_len + 127) / 128; }
   else { p.n_hg = pp.H_Q; p.n_rb = (max_len + 255) / 256; }
   const long long n_items = (long long)p.n_rb * pp.batch * p.n_hg;
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  grid = dim3((unsigned)(n_items < sms ? n_items : sms));
-  if (n_items > sms) {           // (else CTA i has item i, without a trip to the counter)
-    e = next_item_counter(&p.item_counter);
-    if (e != cudaSuccess) return e;
-  }
-  return launch_attention(pp.after_clear != 0, kern, grid.x, 640, smem, stream, qmap, kmap, vmap, qmap, kmap, p);
+  p.take_over = n_items > sms ? 1 : 0;
+  return launch_attention(pp.after_clear != 0, kern, item_grid(n_items), 640, smem, stream, qmap, kmap, vmap, qmap, kmap, p);
 }
 
 }  // namespace

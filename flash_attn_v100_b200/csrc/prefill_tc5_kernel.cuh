@@ -23,8 +23,9 @@
 // in fp16 range and compensated in the fp32 row sum).  Causal tiles above the diagonal are
 // skipped; only the diagonal tile and the ragged last tile are masked per element.
 //
-// The kernel is persistent: one CTA per SM claims work items (tile pairs, heaviest first) from
-// a global counter; barrier phases are running counters, so the copy and MMA lanes start the
+// The grid has one CTA per work item (tile pairs, heaviest first), and a CTA that is nearly done takes
+// over the item of one that has not started (take_item): as many run as there are free SMs.
+// Barrier phases are running counters, so the copy and MMA lanes start the
 // next item while the softmax groups still write the previous item's output.
 //
 // Tensor-memory map (512 columns x 128 lanes): S_0 [0,128) S_1 [128,256) O_0 [256,256+D)
@@ -34,8 +35,6 @@
 #include "tc5.cuh"
 #include "tma3.cuh"
 
-#include <atomic>
-#include <mutex>
 #include <type_traits>
 
 namespace fa {
@@ -91,7 +90,7 @@ struct Tc5Params {
   int dense;
   int out_bf16;    // store O as bfloat16 instead of fp16
   int n_hg, n_rb;  // head groups and row blocks of the item grid (items = n_rb * batch * n_hg)
-  unsigned long long* item_counter;  // next unclaimed item of this launch (zeroed in-stream before it); null: CTA i has item i
+  int take_over;   // CTAs go on with the items of CTAs that have not started (0: there are no more items than SMs)
   float scale_log2;
 };
 // Builds with a shared key part (a type of its own: the wider parameter block costs the plain builds registers).
@@ -130,14 +129,36 @@ __device__ __forceinline__ void drain_wait(uint32_t bar, uint32_t parity, volati
   atomicOr(&g_prefill_status, kStatusWaitTimeout);
 }
 
-// The next item of a launch; `n_items` or more: there is none.  Every CTA gets exactly one such answer, so the one that is given out last is known, and whoever
-// gets it puts the counter back to zero for the next launch.
-__device__ __forceinline__ long long claim_item(unsigned long long* counter, long long n_items) {
-  const long long item = (long long)atomicAdd(counter, 1ULL);
-  if (item == n_items + gridDim.x - 1) atomicExch(counter, 0ULL);
-  return item;
+// The item of this CTA, and the next item: that of a CTA of the launch which has not started and now will not (-1: all have).  CTAs start and are taken over
+// in the order of their numbers.  The work is dealt out by the launch itself, so nothing in memory is shared with another launch, on whatever stream or in
+// whatever graph.  One thread calls it; `reply` holds 16 bytes, `taken` counts the phases of `bar`.
+__device__ __forceinline__ long long first_item() { return (long long)blockIdx.y * gridDim.x + blockIdx.x; }
+__device__ __forceinline__ long long take_item(uint32_t reply, uint32_t bar, uint32_t& taken, volatile int* abort_flag) {
+  mbar_expect_tx(bar, 16);
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(reply), "r"(bar) : "memory");
+  if (!wait_or_abort(bar, taken & 1u, abort_flag)) {
+    drain_wait(bar, taken & 1u, abort_flag);         // (the reply must not come after this CTA)
+    return -1;
+  }
+  ++taken;
+  uint32_t ok, x, y;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b128 r;\n\t"
+      "ld.shared.b128 r, [%3];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, r;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\tmov.u32 %1, 0;\n\tmov.u32 %2, 0;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {%1, %2, _, _}, r;\n\t}"
+      : "=&r"(ok), "=&r"(x), "=&r"(y)
+      : "r"(reply)
+      : "memory");
+  fence_proxy_async();                               // (read before the next reply is written there)
+  return ok ? (long long)y * gridDim.x + x : -1;
 }
-
+// Grid of a launch with that many items.
+inline dim3 item_grid(long long n_items) {
+  constexpr long long kMaxX = 1ll << 30;
+  return n_items <= kMaxX ? dim3((unsigned)n_items) : dim3((unsigned)kMaxX, (unsigned)((n_items + kMaxX - 1) / kMaxX));
+}
 // P quarter i / 2 holds the keys of score chunk {0, 1, 3, 2}[i / 2]: the matching rows of V.
 struct PvSteps {
   static constexpr uint32_t a(int i) { return (uint32_t)i * 8u; }
@@ -224,9 +245,9 @@ struct Tc5Layout {
 
 // Work item = one pair of query tiles.  Items are numbered with the row block as the slowest
 // index, running backwards, so the items with the most KV tiles (late causal blocks of the long
-// sequences) come first.  CTAs claim items from a global counter (heaviest-first greedy
-// scheduling): the copy lane claims, skips empty items, and publishes the item number to the
-// other roles of its CTA through a small shared-memory queue.
+// sequences) come first (heaviest-first greedy scheduling): a warp of its own takes items, skips
+// empty ones, and publishes the item number to the other roles of its CTA through a small
+// shared-memory queue.
 struct Tc5Item {
   int head[2], row0[2], n_kv[2];
   int q_c1[2], q_c2[2], kv_c1, kv_c2;
@@ -344,8 +365,8 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_consta
                 B_VFULL = B_KEMPTY + K_STAGES, B_VEMPTY = B_VFULL + V_STAGES, B_SFULL = B_VEMPTY + V_STAGES,
                 B_PFULL = B_SFULL + 2 * kBatchBars, B_TOKEN = B_PFULL + 2,
                 B_IFULL = B_TOKEN + 2, B_IEMPTY = B_IFULL + kItemQ, B_CLAIM = B_IEMPTY + kItemQ, B_PAIR = B_CLAIM + 1,
-                B_DRAIN = B_PAIR + 8, B_TURN = B_DRAIN + 2, B_COUNT = B_TURN + 2;
-  static_assert(B_COUNT + kItemQ + 1 <= 64, "barriers, item slots and the tensor-memory slot share 64 words");
+                B_DRAIN = B_PAIR + 8, B_TURN = B_DRAIN + 2, B_TAKEN = B_TURN + 2, B_COUNT = B_TAKEN + 1;
+  static_assert(B_COUNT + kItemQ + 1 <= 62, "barriers, item slots, the tensor-memory slot and the reply of take_item share 64 words");
   volatile long long* item_slot = reinterpret_cast<volatile long long*>(bars + B_COUNT);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + B_COUNT + kItemQ);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -355,6 +376,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_consta
   auto bar = [&](int i) -> uint32_t { return smem_u32(bars + i); };
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t reply = smem_u32(bars + 62);
   const long long n_items = (long long)p.n_rb * p.batch * p.n_hg;
 #ifdef FA_TC5_PROF
   unsigned long long* prof_smem = reinterpret_cast<unsigned long long*>(xchg + 2 * 3 * 2 * 128 + 8);
@@ -388,6 +410,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_consta
       mbar_init(bar(B_IEMPTY + i), kItemConsumers);
     }
     mbar_init(bar(B_CLAIM), 1);
+    mbar_init(bar(B_TAKEN), 1);
     *abort_flag = 0;
     for (int i = 0; i < 8; ++i) redo_tag[i] = 0u;
     mbar_fence_init();
@@ -611,26 +634,25 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_consta
     }
   } else if (warp == 2) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
-    // ============================ item claimer ======================================
-    // Claims work items from the global counter, skips the empty ones (row blocks past the end of a
-    // sequence) and publishes the others through the item queue: an item is claimed while the copies of the last three
-    // KV tiles of the one before are issued, which keeps the latency of the global atomic off every other role's path.
-    // Claims of up to kItemQ items ahead dealt the items out in turn, whatever they cost, where a CTA has few of them.
+    // ============================ items =============================================
+    // Takes work items, skips the empty ones (row blocks past the end of a
+    // sequence) and publishes the others through the item queue: an item is taken while the copies of the last three
+    // KV tiles of the one before are issued, which keeps the latency of take_item off every other role's path.
+    // Items taken up to kItemQ ahead were dealt out in turn, whatever they cost, where a CTA has few of them.
     if (lane == 0) {
-      bool first = true, ended = p.item_counter == nullptr;
+      bool first = true;
+      uint32_t taken = 0;
       for (uint32_t ic = 0;; ++ic) {
         if (*abort_flag) break;
         Tc5Item it;
         long long item;
         bool have = false;
-        // not before the copies of the last steps of the item before begin: earlier claims would deal the items out in turn, whatever they cost
         if (ic > 0) wait_or_abort(bar(B_CLAIM), (ic - 1) & 1u, abort_flag);
         while (true) {
-          if (p.item_counter != nullptr) item = claim_item(p.item_counter, n_items);
-          else item = first ? (long long)blockIdx.x : n_items;
+          item = first ? first_item() : (p.take_over ? take_item(reply, bar(B_TAKEN), taken, abort_flag) : -1);
           first = false;
-          if (item >= n_items) { ended = true; break; }
-          if (tc5_decode_item<EXT>(p, item, it)) { have = true; break; }
+          if (item < 0) break;
+          if (item < n_items && tc5_decode_item<EXT>(p, item, it)) { have = true; break; }
         }
         const int slot = ic % kItemQ;
         if (ic >= kItemQ) wait_or_abort(bar(B_IEMPTY + slot), ((ic / kItemQ) & 1u) ^ 1u, abort_flag);
@@ -638,7 +660,6 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_consta
         mbar_arrive(bar(B_IFULL + slot));
         if (!have) break;
       }
-      while (!ended) ended = claim_item(p.item_counter, n_items) >= n_items;      // (left early: the counter is put back all the same)
     }
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
@@ -1024,33 +1045,6 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_consta
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
   }
-}
-
-// Item counters of in-flight launches (one per launch, used round-robin).  A launch finds its counter at zero and leaves it so (claim_item), so none of
-// them has to be cleared by a launch of its own (2 to 3 us of a prefill of 40).  More than kCounterPool prefill launches in flight at once on
-// one device would share a counter; launches ordered on one stream never do.
-constexpr int kCounterPool = 64;
-__device__ unsigned long long g_tc5_item_counters[kCounterPool];
-unsigned long long* g_counter_base[64] = {nullptr};
-std::atomic<unsigned int> g_counter_next{0};
-std::mutex g_counter_mu;
-
-cudaError_t next_item_counter(unsigned long long** out) {
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-  {
-    std::lock_guard<std::mutex> lk(g_counter_mu);
-    if (g_counter_base[dev] == nullptr) {
-      void* ptr = nullptr;
-      e = cudaGetSymbolAddress(&ptr, g_tc5_item_counters);
-      if (e != cudaSuccess) return e;
-      g_counter_base[dev] = static_cast<unsigned long long*>(ptr);
-    }
-  }
-  *out = g_counter_base[dev] + (g_counter_next.fetch_add(1) % kCounterPool);
-  return cudaSuccess;
 }
 
 }  // namespace

@@ -18,7 +18,7 @@
 // Measured: 16 x 2048 tokens, 2 heads of 256, causal: 134 us against 401 of the mma.sync kernel (prefill_mma.cu); 1 x 2048, 16 heads on 8: 79 and 229; 4
 // x 1024, 8 on 1: 51 and 127.  The smallest launch takes 12 us.  Releasing every unit with a commit of its own, earlier, changed nothing.
 //
-// Warps: 0 copies (TMA), 1 issues the MMAs, 2 owns tensor memory and claims work, 4-7 and 8-11 softmax of the even and of the odd steps (a
+// Warps: 0 copies (TMA), 1 issues the MMAs, 2 owns tensor memory and takes work items, 4-7 and 8-11 softmax of the even and of the odd steps (a
 // thread per row, its 128 scores in registers), 12-15 write the output of a finished tile while the softmax is on the next one.  (With one
 // softmax group a step took 3800 cycles: a single warp per scheduler waits for its own loads, maxima and stores.)  Shared memory: Q (64 KB) and a ring of
 // five units of 32 KB.  A K unit is 128 keys x 128 columns (QK accumulates over two units), a V unit 64 keys x all columns, so that every
@@ -40,8 +40,8 @@ constexpr int kQBytes = 64 * 1024;
 constexpr int kWideItemQ = 4;
 constexpr int kWideConsumers = 1 + 1 + 8 + 4;             // copy lane, MMA warp, softmax and output warps
 enum WideBar { kQFull = 0, kUFull = 1, kSFull = kUFull + kUnits, kPLo = kSFull + 2, kPHi = kPLo + 2, kODone = kPHi + 2, kOEmpty = kODone + 2, kLFull, kMReady,
-               kIFull = kMReady + 2, kIEmpty = kIFull + kWideItemQ, kClaim = kIEmpty + kWideItemQ, kWideBars };
-constexpr int kWideSmem = kQBytes + kUnits * kUnitBytes + kWideBars * 8 + kWideItemQ * 8 + 4 * 128 * 4 + 16;
+               kIFull = kMReady + 2, kIEmpty = kIFull + kWideItemQ, kClaim = kIEmpty + kWideItemQ, kTaken, kWideBars };
+constexpr int kWideSmem = kQBytes + kUnits * kUnitBytes + 16 + kWideBars * 8 + kWideItemQ * 8 + 4 * 128 * 4 + 16;
 static_assert(kWideSmem <= 227 * 1024, "shared memory plan exceeds the SM");
 
 struct WideParams {
@@ -52,7 +52,7 @@ struct WideParams {
   long long o_batch_stride, o_head_stride, o_tok_stride;
   int causal, D_real, dense, out_bf16;
   int n_rb;                                // row blocks of the item grid (items = n_rb * batch * H_Q)
-  unsigned long long* item_counter;        // next unclaimed item; null: CTA i has item i
+  int take_over;                           // CTAs go on with the items of CTAs that have not started (see take_item)
   int* status;
   float scale_log2;
 };
@@ -123,7 +123,8 @@ prefill_wide_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
     if (threadIdx.x == 0) atomicOr(p.status, kStatusWaitTimeout);
     return;
   }
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kQBytes + kUnits * kUnitBytes);
+  const uint32_t reply = sU + kUnits * kUnitBytes;             // of take_item
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kQBytes + kUnits * kUnitBytes + 16);
   volatile long long* item_slot = reinterpret_cast<volatile long long*>(bars + kWideBars);
   float* l_rows = reinterpret_cast<float*>(bars + kWideBars + kWideItemQ);       // [softmax group][row]: parts of the row sums
   float* m_rows = l_rows + 256;                                                  // [step & 1][row]: reference exponents
@@ -146,6 +147,7 @@ prefill_wide_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
     }
     mbar_init(bar(kOEmpty), 4);
     mbar_init(bar(kClaim), 1);
+    mbar_init(bar(kTaken), 1);
     mbar_init(bar(kLFull), 8);
     for (int i = 0; i < kWideItemQ; ++i) {
       mbar_init(bar(kIFull + i), 1);
@@ -299,19 +301,18 @@ prefill_wide_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
   } else if (warp == 2) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
     if (lane == 0) {
-      bool first = true, ended = p.item_counter == nullptr;
+      bool first = true;
+      uint32_t taken = 0;
       for (uint32_t ic = 0;; ++ic) {
         if (*abort_flag) break;
         WideItem it;
         long long item = -1;
-        // an item is claimed when the copies of the last steps of the one before begin: earlier claims would deal the items out in turn, whatever they cost
+        // an item is taken when the copies of the last steps of the one before begin: taken earlier, items were dealt out in turn, whatever they cost
         if (ic > 0) wait_or_abort(bar(kClaim), (ic - 1) & 1u, abort_flag);
         while (true) {
-          if (p.item_counter != nullptr) item = claim_item(p.item_counter, n_items);
-          else item = first ? (long long)blockIdx.x : n_items;
+          item = first ? first_item() : (p.take_over ? take_item(reply, bar(kTaken), taken, abort_flag) : -1);
           first = false;
-          if (item >= n_items) { item = -1; ended = true; break; }
-          if (wide_item(p, item, it)) break;
+          if (item < 0 || (item < n_items && wide_item(p, item, it))) break;
         }
         const int slot = ic % kWideItemQ;
         if (ic >= kWideItemQ) wait_or_abort(bar(kIEmpty + slot), ((ic / kWideItemQ) & 1u) ^ 1u, abort_flag);
@@ -319,7 +320,6 @@ prefill_wide_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
         mbar_arrive(bar(kIFull + slot));
         if (item < 0) break;
       }
-      while (!ended) ended = claim_item(p.item_counter, n_items) >= n_items;      // (left early: the counter is put back all the same)
     }
   } else if (warp == 3) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
@@ -539,12 +539,8 @@ cudaError_t launch_prefill_wide(const PrefillParams& pp, int sm_count, void* enc
   e = limit.raise(reinterpret_cast<const void*>(prefill_wide_kernel), kWideSmem);
   if (e != cudaSuccess) return e;
   const long long n_items = (long long)p.n_rb * pp.batch * pp.H_Q;
-  if (n_items > sm_count) {
-    e = next_item_counter(&p.item_counter);
-    if (e != cudaSuccess) return e;
-  }
-  return launch_attention(pp.after_clear != 0, prefill_wide_kernel, (unsigned)(n_items < sm_count ? n_items : sm_count), kWideThreads, kWideSmem, stream, qmap, kmap,
-                          vmap, p);
+  p.take_over = n_items > sm_count ? 1 : 0;
+  return launch_attention(pp.after_clear != 0, prefill_wide_kernel, item_grid(n_items), kWideThreads, kWideSmem, stream, qmap, kmap, vmap, p);
 }
 
 }  // namespace fa
