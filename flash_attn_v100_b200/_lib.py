@@ -6,9 +6,11 @@ fallback: if a library is missing, the use of any of its operators raises, with 
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import os
+import warnings
 
-from .build import LIBRARIES
+from .build import CALL_PATH, LIBRARIES, call_fits
 
 _c = ctypes
 _vp, _i, _i64, _sz = _c.c_void_p, _c.c_int, _c.c_int64, _c.c_size_t
@@ -169,17 +171,18 @@ def check(rc: int, name: str = "attention") -> None:
 
 
 def call_module(workspaces):
-    """The native host side of the calls (`_call`), bound to the library's entry points and to the scratch buffers by (device, stream); None if it has
-    not been built, or for another torch."""
+    """The native host side of the calls (`_call`), bound to the library's entry points and to the scratch buffers by (device, stream); None, with a
+    warning, if it has not been built, or for another torch or Python."""
+    lib = load()
     try:
-        import torch
-
-        from . import _call
-        if _call.torch_version != torch.__version__.split("+")[0]:
-            return None
-        lib = load()
-        entries = [n for n in SIGNATURES if n.startswith(("fa_last", "fa_decode", "fa_paged", "fa_prefill"))]
-        _call.bind({n: _c.cast(getattr(lib, n), _vp).value for n in entries}, workspaces)
-        return _call
-    except ImportError:
+        if not call_fits(CALL_PATH):
+            raise ImportError("not there, or built for another torch")
+        spec = importlib.util.spec_from_file_location(f"{__package__}._call", CALL_PATH)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+    except ImportError as e:
+        warnings.warn(f"{CALL_PATH}: {e}; small calls cost more. Run `python -m flash_attn_v100_b200.build`.", RuntimeWarning, stacklevel=2)
         return None
+    entries = [n for n in SIGNATURES if n.startswith(("fa_last", "fa_decode", "fa_paged", "fa_prefill"))]
+    module.bind({n: _c.cast(getattr(lib, n), _vp).value for n in entries}, workspaces)
+    return module

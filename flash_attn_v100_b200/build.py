@@ -10,7 +10,8 @@ model needs.
     python -m flash_attn_v100_b200.build --force
     python -m flash_attn_v100_b200.build -v         # also print ptxas resource usage
 
-`_call` (csrc/host/call.cpp) is the host side of the attention operators' calls, a CPython extension built against the installed torch.
+`_call` (csrc/host/call.cpp) is the host side of the attention operators' calls, a CPython extension built against the installed torch and built again when that
+or Python changes.
 
 Every `.cu` file is compiled to an object of its own (in parallel, cached under
 `_build/` by source time stamps and flags) and the objects of a library are linked
@@ -26,6 +27,8 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
+import warnings
 from concurrent.futures import ThreadPoolExecutor
 
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
@@ -125,16 +128,28 @@ def build(force: bool = False, verbose: bool = False, extra_flags=None, lib_path
 
 
 CALL_SOURCE = os.path.join(CSRC, "host", "call.cpp")
-CALL_PATH = os.path.join(PKG_DIR, "_call.so")
+CALL_PATH = os.path.join(PKG_DIR, "_call" + sysconfig.get_config_var("EXT_SUFFIX"))      # (another Python does not take it for its own)
+
+
+def call_built_for() -> str:
+    """What the host side of the calls is compiled against; the module carries it (`_call.built_for`)."""
+    import torch
+    return f"torch {torch.__version__}, C++11 ABI {int(torch.compiled_with_cxx11_abi())}, {sysconfig.get_config_var('SOABI')}"
+
+
+def call_fits(path: str) -> bool:
+    """Whether the module at `path` is there and built for this torch and Python: read from the file, as one that was not must not be loaded."""
+    if not os.path.exists(path):
+        return False
+    with open(path, "rb") as f:
+        return call_built_for().encode() + b"\0" in f.read()
 
 
 def build_call(force: bool = False) -> str:
     """Compile the host side of the calls.  The operators work without it, through ctypes, at a higher cost per call."""
     deps = (CALL_SOURCE, os.path.join(INCLUDE, "fa_b200.h"))
-    if not force and os.path.exists(CALL_PATH) and os.path.getmtime(CALL_PATH) >= max(os.path.getmtime(d) for d in deps):
+    if not force and call_fits(CALL_PATH) and os.path.getmtime(CALL_PATH) >= max(os.path.getmtime(d) for d in deps):
         return CALL_PATH
-    import sysconfig
-
     import torch
     root = os.path.join(os.path.dirname(torch.__file__), "")
     cuda = os.path.dirname(os.path.dirname(os.path.realpath(find_nvcc())))
@@ -142,13 +157,22 @@ def build_call(force: bool = False) -> str:
     with _build_lock():
         part = f"{CALL_PATH}.{os.getpid()}.tmp"
         abi = f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}"
-        _run([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", abi, *[f"-I{d}" for d in include], CALL_SOURCE, "-o", part, f"-L{root}lib",
+        built_for = f'-DFA_BUILT_FOR="{call_built_for()}"'
+        _run([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", abi, built_for, *[f"-I{d}" for d in include], CALL_SOURCE, "-o", part, f"-L{root}lib",
               "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"])
         os.replace(part, CALL_PATH)
     return CALL_PATH
 
 
+def build_all(force: bool = False, verbose: bool = False) -> list:
+    """Build what is out of date; the paths.  Without a host compiler or torch's headers the libraries alone, with a warning."""
+    paths = [build(force=force, verbose=verbose, library=name) for name in LIBRARIES]
+    try:
+        paths.append(build_call(force))
+    except (OSError, RuntimeError) as e:
+        warnings.warn(f"the native host side of the calls is not built, small calls cost more: {e}", RuntimeWarning, stacklevel=2)
+    return paths
+
+
 if __name__ == "__main__":
-    for name in LIBRARIES:
-        print(build(force="--force" in sys.argv, verbose="-v" in sys.argv, library=name))
-    print(build_call(force="--force" in sys.argv))
+    print("\n".join(build_all("--force" in sys.argv, "-v" in sys.argv)))

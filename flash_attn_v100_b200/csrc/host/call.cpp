@@ -354,6 +354,6 @@ PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_call", nullptr, -1, g_methods, 
 
 PyMODINIT_FUNC PyInit__call(void) {
   PyObject* m = PyModule_Create(&g_module);
-  if (m != nullptr && PyModule_AddStringConstant(m, "torch_version", TORCH_VERSION) != 0) Py_CLEAR(m);
+  if (m != nullptr && (PyModule_AddStringConstant(m, "torch_version", TORCH_VERSION) != 0 || PyModule_AddStringConstant(m, "built_for", FA_BUILT_FOR) != 0)) Py_CLEAR(m);
   return m;
 }
