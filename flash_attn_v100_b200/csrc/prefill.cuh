@@ -31,7 +31,7 @@ struct PrefillParams {
 
 // Launch of an attention kernel; `overlap`: beside the end of the clear in front of it, which lets its successor start as soon as its own blocks have.  That clear
 // started behind everything before it, so the attention may read its inputs at once; before its first store it waits for the clear (wait_for_clear), whose rows it
-// may share where offsets overlap.
+// may share where offsets overlap, and every thread does before it leaves: what follows on the stream waits for the attention alone.
 template <class Kernel, class... Args>
 cudaError_t launch_attention(bool overlap, Kernel kern, dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, const Args&... args) {
   cudaLaunchAttribute attr;

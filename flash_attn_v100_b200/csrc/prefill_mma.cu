@@ -69,6 +69,7 @@ __global__ void __launch_bounds__(BM * 2) prefill_mma_kernel(const PrefillParams
   const int h_q = blockIdx.y, seq = blockIdx.z;
   const int h_kv = h_q / (p.H_Q / p.H_KV);
 
+  // (a block without rows waits for the clear as well: the launch must not end before it)
   long long tok0;
   int len;
   if (p.cu_seqlens != nullptr) {
@@ -76,14 +77,14 @@ __global__ void __launch_bounds__(BM * 2) prefill_mma_kernel(const PrefillParams
     tok0 = a;
     len = e - a;
     if ((long long)e > p.total) len = (int)(p.total - a);
-    if (a < 0 || (long long)a > p.total) return;
+    if (a < 0 || (long long)a > p.total) return wait_for_clear();
   } else {
     tok0 = 0;
     len = p.N;
   }
   if (len > p.max_seqlen) len = p.max_seqlen;
   const int q0 = m_block * BM;
-  if (q0 >= len) return;
+  if (q0 >= len) return wait_for_clear();
 
   const __half* qg = p.q + seq * p.q_batch_stride + (long long)h_q * p.q_head_stride + tok0 * p.q_tok_stride;
   const __half* kg = p.k + seq * p.kv_batch_stride + (long long)h_kv * p.kv_head_stride + tok0 * p.kv_tok_stride;

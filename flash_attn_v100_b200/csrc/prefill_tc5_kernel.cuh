@@ -985,7 +985,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_consta
         }
       }
       // u[k] now holds unit gi of the row (lane - gi + k) of this warp's quadrant
-      if (ic == 0) wait_for_clear();
+      wait_for_clear();                      // (at once but for the first time)
       PROF_MARK(pe3);
       const int row_g = wq * 32 + (lane - gi);            // first row of my lane group within the tile
       const int col = h * (D / 2) + gi * 8;               // first column of the unit I store
@@ -1032,6 +1032,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_consta
     prof_smem[role * 16 + 15] += (unsigned long long)(clock64() - prof_start);
   }
 #endif
+  wait_for_clear();     // (CTAs without items too: the launch must not end before the clear)
   tc_fence_before();
   __syncthreads();
 #ifdef FA_TC5_PROF

@@ -120,6 +120,7 @@ prefill_wide_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
   uint8_t* smem = smem_wide;
   const uint32_t sQ = smem_u32(smem), sU = sQ + kQBytes;
   if ((sQ & 1023u) != 0u) {
+    wait_for_clear();
     if (threadIdx.x == 0) atomicOr(p.status, kStatusWaitTimeout);
     return;
   }

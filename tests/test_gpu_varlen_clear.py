@@ -74,3 +74,23 @@ def test_long_gap_at_the_rate_of_a_fill(batch):
             times.append(a.elapsed_time(b))
         return min(times)
     assert fastest(lambda: _clear(out, cu, 1)) < 4 * fastest(out.zero_)
+
+
+@pytest.mark.parametrize("D,longest", [(128, 1000), (64, 30), (128, 64), (256, 1000), (256, 20)])
+def test_no_sequence_has_rows(D, longest):
+    """All sequences empty, the whole of a large output to be cleared: nothing that follows on the stream sees it before, although no block of the attention
+    has anything to store."""
+    from flash_attn_v100_b200 import ops
+    total, H = 16384, 32768 // D
+    q, k, v = (torch.randn(total, h, D, dtype=torch.float16, device="cuda") for h in (H, 1, 1))
+    cu = torch.full((4,), 7, dtype=torch.int32, device="cuda")
+    run = lambda: ops.forward_varlen_prefill_fp16(q, k, v, cu, longest, True)
+    run()
+    for _ in range(5):
+        stale = torch.full((total, H, D), float("nan"), dtype=torch.float16, device="cuda")
+        del stale
+        torch.cuda._sleep(1000000)                     # everything below is in the queue by the time it starts
+        got = run()
+        rows = got[1023::1024].clone()
+        assert not rows.any() and not got.any()
+        del got
