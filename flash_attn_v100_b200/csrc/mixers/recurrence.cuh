@@ -1,7 +1,7 @@
 // Gated linear recurrences with a matrix state per head (see recurrence.cu, recurrence_gates.cu, recurrence_tc5.cu).
 //
 //     S_t = e^(la_t) S_(t-1) + b_t k_t v_t^T,      y_t = S_t^T q_t,
-// la (at most 0) and b being fp32 numbers per token and head.  Optionally a normaliser n_t = e^(la_t) n_(t-1) + b_t k_t divides:
+// la (usually at most 0) and b being fp32 numbers per token and head.  Optionally a normaliser n_t = e^(la_t) n_(t-1) + b_t k_t divides:
 // y_t = S_t^T q_t / (max(|n_t . q_t|, floor_t) + norm_eps); optionally skip_h v_t is added.  S and n are fp32.
 #pragma once
 #include <cuda_runtime.h>

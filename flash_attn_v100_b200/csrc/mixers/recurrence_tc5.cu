@@ -62,6 +62,7 @@ struct Small {                 // behind the tiles
   uint64_t bars[16];
   uint32_t tmem_slot;
   volatile int gave_up;
+  int grows[2];                // [buffer] (pairs of heads) some log decay of the chunk is above 0
 };
 // Barriers: a copy has landed; MMAs are done; the computing warps have written (or, the last, may be read) what the name says; gates are there.
 enum Bar { kFullQ, kFullV, kFullK, kScores = kFullK + 2, kOld, kNew, kState, kStateIn, kWeights, kValues, kOut, kGates, kDrain = kGates + 2, kBars };
@@ -183,6 +184,13 @@ recurrence_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
     }
   };
   auto put_gates = [&](int buf) {
+    if (NH == 2 && !STATE_ONLY) {
+      bool up = false;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) up |= gl[0][i] > 0.f || gl[NH - 1][i] > 0.f;
+      up = __any_sync(0xffffffffu, up);
+      if (lane == 0) sm.grows[buf] = up ? 1 : 0;
+    }
 #pragma unroll
     for (int h = 0; h < NH; ++h) {
       float* g = gl[h];
@@ -470,9 +478,10 @@ recurrence_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
         const int over = row - cg * 32;                         // my columns up to this one are at or before my row
         const bool below = __any_sync(0xffffffffu, over >= 0);
         // All of my columns' tokens are in blocks before my row's: e^(L_i - L_j) is a factor per row, from the end of the columns' block on, and one per column,
-        // which come with the gates (both at most 1), in place of an exponential per element and head.  Pairs of heads, 8 x 2048 tokens of 64 heads: 166 -> 154 us,
+        // which come with the gates, in place of an exponential per element and head.  Both are at most 1 where nothing grows; a chunk with a log decay above 0 goes by the
+        // differences, as a factor could overflow where they do not.  Pairs of heads, 8 x 2048 tokens of 64 heads: 166 -> 154 us,
         // 8 x 1024 of 32 48.4 -> 46.9; with one head per CTA the exponentials are not what a chunk waits for (157.4 and 156.3 us, long sequences 2 % slower).
-        const bool apart = NH == 2 && cg < (warp & 3);
+        const bool apart = NH == 2 && cg < (warp & 3) && sm.grows[buf] == 0;
 #pragma unroll
         for (int hh = 0; hh < NH; ++hh) {
           const float2* lb = sm.lb[buf][hh] + cg * 32;

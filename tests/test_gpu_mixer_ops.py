@@ -194,6 +194,29 @@ def test_recurrence_over_prompts(H, G, K, V, normed, dtype):
     assert torch.equal(sg[untouched].cpu(), state[untouched])
 
 
+@pytest.mark.parametrize("H, G, K, V", [(2, 1, 64, 64), (6, 3, 128, 32), (2, 2, 64, 64)])
+@pytest.mark.parametrize("at, rise", [(31, 100.0), (63, 95.0), (20, 60.0)])
+def test_decays_of_both_signs(H, G, K, V, at, rise):
+    """A log decay above 0 and one that takes it back: the weights of a row's tokens stay in range, whatever e to the sum of either part is."""
+    g, T = gen(at + H), 200
+    x = rnd(g, T, 2 * G * K + H * V, dtype=torch.bfloat16)
+    la, b = gates(g, H, T, 0.1)
+    la.clamp_(min=-1.0)
+    la[:, at - 1:at + 1] = rise / 2
+    la[:, at + 1] = -rise
+    b[:, :at + 1] *= 1e-30                             # (the state itself stays in range)
+    state, st = torch.zeros(1, H, K, V, device="cuda"), status()
+    seqs = mops().Sequences(i32(0), i32(0), i32(0, T), T)
+    got = mops().recurrence(x.cuda(), (0, G * K, 2 * G * K), H, G, K, V, la.cuda(), b.cuda(), state, seqs, st)
+    xd = x.double()
+    rep = lambda off: xd[:, off:off + G * K].view(T, G, K).repeat_interleave(H // G, 1)
+    want, S, _ = scan(rep(0), rep(G * K), xd[:, 2 * G * K:].view(T, H, V), la.double(), b.double())
+    assert int(st.item()) == 0
+    later = slice(at + 1, T)
+    close(got.view(T, H, V)[later], want[later], TOL[torch.bfloat16])
+    close(state[0], S, 2e-5)
+
+
 @pytest.mark.parametrize("H, G, K, V, normed", [(2, 1, 128, 64, False), (1, 1, 64, 128, True), (2, 2, 32, 16, True)])
 def test_long_sequences_in_segments(H, G, K, V, normed):
     """Few heads and long sequences are cut into segments that run side by side."""
