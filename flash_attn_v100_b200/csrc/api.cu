@@ -138,7 +138,7 @@ fa::DecodeLaunchConfig pick_decode_config(int D, int G, int slot_rows, int B, in
                                           long long segments, long long units, const DeviceInfo& di) {
   fa::DecodeLaunchConfig c;
   const bool half_m = G <= 8;  // kernels for at most 8 query heads per KV head: 128 threads, more CTAs per SM
-  // The int8 kinds are bound by instructions, so as many CTAs per SM as registers and shared memory allow, up to where the rings of more CTAs only
+  // The int8 kinds are bound by the latency of dependent instructions (half of the issue slots taken with 12 warps per SM), so as many CTAs per SM as registers and shared memory allow, up to where the rings of more CTAs only
   // cut the work finer.  Over 235 shapes each (1 to 32 sequences of 16 to 8000 tokens; 32 heads on 8, 4 on 4, 16 on 4, 16 on 2, 5 on 1), times of the choice
   // against one CTA per SM fewer: int8 cache 128 columns 0.98 (0.90 to 1.03 by length), 256 columns 0.94 (0.84 to 1.01); scores in whole
   // numbers, 64 columns 0.97 (0.89 to 1.03).  At 256 columns, scores in whole numbers, two CTAs fit only with three warps each (and up to five or six heads), whose
