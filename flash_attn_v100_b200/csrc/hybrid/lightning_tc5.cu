@@ -230,16 +230,13 @@ __global__ void __launch_bounds__(kThreads, 1) lightning_tc5_kernel(const Lightn
       tc_fence_after();
       __syncwarp();
       const uint64_t qd = smem_desc(sQ, 16, 1024), kd = smem_desc(sK, 16, 1024);
-      const uint64_t vd = smem_desc(sV, SLAB, 1024), khd = smem_desc(sKh, SLAB, 1024), kld = smem_desc(sKl, SLAB, 1024);
-      const uint64_t shd = smem_desc(sSh, SLAB, 1024), sld = smem_desc(sSl, SLAB, 1024);
+      const uint64_t vd = smem_desc(sV, SLAB, 1024), khd = smem_desc(sKh, SLAB, 1024), shd = smem_desc(sSh, SLAB, 1024);
       if (!STATE_ONLY) {
         tc_mma_ss8<StepsAlongK<SLAB, SLAB>>(tmem, qd, kd, IDESC_QK, 0u);
         tc_commit(bar_a);
-        tc_mma_ss8<StepsByRowsB<SLAB>>(tmem + 128u, qd, shd, IDESC_B, 0u);
-        tc_mma_ss8<StepsByRowsB<SLAB>>(tmem + 128u, qd, sld, IDESC_B, 1u);
+        tc_mma_ss8_parts<StepsByRowsB<SLAB>, 0, (TILE >> 4)>(tmem + 128u, qd, shd, IDESC_B, 0u);
       }
-      tc_mma_ss8<StepsByRows>(tmem + 384u, khd, vd, IDESC_AB, 0u);
-      tc_mma_ss8<StepsByRows>(tmem + 384u, kld, vd, IDESC_AB, 1u);
+      tc_mma_ss8_parts<StepsByRows, (TILE >> 4), 0>(tmem + 384u, khd, vd, IDESC_AB, 0u);
       tc_commit(bar_s);
     }
     if (!STATE_ONLY) {
@@ -272,8 +269,7 @@ __global__ void __launch_bounds__(kThreads, 1) lightning_tc5_kernel(const Lightn
         tc_fence_after();
         __syncwarp();
         const uint64_t vd = smem_desc(sV, SLAB, 1024);
-        tc_mma_ts8<StepsTmemA<>>(tmem + 256u, tmem, vd, IDESC_B, 0u);
-        tc_mma_ts8<StepsTmemA<>>(tmem + 256u, tmem + 64u, vd, IDESC_B, 1u);
+        tc_mma_ts8_parts<StepsTmemA<>, 64>(tmem + 256u, tmem, vd, IDESC_B, 0u);
         tc_commit(bar_o);
       }
     }

@@ -269,7 +269,7 @@ recurrence_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
   if (mma_warp) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
     const uint64_t qd = smem_desc(sQ, 16, 1024), qkd = smem_desc(sK0, 16, 1024), khd = smem_desc(sK0, SLAB, 1024), vd = smem_desc(sV, SLAB, 1024);
-    const uint64_t shd = smem_desc(sSh, SLAB, 1024), sld = smem_desc(sSl, SLAB, 1024), ed = smem_desc(sE, SLAB, 1024);
+    const uint64_t shd = smem_desc(sSh, SLAB, 1024), ed = smem_desc(sE, SLAB, 1024);
     auto issue_scores = [&](int c) {
       wait(kFullQ, (uint32_t)c & 1u);
       wait(kFullK + (c & 1), (uint32_t)(c >> 1) & 1u);
@@ -287,8 +287,7 @@ recurrence_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
         wait(kStateIn, ph);
         tc_fence_after();
         __syncwarp();
-        tc_mma_ss8<StepsByRowsB<SLAB>>(tmem + 128u, qd, shd, IDESC_B, 0u);
-        tc_mma_ss8<StepsByRowsB<SLAB>>(tmem + 128u, qd, sld, IDESC_B, 1u);
+        tc_mma_ss8_parts<StepsByRowsB<SLAB>, 0, (TILE >> 4)>(tmem + 128u, qd, shd, IDESC_B, 0u);
         if constexpr (NORM) {
           tc_mma_ss8<StepsByRowsB<SLAB>>(tmem + 256u, qd, ed, IDESC_B32, 0u);
           tc_mma_ss8<StepsByRows>(tmem + 288u, kc, ed, IDESC_AB32, 0u);
@@ -302,8 +301,7 @@ recurrence_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
         for (int hh = 0; hh < NH; ++hh) {
           const uint64_t vh = vd + (uint64_t)(hh * (SLAB >> 4));
           const uint32_t d = tmem + 256u + (uint32_t)hh * 64u, p = tmem + (uint32_t)hh * 384u;
-          tc_mma_ts8<StepsTmemA<>>(d, p, vh, IDESC_PV, 0u);
-          tc_mma_ts8<StepsTmemA<>>(d, p + 64u, vh, IDESC_PV, 1u);
+          tc_mma_ts8_parts<StepsTmemA<>, 64>(d, p, vh, IDESC_PV, 0u);
         }
         tc_commit(bar(kNew));
       }
@@ -311,8 +309,7 @@ recurrence_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
       if constexpr (STATE_ONLY) wait(kFullK + (c & 1), (uint32_t)(c >> 1) & 1u);
       tc_fence_after();
       __syncwarp();
-      tc_mma_ss8<StepsByRows>(tmem + 384u, kc, shd, IDESC_AB, 0u);       // (in order behind the products that read the second head's P there)
-      tc_mma_ss8<StepsByRows>(tmem + 384u, kc, sld, IDESC_AB, 1u);
+      tc_mma_ss8_parts<StepsByRows, 0, (TILE >> 4)>(tmem + 384u, kc, shd, IDESC_AB, 0u);       // (in order behind the products that read the second head's P there)
       if constexpr (NORM && STATE_ONLY) tc_mma_ss8<StepsByRows>(tmem + 288u, kc, ed, IDESC_AB32, 0u);
       tc_commit(bar(kState));
       if constexpr (!STATE_ONLY)
