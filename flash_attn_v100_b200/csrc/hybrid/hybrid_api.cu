@@ -1,6 +1,4 @@
 // C-ABI entry points of the hybrid decoder's operators (see include/fa_b200_hybrid.h): argument checks and launches.
-#include <algorithm>
-
 #include "../../../include/fa_b200_hybrid.h"
 
 #include "../api_common.cuh"
@@ -87,8 +85,7 @@ int fah_rotate_heads(void* q, const float* cos_t, const float* sin_t, int64_t ro
 
 size_t fah_latent_attention_workspace(int heads, int kv_rank, int rot_dim, int64_t rows, int dtype) {
   if (dtype != FAH_BF16 || heads <= 0 || rows <= 0 || kv_rank <= 0) return 0;
-  int64_t n = 0;                     // of the grids that a call may have, whatever its table's width
-  for (long long tokens : {0ll, 1ll << 40}) n = std::max<int64_t>(n, fa::hybrid::latent_decode_ctas(heads, kv_rank, rot_dim, tokens, sm_count()));
+  const int64_t n = fa::hybrid::latent_decode_max_ctas(heads, kv_rank, rot_dim, sm_count());     // whatever the call's table is like
   return (size_t)(n * 2 * heads * ((int64_t)kv_rank + 2) * 4 + (rows + 1) * 4);
 }
 
@@ -111,7 +108,9 @@ int fah_latent_attention(const void* q_abs, const void* q, int q_stride, int q_o
     const size_t need = fah_latent_attention_workspace(heads, kv_rank, rot_dim, rows, dtype);
     FA_REQUIRE(workspace_bytes >= need && (need == 0 || (workspace != nullptr && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0)),
                 "the workspace has %zu bytes, %zu (16-byte aligned) are needed", workspace_bytes, need);
-    a.n_cta = fa::hybrid::latent_decode_ctas(heads, kv_rank, rot_dim, rows * max_blocks * 16, sm_count());
+    const fa::hybrid::LatentPlan plan = fa::hybrid::latent_decode_plan(heads, kv_rank, rot_dim, rows, max_blocks, sm_count());
+    a.n_cta = plan.n_cta;
+    a.block_heads = plan.block_heads;
     a.part_o = static_cast<float*>(workspace);
     a.part_ml = a.part_o + (int64_t)a.n_cta * 2 * heads * kv_rank;
     a.row_tiles = reinterpret_cast<int32_t*>(a.part_ml + (int64_t)a.n_cta * 2 * heads * 2);

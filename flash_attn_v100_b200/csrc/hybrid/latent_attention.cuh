@@ -27,6 +27,7 @@ struct LatentAttentionArgs {
   int* status;
   // tensor-core kernel: work is cut into equal runs of key tiles, one per CTA and head block
   int n_cta;
+  int block_heads;           // (see LatentPlan)
   float* part_o;             // [n_cta, 2, heads, kv_rank] unnormalised sums of the rows that are cut
   float* part_ml;            // [n_cta, 2, heads, 2]: their maxima (log2 units) and weights
   int32_t* row_tiles;        // [rows + 1] prefix sums of the rows' key tiles, written by the kernel for the merge
@@ -38,12 +39,18 @@ template <typename T> cudaError_t launch_latent_attention(const LatentAttentionA
 
 // Tensor cores (bfloat16; kv_rank + rot_dim <= 576, both multiples of 8).
 bool latent_decode_supported(const LatentAttentionArgs& a);
-int latent_decode_ctas(int heads, int kv_rank, int rot_dim, long long tokens, int sm_count);   // per head block
+// Which kernel a call takes, and its grid.
+struct LatentPlan {
+  int block_heads;           // heads per CTA of the kernel in latent_decode_tc5.cu; 0: the one in latent_decode.cu
+  int n_cta;                 // per head block
+};
+LatentPlan latent_decode_plan(int heads, int kv_rank, int rot_dim, long long rows, int max_blocks, int sm_count);
+int latent_decode_max_ctas(int heads, int kv_rank, int rot_dim, int sm_count);   // n_cta of any plan, at most
 cudaError_t launch_latent_decode(const LatentAttentionArgs& a, int sm_count, void* encode_fn, cudaStream_t s);   // cuTensorMapEncodeTiled
 
 // The kernel of latents of 128 to 512 columns in blocks of 128, with rotated parts of 16 to 64 columns (latent_decode_tc5.cu).
 bool latent_decode_tc5_supported(int kv_rank, int rot_dim);
-int latent_decode_tc5_ctas(int heads, int kv_rank, long long tokens, int sm_count);   // tokens: a bound on those of all rows
+int latent_decode_tc5_ctas(int heads, int kv_rank, int block_heads, int sm_count);
 cudaError_t launch_latent_decode_tc5(const LatentAttentionArgs& a, const CUtensorMap& pool_map, cudaStream_t s);
 
 }  // namespace hybrid

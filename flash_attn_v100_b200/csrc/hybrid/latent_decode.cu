@@ -1,5 +1,5 @@
 // Attention in the latent space on the tensor cores (mma.sync, bfloat16 operands, fp32 scores, weights' sums and
-// accumulators), sm_100a: decode steps and short portions of prompts, of the sizes that latent_decode_tc5.cu does not serve.
+// accumulators), sm_100a: decode steps and short portions of prompts, of the sizes that latent_decode_tc5.cu does not serve, and the smallest (latent_decode_plan).
 //
 // All heads read the same cached rows, so a key tile (64 tokens) is fetched once and serves every head of the block (16 or
 // 32, the M rows of the MMAs) as key and as value.  The (row, key tile) units of the batch are numbered row by row and cut
@@ -444,11 +444,36 @@ bool latent_decode_supported(const LatentAttentionArgs& a) {
          (reinterpret_cast<uintptr_t>(a.out) & 15) == 0;
 }
 
-int latent_decode_ctas(int heads, int kv_rank, int rot_dim, long long tokens, int sm_count) {
-  if (latent_decode_tc5_supported(kv_rank, rot_dim)) return latent_decode_tc5_ctas(heads, kv_rank, tokens, sm_count);
-  const int blocks = heads <= 16 ? 1 : (heads + 31) / 32;
-  const int n = sm_count / blocks;
-  return n > 0 ? n : 1;
+namespace {
+int head_blocks(int heads) { return heads <= 16 ? 1 : (heads + 31) / 32; }
+int mma_ctas(int heads, int sm_count) { return sm_count >= head_blocks(heads) ? sm_count / head_blocks(heads) : 1; }
+}  // namespace
+
+LatentPlan latent_decode_plan(int heads, int kv_rank, int rot_dim, long long rows, int max_blocks, int sm_count) {
+  const LatentPlan mma = {0, mma_ctas(heads, sm_count)};
+  if (!latent_decode_tc5_supported(kv_rank, rot_dim)) return mma;
+  // Few heads, or the narrowest latents, and about one tile of a short context per CTA: the other kernel's start and hand-overs take 1 to 1.5 us more than they save.  4 to 16
+  // heads, its time against this one's: up to 64 cached tokens, 1 to 64 rows 1.0 to 1.2, 200 rows 0.84 to 1.0; 200 tokens, 16 rows 1.0 to 1.09, 64 rows 0.9 to 1.04; from 700
+  // on 0.94 to 1.1 with one or two rows, else below.  64 heads of 128 + 16: up to 200 tokens 1.0 to 1.15
+  // in this range.  32 heads or more of wider latents: 0.85 to 1.07 at these sizes.
+  if ((heads <= 16 || (heads > 32 && kv_rank == 128)) && max_blocks <= 16 && rows * ((max_blocks + 3) / 4) * head_blocks(heads) <= sm_count * 9ll / 8) return mma;
+  // Heads per CTA of 64 in blocks of 32 (of 64), us, L2 flushed: fewer queries to stage and pieces to merge, 1 row of 4096 22 (27), 8 of 700 20 (25), 16 of
+  // 4096 41 (43), 64 of 700 41 (43); but every tile is fetched twice: 24 of 4096 53 (51), 32 61 (59), 64 102 (90).  The host knows the table's width, not the contexts: behind
+  // a table of 16384 tokens 8 to 16 rows of 200 to 700 take the large blocks, 1.06 to 1.17 times as long, as 8 to 19 rows of 16000 would in small ones, 1.05 to 1.21 times.
+  const long long tokens = rows * max_blocks * 16;
+  const int block = heads <= 16 ? 16 : (heads <= 32 || tokens <= 80 * 1024 ? 32 : 64);
+  return {block, latent_decode_tc5_ctas(heads, kv_rank, block, sm_count)};
+}
+
+int latent_decode_max_ctas(int heads, int kv_rank, int rot_dim, int sm_count) {
+  int n = mma_ctas(heads, sm_count);
+  if (latent_decode_tc5_supported(kv_rank, rot_dim))
+    for (int block : {16, 32, 64}) {
+      if (block == 16 && heads > 16) continue;
+      const int m = latent_decode_tc5_ctas(heads, kv_rank, block, sm_count);
+      if (m > n) n = m;
+    }
+  return n;
 }
 
 cudaError_t launch_latent_decode(const LatentAttentionArgs& a, int sm_count, void* encode_fn, cudaStream_t s) {
@@ -463,7 +488,7 @@ cudaError_t launch_latent_decode(const LatentAttentionArgs& a, int sm_count, voi
     return cudaErrorInvalidValue;
   cudaError_t e;
   const int ks = ks_of(a.kv_rank + a.rot_dim);
-  if (latent_decode_tc5_supported(a.kv_rank, a.rot_dim)) e = launch_latent_decode_tc5(a, map, s);
+  if (a.block_heads > 0) e = launch_latent_decode_tc5(a, map, s);
   else if (a.heads <= 16) e = ks == 2 ? launch_t<2, 1>(a, map, s) : (ks == 3 ? launch_t<3, 1>(a, map, s) : (ks == 5 ? launch_t<5, 1>(a, map, s) : launch_t<9, 1>(a, map, s)));
   else e = ks == 2 ? launch_t<2, 2>(a, map, s) : (ks == 3 ? launch_t<3, 2>(a, map, s) : (ks == 5 ? launch_t<5, 2>(a, map, s) : launch_t<9, 2>(a, map, s)));
   return e == cudaSuccess ? launch_merge(a, sm_count, s) : e;

@@ -606,12 +606,9 @@ cudaError_t launch_t(const LatentAttentionArgs& a, const CUtensorMap& map, cudaS
   latent_decode_tc5_kernel<NB, N><<<dim3((unsigned)a.n_cta, (unsigned)((a.heads + N - 1) / N)), Plan<NB, N>::kThreads, smem, s>>>(map, a);
   return cudaGetLastError();
 }
-// Heads per CTA, `tokens` a bound on the cached tokens of all rows.  64 heads in blocks of 32 (of 64), us, L2 flushed: fewer queries to stage and pieces to merge, 1 row of
-// 4096 22 (27), 8 of 700 20 (25), 16 of 4096 41 (43), 64 of 700 41 (43); but every tile is fetched twice: 24 of 4096 53 (51), 32 61 (59), 64 102 (90).
-int block_heads(int heads, long long tokens) { return heads <= 16 ? 16 : (heads <= 32 || tokens <= 80 * 1024 ? 32 : 64); }
 template <int NB>
 cudaError_t launch_n(const LatentAttentionArgs& a, const CUtensorMap& map, cudaStream_t s) {
-  switch (block_heads(a.heads, a.rows * a.max_blocks * 16)) {
+  switch (a.block_heads) {
     case 16: return launch_t<NB, 16>(a, map, s);
     case 32: return launch_t<NB, 32>(a, map, s);
     default: return launch_t<NB, 64>(a, map, s);
@@ -624,8 +621,8 @@ bool latent_decode_tc5_supported(int kv_rank, int rot_dim) {
   return kv_rank % 128 == 0 && kv_rank <= 512 && rot_dim > 0 && rot_dim <= 64 && rot_dim % 16 == 0;
 }
 
-int latent_decode_tc5_ctas(int heads, int kv_rank, long long tokens, int sm_count) {
-  const int per_block = block_heads(heads, tokens), blocks = (heads + per_block - 1) / per_block, per_sm = kv_rank <= 256 && per_block <= 32 ? 2 : 1;
+int latent_decode_tc5_ctas(int heads, int kv_rank, int block_heads, int sm_count) {
+  const int blocks = (heads + block_heads - 1) / block_heads, per_sm = kv_rank <= 256 && block_heads <= 32 ? 2 : 1;
   const int n = sm_count * per_sm / blocks;
   return n > 0 ? n : 1;
 }

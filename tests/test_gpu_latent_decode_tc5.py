@@ -98,3 +98,13 @@ def test_captured():
     pos.fill_(150)
     graph.replay()
     assert torch.equal(out, call()) and int(st) == 0
+
+
+SHORT = [1, 63, 64, 200, 256]
+
+
+@pytest.mark.parametrize("H,r,rot", [(1, 256, 32), (8, 512, 64), (16, 384, 64), (33, 128, 16), (64, 128, 64), (64, 512, 64)])
+@pytest.mark.parametrize("lens,rows", [([40, 64, 1, 63], 40), ([40, 64, 1, 63], 166), ([40, 64, 1, 63], 167), (SHORT, 20), (SHORT, 41), (SHORT, 42), ([257, 30], 3)])
+def test_short_tables(lens, rows, H, r, rot):
+    """Either side of the line up to which the mma.sync kernel has the short contexts (on 148 SMs: 166 tiles of a table of up to 16 blocks)."""
+    run(H, r, rot, lens, [(t % len(lens), (7 * t) % lens[t % len(lens)]) for t in range(rows)], rows + H)
