@@ -612,23 +612,14 @@ static int run_prefill(fa::PrefillParams& p, int D, cudaStream_t stream) {
     return fail(FA_ERR_UNSUPPORTED, "no tcgen05 prefill kernel supports this call");
   if (p.in_bf16 && !tc5_ok)
     return fail(FA_ERR_UNSUPPORTED, "bfloat16 prefill is served by the tcgen05 kernel: head dimension up to 128");
+  // Up to 128 columns the tcgen05 kernel serves every call, so a sequence's bits are the same whatever it is called with.  (Up to 64 rows the mma.sync kernel would take 0.2 to
+  // 0.7 of its time.  Chosen by a call's longest sequence, or its number of blocks, it gave a prompt other bits beside longer ones; chosen by each sequence's own rows it is a launch
+  // more in packed calls, 2 us, or 5 us in front of the longer sequences: three prompts of up to 331 tokens 14.3 -> 16.4 us.)
   // Wide heads: the mma.sync kernel keeps the short prompts.  Its blocks of 64 rows and 64 keys are done sooner than one step of 128 x 128 and the
   // hand-overs of the tcgen05 kernel: up to 64 tokens 0.58 to 0.80 times its time, whatever the batch; of 72 to 128 tokens 0.9 to 1.2 times with few
   // heads in all, 1.4 to 2 times where they fill half the SMs; from 144 on more than its time.
   const bool wide = wide_ok && (g_prefill_impl == 2 || p.max_seqlen > ((long long)p.batch * p.H_Q * 2 > di.sm_count ? 64 : 128));
-  // Up to 128 columns (an item of the tcgen05 kernel starts with 9 us, whatever its size; figures for 8 to 4096 blocks of 64 rows, 8 to 32 heads):
-  // - one tile of keys: 0.22 to 0.71 times its time, however many blocks
-  // - D = 64 up to 192 tokens: 0.43 to 0.88 packed; dense 0.5 to 0.91 with eight blocks per SM, 1.02 with 28
-  // - D = 128 up to 192 tokens: 0.59 to 0.87 where two blocks per SM are enough, above 1.1 to 1.7
-  // - both up to 384 tokens: 0.75 to 0.91 where every block has an SM of its own, then 0.9 to 1.5; longer ones take as long or longer.
-  // Packed calls go by the length alone: a sequence's bits do not depend on how many others are packed with it.
-  const bool packed = p.cu_seqlens != nullptr;
-  const int max_len = packed ? p.max_seqlen : p.N;
-  const long long blocks = (max_len + 63ll) / 64 * p.H_Q * p.batch;
-  const bool brief = tc5_ok && g_prefill_impl == 0 &&
-                     (max_len <= 64 || (max_len <= 192 && (packed ? D == 64 : blocks <= (D == 64 ? 8ll : 2ll) * di.sm_count)) ||
-                      (!packed && max_len <= 384 && blocks <= di.sm_count));
-  if ((tc5_ok || wide) && g_prefill_impl != 1 && !brief) {
+  if ((tc5_ok || wide) && (g_prefill_impl != 1 || p.in_bf16)) {
     EncodeTiledFn enc;
     rc = get_encode(&enc);
     if (rc != FA_OK) return rc;

@@ -1,15 +1,9 @@
 // Tiled GQA prefill on mma.sync tensor cores (dense [B,H,N,D] and packed varlen).
 //
 // Replaces the reference's one-thread-per-query-row prefill kernels
-// (flash_attn_kernel.cu:1138-1299, 2471-2605, 3005-3148), for short prompts, and is
-// what the tcgen05 kernels (prefill_tc5.cu up to D = 128, prefill_wide.cu above) are checked
-// against (fa_prefill_set_impl(1)).  Which prompts are short: see run_prefill in api.cu.
-//
-// Bound there by one chain of loads, MMAs and softmax per tile: 1.5 us per 64 keys at D = 64, behind 3 us of
-// launch and first loads, where the tcgen05 kernel takes 9 us for its roles' start, a step and the hand-overs.
-// 64 rows per CTA: with 128 a prompt of 64 tokens leaves half of the warps idle and one of 256 takes 1.2 times as long.
-// A prompt of one tile gets one K and V buffer, so that twice as many CTAs are resident: 64 x 64 tokens of 32
-// heads of 128, 1.5 -> 0.7 times the tcgen05 kernel's time with both.
+// (flash_attn_kernel.cu:1138-1299, 2471-2605, 3005-3148).  The tcgen05
+// kernels (prefill_tc5.cu up to D = 128, prefill_wide.cu above) take over, but for short prompts of
+// wide heads, unless this one is asked for (fa_prefill_set_impl(1)): it is what they are checked against.
 //
 // One CTA = BM query rows of one (sequence, query head); each warp owns 16 rows.
 // K/V tiles of 64 keys are double-buffered in shared memory with cp.async and an
@@ -18,12 +12,11 @@
 // are skipped; only the diagonal and the ragged last tile are masked per element.
 #include "common.cuh"
 #include "prefill.cuh"
-#include "smem_limit.cuh"
 
 namespace fa {
 namespace {
 
-constexpr int BM = 64, BN = 64;
+constexpr int BN = 64;
 
 template <int D>
 __device__ __forceinline__ uint32_t swz(int row, int chunk) {
@@ -46,22 +39,15 @@ __device__ __forceinline__ void load_tile(uint32_t smem_base, const __half* gbas
   }
 }
 
-template <bool BF> __device__ __forceinline__ void mma16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  if constexpr (BF) mma_bf16_16816(c, a, b0, b1);
-  else mma_f16_16816(c, a, b0, b1);
-}
-template <bool BF> __device__ __forceinline__ uint32_t pack16(float lo, float hi) { return BF ? pack_bf162(lo, hi) : pack_half2(lo, hi); }
-
-// BF: q, k, v, the weights and the output are bfloat16.  `buffers`: of a K and a V tile each (one where no sequence has more keys).
-template <int D, bool BF>
-__global__ void __launch_bounds__(BM * 2) prefill_mma_kernel(const PrefillParams p, int buffers) {
+template <int D, int BM>
+__global__ void __launch_bounds__(BM * 2) prefill_mma_kernel(const PrefillParams p) {
   constexpr int THREADS = BM * 2;
   constexpr int NT_S = BN / 8;   // score n-tiles per warp row block
   constexpr int NT_O = D / 8;
   extern __shared__ __align__(128) uint8_t smem_raw[];
   const uint32_t sQ = smem_u32(smem_raw);
   const uint32_t sK0 = sQ + BM * D * 2;
-  const uint32_t sV0 = sK0 + buffers * BN * D * 2;
+  const uint32_t sV0 = sK0 + 2 * BN * D * 2;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, cq = (lane & 3) * 2;
@@ -69,7 +55,6 @@ __global__ void __launch_bounds__(BM * 2) prefill_mma_kernel(const PrefillParams
   const int h_q = blockIdx.y, seq = blockIdx.z;
   const int h_kv = h_q / (p.H_Q / p.H_KV);
 
-  // (a block without rows waits for the clear as well: the launch must not end before it)
   long long tok0;
   int len;
   if (p.cu_seqlens != nullptr) {
@@ -77,14 +62,14 @@ __global__ void __launch_bounds__(BM * 2) prefill_mma_kernel(const PrefillParams
     tok0 = a;
     len = e - a;
     if ((long long)e > p.total) len = (int)(p.total - a);
-    if (a < 0 || (long long)a > p.total) return wait_for_clear();
+    if (a < 0 || (long long)a > p.total) return;
   } else {
     tok0 = 0;
     len = p.N;
   }
   if (len > p.max_seqlen) len = p.max_seqlen;
   const int q0 = m_block * BM;
-  if (q0 >= len) return wait_for_clear();
+  if (q0 >= len) return;
 
   const __half* qg = p.q + seq * p.q_batch_stride + (long long)h_q * p.q_head_stride + tok0 * p.q_tok_stride;
   const __half* kg = p.k + seq * p.kv_batch_stride + (long long)h_kv * p.kv_head_stride + tok0 * p.kv_tok_stride;
@@ -141,8 +126,8 @@ __global__ void __launch_bounds__(BM * 2) prefill_mma_kernel(const PrefillParams
           const int r = jp * 16 + (lane & 7) + (mi >> 1) * 8;
           uint32_t kb[4];
           ldmatrix_x4(kb, sK + swz<D>(r, 2 * kk + (mi & 1)));
-          mma16<BF>(s[2 * jp], qa, kb[0], kb[1]);
-          mma16<BF>(s[2 * jp + 1], qa, kb[2], kb[3]);
+          mma_f16_16816(s[2 * jp], qa, kb[0], kb[1]);
+          mma_f16_16816(s[2 * jp + 1], qa, kb[2], kb[3]);
         }
       }
       const bool need_mask = (k0 + BN > len) || (p.causal && (k0 + BN - 1 > q0 + warp * 16));
@@ -183,8 +168,8 @@ __global__ void __launch_bounds__(BM * 2) prefill_mma_kernel(const PrefillParams
         const float p2 = fast_exp2(s[j][2] - ms1), p3 = fast_exp2(s[j][3] - ms1);
         r0 += p0 + p1;
         r1 += p2 + p3;
-        pa[j >> 1][(j & 1) * 2 + 0] = pack16<BF>(p0, p1);
-        pa[j >> 1][(j & 1) * 2 + 1] = pack16<BF>(p2, p3);
+        pa[j >> 1][(j & 1) * 2 + 0] = pack_half2(p0, p1);
+        pa[j >> 1][(j & 1) * 2 + 1] = pack_half2(p2, p3);
       }
       l0 = l0 * a0 + r0;
       l1 = l1 * a1 + r1;
@@ -203,8 +188,8 @@ __global__ void __launch_bounds__(BM * 2) prefill_mma_kernel(const PrefillParams
           const int r = ks * 16 + (lane & 7) + (mi & 1) * 8;
           uint32_t vb[4];
           ldmatrix_x4_trans(vb, sV + swz<D>(r, 2 * c2 + (mi >> 1)));
-          mma16<BF>(acc[2 * c2], pa[ks], vb[0], vb[1]);
-          mma16<BF>(acc[2 * c2 + 1], pa[ks], vb[2], vb[3]);
+          mma_f16_16816(acc[2 * c2], pa[ks], vb[0], vb[1]);
+          mma_f16_16816(acc[2 * c2 + 1], pa[ks], vb[2], vb[3]);
         }
       }
     }
@@ -215,42 +200,42 @@ __global__ void __launch_bounds__(BM * 2) prefill_mma_kernel(const PrefillParams
   l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
   l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
   l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
-  wait_for_clear();
   const float inv0 = l0 > 0.f ? 1.f / l0 : 0.f, inv1 = l1 > 0.f ? 1.f / l1 : 0.f;
   if (qrow0 < len) {
     __half* o = og + (long long)qrow0 * p.q_tok_stride;
 #pragma unroll
     for (int i = 0; i < NT_O; ++i)
       if (i * 8 < p.D_real)
-        *reinterpret_cast<uint32_t*>(o + i * 8 + cq) = pack_out16x2(acc[i][0] * inv0, acc[i][1] * inv0, BF || p.out_bf16 != 0);
+        *reinterpret_cast<uint32_t*>(o + i * 8 + cq) = pack_out16x2(acc[i][0] * inv0, acc[i][1] * inv0, p.out_bf16 != 0);
   }
   if (qrow0 + 8 < len) {
     __half* o = og + (long long)(qrow0 + 8) * p.q_tok_stride;
 #pragma unroll
     for (int i = 0; i < NT_O; ++i)
       if (i * 8 < p.D_real)
-        *reinterpret_cast<uint32_t*>(o + i * 8 + cq) = pack_out16x2(acc[i][2] * inv1, acc[i][3] * inv1, BF || p.out_bf16 != 0);
+        *reinterpret_cast<uint32_t*>(o + i * 8 + cq) = pack_out16x2(acc[i][2] * inv1, acc[i][3] * inv1, p.out_bf16 != 0);
   }
 }
 
-template <int D, bool BF>
+template <int D, int BM>
 cudaError_t launch_mma_t(const PrefillParams& p, cudaStream_t stream) {
-  auto kern = prefill_mma_kernel<D, BF>;
-  const int max_len = p.cu_seqlens ? p.max_seqlen : p.N, buffers = max_len > BN ? 2 : 1;
-  constexpr size_t smem = (size_t)BM * D * 2 + 4 * (size_t)BN * D * 2;
-  static SharedMemoryLimit limit;
-  const cudaError_t e = limit.raise(reinterpret_cast<const void*>(kern), (int)smem);
+  auto kern = prefill_mma_kernel<D, BM>;
+  const size_t smem = (size_t)BM * D * 2 + 4 * (size_t)BN * D * 2;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  const dim3 grid((max_len + BM - 1) / BM, p.H_Q, p.batch);
-  return launch_attention(p.after_clear != 0, kern, grid, BM * 2, smem - (2 - buffers) * 2 * (size_t)BN * D * 2, stream, p, buffers);
+  const int max_len = p.cu_seqlens ? p.max_seqlen : p.N;
+  dim3 grid((max_len + BM - 1) / BM, p.H_Q, p.batch);
+  kern<<<grid, BM * 2, smem, stream>>>(p);
+  return cudaGetLastError();
 }
+
 }  // namespace
 
 cudaError_t launch_prefill_mma(const PrefillParams& p, int D, cudaStream_t stream) {
   switch (D) {
-    case 64: return p.in_bf16 ? launch_mma_t<64, true>(p, stream) : launch_mma_t<64, false>(p, stream);
-    case 128: return p.in_bf16 ? launch_mma_t<128, true>(p, stream) : launch_mma_t<128, false>(p, stream);
-    case 256: return p.in_bf16 ? cudaErrorInvalidValue : launch_mma_t<256, false>(p, stream);
+    case 64: return launch_mma_t<64, 128>(p, stream);
+    case 128: return launch_mma_t<128, 128>(p, stream);
+    case 256: return launch_mma_t<256, 64>(p, stream);
     default: return cudaErrorInvalidValue;
   }
 }

@@ -380,8 +380,8 @@ int fa_silu_mul_bf16(const void* gate_up, void* out, int64_t T, int I, void* str
 int fa_half_to_bf16(const void* in, void* out, int64_t n, void* stream);
 
 /* Kernel choice for the prefill entry points: 0 = automatic (a tcgen05 kernel, but for short
- * prompts, which the mma.sync kernel serves: up to 64 tokens, up to 384 where there are few
- * blocks of 64 rows), 1 = the mma.sync kernel, 2 =
+ * prompts of head dimensions above 128, which the mma.sync kernel serves), 1 = the mma.sync
+ * kernel (bfloat16 operands, which it has no build for, stay with the tcgen05 kernel), 2 =
  * require a tcgen05 kernel, 3 = automatic, with every fourth pair of exp2 evaluated as a
  * polynomial on the FMA pipes up to head dimension 128.  Process-wide, a plain global like
  * fa_decode_set_tuning: meant for tests and measurements, not to be changed while another thread
