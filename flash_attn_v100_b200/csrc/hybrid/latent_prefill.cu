@@ -81,7 +81,7 @@ cudaError_t launch_t(const LatentPrefillArgs& a, EncodeTiledFn enc, cudaStream_t
   p.scale_log2 = a.scale * 1.4426950408889634f;
   p.n_hg = H;
   p.n_rb = (a.max_q + 255) / 256;
-  const long long n_items = (long long)p.n_rb * p.batch * p.n_hg;
+  const long long n_items = items_of_grid(true, a.total_q, 256, p.batch, p.n_rb, p.n_hg);
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -89,6 +89,7 @@ cudaError_t launch_t(const LatentPrefillArgs& a, EncodeTiledFn enc, cudaStream_t
   constexpr int smem = Tc5Layout<NA, 1, D>::BYTES;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
+  p.n_grid = n_items;
   p.take_over = n_items > sms ? 1 : 0;
   kern<<<item_grid(n_items), 640, smem, stream>>>(qmap, kmap, vmap, qmap_b, kmap_b, p);
   return cudaGetLastError();

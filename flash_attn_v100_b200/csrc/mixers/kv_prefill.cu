@@ -40,7 +40,7 @@ cudaError_t launch_t(const KvPrefillArgs& a, EncodeTiledFn enc, cudaStream_t str
   p.scale_log2 = a.scale * 1.4426950408889634f;
   p.n_hg = p.pair_heads ? H / 2 : H;
   p.n_rb = p.pair_heads ? (a.max_q + 127) / 128 : (a.max_q + 255) / 256;
-  const long long n_items = (long long)p.n_rb * p.batch * p.n_hg;
+  const long long n_items = items_of_grid(true, a.total_q, p.pair_heads ? 128 : 256, p.batch, p.n_rb, p.n_hg);
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -48,6 +48,7 @@ cudaError_t launch_t(const KvPrefillArgs& a, EncodeTiledFn enc, cudaStream_t str
   constexpr int smem = Tc5Layout<NA, 0, D>::BYTES;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
+  p.n_grid = n_items;
   p.take_over = n_items > sms ? 1 : 0;
   kern<<<item_grid(n_items), 640, smem, stream>>>(qmap, kmap, vmap, qmap, kmap, p);
   return cudaGetLastError();

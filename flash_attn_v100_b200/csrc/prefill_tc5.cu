@@ -58,10 +58,11 @@ cudaError_t launch_tc5_t(const PrefillParams& pp, void* encode_fn, cudaStream_t 
   const int max_len = dense ? pp.N : pp.max_seqlen;
   if (p.pair_heads) { p.n_hg = pp.H_Q / 2; p.n_rb = (max_len + 127) / 128; }
   else { p.n_hg = pp.H_Q; p.n_rb = (max_len + 255) / 256; }
-  const long long n_items = (long long)p.n_rb * pp.batch * p.n_hg;
+  const long long n_items = items_of_grid(!dense, pp.total, p.pair_heads ? 128 : 256, pp.batch, p.n_rb, p.n_hg);
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  p.n_grid = n_items;
   p.take_over = n_items > sms ? 1 : 0;
   return launch_attention(pp.after_clear != 0, kern, item_grid(n_items), 640, smem, stream, qmap, kmap, vmap, qmap, kmap, p);
 }

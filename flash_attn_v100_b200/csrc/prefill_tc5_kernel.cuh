@@ -90,6 +90,7 @@ struct Tc5Params {
   int dense;
   int out_bf16;    // store O as bfloat16 instead of fp16
   int n_hg, n_rb;  // head groups and row blocks of the item grid (items = n_rb * batch * n_hg)
+  long long n_grid;  // items that the grid is made for (items_of_grid)
   int take_over;   // CTAs go on with the items of CTAs that have not started (0: there are no more items than SMs)
   float scale_log2;
 };
@@ -153,6 +154,99 @@ __device__ __forceinline__ long long take_item(uint32_t reply, uint32_t bar, uin
       : "memory");
   fence_proxy_async();                               // (read before the next reply is written there)
   return ok ? (long long)y * gridDim.x + x : -1;
+}
+// A work item: row block, sequence and head (group).  rb < 0: there is none.
+struct ItemPlace {
+  int rb, seq, hg;
+};
+__device__ __forceinline__ ItemPlace read_place(const volatile int* slot) { return {slot[0], slot[1], slot[2]}; }
+__device__ __forceinline__ void write_place(volatile int* slot, const ItemPlace& at) {
+  slot[0] = at.rb;
+  slot[1] = at.seq;
+  slot[2] = at.hg;
+}
+__device__ __forceinline__ long long divide(long long n, int by, int& rest) {
+  if (n <= 0xffffffffll) {                           // (a division of 64 bits is a hundred instructions)
+    const uint32_t q = (uint32_t)n / (uint32_t)by;
+    rest = (int)((uint32_t)n - q * (uint32_t)by);
+    return q;
+  }
+  rest = (int)(n % by);
+  return n / by;
+}
+// Items by number, those with the most KV tiles first: late row blocks of the long sequences; the head groups of a row block are neighbours.  Dense: row block, sequence, head
+// group, from the last row block on.  Packed sequences: the same, but without the row blocks that a sequence does not have.  One warp finds them, walking the sequences 32 at a time,
+// row block by row block; numbers that only grow are found in one walk.  (With a number for every row block that the longest sequence has, the warp took one empty item after the other
+// where one prompt is long and many are short, a trip each, while its CTA waited: 1 x 8192 tokens beside 255 x 100, 32 heads on 8 of 128, 1836 us, 720 so.)
+struct ItemWalk {
+  long long blocks = 0;            // of all packed sequences
+  int level = -1, top = -1;        // the row block in hand, and the last one that a sequence has
+  int seq = 0;                     // walked up to this sequence of it
+  int mine = 0;                    // row blocks of sequence `lane`
+  long long before = 0;            // blocks walked
+  template <class Blocks>
+  __device__ __forceinline__ void start(int batch, Blocks blocks_of) {
+    const int lane = threadIdx.x & 31;
+    int most = 0;
+    for (int s0 = 0; s0 < batch; s0 += 32) {
+      const int n = s0 + lane < batch ? blocks_of(s0 + lane) : 0;
+      if (s0 == 0) mine = n;
+      most = n > most ? n : most;
+      blocks += __reduce_add_sync(0xffffffffu, (unsigned)n);       // (at most 32 x 2^24)
+    }
+    level = top = __reduce_max_sync(0xffffffffu, most) - 1;
+  }
+  // Place of packed block `number`.
+  template <class Blocks>
+  __device__ __forceinline__ bool find(long long number, int batch, Blocks blocks_of, ItemPlace& at) {
+    if (number >= blocks) return false;
+    if (number < before) {         // (not reached while numbers grow)
+      level = top;
+      seq = 0;
+      before = 0;
+    }
+    for (; level >= 0; --level, seq = 0) {
+      for (; seq < batch; seq += 32) {
+        const int s = seq + (int)(threadIdx.x & 31);
+        uint32_t has = __ballot_sync(0xffffffffu, (seq == 0 ? mine : (s < batch ? blocks_of(s) : 0)) > level);
+        const int n = __popc(has);
+        if (number < before + n) {
+          for (int i = (int)(number - before); i > 0; --i) has &= has - 1u;
+          at.seq = seq + __ffs((int)has) - 1;
+          at.rb = level;
+          return true;
+        }
+        before += n;
+      }
+    }
+    return false;
+  }
+};
+// The next item of this CTA, by one warp.  `number`: of the last one (-1: none left); `first`: it is this CTA's own, not looked at yet.  A CTA whose grid is smaller than the
+// number of items (packed offsets out of order, see items_of_grid) has every n_grid-th.
+template <class Take, class Blocks>
+__device__ __forceinline__ ItemPlace next_place(ItemWalk& walk, bool first, long long& number, long long count, long long n_grid, bool packed, int n_rb, int batch, int n_hg,
+                                                Take take, Blocks blocks_of) {
+  ItemPlace at = {-1, 0, 0};
+  for (; number >= 0; first = false) {
+    if (!first) {
+      if (number + n_grid < count) number += n_grid;
+      else number = __shfl_sync(0xffffffffu, (threadIdx.x & 31) == 0 ? take() : 0ll, 0);
+    }
+    if (number < 0 || number >= count) continue;
+    const long long block = divide(number, n_hg, at.hg);
+    if (!packed) {
+      at.rb = n_rb - 1 - (int)divide(block, batch, at.seq);
+      break;
+    }
+    if (walk.find(block, batch, blocks_of, at)) break;
+  }
+  return at;
+}
+// How many items a launch is made for: all of dense sequences; of packed ones as many as sequences without common rows can have (`rows`: of a block).
+inline long long items_of_grid(bool packed, long long total, int rows, int batch, int n_rb, int n_hg) {
+  const long long all = (long long)n_rb * batch, most = total / rows + batch;
+  return (packed && most < all ? most : all) * n_hg;
 }
 // Grid of a launch with that many items.
 inline dim3 item_grid(long long n_items) {
@@ -243,11 +337,9 @@ struct Tc5Layout {
   static_assert(BYTES <= 227 * 1024, "shared memory plan exceeds the SM");
 };
 
-// Work item = one pair of query tiles.  Items are numbered with the row block as the slowest
-// index, running backwards, so the items with the most KV tiles (late causal blocks of the long
-// sequences) come first (heaviest-first greedy scheduling): a warp of its own takes items, skips
-// empty ones, and publishes the item number to the other roles of its CTA through a small
-// shared-memory queue.
+// Work item = one pair of query tiles.  Those with the most KV tiles come first (heaviest-first greedy
+// scheduling): a warp of its own takes items and publishes their places to the other roles of its CTA
+// through a small shared-memory queue.
 struct Tc5Item {
   int head[2], row0[2], n_kv[2];
   int q_c1[2], q_c2[2], kv_c1, kv_c2;
@@ -256,13 +348,21 @@ struct Tc5Item {
   long long tok0;
 };
 
+// Rows of packed sequence `seq`, from row `first` on; one that starts below 0 has none.
+template <typename P>
+__device__ __forceinline__ int packed_rows(const P& p, int seq, int& first) {
+  const int a = __ldg(p.cu_seqlens + seq), e = __ldg(p.cu_seqlens + seq + 1);
+  first = a;
+  int len = e - a;
+  if ((long long)e > p.total) len = (int)(p.total - a);
+  if (len > p.max_seqlen) len = p.max_seqlen;
+  return a < 0 || len < 0 ? 0 : len;
+}
+
 template <bool EXT, typename P>
-__device__ __forceinline__ bool tc5_decode_item(const P& p, long long item, Tc5Item& it) {
+__device__ __forceinline__ bool tc5_decode_item(const P& p, const ItemPlace& at, Tc5Item& it) {
   constexpr int BM = 128, BN = 128;
-  const int hg = (int)(item % p.n_hg);
-  const long long r1 = item / p.n_hg;
-  const int seq = (int)(r1 % p.batch);
-  const int rb = p.n_rb - 1 - (int)(r1 / p.batch);
+  const int hg = at.hg, seq = at.seq, rb = at.rb;
   if (p.pair_heads) {
     it.head[0] = 2 * hg; it.head[1] = it.head[0] + 1;
     it.row0[0] = it.row0[1] = rb * BM;
@@ -273,15 +373,13 @@ __device__ __forceinline__ bool tc5_decode_item(const P& p, long long item, Tc5I
   const int h_kv = it.head[0] / (p.H_Q / p.H_KV);
   int len;
   if (p.cu_seqlens != nullptr) {
-    const int a = __ldg(p.cu_seqlens + seq), e = __ldg(p.cu_seqlens + seq + 1);
+    int a;
+    len = packed_rows(p, seq, a);
     it.tok0 = a;
-    len = e - a;
-    if ((long long)e > p.total) len = (int)(p.total - a);
   } else {
     it.tok0 = 0;
     len = p.N;
   }
-  if (len > p.max_seqlen) len = p.max_seqlen;
   it.len = len;
   int klen = len;
   long long ktok0 = it.tok0;
@@ -366,9 +464,9 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_consta
                 B_PFULL = B_SFULL + 2 * kBatchBars, B_TOKEN = B_PFULL + 2,
                 B_IFULL = B_TOKEN + 2, B_IEMPTY = B_IFULL + kItemQ, B_CLAIM = B_IEMPTY + kItemQ, B_PAIR = B_CLAIM + 1,
                 B_DRAIN = B_PAIR + 8, B_TURN = B_DRAIN + 2, B_TAKEN = B_TURN + 2, B_COUNT = B_TAKEN + 1;
-  static_assert(B_COUNT + kItemQ + 1 <= 62, "barriers, item slots, the tensor-memory slot and the reply of take_item share 64 words");
-  volatile long long* item_slot = reinterpret_cast<volatile long long*>(bars + B_COUNT);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + B_COUNT + kItemQ);
+  static_assert(B_COUNT + 2 * kItemQ + 1 <= 62, "barriers, item slots, the tensor-memory slot and the reply of take_item share 64 words");
+  volatile int* item_slot = reinterpret_cast<volatile int*>(bars + B_COUNT);       // [kItemQ][4]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + B_COUNT + 2 * kItemQ);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   // exchange area of the softmax role: per tile, three slots of [half][row] floats, and one redo tag per row quadrant
   float* xchg = reinterpret_cast<float*>(bars + 64);
@@ -377,7 +475,6 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_consta
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t reply = smem_u32(bars + 62);
-  const long long n_items = (long long)p.n_rb * p.batch * p.n_hg;
 #ifdef FA_TC5_PROF
   unsigned long long* prof_smem = reinterpret_cast<unsigned long long*>(xchg + 2 * 3 * 2 * 128 + 8);
   if (threadIdx.x < 5 * 16) prof_smem[threadIdx.x] = 0ull;
@@ -452,9 +549,9 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_consta
         // next item from the queue that warp 2 fills (-1: no more items)
         const int slot = ic % kItemQ;
         PROF_WAIT(0, 0, wait_or_abort(bar(B_IFULL + slot), (ic / kItemQ) & 1u, abort_flag));
-        const long long item = item_slot[slot];
+        const ItemPlace item = read_place(item_slot + 4 * slot);
         mbar_arrive(bar(B_IEMPTY + slot));
-        if (item < 0 || item >= n_items) break;
+        if (item.rb < 0) break;
         Tc5Item it;
         tc5_decode_item<EXT>(p, item, it);
         const int n_act = it.n_kv[1] > 0 ? 2 : 1;
@@ -542,10 +639,10 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_consta
         if (*abort_flag) break;
         const int slot = ic % kItemQ;
         PROF_WAIT(1 + t, 0, wait_or_abort(bar(B_IFULL + slot), (ic / kItemQ) & 1u, abort_flag));
-        const long long item = item_slot[slot];
+        const ItemPlace item = read_place(item_slot + 4 * slot);
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(B_IEMPTY + slot));
-        if (item < 0 || item >= n_items) break;
+        if (item.rb < 0) break;
         Tc5Item it;
         tc5_decode_item<EXT>(p, item, it);
         const bool other_active = it.n_kv[1] > 0;   // tile 0 is always active in a non-empty item
@@ -635,31 +732,40 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_consta
   } else if (warp == 2) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
     // ============================ items =============================================
-    // Takes work items, skips the empty ones (row blocks past the end of a
-    // sequence) and publishes the others through the item queue: an item is taken while the copies of the last three
+    // Takes work items and publishes their places through the item queue: an item is taken while the copies of the last three
     // KV tiles of the one before are issued, which keeps the latency of take_item off every other role's path.
     // Items taken up to kItemQ ahead were dealt out in turn, whatever they cost, where a CTA has few of them.
-    if (lane == 0) {
-      bool first = true;
-      uint32_t taken = 0;
-      for (uint32_t ic = 0;; ++ic) {
-        if (*abort_flag) break;
+    ItemWalk walk;
+    auto blocks_of = [&](int s) {
+      int a;
+      const int len = packed_rows(p, s, a);
+      return p.pair_heads ? (len + BM - 1) / BM : (len + 2 * BM - 1) / (2 * BM);
+    };
+    uint32_t taken = 0;
+    auto take = [&]() { return p.take_over ? take_item(reply, bar(B_TAKEN), taken, abort_flag) : -1ll; };
+    const bool packed = p.cu_seqlens != nullptr;
+    if (packed) walk.start(p.batch, blocks_of);
+    const long long count = packed ? walk.blocks * p.n_hg : p.n_grid;
+    long long number = first_item();
+    for (uint32_t ic = 0;; ++ic) {
+      if (__any_sync(0xffffffffu, *abort_flag != 0)) break;
+      if (ic > 0) wait_or_abort(bar(B_CLAIM), (ic - 1) & 1u, abort_flag);
+      __syncwarp();
+      ItemPlace at = next_place(walk, ic == 0, number, count, p.n_grid, packed, p.n_rb, p.batch, p.n_hg, take, blocks_of);
+      if constexpr (EXT) {
+        // (rows without keys are no work)
         Tc5Item it;
-        long long item;
-        bool have = false;
-        if (ic > 0) wait_or_abort(bar(B_CLAIM), (ic - 1) & 1u, abort_flag);
-        while (true) {
-          item = first ? first_item() : (p.take_over ? take_item(reply, bar(B_TAKEN), taken, abort_flag) : -1);
-          first = false;
-          if (item < 0) break;
-          if (item < n_items && tc5_decode_item<EXT>(p, item, it)) { have = true; break; }
-        }
-        const int slot = ic % kItemQ;
-        if (ic >= kItemQ) wait_or_abort(bar(B_IEMPTY + slot), ((ic / kItemQ) & 1u) ^ 1u, abort_flag);
-        item_slot[slot] = have ? item : -1;
-        mbar_arrive(bar(B_IFULL + slot));
-        if (!have) break;
+        while (at.rb >= 0 && !tc5_decode_item<EXT>(p, at, it)) at = next_place(walk, false, number, count, p.n_grid, packed, p.n_rb, p.batch, p.n_hg, take, blocks_of);
       }
+      const int slot = ic % kItemQ;
+      if (ic >= kItemQ) wait_or_abort(bar(B_IEMPTY + slot), ((ic / kItemQ) & 1u) ^ 1u, abort_flag);
+      __syncwarp();
+      if (lane == 0) {
+        write_place(item_slot + 4 * slot, at);
+        mbar_arrive(bar(B_IFULL + slot));
+      }
+      __syncwarp();
+      if (at.rb < 0) break;
     }
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
@@ -753,10 +859,10 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_consta
       if (*abort_flag) break;
       const int slot = ic % kItemQ;
       PROF_WAIT(3 + t, 0, wait_or_abort(bar(B_IFULL + slot), (ic / kItemQ) & 1u, abort_flag));
-      const long long item = item_slot[slot];
+      const ItemPlace item = read_place(item_slot + 4 * slot);
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(B_IEMPTY + slot));
-      if (item < 0 || item >= n_items) break;
+      if (item.rb < 0) break;
       Tc5Item it;
       tc5_decode_item<EXT>(p, item, it);
       const int n_mine = it.n_kv[t];

@@ -41,7 +41,7 @@ constexpr int kWideItemQ = 4;
 constexpr int kWideConsumers = 1 + 1 + 8 + 4;             // copy lane, MMA warp, softmax and output warps
 enum WideBar { kQFull = 0, kUFull = 1, kSFull = kUFull + kUnits, kPLo = kSFull + 2, kPHi = kPLo + 2, kODone = kPHi + 2, kOEmpty = kODone + 2, kLFull, kMReady,
                kIFull = kMReady + 2, kIEmpty = kIFull + kWideItemQ, kClaim = kIEmpty + kWideItemQ, kTaken, kWideBars };
-constexpr int kWideSmem = kQBytes + kUnits * kUnitBytes + 16 + kWideBars * 8 + kWideItemQ * 8 + 4 * 128 * 4 + 16;
+constexpr int kWideSmem = kQBytes + kUnits * kUnitBytes + 16 + kWideBars * 8 + kWideItemQ * 16 + 4 * 128 * 4 + 16;
 static_assert(kWideSmem <= 227 * 1024, "shared memory plan exceeds the SM");
 
 struct WideParams {
@@ -52,6 +52,7 @@ struct WideParams {
   long long o_batch_stride, o_head_stride, o_tok_stride;
   int causal, D_real, dense, out_bf16;
   int n_rb;                                // row blocks of the item grid (items = n_rb * batch * H_Q)
+  long long n_grid;                        // items that the grid is made for (items_of_grid)
   int take_over;                           // CTAs go on with the items of CTAs that have not started (see take_item)
   int* status;
   float scale_log2;
@@ -63,24 +64,20 @@ struct WideItem {
   long long tok0;
 };
 
-// Items with the most KV tiles (late row blocks) come first; the heads of a group are neighbours, so they read K and V from L2 together.
-__device__ __forceinline__ bool wide_item(const WideParams& p, long long item, WideItem& it) {
-  it.head = (int)(item % p.H_Q);
-  const long long r = item / p.H_Q;
-  it.seq = (int)(r % p.batch);
-  it.row0 = (p.n_rb - 1 - (int)(r / p.batch)) * 128;
+// (The heads of a group are neighbours in the order of the items, so they read K and V from L2 together.)
+__device__ __forceinline__ void wide_item(const WideParams& p, const ItemPlace& at, WideItem& it) {
+  it.head = at.hg;
+  it.seq = at.seq;
+  it.row0 = at.rb * 128;
   const int h_kv = it.head / (p.H_Q / p.H_KV);
   if (p.cu_seqlens != nullptr) {
-    const int a = __ldg(p.cu_seqlens + it.seq), e = __ldg(p.cu_seqlens + it.seq + 1);
+    int a;
+    it.len = packed_rows(p, it.seq, a);
     it.tok0 = a;
-    it.len = e - a;
-    if ((long long)e > p.total) it.len = (int)(p.total - a);
   } else {
     it.tok0 = 0;
     it.len = p.N;
   }
-  if (it.len > p.max_seqlen) it.len = p.max_seqlen;
-  if (it.row0 >= it.len) return false;
   const int kv_end = p.causal && it.row0 + 128 < it.len ? it.row0 + 128 : it.len;
   it.n_kv = (kv_end + 127) / 128;
   if (p.dense) {
@@ -93,7 +90,6 @@ __device__ __forceinline__ bool wide_item(const WideParams& p, long long item, W
     it.q_c2 = (int)it.tok0 + it.row0;
     it.kv_c2 = (int)it.tok0;
   }
-  return true;
 }
 
 // One 32-column chunk of a score row: P = exp2(s * scale - m) in two fp16 terms, the weight and what its rounding left, written to tensor memory
@@ -126,15 +122,14 @@ prefill_wide_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
   }
   const uint32_t reply = sU + kUnits * kUnitBytes;             // of take_item
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kQBytes + kUnits * kUnitBytes + 16);
-  volatile long long* item_slot = reinterpret_cast<volatile long long*>(bars + kWideBars);
-  float* l_rows = reinterpret_cast<float*>(bars + kWideBars + kWideItemQ);       // [softmax group][row]: parts of the row sums
+  volatile int* item_slot = reinterpret_cast<volatile int*>(bars + kWideBars);   // [kWideItemQ][4]
+  float* l_rows = reinterpret_cast<float*>(bars + kWideBars + 2 * kWideItemQ);   // [softmax group][row]: parts of the row sums
   float* m_rows = l_rows + 256;                                                  // [step & 1][row]: reference exponents
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(m_rows + 256);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   auto bar = [&](int i) -> uint32_t { return smem_u32(bars + i); };
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_slab = (p.D_real + 63) >> 6;         // 3 or 4 slabs of 64 columns
-  const long long n_items = (long long)p.n_rb * p.batch * p.H_Q;
 
   if (threadIdx.x == 0) {
     mbar_init(bar(kQFull), 1);
@@ -169,10 +164,10 @@ prefill_wide_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;                // S_0 [0,128) S_1 [128,256) O [256,512); P over its S: per 64 keys 32 columns and 32 of their rests
-  auto next_item = [&](uint32_t ic) -> long long {
+  auto next_item = [&](uint32_t ic) -> ItemPlace {
     const int slot = ic % kWideItemQ;
     wait_or_abort(bar(kIFull + slot), (ic / kWideItemQ) & 1u, abort_flag);
-    return item_slot[slot];
+    return read_place(item_slot + 4 * slot);
   };
   auto release_item = [&](uint32_t ic) { mbar_arrive(bar(kIEmpty + (int)(ic % kWideItemQ))); };
 
@@ -200,9 +195,9 @@ prefill_wide_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
       };
       for (uint32_t ic = 0;; ++ic) {
         if (*abort_flag) break;
-        const long long item = next_item(ic);
+        const ItemPlace item = next_item(ic);
         release_item(ic);
-        if (item < 0) break;
+        if (item.rb < 0) break;
         WideItem it;
         wide_item(p, item, it);
         if (cnt > 0) wait_or_abort(bar(kSFull + ((cnt - 1) & 1u)), ((cnt - 1) >> 1) & 1u, abort_flag);   // Q has been read
@@ -248,10 +243,10 @@ prefill_wide_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
     uint32_t ic = 0;
     for (;; ++ic) {
       if (*abort_flag) break;
-      const long long item = next_item(ic);
+      const ItemPlace item = next_item(ic);
       __syncwarp();
       if (lane == 0) release_item(ic);
-      if (item < 0) break;
+      if (item.rb < 0) break;
       WideItem it;
       wide_item(p, item, it);
       auto take_unit = [&]() -> uint32_t {
@@ -301,26 +296,32 @@ prefill_wide_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
     if (cnt > 0) drain_wait(bar(kODone + (int)((cnt - 1) & 1u)), ((cnt - 1) >> 1) & 1u, abort_flag);
   } else if (warp == 2) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
-    if (lane == 0) {
-      bool first = true;
-      uint32_t taken = 0;
-      for (uint32_t ic = 0;; ++ic) {
-        if (*abort_flag) break;
-        WideItem it;
-        long long item = -1;
-        // an item is taken when the copies of the last steps of the one before begin: taken earlier, items were dealt out in turn, whatever they cost
-        if (ic > 0) wait_or_abort(bar(kClaim), (ic - 1) & 1u, abort_flag);
-        while (true) {
-          item = first ? first_item() : (p.take_over ? take_item(reply, bar(kTaken), taken, abort_flag) : -1);
-          first = false;
-          if (item < 0 || (item < n_items && wide_item(p, item, it))) break;
-        }
-        const int slot = ic % kWideItemQ;
-        if (ic >= kWideItemQ) wait_or_abort(bar(kIEmpty + slot), ((ic / kWideItemQ) & 1u) ^ 1u, abort_flag);
-        item_slot[slot] = item;
+    ItemWalk walk;
+    auto blocks_of = [&](int s) {
+      int a;
+      return (packed_rows(p, s, a) + 127) / 128;
+    };
+    uint32_t taken = 0;
+    auto take = [&]() { return p.take_over ? take_item(reply, bar(kTaken), taken, abort_flag) : -1ll; };
+    const bool packed = p.cu_seqlens != nullptr;
+    if (packed) walk.start(p.batch, blocks_of);
+    const long long count = packed ? walk.blocks * p.H_Q : p.n_grid;
+    long long number = first_item();
+    for (uint32_t ic = 0;; ++ic) {
+      if (__any_sync(0xffffffffu, *abort_flag != 0)) break;
+      // an item is taken when the copies of the last steps of the one before begin: taken earlier, items were dealt out in turn, whatever they cost
+      if (ic > 0) wait_or_abort(bar(kClaim), (ic - 1) & 1u, abort_flag);
+      __syncwarp();
+      const ItemPlace at = next_place(walk, ic == 0, number, count, p.n_grid, packed, p.n_rb, p.batch, p.H_Q, take, blocks_of);
+      const int slot = ic % kWideItemQ;
+      if (ic >= kWideItemQ) wait_or_abort(bar(kIEmpty + slot), ((ic / kWideItemQ) & 1u) ^ 1u, abort_flag);
+      __syncwarp();
+      if (lane == 0) {
+        write_place(item_slot + 4 * slot, at);
         mbar_arrive(bar(kIFull + slot));
-        if (item < 0) break;
       }
+      __syncwarp();
+      if (at.rb < 0) break;
     }
   } else if (warp == 3) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
@@ -337,10 +338,10 @@ prefill_wide_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
     uint32_t cnt0 = 0;
     for (uint32_t ic = 0;; ++ic) {
       if (*abort_flag) break;
-      const long long item = next_item(ic);
+      const ItemPlace item = next_item(ic);
       __syncwarp();
       if (lane == 0) release_item(ic);
-      if (item < 0) break;
+      if (item.rb < 0) break;
       WideItem it;
       wide_item(p, item, it);
       const int grow = it.row0 + row;
@@ -438,10 +439,10 @@ prefill_wide_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
     wait_for_clear();
     for (uint32_t ic = 0;; ++ic) {
       if (*abort_flag) break;
-      const long long item = next_item(ic);
+      const ItemPlace item = next_item(ic);
       __syncwarp();
       if (lane == 0) release_item(ic);
-      if (item < 0) break;
+      if (item.rb < 0) break;
       WideItem it;
       wide_item(p, item, it);
       cnt += (uint32_t)it.n_kv;
@@ -539,7 +540,8 @@ cudaError_t launch_prefill_wide(const PrefillParams& pp, int sm_count, void* enc
   static SharedMemoryLimit limit;
   e = limit.raise(reinterpret_cast<const void*>(prefill_wide_kernel), kWideSmem);
   if (e != cudaSuccess) return e;
-  const long long n_items = (long long)p.n_rb * pp.batch * pp.H_Q;
+  const long long n_items = items_of_grid(!dense, pp.total, 128, pp.batch, p.n_rb, pp.H_Q);
+  p.n_grid = n_items;
   p.take_over = n_items > sm_count ? 1 : 0;
   return launch_attention(pp.after_clear != 0, prefill_wide_kernel, item_grid(n_items), kWideThreads, kWideSmem, stream, qmap, kmap, vmap, p);
 }
