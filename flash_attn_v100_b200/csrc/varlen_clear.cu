@@ -6,8 +6,8 @@ namespace {
 
 constexpr int kThreads = 256, kRows = 1024, kAhead = 4;      // kRows: rows that a block looks at together
 
-// Gap 0 lies before the first sequence, gap g in 1 .. batch behind the first max_seqlen rows of sequence g - 1, gap batch + 1 behind the last
-// sequence.  A block has an equal share of the rows, marks which of them lie in a gap and clears those, a warp per row: one gap that is most
+// Gap 0 lies before the first sequence, gap g in 1 .. batch behind the first max_seqlen rows of sequence g - 1 (from its start on, where
+// that lies below row 0: it has no rows), gap batch + 1 behind the last sequence.  A block has an equal share of the rows, marks which of them lie in a gap and clears those, a warp per row: one gap that is most
 // of the output, as a buffer padded to a fixed size has it, then keeps every SM writing.  (65536 rows of 32 heads of 128, 300 sequences of 4
 // tokens at their start: the packed prefill takes 290 us so, 340 over a fill of the whole output, and took 4400 with the blocks dealt out to the gaps, two
 // for each.)  Every gap is looked at, not searched for, so offsets in any order are served as they were by a fill; the attention waits for
@@ -31,11 +31,13 @@ varlen_clear_kernel(uint4* out, const int32_t* cu, int batch, long long total, i
         const int g = g0 + i * kThreads;
         from[i] = 0;
         to[i] = g < batch + 2 ? total : 0;
-        if (g > 0 && g < batch + 2) from[i] = (long long)__ldg(cu + g - 1) + (g <= batch ? max_seqlen : 0);
+        if (g > 0 && g < batch + 2) from[i] = __ldg(cu + g - 1);
         if (g <= batch) to[i] = __ldg(cu + g);
       }
 #pragma unroll
       for (int i = 0; i < kAhead; ++i) {
+        const int g = g0 + i * kThreads;
+        if (g > 0 && g <= batch && from[i] >= 0) from[i] += max_seqlen;
         const long long lo = from[i] > r0 ? from[i] - r0 : 0, hi = to[i] < r0 + n ? to[i] - r0 : n;
         if (lo >= hi) continue;
         any = true;

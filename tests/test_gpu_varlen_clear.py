@@ -94,3 +94,22 @@ def test_no_sequence_has_rows(D, longest):
         rows = got[1023::1024].clone()
         assert not rows.any() and not got.any()
         del got
+
+
+@pytest.mark.parametrize("D", [64, 128, 200])
+@pytest.mark.parametrize("cu,longest", [([60, 100, 20], 1000), ([60, 500, 20, 55], 300), ([60, 90, 500, 20], 1000), ([-5, 30, 90, 400], 1000), ([-5, 30, 90], 40), ([590, 700], 300)])
+def test_offsets_out_of_order_or_range(cu, longest, D):
+    """Rows that a sequence covers are its result although they lie in another one's gap, too; all others are zeros; a sequence that starts below 0 has no rows."""
+    from flash_attn_v100_b200 import ops
+    total, H = 600, 4
+    q, k, v = (torch.randn(total, h, D, dtype=torch.float16, device="cuda") for h in (H, 2, 2))
+    call = lambda t, cu: ops.forward_varlen_prefill_fp16(*t, torch.tensor(cu, dtype=torch.int32, device="cuda"), longest, True)
+    want = torch.zeros(total, H, D, dtype=torch.float16, device="cuda")
+    for a, e in zip(cu, cu[1:]):
+        n = min(e, total, a + longest) - a
+        if a >= 0 and n > 0:
+            want[a:a + n] = call([t[a:a + n].contiguous() for t in (q, k, v)], [0, n])
+    for _ in range(10):
+        stale = torch.full((total, H, D), float("nan"), dtype=torch.float16, device="cuda")
+        del stale
+        assert torch.equal(call((q, k, v), cu), want)
