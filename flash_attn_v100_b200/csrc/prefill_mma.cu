@@ -1,9 +1,12 @@
 // Tiled GQA prefill on mma.sync tensor cores (dense [B,H,N,D] and packed varlen).
 //
 // Replaces the reference's one-thread-per-query-row prefill kernels
-// (flash_attn_kernel.cu:1138-1299, 2471-2605, 3005-3148).  The tcgen05
-// kernels (prefill_tc5.cu up to D = 128, prefill_wide.cu above) take over, but for short prompts of
-// wide heads, unless this one is asked for (fa_prefill_set_impl(1)): it is what they are checked against.
+// (flash_attn_kernel.cu:1138-1299, 2471-2605, 3005-3148), for short prompts of wide heads
+// (see run_prefill in api.cu), and is what the tcgen05 kernels (prefill_tc5.cu up to D = 128,
+// prefill_wide.cu above) are checked against (fa_prefill_set_impl(1)).
+//
+// A prompt of one tile gets one K and V buffer, so that twice as many CTAs are resident: 16 x 16 tokens
+// of 16 heads of 256, 14.9 -> 10.3 us.
 //
 // One CTA = BM query rows of one (sequence, query head); each warp owns 16 rows.
 // K/V tiles of 64 keys are double-buffered in shared memory with cp.async and an
@@ -12,11 +15,12 @@
 // are skipped; only the diagonal and the ragged last tile are masked per element.
 #include "common.cuh"
 #include "prefill.cuh"
+#include "smem_limit.cuh"
 
 namespace fa {
 namespace {
 
-constexpr int BN = 64;
+constexpr int BM = 64, BN = 64;
 
 template <int D>
 __device__ __forceinline__ uint32_t swz(int row, int chunk) {
@@ -39,15 +43,16 @@ __device__ __forceinline__ void load_tile(uint32_t smem_base, const __half* gbas
   }
 }
 
-template <int D, int BM>
+// Two buffers of a K and a V tile each, or memory for the first alone where no sequence has more keys than a tile.
+template <int D>
 __global__ void __launch_bounds__(BM * 2) prefill_mma_kernel(const PrefillParams p) {
   constexpr int THREADS = BM * 2;
   constexpr int NT_S = BN / 8;   // score n-tiles per warp row block
   constexpr int NT_O = D / 8;
   extern __shared__ __align__(128) uint8_t smem_raw[];
   const uint32_t sQ = smem_u32(smem_raw);
+  constexpr uint32_t kTile = BN * D * 2, kBuffer = 2 * kTile;    // (V at a constant distance from K: at 256 columns there are no registers for a second base)
   const uint32_t sK0 = sQ + BM * D * 2;
-  const uint32_t sV0 = sK0 + 2 * BN * D * 2;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, cq = (lane & 3) * 2;
@@ -55,6 +60,7 @@ __global__ void __launch_bounds__(BM * 2) prefill_mma_kernel(const PrefillParams
   const int h_q = blockIdx.y, seq = blockIdx.z;
   const int h_kv = h_q / (p.H_Q / p.H_KV);
 
+  // (a block without rows waits for the clear as well: the launch must not end before it)
   long long tok0;
   int len;
   if (p.cu_seqlens != nullptr) {
@@ -62,14 +68,14 @@ __global__ void __launch_bounds__(BM * 2) prefill_mma_kernel(const PrefillParams
     tok0 = a;
     len = e - a;
     if ((long long)e > p.total) len = (int)(p.total - a);
-    if (a < 0 || (long long)a > p.total) return;
+    if (a < 0 || (long long)a > p.total) return wait_for_clear();
   } else {
     tok0 = 0;
     len = p.N;
   }
   if (len > p.max_seqlen) len = p.max_seqlen;
   const int q0 = m_block * BM;
-  if (q0 >= len) return;
+  if (q0 >= len) return wait_for_clear();
 
   const __half* qg = p.q + seq * p.q_batch_stride + (long long)h_q * p.q_head_stride + tok0 * p.q_tok_stride;
   const __half* kg = p.k + seq * p.kv_batch_stride + (long long)h_kv * p.kv_head_stride + tok0 * p.kv_tok_stride;
@@ -82,7 +88,7 @@ __global__ void __launch_bounds__(BM * 2) prefill_mma_kernel(const PrefillParams
   const int real_chunks = p.D_real >> 3;
   load_tile<D, BM, THREADS>(sQ, qg, p.q_tok_stride, q0, len, real_chunks, tid);
   load_tile<D, BN, THREADS>(sK0, kg, p.kv_tok_stride, 0, len, real_chunks, tid);
-  load_tile<D, BN, THREADS>(sV0, vg, p.kv_tok_stride, 0, len, real_chunks, tid);
+  load_tile<D, BN, THREADS>(sK0 + kTile, vg, p.kv_tok_stride, 0, len, real_chunks, tid);
   cp_async_commit();
 
   float acc[NT_O][4];
@@ -94,8 +100,8 @@ __global__ void __launch_bounds__(BM * 2) prefill_mma_kernel(const PrefillParams
   for (int t = 0; t < n_tiles; ++t) {
     const int buf = t & 1;
     if (t + 1 < n_tiles) {
-      load_tile<D, BN, THREADS>(sK0 + (buf ^ 1) * BN * D * 2, kg, p.kv_tok_stride, (t + 1) * BN, len, real_chunks, tid);
-      load_tile<D, BN, THREADS>(sV0 + (buf ^ 1) * BN * D * 2, vg, p.kv_tok_stride, (t + 1) * BN, len, real_chunks, tid);
+      load_tile<D, BN, THREADS>(sK0 + (buf ^ 1) * kBuffer, kg, p.kv_tok_stride, (t + 1) * BN, len, real_chunks, tid);
+      load_tile<D, BN, THREADS>(sK0 + (buf ^ 1) * kBuffer + kTile, vg, p.kv_tok_stride, (t + 1) * BN, len, real_chunks, tid);
       cp_async_commit();
       cp_async_wait<1>();
     } else {
@@ -103,7 +109,7 @@ __global__ void __launch_bounds__(BM * 2) prefill_mma_kernel(const PrefillParams
     }
     __syncthreads();
 
-    const uint32_t sK = sK0 + buf * BN * D * 2, sV = sV0 + buf * BN * D * 2;
+    const uint32_t sK = sK0 + buf * kBuffer, sV = sK + kTile;
     const int k0 = t * BN;
     // warp-level skip: under causal masking a warp whose rows all precede the tile has no work
     const bool warp_active = !p.causal || (k0 <= q0 + warp * 16 + 15);
@@ -200,6 +206,7 @@ __global__ void __launch_bounds__(BM * 2) prefill_mma_kernel(const PrefillParams
   l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
   l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
   l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
+  wait_for_clear();
   const float inv0 = l0 > 0.f ? 1.f / l0 : 0.f, inv1 = l1 > 0.f ? 1.f / l1 : 0.f;
   if (qrow0 < len) {
     __half* o = og + (long long)qrow0 * p.q_tok_stride;
@@ -217,25 +224,25 @@ __global__ void __launch_bounds__(BM * 2) prefill_mma_kernel(const PrefillParams
   }
 }
 
-template <int D, int BM>
+template <int D>
 cudaError_t launch_mma_t(const PrefillParams& p, cudaStream_t stream) {
-  auto kern = prefill_mma_kernel<D, BM>;
-  const size_t smem = (size_t)BM * D * 2 + 4 * (size_t)BN * D * 2;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  auto kern = prefill_mma_kernel<D>;
+  const int max_len = p.cu_seqlens ? p.max_seqlen : p.N, buffers = max_len > BN ? 2 : 1;
+  constexpr size_t smem = (size_t)BM * D * 2 + 4 * (size_t)BN * D * 2;
+  static SharedMemoryLimit limit;
+  const cudaError_t e = limit.raise(reinterpret_cast<const void*>(kern), (int)smem);
   if (e != cudaSuccess) return e;
-  const int max_len = p.cu_seqlens ? p.max_seqlen : p.N;
-  dim3 grid((max_len + BM - 1) / BM, p.H_Q, p.batch);
-  kern<<<grid, BM * 2, smem, stream>>>(p);
-  return cudaGetLastError();
+  const dim3 grid((max_len + BM - 1) / BM, p.H_Q, p.batch);
+  return launch_attention(p.after_clear != 0, kern, grid, BM * 2, smem - (2 - buffers) * 2 * (size_t)BN * D * 2, stream, p);
 }
 
 }  // namespace
 
 cudaError_t launch_prefill_mma(const PrefillParams& p, int D, cudaStream_t stream) {
   switch (D) {
-    case 64: return launch_mma_t<64, 128>(p, stream);
-    case 128: return launch_mma_t<128, 128>(p, stream);
-    case 256: return launch_mma_t<256, 64>(p, stream);
+    case 64: return launch_mma_t<64>(p, stream);
+    case 128: return launch_mma_t<128>(p, stream);
+    case 256: return launch_mma_t<256>(p, stream);
     default: return cudaErrorInvalidValue;
   }
 }

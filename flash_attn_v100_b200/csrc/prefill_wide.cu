@@ -15,8 +15,7 @@
 // 136 to 256 columns, flat and peaked scores.  The other way, an exact maximum with O scaled in tensor memory before every PV, is as slow: PV, scale, PV is a
 // serial chain (1 x 4096 tokens, 16 heads on 8, not causal: 375 us; two terms 374; one term 252).
 //
-// Measured: 16 x 2048 tokens, 2 heads of 256, causal: 134 us against 401 of the mma.sync kernel (prefill_mma.cu); 1 x 2048, 16 heads on 8: 79 and 229; 4
-// x 1024, 8 on 1: 51 and 127.  The smallest launch takes 12 us.  Releasing every unit with a commit of its own, earlier, changed nothing.
+// Measured: 2 x 2048 tokens, 16 heads on 8 of 256, causal: 112 us against 401 of the mma.sync kernel (prefill_mma.cu); 1 x 2048 48 and 229.  The smallest launch takes 12 us.  Releasing every unit with a commit of its own, earlier, changed nothing.
 //
 // Warps: 0 copies (TMA), 1 issues the MMAs, 2 owns tensor memory and takes work items, 4-7 and 8-11 softmax of the even and of the odd steps (a
 // thread per row, its 128 scores in registers), 12-15 write the output of a finished tile while the softmax is on the next one.  (With one
