@@ -458,10 +458,11 @@ LatentPlan latent_decode_plan(int heads, int kv_rank, int rot_dim, long long row
   // in this range.  32 heads or more of wider latents: 0.85 to 1.07 at these sizes.
   if ((heads <= 16 || (heads > 32 && kv_rank == 128)) && max_blocks <= 16 && rows * ((max_blocks + 3) / 4) * head_blocks(heads) <= sm_count * 9ll / 8) return mma;
   // Heads per CTA of 64 in blocks of 32 (of 64), us, L2 flushed: fewer queries to stage and pieces to merge, 1 row of 4096 22 (27), 8 of 700 20 (25), 16 of
-  // 4096 41 (43), 64 of 700 41 (43); but every tile is fetched twice: 24 of 4096 53 (51), 32 61 (59), 64 102 (90).  The host knows the table's width, not the contexts: behind
-  // a table of 16384 tokens 8 to 16 rows of 200 to 700 take the large blocks, 1.06 to 1.17 times as long, as 8 to 19 rows of 16000 would in small ones, 1.05 to 1.21 times.
+  // 4096 41 (43), 64 of 700 41 (43); but every tile is fetched twice: 24 of 4096 53 (51), 32 61 (59), 64 102 (90).  The host knows the table's width, not the contexts.  One
+  // of more than 8192 tokens is as wide as the longest request may get: fewer than 20 rows behind it take the small blocks.  Behind 16384, 8 and 16 rows of 200 to 700
+  // would take 1.06 to 1.17 times as long in large ones, 8 to 19 rows of 16000 in small ones 1.05 to 1.21 times.
   const long long tokens = rows * max_blocks * 16;
-  const int block = heads <= 16 ? 16 : (heads <= 32 || tokens <= 80 * 1024 ? 32 : 64);
+  const int block = heads <= 16 ? 16 : (heads <= 32 || tokens <= 80 * 1024 || (rows < 20 && max_blocks > 512) ? 32 : 64);
   return {block, latent_decode_tc5_ctas(heads, kv_rank, block, sm_count)};
 }
 

@@ -108,3 +108,9 @@ SHORT = [1, 63, 64, 200, 256]
 def test_short_tables(lens, rows, H, r, rot):
     """Either side of the line up to which the mma.sync kernel has the short contexts (on 148 SMs: 166 tiles of a table of up to 16 blocks)."""
     run(H, r, rot, lens, [(t % len(lens), (7 * t) % lens[t % len(lens)]) for t in range(rows)], rows + H)
+
+
+@pytest.mark.parametrize("rows,longest", [(19, 8193), (20, 8193), (19, 8192)])
+def test_few_rows_behind_a_wide_table(rows, longest):
+    """64 heads: fewer than 20 rows behind a table of more than 512 blocks come in blocks of 32 heads."""
+    run(64, 512, 64, [longest, 300], [(t % 2, 11 * t) for t in range(rows - 1)] + [(0, longest - 1)], rows)
