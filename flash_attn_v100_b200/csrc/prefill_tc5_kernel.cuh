@@ -503,6 +503,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_consta
     }
     for (int i = 0; i < 8; ++i) mbar_init(bar(B_PAIR + i), 64);   // the two warps that share 32 query rows
     for (int i = 0; i < kItemQ; ++i) {
+      item_slot[4 * i] = -1;               // (a role that gave up waiting reads a place that is none, or an earlier one)
       mbar_init(bar(B_IFULL + i), 1);
       mbar_init(bar(B_IEMPTY + i), kItemConsumers);
     }

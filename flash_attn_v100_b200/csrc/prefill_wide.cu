@@ -145,6 +145,7 @@ prefill_wide_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
     mbar_init(bar(kTaken), 1);
     mbar_init(bar(kLFull), 8);
     for (int i = 0; i < kWideItemQ; ++i) {
+      item_slot[4 * i] = -1;                       // (a role that gave up waiting reads a place that is none, or an earlier one)
       mbar_init(bar(kIFull + i), 1);
       mbar_init(bar(kIEmpty + i), kWideConsumers);
     }
